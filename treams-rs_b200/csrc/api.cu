@@ -130,7 +130,6 @@ struct tcu_factor {
     cplx* d_Z = nullptr;             // stored pair tables of the refinement's FP64 residual (lmax 2..5)
     bool scaled = false;
     tcu_factor* fallback = nullptr;  // FP64 factor of a mixed factor whose refinement stalled
-    unsigned sweep_epoch = 0;        // epochs of the persistent triangular sweeps
 };
 
 namespace {
@@ -448,12 +447,65 @@ tcu_status factor_impl(tcu_context* ctx, int L, double k0, size_t N, const doubl
     return TCU_OK;
 }
 
+// Refinement state of the columns of one solve in groups of 8 that converge separately: a group
+// takes another sweep while its worst relative residual is above the target, the last sweep
+// halved it and sweeps are left; afterwards its columns and their residuals stay as they are.
+struct RefineGroups {
+    static constexpr int WIDTH = 8;
+    struct Group {
+        bool active = true;
+        int sweeps = 1, left = 0;
+        double prev = INFINITY;
+    };
+    std::vector<Group> g;
+    std::vector<double> rn;  // residual norms of the columns' current solutions
+    int p;
+    double target;
+    RefineGroups(int p_, double target_, int max_sweeps) : g((p_ + WIDTH - 1) / WIDTH), rn(p_), p(p_), target(target_) {
+        for (Group& q : g) q.left = max_sweeps;
+    }
+    size_t first(size_t q) const { return q * WIDTH; }
+    int width(size_t q) const { return std::min(WIDTH, p - (int)q * WIDTH); }
+    double worst(size_t q, const std::vector<double>& r, const std::vector<double>& bn) const {
+        double w = 0.0;
+        for (int c = (int)first(q); c < (int)first(q) + width(q); ++c) w = std::max(w, bn[c] > 0 ? r[c] / bn[c] : r[c]);
+        return w;
+    }
+    // r: norms after the latest sweep; true while a group takes another one
+    bool advance(const std::vector<double>& r, const std::vector<double>& bn) {
+        bool any = false;
+        for (size_t q = 0; q < g.size(); ++q) {
+            if (!g[q].active) continue;
+            for (int c = (int)first(q); c < (int)first(q) + width(q); ++c) rn[c] = r[c];
+            const double w = worst(q, r, bn);
+            if (g[q].left == 0 || w <= target || !(w < 0.5 * g[q].prev)) {
+                g[q].active = false;
+                continue;
+            }
+            g[q].prev = w;
+            --g[q].left;
+            ++g[q].sweeps;
+            any = true;
+        }
+        return any;
+    }
+    bool any_above(const std::vector<double>& bn, double limit) const {
+        for (size_t q = 0; q < g.size(); ++q)
+            if (!(worst(q, rn, bn) <= limit)) return true;
+        return false;
+    }
+};
+
+// device scratch of vec_norms over p columns: p norms and 256 partial sums a column
+size_t norm_scratch(int p) { return (size_t)p * 257 * sizeof(double); }
+
 tcu_status solve_impl(tcu_factor* f, const double* B, int p, double* X, tcu_certificate* certs, bool device) {
     if (!f || !B || !X || p <= 0) return fail(TCU_INVALID_INPUT, "require a factor and at least one column");
-    if (p > 8) {  // the norms of a context reduce at most 8 columns at once
-        for (int c0 = 0; c0 < p; c0 += 8) {
+    if (p > SOLVE_MAXC) {
+        for (int c0 = 0; c0 < p; c0 += SOLVE_MAXC) {
             const size_t off = 2 * f->n * (size_t)c0;
-            tcu_status s = solve_impl(f, B + off, std::min(8, p - c0), X + off, certs ? certs + c0 : nullptr, device);
+            tcu_status s =
+                solve_impl(f, B + off, std::min(SOLVE_MAXC, p - c0), X + off, certs ? certs + c0 : nullptr, device);
             if (s) return s;
         }
         return TCU_OK;
@@ -472,30 +524,30 @@ tcu_status solve_impl(tcu_factor* f, const double* B, int p, double* X, tcu_cert
     DevBuf bufs(ctx);
     size_t per = n * p;
     const size_t xf_bytes = f->d_Z ? stored_inputs_bytes(*P, f->N, STORED_FULL, p) : 0;
-    CK(bufs.alloc(6 * per * sizeof(cplx) + xf_bytes), "solve buffers");
+    CK(bufs.alloc(6 * per * sizeof(cplx) + xf_bytes + norm_scratch(p)), "solve buffers");
     cplx* b = (cplx*)bufs.p;
     cplx* tb = b + per;
     cplx* x = tb + per;
     cplx* r = x + per;
     cplx* tmp = r + per;  // 2 per
     cplx* xf = tmp + 2 * per;  // packed inputs of the stored-table residual
+    double* d_norm = (double*)((char*)xf + xf_bytes);  // p norms, then their partial sums
     CK(cudaMemcpyAsync(b, B, per * 16, device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, ctx->stream),
        "copy rhs");
     launch_apply_t(f->L, f->N, f->d_T, b, p, tb, ctx->stream);
     ++ctx->launches;
     std::vector<double> rn(p), bn(p);
-    vec_norms(tb, n, p, ctx->d_small, ctx->d_partial, ctx->stream);
+    vec_norms(tb, n, p, d_norm, d_norm + p, ctx->stream);
     ctx->launches += 2;
-    CK(cudaMemcpyAsync(bn.data(), ctx->d_small, p * 8, cudaMemcpyDeviceToHost, ctx->stream), "norms");
-    int sweeps = 0;
+    CK(cudaMemcpyAsync(bn.data(), d_norm, p * 8, cudaMemcpyDeviceToHost, ctx->stream), "norms");
     auto lu_apply = [&](cplx* v) {
         if (f->scaled) scale_rows(v, f->d_scale, n, p, ctx->stream);  // R v
         if (f->precision == TCU_FP64)
             lu_solve_fp64((const double2*)f->d_A, (int)n, f->wk.perm, f->d_inv, v, tmp, p, ctx->stream,
-                          &ctx->launches, &f->sweep_epoch, f->wk.status);
+                          &ctx->launches, f->wk.status);
         else
             lu_solve_fp32((const float2*)f->d_A, (int)n, f->wk.perm, f->d_inv, v, tmp, p, ctx->stream,
-                          &ctx->launches, &f->sweep_epoch, f->wk.status);
+                          &ctx->launches, f->wk.status);
         if (f->scaled) {
             scale_rows(v, f->d_scale + n, n, p, ctx->stream);  // C (A')^-1 R v
             ctx->launches += 2;
@@ -511,9 +563,9 @@ tcu_status solve_impl(tcu_factor* f, const double* B, int p, double* X, tcu_cert
         } else {
             apply_op(ctx, P, f->N, f->k0, f->d_pos, f->d_T, x, n, p, tb, -1.0, 1.0, true, r);
         }
-        vec_norms(r, n, p, ctx->d_small, ctx->d_partial, ctx->stream);
+        vec_norms(r, n, p, d_norm, d_norm + p, ctx->stream);
         ctx->launches += 2;
-        CK(cudaMemcpyAsync(rn.data(), ctx->d_small, p * 8, cudaMemcpyDeviceToHost, ctx->stream), "norms");
+        CK(cudaMemcpyAsync(rn.data(), d_norm, p * 8, cudaMemcpyDeviceToHost, ctx->stream), "norms");
         CK(cudaMemcpyAsync(&sweep_status, f->wk.status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream), "status");
         tcu_status s2 = sync_status(ctx, "residual");
         if (s2) return s2;
@@ -522,32 +574,23 @@ tcu_status solve_impl(tcu_factor* f, const double* B, int p, double* X, tcu_cert
     };
     CK(cudaMemcpyAsync(x, tb, per * 16, cudaMemcpyDeviceToDevice, ctx->stream), "copy");
     lu_apply(x);
-    sweeps = 1;
     if ((s = residual())) return s;
-    {
-        // iterative refinement in FP64: up to 10 sweeps on mixed factors (20 with two-pass updates), 2 on
-        // FP64 factors
-        const double tol = ctx->refine_target;
-        double prev = INFINITY;
-        const int max_sweeps = f->precision == TCU_MIXED ? (f->wk.two_pass ? 20 : 10) : 2;
-        for (int it = 0; it < max_sweeps; ++it) {
-            double worst = 0.0;
-            for (int c = 0; c < p; ++c) worst = std::max(worst, bn[c] > 0 ? rn[c] / bn[c] : rn[c]);
-            if (worst <= tol || !(worst < 0.5 * prev)) break;
-            prev = worst;
-            lu_apply(r);
-            vec_axpy(x, r, n, p, ctx->stream);
-            ++ctx->launches;
-            ++sweeps;
-            if ((s = residual())) return s;
-        }
+    // iterative refinement in FP64: up to 10 sweeps on mixed factors (20 with two-pass updates), 2 on
+    // FP64 factors
+    RefineGroups groups(p, ctx->refine_target, f->precision == TCU_MIXED ? (f->wk.two_pass ? 20 : 10) : 2);
+    while (groups.advance(rn, bn)) {
+        lu_apply(r);
+        for (size_t g = 0; g < groups.g.size(); ++g)
+            if (groups.g[g].active) {
+                vec_axpy(x + groups.first(g) * n, r + groups.first(g) * n, n, groups.width(g), ctx->stream);
+                ++ctx->launches;
+            }
+        if ((s = residual())) return s;
     }
     if (f->precision == TCU_MIXED) {
         // refinement stalled above the FP64 target (an ill-scaled operator beyond the reach of
         // the TF32 factors): finish with an FP64 factor of the same cluster, kept for later solves
-        double worst = 0.0;
-        for (int c = 0; c < p; ++c) worst = std::max(worst, bn[c] > 0 ? rn[c] / bn[c] : rn[c]);
-        if (!(worst <= ctx->fallback_above)) {
+        if (groups.any_above(bn, ctx->fallback_above)) {
             // FP16 pieces first fall back to a mixed factor with TF32 pieces (which keep 22
             // bits relative to every element), that one in turn to FP64
             if (!f->fallback) {
@@ -561,22 +604,35 @@ tcu_status solve_impl(tcu_factor* f, const double* B, int p, double* X, tcu_cert
                                      nullptr, to_tf32 ? TCU_MIXED : TCU_FP64, &f->fallback, false)))
                     return s;
             }
-            ++ctx->fallbacks;
-            return solve_impl(f->fallback, B, p, X, certs, device);
         }
     }
-    for (int c = 0; c < p; ++c)
-        if (!std::isfinite(rn[c])) return fail(TCU_SINGULAR, "non-finite solution: numerically singular operator");
-    CK(cudaMemcpyAsync(X, x, per * 16, device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, ctx->stream),
-       "copy solution");
-    if ((s = sync_status(ctx, "solve"))) return s;
-    if (certs)
-        for (int c = 0; c < p; ++c) {
-            certs[c].iterations = sweeps;
-            certs[c].residual_norm = rn[c];
-            certs[c].rhs_norm = bn[c];
+    int done = 0;  // columns before it are in X
+    auto copy_out = [&](int end) {  // columns done .. end - 1
+        const int c0 = done;
+        done = end;
+        return end > c0 ? cudaMemcpyAsync((cplx*)X + c0 * n, x + c0 * n, (end - c0) * n * 16,
+                                          device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
+                                          ctx->stream)
+                        : cudaSuccess;
+    };
+    for (size_t q = 0; q < groups.g.size(); ++q) {
+        const int c0 = (int)groups.first(q), w = groups.width(q);
+        if (f->precision == TCU_MIXED && !(groups.worst(q, groups.rn, bn) <= ctx->fallback_above)) {
+            CK(copy_out(c0), "copy solution");
+            ++ctx->fallbacks;
+            const size_t off = 2 * n * (size_t)c0;
+            if ((s = solve_impl(f->fallback, B + off, w, X + off, certs ? certs + c0 : nullptr, device))) return s;
+            done = c0 + w;
+            continue;
         }
-    return TCU_OK;
+        for (int c = c0; c < c0 + w; ++c) {
+            if (!std::isfinite(groups.rn[c]))
+                return fail(TCU_SINGULAR, "non-finite solution: numerically singular operator");
+            if (certs) certs[c] = {groups.g[q].sweeps, groups.rn[c], bn[c]};
+        }
+    }
+    CK(copy_out(p), "copy solution");
+    return sync_status(ctx, "solve");
 }
 
 // Adjoint solve Y = (I - T C)^-H G with a factor (cluster/interaction.rs:221-227 uses it for
@@ -585,11 +641,11 @@ tcu_status solve_impl(tcu_factor* f, const double* B, int p, double* X, tcu_cert
 // the forward solve. th: return T^H Y instead (the incident-field gradient).
 tcu_status solve_adjoint_impl(tcu_factor* f, const double* G, int p, double* Y, tcu_certificate* certs, bool th) {
     if (!f || !G || !Y || p <= 0) return fail(TCU_INVALID_INPUT, "require a factor and at least one column");
-    if (p > 8) {  // the norms of a context reduce at most 8 columns at once
-        for (int c0 = 0; c0 < p; c0 += 8) {
+    if (p > SOLVE_MAXC) {
+        for (int c0 = 0; c0 < p; c0 += SOLVE_MAXC) {
             const size_t off = 2 * f->n * (size_t)c0;
-            tcu_status s =
-                solve_adjoint_impl(f, G + off, std::min(8, p - c0), Y + off, certs ? certs + c0 : nullptr, th);
+            tcu_status s = solve_adjoint_impl(f, G + off, std::min(SOLVE_MAXC, p - c0), Y + off,
+                                              certs ? certs + c0 : nullptr, th);
             if (s) return s;
         }
         return TCU_OK;
@@ -607,7 +663,7 @@ tcu_status solve_adjoint_impl(tcu_factor* f, const double* G, int p, double* Y, 
     DevBuf bufs(ctx);
     const size_t tmpc = adjoint_solve_tmp((int)n, p);
     const size_t xfc = f->d_Z ? stored_inputs_bytes(*P, f->N, STORED_FULL, p) / sizeof(cplx) : 0;
-    CK(bufs.alloc((5 * per + tmpc + xfc) * sizeof(cplx)), "adjoint solve buffers");
+    CK(bufs.alloc((5 * per + tmpc + xfc) * sizeof(cplx) + norm_scratch(p)), "adjoint solve buffers");
     cplx* g = (cplx*)bufs.p;
     cplx* y = g + per;
     cplx* r = y + per;
@@ -615,53 +671,45 @@ tcu_status solve_adjoint_impl(tcu_factor* f, const double* G, int p, double* Y, 
     cplx* t2 = t1 + per;
     cplx* xf = t2 + per;  // packed inputs of the stored-table coupling product
     cplx* tmp = xf + xfc;
+    double* d_norm = (double*)(tmp + tmpc);  // p norms, then their partial sums
     CK(cudaMemsetAsync(ctx->d_status, 0, 4, ctx->stream), "status");
     CK(cudaMemcpyAsync(g, G, per * 16, cudaMemcpyHostToDevice, ctx->stream), "copy rhs");
     std::vector<double> rn(p), bn(p);
-    vec_norms(g, n, p, ctx->d_small, ctx->d_partial, ctx->stream);
-    CK(cudaMemcpyAsync(bn.data(), ctx->d_small, p * 8, cudaMemcpyDeviceToHost, ctx->stream), "norms");
+    vec_norms(g, n, p, d_norm, d_norm + p, ctx->stream);
+    CK(cudaMemcpyAsync(bn.data(), d_norm, p * 8, cudaMemcpyDeviceToHost, ctx->stream), "norms");
     auto lu_adjoint = [&](cplx* v) {
         if (f->scaled) scale_rows(v, f->d_scale + n, n, p, ctx->stream);  // C g
         if (f->precision == TCU_FP64)
             lu_solve_adjoint_fp64((const double2*)f->d_A, (int)n, f->wk.perm, f->d_inv, v, tmp, p, ctx->stream,
-                                  &ctx->launches);
+                                  &ctx->launches, ctx->d_status);
         else
             lu_solve_adjoint_fp32((const float2*)f->d_A, (int)n, f->wk.perm, f->d_inv, v, tmp, p, ctx->stream,
-                                  &ctx->launches);
+                                  &ctx->launches, ctx->d_status);
         if (f->scaled) scale_rows(v, f->d_scale, n, p, ctx->stream);  // R
     };
     auto residual = [&]() -> tcu_status {  // r = g - A^H y
         launch_apply_adjoint(*P, f->N, f->k0, f->d_pos, f->d_T, y, n, p, r, t1, t2, ctx->stream, &ctx->launches,
                              f->d_Z, xf, ctx->d_status);
         vec_sub(r, g, r, n, p, ctx->stream);
-        vec_norms(r, n, p, ctx->d_small, ctx->d_partial, ctx->stream);
+        vec_norms(r, n, p, d_norm, d_norm + p, ctx->stream);
         ctx->launches += 3;
-        CK(cudaMemcpyAsync(rn.data(), ctx->d_small, p * 8, cudaMemcpyDeviceToHost, ctx->stream), "norms");
+        CK(cudaMemcpyAsync(rn.data(), d_norm, p * 8, cudaMemcpyDeviceToHost, ctx->stream), "norms");
         return read_status(ctx, "adjoint residual");
     };
     CK(cudaMemcpyAsync(y, g, per * 16, cudaMemcpyDeviceToDevice, ctx->stream), "copy");
     lu_adjoint(y);
-    int sweeps = 1;
     if ((s = residual())) return s;
-    const double tol = ctx->refine_target;
-    double prev = INFINITY;
-    const int max_sweeps = f->precision == TCU_MIXED ? (f->wk.two_pass ? 20 : 10) : 2;
-    auto worst_of = [&]() {
-        double w = 0.0;
-        for (int c = 0; c < p; ++c) w = std::max(w, bn[c] > 0 ? rn[c] / bn[c] : rn[c]);
-        return w;
-    };
-    for (int it = 0; it < max_sweeps; ++it) {
-        const double worst = worst_of();
-        if (worst <= tol || !(worst < 0.5 * prev)) break;
-        prev = worst;
+    RefineGroups groups(p, ctx->refine_target, f->precision == TCU_MIXED ? (f->wk.two_pass ? 20 : 10) : 2);
+    while (groups.advance(rn, bn)) {
         lu_adjoint(r);
-        vec_axpy(y, r, n, p, ctx->stream);
-        ++ctx->launches;
-        ++sweeps;
+        for (size_t q = 0; q < groups.g.size(); ++q)
+            if (groups.g[q].active) {
+                vec_axpy(y + groups.first(q) * n, r + groups.first(q) * n, n, groups.width(q), ctx->stream);
+                ++ctx->launches;
+            }
         if ((s = residual())) return s;
     }
-    if (f->precision == TCU_MIXED && !(worst_of() <= ctx->fallback_above)) {
+    if (f->precision == TCU_MIXED && groups.any_above(bn, ctx->fallback_above)) {
         if (!f->fallback) {
             std::vector<double> hr(f->N), he(2 * (size_t)f->N), hp(3 * (size_t)f->N);
             CK(cudaMemcpyAsync(hr.data(), f->d_radii, f->N * 8, cudaMemcpyDeviceToHost, ctx->stream), "copy");
@@ -673,24 +721,38 @@ tcu_status solve_adjoint_impl(tcu_factor* f, const double* G, int p, double* Y, 
                                  to_tf32 ? TCU_MIXED : TCU_FP64, &f->fallback, false)))
                 return s;
         }
-        ++ctx->fallbacks;
-        return solve_adjoint_impl(f->fallback, G, p, Y, certs, th);
     }
-    for (int c = 0; c < p; ++c)
-        if (!std::isfinite(rn[c])) return fail(TCU_SINGULAR, "non-finite solution: numerically singular operator");
     if (th) {
         launch_apply_th(f->L, f->N, f->d_T, y, n, p, r, ctx->stream);
         ++ctx->launches;
     }
-    CK(cudaMemcpyAsync(Y, th ? r : y, per * 16, cudaMemcpyDeviceToHost, ctx->stream), "copy solution");
-    if ((s = sync_status(ctx, "adjoint solve"))) return s;
-    if (certs)
-        for (int c = 0; c < p; ++c) {
-            certs[c].iterations = sweeps;
-            certs[c].residual_norm = rn[c];
-            certs[c].rhs_norm = bn[c];
+    int done = 0;  // columns before it are in Y
+    auto copy_out = [&](int end) {  // columns done .. end - 1
+        const int c0 = done;
+        done = end;
+        return end > c0 ? cudaMemcpyAsync((cplx*)Y + c0 * n, (th ? r : y) + c0 * n, (end - c0) * n * 16,
+                                          cudaMemcpyDeviceToHost,
+                                          ctx->stream)
+                        : cudaSuccess;
+    };
+    for (size_t q = 0; q < groups.g.size(); ++q) {
+        const int c0 = (int)groups.first(q), w = groups.width(q);
+        if (f->precision == TCU_MIXED && !(groups.worst(q, groups.rn, bn) <= ctx->fallback_above)) {
+            CK(copy_out(c0), "copy solution");
+            ++ctx->fallbacks;
+            const size_t off = 2 * n * (size_t)c0;
+            if ((s = solve_adjoint_impl(f->fallback, G + off, w, Y + off, certs ? certs + c0 : nullptr, th))) return s;
+            done = c0 + w;
+            continue;
         }
-    return TCU_OK;
+        for (int c = c0; c < c0 + w; ++c) {
+            if (!std::isfinite(groups.rn[c]))
+                return fail(TCU_SINGULAR, "non-finite solution: numerically singular operator");
+            if (certs) certs[c] = {groups.g[q].sweeps, groups.rn[c], bn[c]};
+        }
+    }
+    CK(copy_out(p), "copy solution");
+    return sync_status(ctx, "adjoint solve");
 }
 
 // A factor applied once (no refinement): v <- A^-1 v with the row/column scales; the coarse
@@ -708,10 +770,10 @@ struct FactorCoarse : CoarseSolve {
         if (f->scaled) scale_rows(v, f->d_scale, n, 1, st);
         if (f->precision == TCU_FP64)
             lu_solve_fp64((const double2*)f->d_A, (int)n, f->wk.perm, f->d_inv, v, tmp, 1, st, &ctx->launches,
-                          &f->sweep_epoch, f->wk.status);
+                          f->wk.status);
         else
             lu_solve_fp32((const float2*)f->d_A, (int)n, f->wk.perm, f->d_inv, v, tmp, 1, st, &ctx->launches,
-                          &f->sweep_epoch, f->wk.status);
+                          f->wk.status);
         if (f->scaled) scale_rows(v, f->d_scale + n, n, 1, st);
         return TCU_OK;
     }

@@ -188,9 +188,9 @@ void launch_apply_adjoint(const DevPlan& P, int N, double k0, const double* pos,
 void launch_apply_th(int L, int N, const cplx* T, const cplx* x, size_t ldx, int ncol, cplx* y, cudaStream_t st);
 size_t adjoint_solve_tmp(int n, int ncol);
 void lu_solve_adjoint_fp64(const double2* A, int n, const int* perm, const double2* inv, double2* x, double2* tmp,
-                           int ncol, cudaStream_t st, long long* launches);
+                           int ncol, cudaStream_t st, long long* launches, int* status);
 void lu_solve_adjoint_fp32(const float2* A, int n, const int* perm, const double2* inv, double2* x, double2* tmp,
-                           int ncol, cudaStream_t st, long long* launches);
+                           int ncol, cudaStream_t st, long long* launches, int* status);
 
 // equil.cu — power-of-two row/column equilibration of an n x n column-major matrix (FP64 or
 // FP32 storage) when its largest entry exceeds `threshold`; r, c: n scales each.
@@ -293,16 +293,22 @@ int lu_factor_fp64(double2* A, int n, LuWork& w, cudaStream_t st, long long* lau
 void launch_barrier_selftest(unsigned* bar, int* status, double limit_s, cudaStream_t st);
 int lu_factor_fp32(float2* A, int n, LuWork& w, cudaStream_t st, long long* launches, bool tensor_cores);
 // solve.cu — inverses of the 64 x 64 diagonal blocks of L and U (FP64, lu_inverse_bytes),
-// then x (n x ncol, FP64) <- A^-1 x; tmp holds 2 n min(ncol, 8) complex.
+// then x (n x ncol, FP64) <- A^-1 x, ncol <= SOLVE_MAXC; tmp holds 2 n ncol complex.
+constexpr int SOLVE_MAXC = 128;
 size_t lu_inverse_bytes(int n);
 void lu_block_inverses_fp64(const double2* A, int n, double2* inv, cudaStream_t st, long long* launches);
 void lu_block_inverses_fp32(const float2* A, int n, double2* inv, cudaStream_t st, long long* launches);
-// epoch: the factor's sweep counter (host), status: its device status word (8 when a sweep's
-// bounded wait gave up); both null select one launch per block step.
+// status: a device status word (8 when a sweep's bounded wait gave up); null selects one launch
+// per block step.
 void lu_solve_fp64(const double2* A, int n, const int* perm, const double2* inv, double2* x, double2* tmp, int ncol,
-                   cudaStream_t st, long long* launches, unsigned* epoch = nullptr, int* status = nullptr);
+                   cudaStream_t st, long long* launches, int* status = nullptr);
 void lu_solve_fp32(const float2* A, int n, const int* perm, const double2* inv, double2* x, double2* tmp, int ncol,
-                   cudaStream_t st, long long* launches, unsigned* epoch = nullptr, int* status = nullptr);
+                   cudaStream_t st, long long* launches, int* status = nullptr);
+// The persistent sweeps alone (no permutation): out = (L U)^-1 rhs or its adjoint, through mid;
+// false when they cannot run (TCU_SOLVE=steps, no status word, a refused launch; rhs is intact).
+template <typename C>
+bool lu_sweeps(const C* A, int n, const double2* inv, const double2* rhs, double2* mid, double2* out, int ncol,
+               bool adjoint, int* status, cudaStream_t st, long long* launches);
 size_t lu_workspace_bytes(int n, bool fp32);
 size_t tf32_pack_bytes(int n);  // packed tensor-core operands of the mixed LU
 void lu_init_attributes();

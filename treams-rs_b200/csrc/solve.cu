@@ -8,11 +8,8 @@
 // updated in place while the block solutions go to a separate array, so no CTA reads a
 // row that another CTA writes in the same step.
 //
-// The default sweep is one persistent kernel per triangle instead (trsv_chain_kernel): CTA c
-// takes the block rows c, c + G, ... in solve order and accumulates L_ij y_j over its
-// dependencies in a fixed order, consuming each y_j as soon as the block's completion flag
-// carries this launch's epoch (release/acquire, bounded waits), so a sweep costs the chain
-// of diagonal steps plus one pass over the factor instead of one launch per block.
+// The default is one persistent kernel per triangle instead (sweep_kernel), which also serves the
+// adjoint solves; the block steps stay for TCU_SOLVE=steps and for a refused cooperative launch.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -25,7 +22,8 @@
 namespace tcu {
 
 constexpr int SB = 64;      // diagonal block size
-constexpr int SMAXC = 8;    // right-hand sides per sweep
+constexpr int SMAXC = 8;    // right-hand sides per block step
+enum SweepOp { SW_L, SW_U, SW_UH, SW_LH };
 
 template <typename C>
 __device__ __forceinline__ double2 to_d2(C v) {
@@ -218,186 +216,203 @@ __global__ void __launch_bounds__(256) trsv_inv_step_kernel(const C* __restrict_
     }
 }
 
-// ---- persistent sweep ------------------------------------------------------------------
-constexpr int CH_JB = 8;  // block solutions staged per batch
+// ---- persistent sweeps -----------------------------------------------------------------
+// One cooperative launch per triangle and direction. Grid (G, chunks): chunk y solves NC of the
+// right-hand-side columns, its CTA x takes the block rows x, x + G, ... in solve order. A block
+// row t accumulates s = b_t - sum_(j < t) T_tj y_j tile by tile (64 x 64, a fixed order) and ends
+// with y_t = Dinv_t s. The block solutions are their own completion flags: the solution array
+// starts as all-ones bit patterns (a NaN no computation produces), a consumer polls the entries it
+// needs until both halves differ, so a step of the chain costs one store and one load through L2
+// and no fence, flag or second read.
+//
+// What bounds it: with few columns the chain of n / 64 dependent steps (a step: poll, one tile,
+// reduction, the diagonal product), with many columns the FP64 arithmetic, n^2 NC / 2 complex
+// multiply-adds a chunk. Hence at most 4 columns a chunk, all chunks side by side on the SMs:
+// a tile of 4 columns takes about 0.5 us of an SM's FP64 rate, below the latency of a step.
+// Tiles arrive by cp.async (3 stages of 32 KB for FP32 factors, 2 of 64 KB for FP64), padded to 65
+// rows so that the transposed reads of the adjoint sweeps have no bank conflicts either.
+// Measured against one launch per 8 columns with completion flags behind fences (both sides us per
+// triangle): n = 9600, 17 columns, FP32 factor 2320 -> 840; n = 1920, 96 columns, FP64 2340 -> 190;
+// n = 24576, 3 columns, FP32 1980 -> 1150; one column 2.6 -> 1.5 us per block step.
+// Every poll is bounded (4 s): status 8 and all CTAs return.
+constexpr int SW_THREADS = 512;
+constexpr int SW_Q = SW_THREADS / SB;  // contraction groups of a tile
+constexpr int SW_K = SB / SW_Q;        // contraction entries per thread and tile
+constexpr int SW_LD = SB + 1;
+constexpr int SW_MAXC = 4;             // columns per chunk
 
-__device__ __forceinline__ unsigned ch_ld_acquire(const unsigned* p) {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ unsigned long long ch_ns() {
+__device__ __forceinline__ unsigned long long sw_ns() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
-__device__ __forceinline__ void ch_cp16(void* smem, const void* gmem) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(smem)),
-                 "l"(gmem)
-                 : "memory");
+__device__ __forceinline__ double2 sw_load(const double2* p) {
+    double2 v;
+    asm volatile("ld.relaxed.gpu.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p) : "memory");
+    return v;
 }
-
-// Bounded wait (4 s) for flag == epoch; false (and status 8) when it gives up.
-__device__ bool ch_wait(const unsigned* flag, unsigned epoch, int* status) {
-    if (ch_ld_acquire(flag) == epoch) return true;
-    const unsigned long long t0 = ch_ns();
-    unsigned spins = 0;
-    while (ch_ld_acquire(flag) != epoch) {
-        if ((++spins & 255u) == 0 && (*(volatile int*)status == 8 || ch_ns() - t0 > 4000000000ull)) {
-            atomicExch(status, 8);
-            return false;
+__device__ __forceinline__ void sw_store(double2* p, double2 v) {
+    asm volatile("st.relaxed.gpu.global.v2.f64 [%0], {%1, %2};" ::"l"(p), "d"(v.x), "d"(v.y) : "memory");
+}
+__device__ __forceinline__ bool sw_empty(double v) { return __double_as_longlong(v) == -1ll; }
+__device__ __forceinline__ double sw_value(double v) {  // never the empty pattern
+    return sw_empty(v) ? __longlong_as_double(0x7ff8000000000000ll) : v;
+}
+// Polls one entry until it is written; false (and status 8) after 4 s or when another wait gave up.
+__device__ __forceinline__ bool sw_wait(const double2* p, double2& v, int* status) {
+    unsigned long long t0 = 0;
+    for (unsigned spins = 1; sw_empty(v.x) || sw_empty(v.y); ++spins) {
+        if ((spins & 255u) == 0) {  // the clock is read on long waits only: it costs about a microsecond
+            const unsigned long long now = sw_ns();
+            if (!t0) t0 = now;
+            if (*(volatile int*)status == 8 || now - t0 > 4000000000ull) {
+                atomicExch(status, 8);
+                return false;
+            }
         }
+        v = sw_load(p);
     }
     return true;
 }
-
 template <typename C>
-__host__ __device__ constexpr size_t chain_smem_bytes(int nc) {
-    return ((size_t)SB * SB + (size_t)CH_JB * nc * SB + 4 * (size_t)nc * SB + (size_t)nc * SB) * sizeof(double2);
+__device__ __forceinline__ void sw_copy(C* smem, const C* gmem, bool valid) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    const int sz = valid ? (int)sizeof(C) : 0;
+    if (sizeof(C) == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(s), "l"(gmem), "r"(sz) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(s), "l"(gmem), "r"(sz) : "memory");
 }
 
-// y = T^-1 b for the unit lower (LOWER) or upper triangle T of the factor, with the FP64
-// inverses of its diagonal blocks. rhs: b (n x NC, read only); sol: y. Block row i (solve
-// order t) forms s = b_i - sum_j T_ij y_j over its dependencies in solve order, then
-// y_i = Dinv_i s, stores it and releases flags[i] = epoch.
-template <typename C, bool LOWER, int NC>
-__global__ void __launch_bounds__(256) trsv_chain_kernel(const C* __restrict__ A, size_t lda, int n, int nb,
-                                                         const double2* __restrict__ dinv,
-                                                         const double2* __restrict__ rhs, double2* __restrict__ sol,
-                                                         unsigned* __restrict__ flags, unsigned epoch,
-                                                         int* __restrict__ status) {
-    extern __shared__ __align__(16) double2 ch_smem[];
-    double2* dsm = ch_smem;                    // Dinv of the current block row, column-major 64 x 64
-    double2* ys = dsm + SB * SB;               // [CH_JB][NC][SB] staged block solutions
-    double2* part = ys + CH_JB * NC * SB;      // [4][NC][SB]
-    double2* sb = part + 4 * NC * SB;          // [NC][SB] right-hand side block
-    __shared__ int s_ready;
-    const int tid = threadIdx.x, ir = tid % SB, q = tid / SB;
-    auto blk = [&](int t) { return LOWER ? t : nb - 1 - t; };
-    int ready = 0;  // solve-order blocks known to be complete
+template <typename C>
+constexpr int sw_stages() {
+    return sizeof(C) == 8 ? 3 : 2;
+}
+template <typename C>
+constexpr size_t sweep_smem_bytes(int nc) {
+    return (size_t)sw_stages<C>() * SB * SW_LD * sizeof(C) + (size_t)(2 + SW_Q + 1) * nc * SB * sizeof(double2);
+}
+
+// sol = op(T)^-1 rhs for ncol columns (n x ncol, sol preset to the empty pattern) with T the unit
+// lower or the upper triangle of the factor. OP: SW_L and SW_UH run down the block rows (L y = b,
+// U^H y = b), SW_U and SW_LH up. clear: presets the solution array of the next sweep.
+template <typename C, int OP, int NC>
+__global__ void __launch_bounds__(SW_THREADS, 1)
+    sweep_kernel(const C* __restrict__ A, size_t lda, int n, int nb, int ncol, const double2* __restrict__ dinv,
+                 const double2* __restrict__ rhs, double2* sol, double2* clear, int* status) {
+    constexpr bool DOWN = OP == SW_L || OP == SW_UH, ADJ = OP == SW_UH || OP == SW_LH;
+    constexpr int ST = sw_stages<C>();
+    extern __shared__ __align__(16) unsigned char sw_smem[];
+    double2* ys = reinterpret_cast<double2*>(sw_smem);  // [2][NC][SB]
+    double2* part = ys + 2 * NC * SB;                   // [SW_Q][NC][SB]
+    double2* sb = part + SW_Q * NC * SB;                // [NC][SB]
+    C* tiles = reinterpret_cast<C*>(sb + NC * SB);      // [ST][SB][SW_LD]: column k at k * SW_LD
+    const int tid = threadIdx.x, o = tid % SB, q = tid / SB;
+    const int col0 = blockIdx.y * NC, nc = min(NC, ncol - col0);
+    rhs += (size_t)col0 * n;
+    sol += (size_t)col0 * n;
+    if (clear) {
+        clear += (size_t)col0 * n;
+        const double e = __longlong_as_double(-1ll);
+        for (size_t i = (size_t)blockIdx.x * SW_THREADS + tid; i < (size_t)nc * n; i += (size_t)gridDim.x * SW_THREADS)
+            clear[i] = make_double2(e, e);
+    }
+    auto blk = [&](int t) { return DOWN ? t : nb - 1 - t; };
+    // this thread's entry (column q, row o of a block) of the solution and right-hand-side blocks
+    const bool entry = q < nc;
     for (int t = blockIdx.x; t < nb; t += gridDim.x) {
-        const int bi = blk(t), r0 = bi * SB, bw = min(SB, n - r0);
-        const bool has_row = ir < bw;
-        const size_t row = (size_t)r0 + (has_row ? ir : 0);
-        // the diagonal inverse and the right-hand side block arrive in the background
-        const double2* dsrc = dinv + (size_t)bi * SB * SB;
-        for (int idx = tid; idx < SB * SB; idx += blockDim.x) ch_cp16(&dsm[idx], &dsrc[idx]);
-        for (int idx = tid; idx < NC * SB; idx += blockDim.x) {
-            const int ii = idx % SB, c = idx / SB;
-            if (ii < bw)
-                ch_cp16(&sb[idx], &rhs[(size_t)c * n + r0 + ii]);
-            else
-                sb[idx] = make_double2(0.0, 0.0);
+        const int bi = blk(t), r0 = bi * SB;
+        double2 d[SW_K], rb = make_double2(0.0, 0.0);
+#pragma unroll
+        for (int u = 0; u < SW_K; ++u) {
+            const size_t at = ADJ ? (size_t)o * SB + q * SW_K + u : (size_t)(q * SW_K + u) * SB + o;
+            d[u] = __ldg(&dinv[(size_t)bi * SB * SB + at]);
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (entry && r0 + o < n) rb = rhs[(size_t)q * n + r0 + o];
+        auto load_tile = [&](int ts) {  // T_(t, ts), or the tile it is the adjoint of
+            if (ts < t) {
+                const int ri = ADJ ? blk(ts) * SB : r0, ci = ADJ ? r0 : blk(ts) * SB;
+                C* dst = tiles + (size_t)(ts % ST) * SB * SW_LD;
+                const bool rok = ri + o < n;
+#pragma unroll
+                for (int u = 0; u < SW_K; ++u) {
+                    const int k = q + SW_Q * u;
+                    const bool ok = rok && ci + k < n;
+                    sw_copy(&dst[k * SW_LD + o], ok ? &A[(size_t)(ci + k) * lda + ri + o] : A, ok);
+                }
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+#pragma unroll
+        for (int s = 0; s < ST - 1; ++s) load_tile(s);
         double2 acc[NC];
 #pragma unroll
         for (int c = 0; c < NC; ++c) acc[c] = make_double2(0.0, 0.0);
-        C cur[16];
-        auto load_block = [&](int ts, C (&v)[16]) {
-            const int c0 = blk(ts) * SB + q * 16;
+        const double2* yp = sol + (size_t)(entry ? q : 0) * n + o;
+        double2 pre = make_double2(0.0, 0.0);
+        auto in_range = [&](int ts) { return entry && blk(ts) * SB + o < n; };
+        if (t > 0 && in_range(0)) pre = sw_load(yp + blk(0) * SB);
+        for (int ts = 0; ts < t; ++ts) {
+            int gave_up = 0;
+            if (q < NC) {
+                if (in_range(ts))
+                    gave_up = !sw_wait(yp + blk(ts) * SB, pre, status);
+                else
+                    pre = make_double2(0.0, 0.0);
+                ys[((ts & 1) * NC + q) * SB + o] = pre;
+            }
+            asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
+            // tile ts and y_ts are in shared memory; the stage of tile ts - 1 is free
+            if (__syncthreads_or(gave_up)) {
+                asm volatile("cp.async.wait_all;" ::: "memory");
+                return;
+            }
+            load_tile(ts + ST - 1);
+            if (ts + 1 < t && in_range(ts + 1)) pre = sw_load(yp + blk(ts + 1) * SB);
+            const C* tile = tiles + (size_t)(ts % ST) * SB * SW_LD;
+            const double2* yv = ys + (ts & 1) * NC * SB + q * SW_K;
 #pragma unroll
-            for (int u = 0; u < 16; ++u) {
-                if (has_row && c0 + u < n)
-                    v[u] = A[(size_t)(c0 + u) * lda + row];
-                else {
-                    v[u].x = 0;
-                    v[u].y = 0;
+            for (int u = 0; u < SW_K; ++u) {
+                const double2 v = to_d2(ADJ ? tile[o * SW_LD + q * SW_K + u] : tile[(q * SW_K + u) * SW_LD + o]);
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    if (ADJ)
+                        cfma_conj(acc[c], v, yv[c * SB + u]);
+                    else
+                        cfma(acc[c], v, yv[c * SB + u]);
                 }
             }
-        };
-        if (t > 0) load_block(0, cur);
-        int ts = 0;
-        while (ts < t) {
-            if (ready <= ts) {
-                __syncthreads();  // s_ready of the previous wait has been read by every thread
-                if (tid == 0) {
-                    int rdy = -1;
-                    if (ch_wait(&flags[blk(ts)], epoch, status)) {
-                        rdy = ts + 1;
-                        while (rdy < t && rdy < ts + CH_JB && ch_ld_acquire(&flags[blk(rdy)]) == epoch) ++rdy;
-                    }
-                    s_ready = rdy;
-                }
-                __syncthreads();
-                ready = s_ready;
-                if (ready < 0) {
-                    asm volatile("cp.async.wait_all;" ::: "memory");
-                    return;
-                }
-            }
-            const int cnt = min(CH_JB, ready - ts);
-            for (int idx = tid; idx < cnt * NC * SB; idx += blockDim.x) {
-                const int ii = idx % SB, c = (idx / SB) % NC, jj = idx / (SB * NC);
-                const int gi = blk(ts + jj) * SB + ii;
-                ys[idx] = gi < n ? __ldcg(&sol[(size_t)c * n + gi]) : make_double2(0.0, 0.0);
-            }
-            __syncthreads();
-            for (int jj = 0; jj < cnt; ++jj) {
-                C nxt[16];
-                const bool more = ts + jj + 1 < t;
-                if (more) load_block(ts + jj + 1, nxt);
-#pragma unroll
-                for (int u = 0; u < 16; ++u) {
-                    const double lr = cur[u].x, li = cur[u].y;
-#pragma unroll
-                    for (int c = 0; c < NC; ++c) {
-                        const double2 y = ys[(jj * NC + c) * SB + q * 16 + u];
-                        acc[c].x += lr * y.x - li * y.y;
-                        acc[c].y += lr * y.y + li * y.x;
-                    }
-                }
-                if (more)
-#pragma unroll
-                    for (int u = 0; u < 16; ++u) cur[u] = nxt[u];
-            }
-            ts += cnt;
-            __syncthreads();  // ys is restaged by the next batch
         }
 #pragma unroll
-        for (int c = 0; c < NC; ++c) part[(q * NC + c) * SB + ir] = acc[c];
-        asm volatile("cp.async.wait_all;" ::: "memory");
+        for (int c = 0; c < NC; ++c) part[(q * NC + c) * SB + o] = acc[c];
         __syncthreads();
-        for (int idx = tid; idx < NC * SB; idx += blockDim.x) {
-            const int ii = idx % SB, c = idx / SB;
-            double2 v = sb[idx];
+        if (q < NC) {
+            double2 s = rb;
 #pragma unroll
-            for (int qq = 0; qq < 4; ++qq) {
-                v.x -= part[(qq * NC + c) * SB + ii].x;
-                v.y -= part[(qq * NC + c) * SB + ii].y;
-            }
-            sb[idx] = v;
+            for (int g = 0; g < SW_Q; ++g) s = csub(s, part[(g * NC + q) * SB + o]);
+            sb[q * SB + o] = s;
         }
         __syncthreads();
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
             double2 y = make_double2(0.0, 0.0);
 #pragma unroll
-            for (int u = 0; u < 16; ++u) {
-                const double2 d = dsm[(q * 16 + u) * SB + ir], v = sb[c * SB + q * 16 + u];
-                y.x += d.x * v.x - d.y * v.y;
-                y.y += d.x * v.y + d.y * v.x;
+            for (int u = 0; u < SW_K; ++u) {
+                if (ADJ)
+                    cfma_conj(y, d[u], sb[c * SB + q * SW_K + u]);
+                else
+                    cfma(y, d[u], sb[c * SB + q * SW_K + u]);
             }
-            part[(q * NC + c) * SB + ir] = y;
+            part[(q * NC + c) * SB + o] = y;
         }
         __syncthreads();
-        for (int idx = tid; idx < NC * SB; idx += blockDim.x) {
-            const int ii = idx % SB, c = idx / SB;
-            if (ii < bw) {
-                double2 y = part[c * SB + ii];
+        if (entry && r0 + o < n) {
+            double2 y = part[q * SB + o];
 #pragma unroll
-                for (int qq = 1; qq < 4; ++qq) {
-                    y.x += part[(qq * NC + c) * SB + ii].x;
-                    y.y += part[(qq * NC + c) * SB + ii].y;
-                }
-                sol[(size_t)c * n + r0 + ii] = y;
-            }
+            for (int g = 1; g < SW_Q; ++g) y = cadd(y, part[(g * NC + q) * SB + o]);
+            sw_store(&sol[(size_t)q * n + r0 + o], make_double2(sw_value(y.x), sw_value(y.y)));
         }
-        __syncthreads();
-        if (tid == 0) {
-            __threadfence();
-            asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(&flags[bi]), "r"(epoch) : "memory");
-        }
+        __syncthreads();  // part and the tile stages are free for the next block row
     }
 }
 
@@ -430,14 +445,10 @@ static void step_launch(int nc, cudaStream_t st, const C* A, int n, int b0, int 
     }
 }
 
-// the two sets of block inverses, then one completion flag per block (persistent sweeps)
+// the two sets of block inverses
 size_t lu_inverse_bytes(int n) {
     const size_t nb = (n + SB - 1) / SB;
-    return (size_t)2 * nb * SB * SB * sizeof(double2) + (nb + 64) * sizeof(unsigned);
-}
-static unsigned* chain_flags(const double2* inv, int n) {
-    const size_t nb = (n + SB - 1) / SB;
-    return (unsigned*)(inv + 2 * nb * SB * SB);
+    return (size_t)2 * nb * SB * SB * sizeof(double2);
 }
 
 template <typename C>
@@ -452,7 +463,6 @@ static void inverses_impl(const C* A, int n, double2* inv, cudaStream_t st, long
         cudaFuncSetAttribute(tri_block_inverse_kernel<float2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         cudaFuncSetAttribute(tri_block_inverse_kernel<float2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     });
-    cudaMemsetAsync(chain_flags(inv, n), 0, (size_t)(nb + 64) * sizeof(unsigned), st);
     tri_block_inverse_kernel<C, true><<<nb, 256, smem, st>>>(A, n, n, inv);
     tri_block_inverse_kernel<C, false><<<nb, 256, smem, st>>>(A, n, n, inv + (size_t)nb * SB * SB);
     *launches += 2;
@@ -473,70 +483,89 @@ static bool chain_enabled() {
     return v;
 }
 
-template <typename C, bool LOWER, int NC>
-static bool chain_launch_nc(cudaStream_t st, const C* A, int n, const double2* dinv, const double2* rhs,
-                            double2* sol, unsigned* flags, unsigned epoch, int* status) {
-    static PerDeviceOnce attr;
-    const size_t smem = chain_smem_bytes<C>(NC);
-    // a refused attribute makes the cooperative launch below fail, and the caller takes the step path
-    once_per_device(attr, [&] {
-        cudaFuncSetAttribute(trsv_chain_kernel<C, LOWER, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    });
-    const int nb = (n + SB - 1) / SB;
-    const int grid = std::min(nb, g_sms);
-    size_t lda = (size_t)n;
-    void* args[] = {(void*)&A, &lda, &n, (void*)&nb, (void*)&dinv, (void*)&rhs, &sol, &flags, &epoch, &status};
-    return cudaLaunchCooperativeKernel((void*)trsv_chain_kernel<C, LOWER, NC>, dim3(grid), dim3(256), args, smem,
-                                       st) == cudaSuccess;
-}
-
-template <typename C, bool LOWER>
-static bool chain_launch(int nc, cudaStream_t st, const C* A, int n, const double2* dinv, const double2* rhs,
-                         double2* sol, unsigned* flags, unsigned epoch, int* status) {
-    switch (nc) {
-#define CH_CASE(K) \
-    case K: return chain_launch_nc<C, LOWER, K>(st, A, n, dinv, rhs, sol, flags, epoch, status);
-        CH_CASE(1) CH_CASE(2) CH_CASE(3) CH_CASE(4) CH_CASE(5) CH_CASE(6) CH_CASE(7) CH_CASE(8)
-#undef CH_CASE
-    }
-    return false;
-}
-
-// x (n x ncol) <- A^-1 x; tmp holds 2 n ncol complex.
-template <typename C>
-static void solve_impl(const C* A, int n, const int* perm, const double2* inv, double2* x, double2* tmp, int ncol,
-                       cudaStream_t st, long long* launches, unsigned* epoch, int* status) {
+static void sweep_init() {
     static PerDeviceOnce sms_once;
     once_per_device(sms_once, [] {
         int dev = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev);
     });
+}
+
+template <typename C, int OP, int NC>
+static bool sweep_launch_nc(cudaStream_t st, const C* A, int n, const double2* dinv, const double2* rhs, double2* sol,
+                            double2* clear, int ncol, int* status) {
+    static PerDeviceOnce attr;
+    const size_t smem = sweep_smem_bytes<C>(NC);
+    // a refused attribute makes the cooperative launch below fail, and the caller takes the step path
+    once_per_device(attr, [&] {
+        cudaFuncSetAttribute(sweep_kernel<C, OP, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    });
+    const int nb = (n + SB - 1) / SB, chunks = (ncol + NC - 1) / NC;
+    const int G = std::min(nb, g_sms / chunks);
+    if (G < 1) return false;
+    size_t lda = (size_t)n;
+    void* args[] = {(void*)&A, &lda, &n, (void*)&nb, &ncol, (void*)&dinv, (void*)&rhs, &sol, &clear, &status};
+    return cudaLaunchCooperativeKernel((void*)sweep_kernel<C, OP, NC>, dim3(G, chunks), dim3(SW_THREADS), args, smem,
+                                       st) == cudaSuccess;
+}
+
+template <typename C, int OP>
+static bool sweep_launch(cudaStream_t st, const C* A, int n, const double2* dinv, const double2* rhs, double2* sol,
+                         double2* clear, int ncol, int* status) {
+    switch (std::min(ncol, SW_MAXC)) {
+#define SW_CASE(K) \
+    case K: return sweep_launch_nc<C, OP, K>(st, A, n, dinv, rhs, sol, clear, ncol, status);
+        SW_CASE(1) SW_CASE(2) SW_CASE(3) SW_CASE(4)
+#undef SW_CASE
+    }
+    return false;
+}
+
+// The two sweeps of a solve over ncol <= SOLVE_MAXC columns, rhs -> mid -> out; false when they are
+// turned off or a launch was refused (mid and out are then undefined, rhs is intact).
+template <typename C>
+bool lu_sweeps(const C* A, int n, const double2* inv, const double2* rhs, double2* mid, double2* out, int ncol,
+               bool adjoint, int* status, cudaStream_t st, long long* launches) {
+    if (!chain_enabled() || !status || ncol > SOLVE_MAXC) return false;
+    sweep_init();
+    const size_t nb = (n + SB - 1) / SB;
+    const double2 *linv = inv, *uinv = inv + nb * SB * SB;
+    cudaMemsetAsync(mid, 0xff, (size_t)n * ncol * sizeof(double2), st);  // the empty pattern
+    const bool ok = adjoint ? sweep_launch<C, SW_UH>(st, A, n, uinv, rhs, mid, out, ncol, status) &&
+                                  sweep_launch<C, SW_LH>(st, A, n, linv, mid, out, nullptr, ncol, status)
+                            : sweep_launch<C, SW_L>(st, A, n, linv, rhs, mid, out, ncol, status) &&
+                                  sweep_launch<C, SW_U>(st, A, n, uinv, mid, out, nullptr, ncol, status);
+    if (ok) {
+        if (launches) *launches += 2;
+    } else {
+        cudaGetLastError();  // a launch that was refused leaves no work behind
+    }
+    return ok;
+}
+template bool lu_sweeps<float2>(const float2*, int, const double2*, const double2*, double2*, double2*, int, bool, int*,
+                                cudaStream_t, long long*);
+template bool lu_sweeps<double2>(const double2*, int, const double2*, const double2*, double2*, double2*, int, bool,
+                                 int*, cudaStream_t, long long*);
+
+// x (n x ncol) <- A^-1 x; tmp holds 2 n ncol complex.
+template <typename C>
+static void solve_impl(const C* A, int n, const int* perm, const double2* inv, double2* x, double2* tmp, int ncol,
+                       cudaStream_t st, long long* launches, int* status) {
+    sweep_init();
     StageScope sc(ST_SOLVE, st);
     const int nb = (n + SB - 1) / SB;
+    const size_t tot = (size_t)n * ncol;
+    gather_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(x, tmp, perm, n, ncol);
+    ++*launches;
+    if (lu_sweeps<C>(A, n, inv, tmp, tmp + tot, x, ncol, false, status, st, launches)) return;
     const double2* linv = inv;
     const double2* uinv = inv + (size_t)nb * SB * SB;
     for (int c0 = 0; c0 < ncol; c0 += SMAXC) {
-        int nc = std::min(SMAXC, ncol - c0);
+        const int nc = std::min(SMAXC, ncol - c0);
         double2* xc = x + (size_t)c0 * n;
-        double2* y = tmp;                  // P b, then updated in place by the forward sweep
-        double2* z = tmp + (size_t)n * nc; // forward solution, updated in place by the backward sweep
-        size_t tot = (size_t)n * nc;
-        gather_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(xc, y, perm, n, nc);
-        ++*launches;
-        if (chain_enabled() && epoch && status) {
-            // forward sweep y -> z, backward sweep z -> x; each launch has its own epoch
-            unsigned* flags = chain_flags(inv, n);
-            if (chain_launch<C, true>(nc, st, A, n, linv, y, z, flags, ++*epoch, status) &&
-                chain_launch<C, false>(nc, st, A, n, uinv, z, xc, flags, ++*epoch, status)) {
-                *launches += 2;
-                continue;
-            }
-            // a launch that was refused leaves no work behind (the flags of later launches
-            // carry new epochs); the step path below recomputes this column chunk
-            cudaGetLastError();
-            cudaMemsetAsync(z, 0, tot * sizeof(double2), st);
-        }
+        double2* y = tmp + (size_t)c0 * n;        // P b, then updated in place by the forward sweep
+        double2* z = tmp + tot + (size_t)c0 * n;  // forward solution, updated in place by the backward sweep
         for (int b = 0; b < nb; ++b) {
             int b0 = b * SB, bw = std::min(SB, n - b0);
             step_launch<C, true>(nc, st, A, n, b0, bw, linv + (size_t)b * SB * SB, y, z);
@@ -551,12 +580,12 @@ static void solve_impl(const C* A, int n, const int* perm, const double2* inv, d
 }
 
 void lu_solve_fp64(const double2* A, int n, const int* perm, const double2* inv, double2* x, double2* tmp, int ncol,
-                   cudaStream_t st, long long* launches, unsigned* epoch, int* status) {
-    solve_impl<double2>(A, n, perm, inv, x, tmp, ncol, st, launches, epoch, status);
+                   cudaStream_t st, long long* launches, int* status) {
+    solve_impl<double2>(A, n, perm, inv, x, tmp, ncol, st, launches, status);
 }
 void lu_solve_fp32(const float2* A, int n, const int* perm, const double2* inv, double2* x, double2* tmp, int ncol,
-                   cudaStream_t st, long long* launches, unsigned* epoch, int* status) {
-    solve_impl<float2>(A, n, perm, inv, x, tmp, ncol, st, launches, epoch, status);
+                   cudaStream_t st, long long* launches, int* status) {
+    solve_impl<float2>(A, n, perm, inv, x, tmp, ncol, st, launches, status);
 }
 
 }  // namespace tcu
