@@ -379,7 +379,7 @@ tcu_status factor_impl(tcu_context* ctx, int L, double k0, size_t N, const doubl
         if ((e = read_status(ctx, "Mie coefficients"))) break;
         launch_assemble(*P, (int)N, k0, f->d_pos, f->d_T, f->d_A, n, precision == TCU_MIXED, ctx->stream);
         ++ctx->launches;
-        if (apply_gemm_supported(*P) && stored_tables_enabled()) {
+        if (stored_full_supported(*P) && stored_tables_enabled()) {
             // the refinement's residuals apply the FP64 operator from stored pair tables (at most a
             // fifth of the matrix's bytes); without room they rebuild the tables per application
             void* z = nullptr;
@@ -786,11 +786,11 @@ int batch_workers() {
     return std::max(1, std::min(8, v));
 }
 
-// The stored-table operator for the applications of GMRES: lmax 2..5 in product form, unless
+// The stored-table operator for the applications of GMRES: lmax 2..7 in product form, unless
 // TCU_APPLY is "fly" or "terms", and only while the tables take at most half of the free device
 // memory (and at most 64 GB).
 bool use_stored_tables(const DevPlan& P, int N) {
-    if (!apply_gemm_supported(P) || !stored_tables_enabled()) return false;
+    if (!stored_full_supported(P) || !stored_tables_enabled()) return false;
     const size_t bytes = stored_tables_bytes(P, N, STORED_FULL);
     if (bytes == 0 || bytes > ((size_t)64 << 30)) return false;
     size_t fr = 0, tot = 0;
@@ -1049,7 +1049,21 @@ tcu_status tcu_cross_sections(tcu_context* ctx, int lmax, double k0, size_t N, c
     CK(cudaMemcpyAsync(pos, positions, N * 24, cudaMemcpyHostToDevice, ctx->stream), "copy");
     CK(cudaMemcpyAsync(dx, x, per * 16, cudaMemcpyHostToDevice, ctx->stream), "copy");
     CK(cudaMemcpyAsync(db, b, per * 16, cudaMemcpyHostToDevice, ctx->stream), "copy");
-    apply_op(ctx, P, (int)N, k0, pos, nullptr, dx, n, p, nullptr, 1.0, 1.0, false, ox);
+    DevBuf zbuf(ctx), xfbuf(ctx);
+    const bool stored = !apply_gemm_supported(*P) && use_stored_tables(*P, (int)N);
+    if (stored && zbuf.alloc(stored_tables_bytes(*P, (int)N, STORED_FULL)) == cudaSuccess &&
+        xfbuf.alloc(stored_inputs_bytes(*P, (int)N, STORED_FULL, p)) == cudaSuccess) {
+        // lmax 6 and 7: the regular operator from its pair tables, like the outgoing one
+        CK(cudaMemsetAsync(ctx->d_status, 0, 4, ctx->stream), "status");
+        build_stored_tables(*P, (int)N, k0, pos, STORED_FULL, (cplx*)zbuf.p, ctx->stream, false);
+        launch_apply_stored(*P, (int)N, STORED_FULL, (const cplx*)zbuf.p, nullptr, dx, n, p, nullptr, 1.0, 1.0, ox,
+                            (cplx*)xfbuf.p, ctx->d_status, ctx->stream, false);
+        ctx->launches += 4;
+        if ((s = read_status(ctx, "cross sections"))) return s;
+    } else {
+        cudaGetLastError();  // no room: the tables per pair
+        apply_op(ctx, P, (int)N, k0, pos, nullptr, dx, n, p, nullptr, 1.0, 1.0, false, ox);
+    }
     std::vector<double> s1(p), s2(p);
     vec_real_dots(dx, ox, n, p, ctx->d_small, ctx->d_partial, ctx->stream);
     CK(cudaMemcpyAsync(s1.data(), ctx->d_small, p * 8, cudaMemcpyDeviceToHost, ctx->stream), "copy");
@@ -1236,10 +1250,12 @@ tcu_status tcu_cluster_apply(tcu_context* ctx, int lmax, double k0, size_t N, co
     if ((s = read_status(ctx, "Mie coefficients"))) return s;
     // Several columns (or TCU_APPLY=stored): the pair tables once, then the stored-table
     // product per column; one column: the product form (building the tables costs about one
-    // application, so storing them gains nothing).
+    // application, so storing them gains nothing), which ends at lmax 5: at lmax 6 and 7 tables
+    // and product (300 spheres lmax 6: 0.11 + 0.57 ms) beat the term sums (4.3 ms) for one column too.
     const char* form = getenv("TCU_APPLY");
     const bool forced = form && strcmp(form, "stored") == 0;
-    if (apply_gemm_supported(*P) && (forced || (p >= 2 && use_stored_tables(*P, (int)N)))) {
+    if (stored_full_supported(*P) &&
+        (forced || ((p >= 2 || !apply_gemm_supported(*P)) && use_stored_tables(*P, (int)N)))) {
         DevBuf zbuf(ctx), xfbuf(ctx);
         CK(zbuf.alloc(stored_tables_bytes(*P, (int)N, STORED_FULL)), "stored tables");
         CK(xfbuf.alloc(stored_inputs_bytes(*P, (int)N, STORED_FULL, p)), "packed inputs");

@@ -69,18 +69,30 @@ size_t gemm_smem(const SubOp& o, const GemmShape& s) {
     const size_t tsz = (size_t)(o.order + 1) * (o.order + 1);
     const size_t rows = (size_t)s.TR * s.RG + 1, cols = (size_t)s.TC * s.CG, npair = (size_t)s.DI * s.KJ;
     const size_t chunk = ((size_t)s.KJ * rows + (size_t)s.KJ * cols + npair * (o.order + 1)) * sizeof(cplx) +
-                         npair * sizeof(double4);
+                         npair * sizeof(double4) + tsz * sizeof(double2);
     const size_t g = (size_t)s.DI * tsz * 2 * o.nsrc * sizeof(cplx);
     return chunk > g ? chunk : g;
 }
 
+// Coefficients of the degree recurrence P_deg = a z P_(deg-1) - b r^2 P_(deg-2) of order column m,
+// at m (order + 1) + deg: the divisions once per CTA instead of once per pair and degree.
+__device__ __forceinline__ void recurrence_table(int order, double2* rec, int tid, int nthr) {
+    const int ord1 = order + 1;
+    for (int t = tid; t < ord1 * ord1; t += nthr) {
+        const int m = t / ord1, deg = t - m * ord1;
+        rec[t] = deg > m ? make_double2(double(2 * deg - 1) / double(deg - m), double(deg + m - 1) / double(deg - m))
+                         : make_double2(0.0, 0.0);
+    }
+}
+
 // Phases A and B of one chunk: the harmonic tables of the pairs (i0 + il, j0 + jj), il < DI,
-// jj < KJ, into Zs (row il * ts + idx, column jj, leading dimension ZLD); Rs and Ds hold the
-// radial sequences and directions. One barrier inside (between A and B), none at the end.
+// jj < KJ, into Zs (row il * ts + idx, column jj, leading dimension ZLD); Rs (entry q of pair p at
+// q npair + p) and Ds hold the radial sequences and directions, rec the recurrence_table. One
+// barrier inside (between A and B), none at the end.
 __device__ __forceinline__ void build_chunk(const DevPlan& P, int order, int N, double k,
                                             const double* __restrict__ pos, bool singular, int i0, int j0,
-                                            int DI, int KJ, int ZLD, cplx* Zs, cplx* Rs, double4* Ds, int tid,
-                                            int nthr) {
+                                            int DI, int KJ, int ZLD, cplx* Zs, cplx* Rs, double4* Ds,
+                                            const double2* rec, int tid, int nthr) {
     const int ord1 = order + 1, ts = ord1 * ord1, npair = DI * KJ;
     // A) per pair: state 2 = a table, 1 = coincident centres of the regular kind (Z = e_0),
     //    0 = no coupling (the pair i = j, sources or destinations past N, coincident outgoing)
@@ -92,15 +104,27 @@ __device__ __forceinline__ void build_chunk(const DevPlan& P, int order, int N, 
             if (unit_direction(pos[3 * i] - pos[3 * j], pos[3 * i + 1] - pos[3 * j + 1],
                                pos[3 * i + 2] - pos[3 * j + 2], r, u)) {
                 state = 2.0;
-                cplx* rad = Rs + (size_t)p * ord1;
-                if (singular) {
+                if (singular && k * r >= 0.5) {
+                    // the recurrence of hankel_sequence, stored as it runs (no local array)
+                    const double inv = 1.0 / (k * r);
+                    double sn, cs;
+                    sincos(k * r, &sn, &cs);
+                    cplx prev = mk(cs * inv, sn * inv), cur = mk(sn * inv, -cs * inv);
+                    for (int q = 0; q <= order; ++q) {
+                        Rs[(size_t)q * npair + p] = cur;
+                        const double f = double(2 * q + 1) * inv;
+                        const cplx next = mk(f * cur.x - prev.x, f * cur.y - prev.y);
+                        prev = cur;
+                        cur = next;
+                    }
+                } else if (singular) {
                     cplx h[MAXP];
                     hankel_sequence<MAXP>(order, k * r, h);
-                    for (int q = 0; q <= order; ++q) rad[q] = h[q];
+                    for (int q = 0; q <= order; ++q) Rs[(size_t)q * npair + p] = h[q];
                 } else {
                     double jv[MAXP];
                     bessel_j_sequence<MAXP>(order, k * r, jv);
-                    for (int q = 0; q <= order; ++q) rad[q] = mk(jv[q], 0.0);
+                    for (int q = 0; q <= order; ++q) Rs[(size_t)q * npair + p] = mk(jv[q], 0.0);
                 }
             } else if (!singular) {
                 state = 1.0;
@@ -109,15 +133,15 @@ __device__ __forceinline__ void build_chunk(const DevPlan& P, int order, int N, 
         Ds[p] = make_double4(u[0], u[1], u[2], state);
     }
     __syncthreads();
-    // B) per (pair, order m >= 0): column m of the table, entries deg = m..order at
-    //    deg^2 + deg + m and deg^2 + deg - m
+    // B) per (order m >= 0, pair), consecutive threads on consecutive pairs so that a warp runs one
+    //    column length: entries deg = m..order at deg^2 + deg + m and deg^2 + deg - m
     for (int it = tid; it < npair * ord1; it += nthr) {
-        const int p = it / ord1, m = it - p * ord1;
+        const int m = it / npair, p = it - m * npair;
         const int il = p / KJ, jj = p - il * KJ;
         cplx* Zp = Zs + (size_t)jj * ZLD + (size_t)il * ts;
         const double4 D = Ds[p];
         if (D.w == 2.0) {
-            const cplx* rad = Rs + (size_t)p * ord1;
+            const cplx* rad = Rs + p;
             const cplx xy = mk(D.x, D.y);
             const double z = D.z, r2 = D.x * D.x + D.y * D.y + D.z * D.z;
             cplx diag = mk(1.0, 0.0);
@@ -125,17 +149,17 @@ __device__ __forceinline__ void build_chunk(const DevPlan& P, int order, int N, 
             cplx pc = diag, prev = mk(0.0, 0.0);
             for (int deg = m; deg <= order; ++deg) {
                 if (deg > m) {
-                    const double a = double(2 * deg - 1) / double(deg - m);
-                    const double b = double(deg + m - 1) / double(deg - m);
-                    const cplx next = mk(a * z * pc.x - b * r2 * prev.x, a * z * pc.y - b * r2 * prev.y);
+                    const double2 ab = rec[m * ord1 + deg];
+                    const double az = ab.x * z, br = ab.y * r2;
+                    const cplx next = mk(az * pc.x - br * prev.x, az * pc.y - br * prev.y);
                     prev = pc;
                     pc = next;
                 }
-                const cplx rd = rad[deg];
+                const cplx rd = rad[(size_t)deg * npair];
                 Zp[deg * deg + deg + m] = cmul(rd, pc);
                 if (m > 0) {
                     const int idx = deg * deg + deg - m;
-                    Zp[idx] = cmul(rd, cscale(cconj(pc), P.reflection[idx]));
+                    Zp[idx] = cmul(rd, cscale(cconj(pc), __ldg(&P.reflection[idx])));
                 }
             }
         } else {
@@ -221,8 +245,10 @@ __global__ void __launch_bounds__(512, 1)
     cplx* Xs = Zs + (size_t)KJ * ZLD;                                // KJ x COLS
     cplx* Rs = Xs + (size_t)KJ * COLS;                               // npair x (order + 1)
     double4* Ds = reinterpret_cast<double4*>(Rs + (size_t)npair * ord1);  // direction, state
+    double2* rec = reinterpret_cast<double2*>(Ds + npair);           // ts
     cplx* Gs = reinterpret_cast<cplx*>(ag_smem);                     // at the end: DI * ts x M
     const int tid = threadIdx.x, nthr = blockDim.x;
+    recurrence_table(order, rec, tid, nthr);
     const int rg = tid / CG, cg = tid - (tid / CG) * CG;
     const bool worker = rg < RG;
     const int i0 = blockIdx.x * DI;
@@ -242,7 +268,7 @@ __global__ void __launch_bounds__(512, 1)
             const int jj = t / COLS, col = t - jj * COLS, j = j0 + jj;
             Xs[t] = (col < M && j < N) ? xc[(size_t)j * O.ldin + col] : mk(0.0, 0.0);
         }
-        build_chunk(P, order, N, k, pos, singular, i0, j0, DI, KJ, ZLD, Zs, Rs, Ds, tid, nthr);
+        build_chunk(P, order, N, k, pos, singular, i0, j0, DI, KJ, ZLD, Zs, Rs, Ds, rec, tid, nthr);
         __syncthreads();
         // C) G += Z_chunk X_chunk
         if (worker) {
@@ -307,22 +333,24 @@ __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
 // (degrees <= order) exactly as the on-the-fly product does and writes them out in the stored
 // order.
 __global__ void __launch_bounds__(256) table_store_kernel(DevPlan P, int order, int N, double k,
-                                                          const double* __restrict__ pos, int DI, int KJ, int RO,
-                                                          int NC, int span, cplx* __restrict__ Z) {
+                                                          const double* __restrict__ pos, bool singular, int DI,
+                                                          int KJ, int RO, int NC, int span, cplx* __restrict__ Z) {
     extern __shared__ __align__(16) unsigned char ts_smem[];
     const int ord1 = order + 1, ts = ord1 * ord1, rows = DI * ts;
     const int ZLD = RO * 8 + 1, npair = DI * KJ;
     cplx* Zs = reinterpret_cast<cplx*>(ts_smem);                          // KJ x ZLD
     cplx* Rs = Zs + (size_t)KJ * ZLD;                                     // npair x (order + 1)
     double4* Ds = reinterpret_cast<double4*>(Rs + (size_t)npair * ord1);  // direction, state
+    double2* rec = reinterpret_cast<double2*>(Ds + npair);                // ts
     const int tid = threadIdx.x, nthr = blockDim.x;
+    recurrence_table(order, rec, tid, nthr);
     const int i0 = blockIdx.x * DI;
     for (int t = tid; t < KJ * ZLD; t += nthr) Zs[t] = mk(0.0, 0.0);  // padding rows stay zero
     const int jbeg = blockIdx.y * span, jend = min(N, jbeg + span);
     cplx* Zb = Z + (size_t)blockIdx.x * NC * RO * 128;
     for (int j0 = jbeg; j0 < jend; j0 += KJ) {
         __syncthreads();  // the previous chunk is written out
-        build_chunk(P, order, N, k, pos, true, i0, j0, DI, KJ, ZLD, Zs, Rs, Ds, tid, nthr);
+        build_chunk(P, order, N, k, pos, singular, i0, j0, DI, KJ, ZLD, Zs, Rs, Ds, rec, tid, nthr);
         __syncthreads();
         // out: per 16-source chunk c, group q of 4 sources, row octet o, lane
         const int total = (KJ / SRC_CHUNK) * 4 * RO * 32;
@@ -336,20 +364,30 @@ __global__ void __launch_bounds__(256) table_store_kernel(DevPlan P, int order, 
     }
 }
 
-// Inputs of ncol columns in the B-fragment order: per chunk, group q, column octet c, lane.
+// Inputs of ncol columns in the B-fragment order: per chunk, group q, column octet c, lane. With
+// parts > 1 (the split product below) part h + 2 r holds the helicity-h entries of the sources'
+// lm from r * cnt on, cnt of them.
 __global__ void pack_sources_kernel(const cplx* __restrict__ x, size_t ldx, int ldin, int N, int M, int NC, int CT,
-                                    cplx* __restrict__ Xf) {
+                                    int parts, int cnt, size_t per_col, cplx* __restrict__ Xf) {
     const size_t per = (size_t)NC * 4 * CT * 32;
     const cplx* xc = x + (size_t)blockIdx.y * ldx;
-    cplx* out = Xf + (size_t)blockIdx.y * per;
+    const int part = blockIdx.z, s0 = (part >> 1) * cnt;
+    cplx* out = Xf + (size_t)blockIdx.y * per_col + part * per;
     for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < per; t += (size_t)gridDim.x * blockDim.x) {
         const int lane = (int)(t & 31);
         const size_t w = t >> 5;
         const int c = (int)(w % CT);
         const size_t g = w / CT;  // chunk * 4 + q
         const size_t j = g * 4 + (lane & 3);
-        const int col = c * 8 + (lane >> 2);
-        out[t] = (j < (size_t)N && col < M) ? xc[j * ldin + col] : mk(0.0, 0.0);
+        int col = c * 8 + (lane >> 2);
+        bool ok = j < (size_t)N;
+        if (parts > 1) {
+            ok = ok && col < cnt && s0 + col < M / 2;
+            col = 2 * (s0 + col) + (part & 1);
+        } else {
+            ok = ok && col < M;
+        }
+        out[t] = ok ? xc[j * ldin + col] : mk(0.0, 0.0);
     }
 }
 
@@ -362,7 +400,8 @@ template <int CT, int RPW>
 __global__ void __launch_bounds__(256, 1)
     apply_stored_kernel(DevPlan P, SubOp O, int N, const cplx* __restrict__ Z, const cplx* __restrict__ Xf, int NC,
                         int DI, int RO, const cplx* __restrict__ T, const cplx* __restrict__ x, size_t ldx,
-                        const cplx* __restrict__ zadd, double alpha, double beta, cplx* __restrict__ y) {
+                        const cplx* __restrict__ zadd, double alpha, double beta, bool singular,
+                        cplx* __restrict__ y) {
     extern __shared__ __align__(16) unsigned char as_smem[];
     const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, o0 = (tid >> 5) * RPW;
     const int ABLK = RO * 128, BBLK = CT * 128, SBLK = ABLK + BBLK;  // complex entries per chunk
@@ -434,7 +473,7 @@ __global__ void __launch_bounds__(256, 1)
     }
     __syncthreads();
     const size_t coff = (size_t)blockIdx.y * ldx;
-    terms_epilogue(P, O, Gs, DI, blockIdx.x * DI, N, T, x + coff, coff, zadd, alpha, beta, true, y, tid, nthr);
+    terms_epilogue(P, O, Gs, DI, blockIdx.x * DI, N, T, x + coff, coff, zadd, alpha, beta, singular, y, tid, nthr);
 }
 
 // ---- bulk-copy pipeline of the stored product ---------------------------------------------
@@ -493,21 +532,17 @@ __device__ __forceinline__ void as_bulk_load(uint32_t dst, const void* src, uint
 // and release it through its empty barrier (one arrival per warp), so no CTA-wide barrier
 // sits in the loop. Every wait is bounded (2 s): on a timeout the kernel records status 8,
 // waits (bounded) for the copies in flight and returns without writing y.
+// On success the product Z X is in Gs = smem (rows < rows, columns < cols, row-major).
 template <int CT, int RPW>
-__global__ void __launch_bounds__(288, 1)
-    apply_stored_tma_kernel(DevPlan P, SubOp O, int N, const cplx* __restrict__ Z, const cplx* __restrict__ Xf,
-                            int NC, int DI, int RO, const cplx* __restrict__ T, const cplx* __restrict__ x, size_t ldx,
-                            const cplx* __restrict__ zadd, double alpha, double beta, cplx* __restrict__ y,
-                            int* __restrict__ status) {
-    extern __shared__ __align__(128) unsigned char at_smem[];
+__device__ __forceinline__ bool stored_product(unsigned char* smem, const cplx* __restrict__ Zb,
+                                               const cplx* __restrict__ Xb, int NC, int RO, int rows, int cols,
+                                               int* __restrict__ status) {
     __shared__ __align__(8) uint64_t bars[2 * AT_STAGES];
     __shared__ int s_abort;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int W = (RO + RPW - 1) / RPW;  // product warps; warp W loads
     const int ABLK = RO * 128, BBLK = CT * 128, SBLK = ABLK + BBLK;  // complex entries per chunk
-    cplx* ring = reinterpret_cast<cplx*>(at_smem);
-    const cplx* Zb = Z + (size_t)blockIdx.x * NC * ABLK;
-    const cplx* Xb = Xf + (size_t)blockIdx.y * NC * BBLK;
+    cplx* ring = reinterpret_cast<cplx*>(smem);
     const uint32_t full0 = as_smem_u32(bars), empty0 = full0 + 8 * AT_STAGES;
     if (tid == 0) {
         for (int s = 0; s < AT_STAGES; ++s) {
@@ -578,10 +613,9 @@ __global__ void __launch_bounds__(288, 1)
     __syncthreads();  // every chunk consumed: no copy in flight, the ring is free for G
     if (s_abort) {
         if (tid == 0 && status) atomicExch(status, 8);
-        return;
+        return false;
     }
-    cplx* Gs = reinterpret_cast<cplx*>(at_smem);
-    const int M = 2 * O.nsrc, rows = DI * (O.order + 1) * (O.order + 1);
+    cplx* Gs = ring;
     if (warp < W) {
 #pragma unroll
         for (int r = 0; r < RPW; ++r) {
@@ -590,18 +624,111 @@ __global__ void __launch_bounds__(288, 1)
 #pragma unroll
                 for (int c = 0; c < CT; ++c) {
                     const int col = c * 8 + 2 * (lane & 3);
-                    if (col < M) {
-                        Gs[(size_t)row * M + col] = mk(re[r][c][0], im[r][c][0]);
-                        Gs[(size_t)row * M + col + 1] = mk(re[r][c][1], im[r][c][1]);
-                    }
+                    if (col < cols) Gs[(size_t)row * cols + col] = mk(re[r][c][0], im[r][c][0]);
+                    if (col + 1 < cols) Gs[(size_t)row * cols + col + 1] = mk(re[r][c][1], im[r][c][1]);
                 }
             }
         }
     }
     __syncthreads();
+    return true;
+}
+
+template <int CT, int RPW>
+__global__ void __launch_bounds__(288, 1)
+    apply_stored_tma_kernel(DevPlan P, SubOp O, int N, const cplx* __restrict__ Z, const cplx* __restrict__ Xf,
+                            int NC, int DI, int RO, const cplx* __restrict__ T, const cplx* __restrict__ x, size_t ldx,
+                            const cplx* __restrict__ zadd, double alpha, double beta, bool singular,
+                            cplx* __restrict__ y, int* __restrict__ status) {
+    extern __shared__ __align__(128) unsigned char at_smem[];
+    const int M = 2 * O.nsrc, rows = DI * (O.order + 1) * (O.order + 1);
+    if (!stored_product<CT, RPW>(at_smem, Z + (size_t)blockIdx.x * NC * RO * 128,
+                                 Xf + (size_t)blockIdx.y * NC * CT * 128, NC, RO, rows, M, status))
+        return;
     const size_t coff = (size_t)blockIdx.y * ldx;
-    terms_epilogue(P, O, Gs, DI, blockIdx.x * DI, N, T, x + coff, coff, zadd, alpha, beta, true, y, tid,
-                   blockDim.x);
+    terms_epilogue(P, O, reinterpret_cast<const cplx*>(at_smem), DI, blockIdx.x * DI, N, T, x + coff, coff, zadd, alpha,
+                   beta, singular, y, threadIdx.x, blockDim.x);
+}
+
+// ---- split product (lmax 6 and 7) -----------------------------------------------------------
+// One destination's G (169 x 96 complex at lmax 6) exceeds a CTA's registers, so `parts` CTAs share
+// it: helicity h of the coupling reads the helicity-h source columns only, (C x)[d, +-] =
+// sum_s sum_t +- w_t G[idx_t, s], so part h + 2 r takes helicity h and the cnt source lm from r cnt
+// on (all 48 at lmax 6, 32 at lmax 7) and writes its sums over them to Cp; split_finish_kernel
+// adds the parts in a fixed order and applies the Mie block and the epilogue. The DMMA pipe
+// bounds it as it bounds lmax 2..5. 300 spheres lmax 6, one application: 4.3 ms with the per-pair
+// term sums (CUDA cores, an index, a weight and a gather per term and pair), 0.57 ms here.
+template <int CT, int RPW>
+__global__ void __launch_bounds__(512, 1)
+    apply_split_kernel(DevPlan P, int N, const cplx* __restrict__ Z, const cplx* __restrict__ Xf, size_t per_col,
+                       int NC, int RO, int parts, int cnt, cplx* __restrict__ Cp, int* __restrict__ status) {
+    extern __shared__ __align__(128) unsigned char sp_smem[];
+    const int i = blockIdx.x / parts, part = blockIdx.x - i * parts, s0 = (part >> 1) * cnt;
+    const int ns = min(cnt, P.nlm - s0), nlm = P.nlm;
+    if (!stored_product<CT, RPW>(sp_smem, Z + (size_t)i * NC * RO * 128,
+                                 Xf + (size_t)blockIdx.y * per_col + (size_t)part * NC * CT * 128, NC, RO, P.tsize, cnt,
+                                 status))
+        return;
+    const cplx* G = reinterpret_cast<const cplx*>(sp_smem);
+    // thread (d, group): the group's source lm s = group, group + groups, ...; then a fixed-order sum
+    __shared__ cplx sums[512];
+    const int groups = min((int)blockDim.x / nlm, 8), d = threadIdx.x % nlm, grp = threadIdx.x / nlm;
+    if (grp < groups) {
+        const double sgn = (part & 1) ? -1.0 : 1.0;
+        cplx a = mk(0.0, 0.0), b = mk(0.0, 0.0);
+        for (int s = grp; s < ns; s += groups) {
+            const int2 cb = __ldg(&P.combo[(s0 + s) * nlm + d]);
+            int t = cb.x;
+            const int na = cb.y & 0xffff, nb = cb.y >> 16;
+            for (int e = 0; e < na; ++e, ++t) cfma(a, __ldg(&P.w[t]), G[(size_t)__ldg(&P.idx[t]) * cnt + s]);
+            for (int e = 0; e < nb; ++e, ++t) cfma(b, __ldg(&P.w[t]), G[(size_t)__ldg(&P.idx[t]) * cnt + s]);
+        }
+        sums[grp * nlm + d] = mk(fma(sgn, b.x, a.x), fma(sgn, b.y, a.y));
+    }
+    __syncthreads();
+    if (threadIdx.x < nlm) {
+        cplx c = sums[threadIdx.x];
+        for (int g = 1; g < groups; ++g) c = cadd(c, sums[g * nlm + threadIdx.x]);
+        Cp[(((size_t)blockIdx.y * parts + part) * N + i) * nlm + threadIdx.x] = c;
+    }
+}
+
+// y from the parts' coupling sums: outgoing, y = zadd + alpha x + beta T c; regular, y = x + c.
+__global__ void split_finish_kernel(DevPlan P, int N, int parts, const cplx* __restrict__ Cp,
+                                    const cplx* __restrict__ T, const cplx* __restrict__ x, size_t ldx,
+                                    const cplx* __restrict__ zadd, double alpha, double beta, bool singular,
+                                    cplx* __restrict__ y) {
+    const int nlm = P.nlm;
+    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (size_t)N * nlm) return;
+    const size_t i = t / nlm, per = (size_t)N * nlm;
+    const int d = (int)(t - i * nlm);
+    const cplx* c = Cp + (size_t)blockIdx.y * parts * per + t;
+    cplx sp = c[0], sn = c[per];
+    for (int p = 2; p < parts; p += 2) {
+        sp = cadd(sp, c[p * per]);
+        sn = cadd(sn, c[(p + 1) * per]);
+    }
+    const size_t row = (size_t)blockIdx.y * ldx + 2 * t;
+    const cplx x0 = x[row], x1 = x[row + 1];
+    if (!singular) {
+        y[row] = cadd(x0, sp);
+        y[row + 1] = cadd(x1, sn);
+        return;
+    }
+    cplx tc0 = sp, tc1 = sn;  // T null: the coupling alone
+    if (T) {
+        const cplx* t4 = T + (i * P.L + degree_of(d) - 1) * 4;
+        tc0 = cadd(cmul(t4[0], sp), cmul(t4[1], sn));
+        tc1 = cadd(cmul(t4[2], sp), cmul(t4[3], sn));
+    }
+    cplx y0 = cadd(cscale(x0, alpha), cscale(tc0, beta)), y1 = cadd(cscale(x1, alpha), cscale(tc1, beta));
+    if (zadd) {
+        y0 = cadd(y0, zadd[row]);
+        y1 = cadd(y1, zadd[row + 1]);
+    }
+    y[row] = y0;
+    y[row + 1] = y1;
 }
 
 }  // namespace
@@ -611,11 +738,12 @@ bool stored_tables_enabled() {
     return !(e && (strcmp(e, "fly") == 0 || strcmp(e, "terms") == 0));
 }
 
-bool apply_gemm_supported(const DevPlan& P) {
-    if (P.L < 2 || P.L > 5) return false;
+static bool product_forms_enabled() {
     const char* e = getenv("TCU_APPLY");  // "terms": the per-pair term-sum kernels instead
     return !(e && strcmp(e, "terms") == 0);
 }
+bool apply_gemm_supported(const DevPlan& P) { return P.L >= 2 && P.L <= 5 && product_forms_enabled(); }
+bool stored_full_supported(const DevPlan& P) { return P.L >= 2 && P.L <= 7 && product_forms_enabled(); }
 
 template <int TR, int TC>
 static void launch_shape(const DevPlan& P, const SubOp& O, const GemmShape& s, int N, double k, const double* pos,
@@ -659,10 +787,10 @@ SubOp stored_subop(const DevPlan& P, int kind) {
         default: return {P.nlm, P.nlm, P.order, 2 * P.nlm, 2 * P.nlm};
     }
 }
-// full operator: lmax 2..5; dipole blocks: tables of at most 128 entries (one destination per
+// full operator: lmax 2..5, and in parts lmax 6 and 7; dipole blocks: tables of at most 128 entries (one destination per
 // block then fills at most 16 row octets, the 8 warps of the product)
 bool stored_kind_ok(const DevPlan& P, int kind) {
-    if (kind == STORED_FULL) return P.L >= 2 && P.L <= 5;
+    if (kind == STORED_FULL) return P.L >= 2 && P.L <= 7;
     if (kind != STORED_DIPOLE_SOURCES && kind != STORED_DIPOLE_BLOCK) return false;
     const int order = stored_subop(P, kind).order;
     return (order + 1) * (order + 1) <= 128;
@@ -670,7 +798,8 @@ bool stored_kind_ok(const DevPlan& P, int kind) {
 struct StoredLayout {
     SubOp O;
     int DI, KJ, RO, CT, NC, nblk, RPW;  // RPW: row octets per warp of the product
-    size_t z_elems, xf_per_col;
+    int parts, cnt;                     // split product: CTAs per destination, source lm of each (else 1, 0)
+    size_t z_elems, xf_per_col, cp_per_col;  // cp: the split product's coupling sums
 };
 StoredLayout stored_layout(const DevPlan& P, int N, int kind) {
     StoredLayout l;
@@ -679,22 +808,32 @@ StoredLayout stored_layout(const DevPlan& P, int N, int kind) {
     l.DI = std::max(1, 128 / ts);  // about 128 table rows per destination block
     l.KJ = 32;
     l.RO = (l.DI * ts + 7) / 8;
-    l.CT = (2 * l.O.nsrc + 7) / 8;
+    l.parts = 1;
+    l.cnt = 0;
+    if (kind == STORED_FULL && P.L > 5) {
+        const int halves = P.L == 6 ? 1 : 2;  // of the source lm, per helicity
+        l.parts = 2 * halves;
+        l.cnt = (l.O.nsrc + halves - 1) / halves;
+    }
+    l.CT = ((l.parts > 1 ? l.cnt : 2 * l.O.nsrc) + 7) / 8;
     l.RPW = 2;
     l.NC = (N + l.KJ - 1) / l.KJ * (l.KJ / SRC_CHUNK);
     l.nblk = (N + l.DI - 1) / l.DI;
     l.z_elems = (size_t)l.nblk * l.NC * l.RO * 128;
-    l.xf_per_col = (size_t)l.NC * l.CT * 128;
+    l.xf_per_col = (size_t)l.parts * l.NC * l.CT * 128;
+    l.cp_per_col = l.parts > 1 ? (size_t)l.parts * N * P.nlm : 0;
     return l;
 }
 size_t stored_smem(const StoredLayout& l) {
     const size_t ring = (size_t)AS_STAGES * (l.RO + l.CT) * 128 * sizeof(cplx);
-    const size_t g = (size_t)l.DI * (l.O.order + 1) * (l.O.order + 1) * 2 * l.O.nsrc * sizeof(cplx);
+    const size_t g = (size_t)l.DI * (l.O.order + 1) * (l.O.order + 1) * (l.parts > 1 ? l.cnt : 2 * l.O.nsrc) *
+                     sizeof(cplx);
     return ring > g ? ring : g;
 }
 size_t store_smem(const StoredLayout& l) {
     const size_t npair = (size_t)l.DI * l.KJ;
-    return ((size_t)l.KJ * (l.RO * 8 + 1) + npair * (l.O.order + 1)) * sizeof(cplx) + npair * sizeof(double4);
+    return ((size_t)l.KJ * (l.RO * 8 + 1) + npair * (l.O.order + 1)) * sizeof(cplx) + npair * sizeof(double4) +
+           (size_t)(l.O.order + 1) * (l.O.order + 1) * sizeof(double2);
 }
 }  // namespace
 
@@ -705,10 +844,12 @@ size_t stored_tables_bytes(const DevPlan& P, int N, int kind) {
 
 size_t stored_inputs_bytes(const DevPlan& P, int N, int kind, int ncol) {
     if (!stored_kind_ok(P, kind) || N <= 0) return 0;
-    return stored_layout(P, N, kind).xf_per_col * (size_t)ncol * sizeof(cplx);
+    const StoredLayout l = stored_layout(P, N, kind);
+    return (l.xf_per_col + l.cp_per_col) * (size_t)ncol * sizeof(cplx);
 }
 
-void build_stored_tables(const DevPlan& P, int N, double k, const double* pos, int kind, cplx* Z, cudaStream_t st) {
+void build_stored_tables(const DevPlan& P, int N, double k, const double* pos, int kind, cplx* Z, cudaStream_t st,
+                         bool singular) {
     if (N <= 0 || !stored_kind_ok(P, kind)) return;
     StageScope sc(kind == STORED_FULL ? ST_APPLY : ST_COARSE, st);
     const StoredLayout l = stored_layout(P, N, kind);
@@ -716,21 +857,36 @@ void build_stored_tables(const DevPlan& P, int N, double k, const double* pos, i
     const int ysplit = std::min(nchunk, std::max(1, (4 * 148 + l.nblk - 1) / l.nblk));
     const int span = (nchunk + ysplit - 1) / ysplit * l.KJ;
     const dim3 grid((unsigned)l.nblk, (unsigned)((nchunk * l.KJ + span - 1) / span));
-    table_store_kernel<<<grid, 256, store_smem(l), st>>>(P, l.O.order, N, k, pos, l.DI, l.KJ, l.RO, l.NC, span, Z);
+    table_store_kernel<<<grid, 256, store_smem(l), st>>>(P, l.O.order, N, k, pos, singular, l.DI, l.KJ, l.RO, l.NC, span,
+                                                         Z);
 }
 
 void launch_apply_stored(const DevPlan& P, int N, int kind, const cplx* Z, const cplx* T, const cplx* x, size_t ldx,
                          int ncol, const cplx* zadd, double alpha, double beta, cplx* y, cplx* Xf, int* status,
-                         cudaStream_t st) {
+                         cudaStream_t st, bool singular) {
     if (N <= 0 || ncol <= 0 || !stored_kind_ok(P, kind)) return;
     StageScope sc(kind == STORED_FULL ? ST_APPLY : ST_COARSE, st);
     const StoredLayout l = stored_layout(P, N, kind);
     const int M = 2 * l.O.nsrc;
-    const dim3 pgrid((unsigned)std::min<size_t>((l.xf_per_col + 255) / 256, 1024), (unsigned)ncol);
-    pack_sources_kernel<<<pgrid, 256, 0, st>>>(x, ldx, l.O.ldin, N, M, l.NC, l.CT, Xf);
-    const dim3 grid((unsigned)l.nblk, (unsigned)ncol);
+    const dim3 pgrid((unsigned)std::min<size_t>((l.xf_per_col / l.parts + 255) / 256, 1024), (unsigned)ncol,
+                     (unsigned)l.parts);
+    pack_sources_kernel<<<pgrid, 256, 0, st>>>(x, ldx, l.O.ldin, N, M, l.NC, l.CT, l.parts, l.cnt, l.xf_per_col, Xf);
     const size_t smem = stored_smem(l);
     const int threads = (l.RO + l.RPW - 1) / l.RPW * 32;
+    if (l.parts > 1) {
+        cplx* Cp = Xf + l.xf_per_col * ncol;
+        const dim3 g((unsigned)(N * l.parts), (unsigned)ncol);
+        if (l.CT == 6)
+            apply_split_kernel<6, 2><<<g, threads + 32, smem, st>>>(P, N, Z, Xf, l.xf_per_col, l.NC, l.RO, l.parts,
+                                                                    l.cnt, Cp, status);
+        else
+            apply_split_kernel<4, 2><<<g, threads + 32, smem, st>>>(P, N, Z, Xf, l.xf_per_col, l.NC, l.RO, l.parts,
+                                                                    l.cnt, Cp, status);
+        const dim3 fg((unsigned)(((size_t)N * P.nlm + 255) / 256), (unsigned)ncol);
+        split_finish_kernel<<<fg, 256, 0, st>>>(P, N, l.parts, Cp, T, x, ldx, zadd, alpha, beta, singular, y);
+        return;
+    }
+    const dim3 grid((unsigned)l.nblk, (unsigned)ncol);
     // bulk-copy pipeline, except at 6 column octets (lmax 4) where the cp.async ring measured
     // faster (1.43 against 1.58 ms at 1024 spheres); TCU_STORED_PIPE=cpasync or tma forces one
     const char* pipe = getenv("TCU_STORED_PIPE");
@@ -738,10 +894,11 @@ void launch_apply_stored(const DevPlan& P, int N, int kind, const cplx* Z, const
 #define TCU_STORED(CT, RPW)                                                                                       \
     if (cpasync)                                                                                                  \
         apply_stored_kernel<CT, RPW><<<grid, threads, smem, st>>>(P, l.O, N, Z, Xf, l.NC, l.DI, l.RO, T, x, ldx,   \
-                                                                 zadd, alpha, beta, y);                            \
+                                                                 zadd, alpha, beta, singular, y);                  \
     else                                                                                                          \
         apply_stored_tma_kernel<CT, RPW><<<grid, threads + 32, smem, st>>>(P, l.O, N, Z, Xf, l.NC, l.DI, l.RO, T, \
-                                                                          x, ldx, zadd, alpha, beta, y, status)
+                                                                          x, ldx, zadd, alpha, beta, singular, y,  \
+                                                                          status)
     switch (l.CT) {
         case 1: TCU_STORED(1, 2); break;
         case 2: TCU_STORED(2, 2); break;
@@ -768,6 +925,8 @@ void apply_gemm_init_attributes() {
     cudaFuncSetAttribute(apply_stored_tma_kernel<6, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     cudaFuncSetAttribute(apply_stored_kernel<9, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     cudaFuncSetAttribute(apply_stored_tma_kernel<9, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(apply_split_kernel<6, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(apply_split_kernel<4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
 }
 
 }  // namespace tcu

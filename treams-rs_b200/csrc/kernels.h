@@ -144,21 +144,23 @@ void apply_gemm_init_attributes();
 void launch_apply_dipole(const DevPlan& P, int N, double k, const double* pos, const cplx* T, const cplx* z,
                          bool dipole_rows, const cplx* zadd, double alpha, double beta, cplx* y, cudaStream_t st);
 // Stored-table form of the singular operator and of its two dipole blocks (for repeated
-// applications): the harmonic tables of all ordered pairs built once into Z
+// applications; singular false: the regular operator x + C x): the harmonic tables of all ordered pairs built once into Z
 // (stored_tables_bytes), then every application is an FP64 tensor-core product over Z plus the
-// term lists. kind: STORED_FULL (lmax 2..5) is launch_apply's operator; STORED_DIPOLE_SOURCES and
+// term lists. kind: STORED_FULL (lmax 2..7) is launch_apply's operator; STORED_DIPOLE_SOURCES and
 // STORED_DIPOLE_BLOCK are launch_apply_dipole with dipole_rows false and true (input ldin 6).
 // Xf: scratch of stored_inputs_bytes for the packed inputs. Sizes are 0 where a kind does not
 // apply.
 enum StoredKind { STORED_FULL = 0, STORED_DIPOLE_SOURCES = 1, STORED_DIPOLE_BLOCK = 2 };
+bool stored_full_supported(const DevPlan& P);  // STORED_FULL exists for this lmax and TCU_APPLY allows it
 bool stored_tables_enabled();  // false when TCU_APPLY is "fly" or "terms" (read at every call)
 size_t stored_tables_bytes(const DevPlan& P, int N, int kind);
 size_t stored_inputs_bytes(const DevPlan& P, int N, int kind, int ncol);
-void build_stored_tables(const DevPlan& P, int N, double k, const double* pos, int kind, cplx* Z, cudaStream_t st);
+void build_stored_tables(const DevPlan& P, int N, double k, const double* pos, int kind, cplx* Z, cudaStream_t st,
+                         bool singular = true);
 // status (may be null) receives 8 when a bounded wait of the product gave up (y not written).
 void launch_apply_stored(const DevPlan& P, int N, int kind, const cplx* Z, const cplx* T, const cplx* x, size_t ldx,
                          int ncol, const cplx* zadd, double alpha, double beta, cplx* y, cplx* Xf, int* status,
-                         cudaStream_t st);
+                         cudaStream_t st, bool singular = true);
 void launch_block(const DevPlan& P, double k, const double* d, bool singular, bool helicity, cplx* out,
                   cudaStream_t st);
 void launch_mie(int L, double k0, int N, const double* radii, const cplx* eps, cplx* T, int* status, cudaStream_t st);
