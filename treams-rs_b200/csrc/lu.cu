@@ -2,10 +2,12 @@
 // matrix, FP64 (double2) or FP32 (float2) storage.
 //
 // Per panel of width w (64 complex columns in FP64, 128 in FP32):
-//  1. panel_kernel (cooperative, one CTA per SM): every CTA holds a slab of the panel rows
-//     in shared memory; per column one grid barrier publishes each CTA's pivot candidate
-//     (largest |a|, ties to the lower row) with its row and the current diagonal row, so
-//     every CTA picks the same pivot, swaps locally and applies the rank-1 update.
+//  1. panel_cluster_kernel (panel.cuh): clusters of up to 16 CTAs hold the panel rows in shared
+//     memory and exchange each column's pivot candidates through distributed shared memory. Where
+//     the rows do not fit, panel_kernel (cooperative, one CTA per SM): per column one grid barrier
+//     publishes each CTA's candidate (largest |a|, ties to the lower row) with its row and the
+//     current diagonal row, so every CTA picks the same pivot, swaps locally and applies the
+//     rank-1 update.
 //  2. laswp_kernel: the panel's row swaps on the columns outside it (skips identities).
 //  3. U12 = L11^-1 A12: trsm_kernel (FP64, one warp per column), or in the mixed path the
 //     blocked inverse of L11 (tri_inverse_l_kernel) and a tensor-core GEMM (gemm_tf32.cu).
@@ -334,6 +336,12 @@ __global__ void __launch_bounds__(PANEL_THREADS) panel_kernel(typename Cx<R>::T*
         A[(size_t)(k0 + c) * lda + row0 + r] = tile[(size_t)r * LD + c];
     }
 }
+
+}  // namespace tcu
+
+#include "panel.cuh"
+
+namespace tcu {
 
 // ---- row swaps outside the panel ------------------------------------------------------------
 template <typename C>
@@ -769,10 +777,92 @@ static bool panel_sub_enabled() {
     return v;
 }
 
+// Cluster panels wherever they fit; TCU_PANEL=grid keeps the grid-wide panel_kernel, which also takes
+// what they cannot hold (more than about 24,900 rows in FP32, 24,200 in FP64).
+static bool cluster_panel_enabled() {
+    static const bool v = [] {
+        const char* e = getenv("TCU_PANEL");
+        return !(e && std::string(e) == "grid");
+    }();
+    return v;
+}
+
+// Words of the cluster panels in the LU workspace, behind the grid panel's candidates.
+static uint4* panel_words(const LuWork& wk) {
+    return reinterpret_cast<uint4*>((unsigned char*)wk.cand + 2 * 160 * 8 + 2 * 160 * 128 * sizeof(double) +
+                                    4096);
+}
+
+// The panel on one cluster, or on several clusters of 16; false when it does not fit or is refused.
+template <typename R, int NB>
+static bool run_panel_cluster(typename Cx<R>::T* A, int n, int k0, int w, LuWork& wk, cudaStream_t st) {
+    typedef typename Cx<R>::T C;
+    const void* fn = (const void*)panel_cluster_kernel<R, NB>;
+    constexpr size_t LIMIT = 224 * 1024;  // beside about 2 KB of static shared memory
+    static int most_clusters = 0;  // clusters of 16 that the device holds at once
+    static PerDeviceOnce attr;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 16;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeCooperative;
+    at[1].val.cooperative = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(PC_T);
+    cfg.stream = st;
+    cfg.attrs = at;
+    once_per_device(attr, [&] {
+        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LIMIT);
+        cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        cfg.gridDim = dim3(16);
+        cfg.dynamicSmemBytes = LIMIT;
+        cfg.numAttrs = 1;
+        int c = 0;
+        if (cudaOccupancyMaxActiveClusters(&c, fn, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            c = 0;
+        }
+        most_clusters = std::min(c, PC_MAXCL);
+    });
+    const int rows = n - k0;
+    // About 64 rows a CTA while one cluster holds them (measured per column at 24, 48, 64 and 96 rows:
+    // 1.22, 1.19, 1.19, 1.21 us at 240 rows FP64; 1.23, 1.22, 1.22, 1.25 at 1920 FP32): fewer rows only add
+    // messages, more rows lengthen the rank-16 update. Beyond one cluster about 128 rows a CTA: every
+    // further cluster adds readers to the global exchange (12288 FP32: 1.87 us at 96 and 128 rows, 1.94 at
+    // 160, 1.96 at 192), so the first panels of 24576 rows, which need all 8 clusters, cost 2.7 us a column.
+    int cs = 1;
+    while (cs < 16 && cs * 64 < rows) cs *= 2;
+    if (most_clusters < 1) return false;
+    int ncl = 1, chunk = 0;
+    auto fits = [&]() {
+        chunk = (rows + cs * ncl - 1) / (cs * ncl);
+        return chunk <= PC_T && panel_cluster_smem<C>(chunk, NB, cs) <= LIMIT;
+    };
+    while (cs < 16 && !fits()) cs *= 2;
+    if (!fits()) {
+        ncl = std::min(most_clusters, (rows + 16 * 128 - 1) / (16 * 128));
+        while (!fits())
+            if (++ncl > most_clusters) return false;
+    }
+    cfg.gridDim = dim3(cs * ncl);
+    cfg.dynamicSmemBytes = panel_cluster_smem<C>(chunk, NB, cs);
+    cfg.numAttrs = ncl > 1 ? 2 : 1;
+    at[0].val.clusterDim.x = cs;
+    size_t lda = (size_t)n;
+    unsigned epoch = (unsigned)k0;
+    uint4* gkey = panel_words(wk);
+    uint4* grow = gkey + PC_GKEY;
+    void* args[] = {&A, &lda, &k0, &n, &w, &chunk, &cs, &epoch, &wk.piv, &gkey, &grow, &wk.status};
+    if (cudaLaunchKernelExC(&cfg, fn, args) == cudaSuccess) return true;
+    cudaGetLastError();
+    return false;
+}
+
 template <typename R, int NB>
 static int run_panel(typename Cx<R>::T* A, int n, int k0, int w, LuWork& wk, cudaStream_t st) {
     typedef typename Cx<R>::T C;
     int rows = n - k0;
+    if (cluster_panel_enabled() && run_panel_cluster<R, NB>(A, n, k0, w, wk, st)) return 0;
     // at least panel_rows_per_cta() rows per CTA: fewer CTAs arrive at each column's barrier
     const int per = wk.panel_rows > 0 ? wk.panel_rows : panel_rows_per_cta();
     int P = std::min(g_num_sms, std::max(1, (rows + per - 1) / per));
@@ -865,6 +955,8 @@ static int lu_factor_impl(typename Cx<R>::T* A, int n, LuWork& wk, cudaStream_t 
     typedef typename Cx<R>::T C;
     lu_init_attributes();
     size_t lda = n;
+    // flags of the cluster panels' words: epochs 1 .. n
+    cudaMemsetAsync(panel_words(wk), 0, (PC_GKEY + PC_GROW) * sizeof(uint4), st);
     // (the FP16-piece packers hold one 128-column panel, so FP16 pieces keep one update per panel)
     const bool pairs = sizeof(R) == 4 && tensor_cores && !wk.f16_pieces && lu_pairs_enabled();
     int pend_k0 = -1, pend_w = 0;  // panel a whose update right of panel b is still pending
