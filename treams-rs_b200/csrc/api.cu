@@ -1789,6 +1789,27 @@ tcu_status lattice_setup(int lsum, double k, const double* lat, size_t nk, const
     return TCU_OK;
 }
 
+// The polynomial coefficients of S_lmn as the reduction reads them: per (l, |m|) pair the slots in the
+// order of their use, pp = (l - |m| - s)/2 descending and n ascending (n = s/2 in the plane), slot-major.
+template <typename At>
+std::vector<double2> lattice_coefficients(int lsum, bool offplane, At at) {
+    const int np = lattice_pairs(lsum, offplane), hstep = offplane ? 1 : 2;
+    int slots = 0;
+    for (int pp = lsum / 2; pp >= 0; --pp) slots += offplane ? lsum - 2 * pp - (lsum - 2 * pp + 1) / 2 + 1 : 1;
+    std::vector<double2> out((size_t)slots * np, make_double2(0.0, 0.0));
+    int p = 0;
+    for (int h = 0; h <= lsum; h += hstep)
+        for (int am = 0; am + h <= lsum; ++am, ++p) {
+            const int l = h + am;
+            size_t slot = 0;
+            for (int pp = h / 2; pp >= 0; --pp) {
+                const int s = h - 2 * pp;
+                for (int n = (s + 1) / 2; n <= (offplane ? s : s / 2); ++n, ++slot) out[slot * np + p] = at(l, am, pp, n);
+            }
+        }
+    return out;
+}
+
 // D (device, nk x T) for device Bloch vectors; shares one LatticeSetup
 tcu_status lattice_sums_device(tcu_context* ctx, int lsum, double k, const LatticeSetup& S, size_t nk,
                                const double2* d_kpar, double2* d_out, Arena* scratch_arena, DevBuf& scratch) {
@@ -1797,10 +1818,15 @@ tcu_status lattice_sums_device(tcu_context* ctx, int lsum, double k, const Latti
     const bool offplane = !S.coefz.empty();
     if (lattice_sum_smem(lsum, (int)S.R.size(), offplane) > 200 * 1024 || S.G.size() > (1u << 20))
         return fail(TCU_INVALID_INPUT, "lattice too elongated for the device lattice sums");
+    const std::vector<double2> coef = lattice_coefficients(lsum, offplane, [&](int l, int am, int pp, int n) {
+        const size_t lm = (size_t)l * l + l + am;
+        return make_double2(offplane ? S.coefz[(lm * LS_PMAX + pp) * LS_FMAX + n] : S.coef[lm * LS_NMAX + n], 0.0);
+    });
     Arena ar;
     size_t oR = ar.add(S.R.size() * 16), oG = ar.add(S.G.size() * 16), oN = ar.add(T * 8), oRf = ar.add(T * 8),
-           oC = ar.add((size_t)T * LS_NMAX * 8), oP = ar.add(T * 16), oTab = ar.add(S.R.size() * T * 16),
-           oZ = ar.add(S.coefz.size() * 8), oGl = ar.add(S.Glo.size() * 16);
+           oC = ar.add(coef.size() * 16), oP = ar.add(T * 16),
+           oTab = ar.add(S.R.size() * 2 * lattice_pairs(lsum, offplane) * 16), oGl = ar.add(S.Glo.size() * 16),
+           oF = ar.add(lattice_order_bytes(lsum, offplane, (int)S.G.size(), nk));
     CK(scratch.alloc(ar.total), "lattice scratch");
     void* b = scratch.p;
     CK(cudaMemcpyAsync(ar.at<void>(b, oR), S.R.data(), S.R.size() * 16, cudaMemcpyHostToDevice, ctx->stream), "copy");
@@ -1809,17 +1835,12 @@ tcu_status lattice_sums_device(tcu_context* ctx, int lsum, double k, const Latti
        "copy");
     CK(cudaMemcpyAsync(ar.at<void>(b, oN), S.norm.data(), T * 8, cudaMemcpyHostToDevice, ctx->stream), "copy");
     CK(cudaMemcpyAsync(ar.at<void>(b, oRf), S.reflection.data(), T * 8, cudaMemcpyHostToDevice, ctx->stream), "copy");
-    CK(cudaMemcpyAsync(ar.at<void>(b, oC), S.coef.data(), (size_t)T * LS_NMAX * 8, cudaMemcpyHostToDevice, ctx->stream),
-       "copy");
+    CK(cudaMemcpyAsync(ar.at<void>(b, oC), coef.data(), coef.size() * 16, cudaMemcpyHostToDevice, ctx->stream), "copy");
     CK(cudaMemcpyAsync(ar.at<void>(b, oP), S.pref.data(), T * 16, cudaMemcpyHostToDevice, ctx->stream), "copy");
-    if (offplane)
-        CK(cudaMemcpyAsync(ar.at<void>(b, oZ), S.coefz.data(), S.coefz.size() * 8, cudaMemcpyHostToDevice,
-                           ctx->stream),
-           "copy");
     CK(cudaMemsetAsync(ctx->d_status, 0, 4, ctx->stream), "status");
     double2* tab = ar.at<double2>(b, oTab);
     launch_real_table(lsum, k, S.eta, (int)S.R.size(), ar.at<double2>(b, oR), S.sx, S.sy, S.sz, ar.at<double>(b, oN),
-                      ar.at<double>(b, oRf), tab, ctx->stream);
+                      ar.at<double>(b, oRf), offplane, tab, ctx->stream);
     ++ctx->launches;
     LatticeSumArgs a;
     a.lsum = lsum;
@@ -1831,25 +1852,22 @@ tcu_status lattice_sums_device(tcu_context* ctx, int lsum, double k, const Latti
     a.NG = (int)S.G.size();
     a.G = ar.at<double2>(b, oG);
     a.Glo = ar.at<double2>(b, oGl);
-    a.coef = ar.at<double>(b, oC);
+    a.coef = ar.at<double2>(b, oC);
     a.pref = ar.at<double2>(b, oP);
     a.self0 = S.at_origin ? S.self0 : make_double2(0.0, 0.0);
     a.sx = S.sx;
     a.sy = S.sy;
     a.R0x = S.R0x;
     a.R0y = S.R0y;
-    a.offplane = offplane ? 1 : 0;
+    a.offplane = offplane;
     a.J = S.J;
     a.t = S.t;
-    a.coefz = offplane ? ar.at<double>(b, oZ) : nullptr;
     a.nk = (int)nk;
     a.kpar = d_kpar;
     a.out = d_out;
     a.ldo = T;
     a.status = ctx->d_status;
-    int grid = (int)std::min<size_t>(nk, 148 * 8);
-    launch_lattice_sum(a, grid, ctx->stream);
-    ++ctx->launches;
+    launch_lattice_sum(a, ar.at<cplx>(b, oF), ctx->stream, &ctx->launches);
     int st = 0;
     CK(cudaMemcpyAsync(&st, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream), "status");
     tcu_status s = sync_status(ctx, "lattice sums");
@@ -2112,10 +2130,15 @@ extern "C" tcu_status tcu_lsumsw2d_complex_batch(tcu_context* ctx, int lmax_sum,
     const int T = (lmax_sum + 1) * (lmax_sum + 1);
     if (lattice_sum_ck_smem(lmax_sum, (int)S.R.size()) > 200 * 1024 || S.G.size() > (1u << 20))
         return fail(TCU_INVALID_INPUT, "lattice too elongated for the device lattice sums");
+    const bool offplane = S.sz != 0.0;
+    const std::vector<double2> coef = lattice_coefficients(lmax_sum, offplane, [&](int l, int am, int pp, int n) {
+        return S.coef[(((size_t)l * l + l + am) * LS_PMAX + pp) * LS_FMAX + n];
+    });
     Arena ar;
     size_t oK = ar.add(nk * 16), oO = ar.add(nk * T * 16), oR = ar.add(S.R.size() * 16), oG = ar.add(S.G.size() * 16),
-           oN = ar.add(T * 8), oRf = ar.add(T * 8), oC = ar.add(S.coef.size() * 16), oP = ar.add(T * 16),
-           oTab = ar.add(S.R.size() * T * 16), oGl = ar.add(S.Glo.size() * 16);
+           oN = ar.add(T * 8), oRf = ar.add(T * 8), oC = ar.add(coef.size() * 16), oP = ar.add(T * 16),
+           oTab = ar.add(S.R.size() * 2 * lattice_pairs(lmax_sum, offplane) * 16), oGl = ar.add(S.Glo.size() * 16),
+           oF = ar.add(lattice_order_bytes(lmax_sum, offplane, (int)S.G.size(), nk));
     DevBuf io(ctx);
     CK(io.alloc(ar.total), "lattice-sum buffers");
     void* b = io.p;
@@ -2127,14 +2150,14 @@ extern "C" tcu_status tcu_lsumsw2d_complex_batch(tcu_context* ctx, int lmax_sum,
     CK(cudaMemcpyAsync(ar.at<void>(b, oGl), S.Glo.data(), S.Glo.size() * 16, cudaMemcpyHostToDevice, st), "copy");
     CK(cudaMemcpyAsync(ar.at<void>(b, oN), S.norm.data(), T * 8, cudaMemcpyHostToDevice, st), "copy");
     CK(cudaMemcpyAsync(ar.at<void>(b, oRf), S.reflection.data(), T * 8, cudaMemcpyHostToDevice, st), "copy");
-    CK(cudaMemcpyAsync(ar.at<void>(b, oC), S.coef.data(), S.coef.size() * 16, cudaMemcpyHostToDevice, st), "copy");
+    CK(cudaMemcpyAsync(ar.at<void>(b, oC), coef.data(), coef.size() * 16, cudaMemcpyHostToDevice, st), "copy");
     CK(cudaMemcpyAsync(ar.at<void>(b, oP), S.pref.data(), T * 16, cudaMemcpyHostToDevice, st), "copy");
     CK(cudaMemsetAsync(ctx->d_status, 0, 4, st), "status");
     double2* tab = ar.at<double2>(b, oTab);
     const double2 kd = make_double2(k[0], k[1]);
     if (!S.R.empty()) {
         launch_real_table_ck(lmax_sum, kd, S.eta, (int)S.R.size(), ar.at<double2>(b, oR), S.sx, S.sy, S.sz,
-                             ar.at<double>(b, oN), ar.at<double>(b, oRf), tab, st);
+                             ar.at<double>(b, oN), ar.at<double>(b, oRf), offplane, tab, st);
         ++ctx->launches;
     }
     LatticeSumCkArgs a;
@@ -2148,6 +2171,7 @@ extern "C" tcu_status tcu_lsumsw2d_complex_batch(tcu_context* ctx, int lmax_sum,
     a.G = ar.at<double2>(b, oG);
     a.Glo = ar.at<double2>(b, oGl);
     a.coef = ar.at<double2>(b, oC);
+    a.offplane = offplane;
     a.pref = ar.at<double2>(b, oP);
     a.self0 = S.at_origin ? S.self0 : make_double2(0.0, 0.0);
     a.sx = S.sx;
@@ -2168,8 +2192,7 @@ extern "C" tcu_status tcu_lsumsw2d_complex_batch(tcu_context* ctx, int lmax_sum,
     a.out = ar.at<double2>(b, oO);
     a.ldo = T;
     a.status = ctx->d_status;
-    launch_lattice_sum_ck(a, (int)std::min<size_t>(nk, 148 * 8), st);
-    ++ctx->launches;
+    launch_lattice_sum_ck(a, ar.at<cplx>(b, oF), st, &ctx->launches);
     int stw = 0;
     CK(cudaMemcpyAsync(&stw, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, st), "status");
     if ((s = sync_status(ctx, "lattice sums"))) return s;

@@ -212,22 +212,20 @@ struct LatticeSumArgs {
     double k = 0, eta = 0;
     int NR = 0;                            // real-space lattice points (R != 0)
     const double2* R = nullptr;
-    const double2* realtab = nullptr;      // NR x T real-space terms
+    const double2* realtab = nullptr;      // NR x pairs x 2 real-space terms (lattice_pair_index)
     int NG = 0;                            // reciprocal lattice vectors
     const double2* G = nullptr;
     const double2* Glo = nullptr;          // their low parts (G = G + Glo to twice FP64 precision)
-    const double* coef = nullptr;          // T x LS_NMAX in-plane polynomial coefficients
+    const double2* coef = nullptr;         // slots x pairs: polynomial coefficients (lattice_coefficients)
     const double2* pref = nullptr;         // T reciprocal prefactors
     double2 self0{0, 0};                   // self term of l = 0 (zero for a nonzero shift)
     double sx = 0, sy = 0;                 // in-plane shift r' (reciprocal phase e^{-i q.r'})
     double R0x = 0, R0y = 0;               // lattice vector taken off the shift: e^{-i kpar.R0}
     // shift off the plane (r_z != 0): every order n <= lsum, F'_n from the t-series of
-    // F_(1/2-n)(v, t) with t = (k r_z eta)^2 (J + 1 terms), and S_lmn as a polynomial in beta^2
-    // with coefficients coefz[(lm * LS_PMAX + p) * LS_FMAX + n] (powers of -k r_z folded in)
-    int offplane = 0;
+    // F_(1/2-n)(v, t) with t = (k r_z eta)^2 (J + 1 terms)
+    bool offplane = false;
     int J = 0;
     double t = 0;
-    const double* coefz = nullptr;
     int nk = 0;
     const double2* kpar = nullptr;
     double2* out = nullptr;                // out[kp * ldo + l*l+l+m]
@@ -241,11 +239,12 @@ struct LatticeSumCkArgs {
     double eta = 0;
     int NR = 0;
     const double2* R = nullptr;
-    const double2* realtab = nullptr;      // NR x T real-space terms
+    const double2* realtab = nullptr;      // NR x pairs x 2 real-space terms (lattice_pair_index)
     int NG = 0;
     const double2* G = nullptr;
     const double2* Glo = nullptr;          // low parts of the reciprocal vectors
-    const double2* coef = nullptr;         // T x LS_PMAX x LS_FMAX: S_lmn coefficient of beta^(2p), order n
+    const double2* coef = nullptr;         // slots x pairs: polynomial coefficients (lattice_coefficients)
+    bool offplane = false;                 // shift off the plane: every order n <= lsum
     const double2* pref = nullptr;         // T reciprocal prefactors (1/k^2 included)
     double2 self0{0, 0};
     double sx = 0, sy = 0, R0x = 0, R0y = 0;
@@ -261,13 +260,28 @@ struct LatticeSumCkArgs {
     int* status = nullptr;                 // 9: a diffraction order on its threshold
 };
 void launch_real_table_ck(int lsum, double2 k, double eta, int NR, const double2* R, double sx, double sy, double sz,
-                          const double* norm, const double* reflection, double2* tab, cudaStream_t st);
+                          const double* norm, const double* reflection, bool offplane, double2* tab, cudaStream_t st);
 size_t lattice_sum_ck_smem(int lsum, int NR);
-void launch_lattice_sum_ck(const LatticeSumCkArgs& a, int grid, cudaStream_t st);
 void launch_real_table(int lsum, double k, double eta, int NR, const double2* R, double sx, double sy, double sz,
-                       const double* norm, const double* reflection, double2* tab, cudaStream_t st);
+                       const double* norm, const double* reflection, bool offplane, double2* tab, cudaStream_t st);
 size_t lattice_sum_smem(int lsum, int NR, bool offplane);
-void launch_lattice_sum(const LatticeSumArgs& a, int grid, cudaStream_t st);
+// lattice_sum.cu — the reciprocal part and the reduction. The sums run over the (l, |m|) pairs of
+// even l - |m| in the plane, of all off it, in the order of l - |m|, then |m|.
+int lattice_pairs(int lsum, bool offplane);
+int lattice_orders(int lsum, bool offplane);  // F'_n kept per reciprocal vector
+size_t lattice_order_bytes(int lsum, bool offplane, int NG, size_t nk);  // scratch F of the launches
+// entry of (l, m) in a table row of 2 lattice_pairs entries (-1: vanishes); hstep 2 in the plane, else 1
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline int lattice_pair_index(int lsum, int l, int m, int hstep) {
+    const int am = m < 0 ? -m : m, h = l - am;
+    if (h % hstep) return -1;
+    const int before = hstep == 2 ? h / 2 * (lsum + 1) - h / 2 * (h / 2 - 1) : h * (lsum + 1) - h * (h - 1) / 2;
+    return 2 * (before + am) + (m < 0 ? 1 : 0);
+}
+void launch_lattice_sum(const LatticeSumArgs& a, cplx* F, cudaStream_t st, long long* launches);
+void launch_lattice_sum_ck(const LatticeSumCkArgs& a, cplx* F, cudaStream_t st, long long* launches);
 void launch_array_solve(const DevPlan& P, const double2* D, size_t ldd, const double* norm, const double2* Tm, int nk,
                         double2* X, int* status, int grid, cudaStream_t st);
 

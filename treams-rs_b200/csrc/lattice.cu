@@ -17,11 +17,8 @@
 // F_(1/2-n)(v, t) = sum_j (t/2)^j / j! F_(1/2-n-j)(v, 0), t = (k r_z eta)^2 (reduced.rs:223).
 //
 // Device layout: the real-space terms do not depend on the Bloch vector, so one launch
-// tabulates Treal (NR x T complex, T = (lsum+1)^2) for the lattice points within the cutoff,
-// and one CTA per Bloch vector then forms sum_R e^{i kpar.R} Treal_lm(R) (threads over lm,
-// fixed order over R) plus the reciprocal sum over G in chunks of 256 points (threads over G
-// evaluate F_n into shared memory, then threads over lm add the chunk in a fixed order).
-// Results do not depend on the launch geometry or on timing.
+// tabulates Treal for the lattice points within the cutoff; lattice_sum.cu evaluates the reduced
+// integrals of every (Bloch vector, reciprocal vector) and reduces both parts.
 //
 // Special functions, all FP64 (each from a published method, checked against the binary128
 // oracle to ~1e-14):
@@ -30,9 +27,6 @@
 //     by the upward recurrence R(d+1) = (d R(d) + e^-a)/a from R(1/2) = sqrt(pi) erfc(sqrt a)/sqrt a
 //     (all terms positive); for d < 1/2 by the power series (DLMF 8.7.3) where a < 2, else by
 //     Legendre's continued fraction (DLMF 8.9.2, modified Lentz).
-//   F_(1/2-n)(v, 0) = Gamma(1/2-n, v)/(-v)^(1/2-n) on the lower side of the cut
-//     (lattice/reduced.rs:18-100): for v > 0, -i (-1)^n R(1/2-n, v); for v < 0 (propagating
-//     orders, y = -v), Gamma(b)/y^b + i (-1)^n sum_k y^k/(k! (b+k)).
 #include <cuda_runtime.h>
 
 #include "common.cuh"
@@ -45,7 +39,6 @@ namespace {
 
 constexpr int LS_JMAX = 64;                  // Kambe series terms
 constexpr int LS_LADDER = LS_MAXL + 1 + LS_JMAX;
-constexpr int LS_CHUNK = 256;                // reciprocal points per chunk
 
 // Gamma(d, a)/a^d for real a > 0 and half-integer d < 1/2
 __device__ double scaled_gamma_low(double d, double a) {
@@ -82,7 +75,7 @@ __device__ double scaled_gamma_low(double d, double a) {
 __global__ void __launch_bounds__(128) real_table_kernel(int lsum, double k, double eta, int NR,
                                                          const double2* __restrict__ R, double sx, double sy,
                                                          double sz, const double* __restrict__ norm,
-                                                         const double* __restrict__ reflection,
+                                                         const double* __restrict__ reflection, int hstep, int row,
                                                          double2* __restrict__ tab) {
     __shared__ double ladder[4][LS_LADDER];
     __shared__ double kam[4][LS_MAXL + 1];
@@ -130,183 +123,9 @@ __global__ void __launch_bounds__(128) real_table_kernel(int lsum, double k, dou
         while ((l + 1) * (l + 1) <= lm) ++l;
         double f = s2p * pow(k * dist, (double)l) * norm[lm] * kam[warp][l];
         cplx y = Y[warp][lm];
-        // -i f y
-        tab[(size_t)r * T + lm] = mk(f * y.y, -f * y.x);
-    }
-}
-
-// F'_n = (2 eta^2)^n / (sqrt 2 eta) F_(1/2-n)(v, 0), n = 0..nmax, real v != 0 (lower side)
-__device__ void reduced_limits(int nmax, double v, double eta, cplx* out) {
-    double factor = 1.0 / (1.4142135623730950488 * eta), step = 2.0 * eta * eta;
-    if (v < 0.0) {
-        double y = -v;
-        for (int n = 0; n <= nmax; ++n) {
-            double b = 0.5 - n;
-            double s = 0.0, term = 1.0;
-            for (int kk = 0; kk < 200; ++kk) {
-                if (kk > 0) term *= y / kk;
-                double add = term / (b + kk);
-                s += add;
-                if (kk > y && fabs(add) < 1e-18 * fabs(s)) break;
-            }
-            double re = tgamma(b) * pow(y, -b);
-            double im = (n & 1) ? -s : s;
-            out[n] = mk(factor * re, factor * im);
-            factor *= step;
-        }
-    } else {
-        for (int n = 0; n <= nmax; ++n) {
-            double rr = scaled_gamma_low(0.5 - n, v);
-            if (n == 0 && v >= 2.0) rr = 1.7724538509055160273 * erfc(sqrt(v)) / sqrt(v);
-            // -i (-1)^n R
-            double im = (n & 1) ? rr : -rr;
-            out[n] = mk(0.0, factor * im);
-            factor *= step;
-        }
-    }
-}
-
-// F_(1/2-n)(v, 0) on the lower side of the cut, real v != 0 (the terms of reduced_limits
-// without the factor (2 eta^2)^n / (sqrt 2 eta))
-__device__ cplx reduced_limit(int n, double v) {
-    if (v < 0.0) {
-        const double y = -v, b = 0.5 - n;
-        double s = 0.0, term = 1.0;
-        for (int kk = 0; kk < 200; ++kk) {
-            if (kk > 0) term *= y / kk;
-            double add = term / (b + kk);
-            s += add;
-            if (kk > y && fabs(add) < 1e-18 * fabs(s)) break;
-        }
-        return mk(tgamma(b) * pow(y, -b), (n & 1) ? -s : s);
-    }
-    double rr = scaled_gamma_low(0.5 - n, v);
-    if (n == 0 && v >= 2.0) rr = 1.7724538509055160273 * erfc(sqrt(v)) / sqrt(v);
-    return mk(0.0, (n & 1) ? rr : -rr);  // -i (-1)^n R
-}
-
-// Off the lattice plane (lattice/reduced.rs:223): F'_n = (2 eta^2)^n / (sqrt 2 eta) F_(1/2-n)(v, t)
-// with F_(1/2-n)(v, t) = sum_j (t/2)^j / j! F_(1/2-n-j)(v, 0), j = 0..J (tw[j] = (t/2)^j / j!),
-// n = 0..nmax. Each limit is evaluated once and added to every n it reaches, in increasing j.
-__device__ void reduced_shifted(int nmax, int J, const double* tw, double v, double eta, cplx* out) {
-    for (int n = 0; n <= nmax; ++n) out[n] = mk(0.0, 0.0);
-    for (int i = 0; i <= nmax + J; ++i) {
-        const cplx L = reduced_limit(i, v);
-        for (int n = min(nmax, i); n >= max(0, i - J); --n) cfma(out[n], mk(tw[i - n], 0.0), L);
-    }
-    double factor = 1.0 / (1.4142135623730950488 * eta);
-    const double step = 2.0 * eta * eta;
-    for (int n = 0; n <= nmax; ++n) {
-        out[n] = cscale(out[n], factor);
-        factor *= step;
-    }
-}
-
-// One CTA per Bloch vector. smem: phases NR double2, chunk arrays.
-__global__ void __launch_bounds__(256) lattice_sum_kernel(LatticeSumArgs A) {
-    extern __shared__ double2 ls_smem[];
-    __shared__ double tw[LS_TMAX + 1];                   // (t/2)^j / j! off the plane
-    const int nF = A.offplane ? A.lsum + 1 : A.lsum / 2 + 1;  // orders n kept per point
-    double2* ph = ls_smem;                               // NR
-    double2* gF = ph + A.NR;                             // LS_CHUNK * nF
-    double2* gaz = gF + LS_CHUNK * nF;                   // LS_CHUNK
-    double2* gph = gaz + LS_CHUNK;                       // LS_CHUNK: e^{-i q.r'}
-    double* gb2 = (double*)(gph + LS_CHUNK);             // LS_CHUNK
-    const int T = (A.lsum + 1) * (A.lsum + 1), nmax = nF - 1;
-    const int tid = threadIdx.x;
-    if (A.offplane && tid == 0) {
-        double w = 1.0;
-        for (int j = 0; j <= A.J; ++j) {
-            if (j > 0) w *= 0.5 * A.t / j;
-            tw[j] = w;
-        }
-    }
-    for (int kp = blockIdx.x; kp < A.nk; kp += gridDim.x) {
-        const double2 kpar = A.kpar[kp];
-        for (int r = tid; r < A.NR; r += blockDim.x) {
-            double2 R = A.R[r];
-            double s, c;
-            sincos(kpar.x * R.x + kpar.y * R.y, &s, &c);
-            ph[r] = mk(c, s);
-        }
-        __syncthreads();
-        int lm = tid, l = 0, m = 0;
-        bool active = lm < T;
-        if (active) {
-            while ((l + 1) * (l + 1) <= lm) ++l;
-            m = lm - l * l - l;
-        }
-        const int am = m < 0 ? -m : m;
-        const bool even = ((l - am) & 1) == 0;
-        cplx acc = mk(0.0, 0.0);
-        if (active)
-            for (int r = 0; r < A.NR; ++r) cfma(acc, __ldg(&A.realtab[(size_t)r * T + lm]), ph[r]);
-        cplx rec = mk(0.0, 0.0);
-        for (int g0 = 0; g0 < A.NG; g0 += LS_CHUNK) {
-            __syncthreads();
-            int g = g0 + tid;
-            if (tid < LS_CHUNK && g < A.NG) {
-                const double2 G = A.G[g], Gl = A.Glo[g];
-                double qx, qy, ex, ey;
-                bloch_order(kpar.x, G.x, Gl.x, qx, ex);
-                bloch_order(kpar.y, G.y, Gl.y, qy, ey);
-                double b2 = (qx * qx + qy * qy) / (A.k * A.k);
-                // v = (q.q - k^2) / (2 eta^2 k^2), the difference compensated near a threshold
-                double v = q2_minus_k2(qx, ex, qy, ey, A.k) / (2.0 * A.eta * A.eta * A.k * A.k);
-                if (fabs(v) <= 1e-14) {
-                    atomicExch(A.status, 9);  // on a diffraction threshold (reciprocal.rs:236-241)
-                    for (int n = 0; n <= nmax; ++n) gF[tid * nF + n] = mk(0.0, 0.0);
-                } else if (A.offplane) {
-                    reduced_shifted(nmax, A.J, tw, v, A.eta, gF + tid * nF);
-                } else {
-                    reduced_limits(nmax, v, A.eta, gF + tid * nF);
-                }
-                gb2[tid] = b2;
-                gaz[tid] = mk(qx / A.k, qy / A.k);
-                double ps, pc;
-                sincos(-(qx * A.sx + qy * A.sy), &ps, &pc);
-                gph[tid] = mk(pc, ps);
-            }
-            __syncthreads();
-            if (active && (even || A.offplane)) {
-                const int nm = (l - am) / 2;
-                const double* coef = A.coef + (size_t)lm * LS_NMAX;
-                const int cnt = min(LS_CHUNK, A.NG - g0);
-                for (int t = 0; t < cnt; ++t) {
-                    const double b2 = gb2[t];
-                    const double2* F = gF + t * nF;
-                    cplx s = mk(0.0, 0.0);
-                    if (A.offplane) {
-                        // Horner in beta^2 over p = (l - |m| - s)/2; the orders n with n <= s <= 2n
-                        const double* cz = A.coefz + (size_t)lm * LS_PMAX * LS_FMAX;
-                        for (int p = (l - am) / 2; p >= 0; --p) {
-                            s = cscale(s, b2);
-                            const int sidx = l - am - 2 * p;
-                            for (int n = (sidx + 1) / 2; n <= sidx; ++n)
-                                cfma(s, mk(cz[p * LS_FMAX + n], 0.0), F[n]);
-                        }
-                    } else {
-                        for (int n = 0; n <= nm; ++n) {  // Horner in beta^2
-                            s = cscale(s, b2);
-                            cfma(s, mk(coef[n], 0.0), F[n]);
-                        }
-                    }
-                    cplx az = gaz[t];
-                    if (m < 0) az.y = -az.y;
-                    cplx azm = mk(1.0, 0.0);
-                    for (int q = 0; q < am; ++q) azm = cmul(azm, az);
-                    cfma(rec, s, cmul(azm, gph[t]));
-                }
-            }
-        }
-        if (active) {
-            cplx v = cadd(acc, cmul(A.pref[lm], rec));
-            if (lm == 0) v = cadd(v, A.self0);
-            double cs, cc;  // e^{-i kpar.R0} of the shift reduced into the cell
-            sincos(-(kpar.x * A.R0x + kpar.y * A.R0y), &cs, &cc);
-            A.out[(size_t)kp * A.ldo + lm] = cmul(v, mk(cc, cs));
-        }
-        __syncthreads();
+        // -i f y, where the reduction reads it (in the plane odd l - |m| vanish)
+        const int m = lm - l * l - l, at = lattice_pair_index(lsum, l, m, hstep);
+        if (at >= 0) tab[(size_t)r * row + at] = mk(f * y.y, -f * y.x);
     }
 }
 
@@ -563,21 +382,15 @@ __global__ void __launch_bounds__(384, 1) array_solve_kernel(DevPlan P, const do
 }  // namespace
 
 void launch_real_table(int lsum, double k, double eta, int NR, const double2* R, double sx, double sy, double sz,
-                       const double* norm, const double* reflection, double2* tab, cudaStream_t st) {
+                       const double* norm, const double* reflection, bool offplane, double2* tab, cudaStream_t st) {
     StageScope sc(ST_LATTICE, st);
-    real_table_kernel<<<(NR + 3) / 4, 128, 0, st>>>(lsum, k, eta, NR, R, sx, sy, sz, norm, reflection, tab);
+    real_table_kernel<<<(NR + 3) / 4, 128, 0, st>>>(lsum, k, eta, NR, R, sx, sy, sz, norm, reflection, offplane ? 1 : 2,
+                                                    2 * lattice_pairs(lsum, offplane), tab);
 }
 
 size_t lattice_sum_smem(int lsum, int NR, bool offplane) {
     const size_t nF = offplane ? lsum + 1 : lsum / 2 + 1;
-    return (size_t)NR * 16 + (size_t)LS_CHUNK * nF * 16 + 2 * LS_CHUNK * 16 + LS_CHUNK * 8;
-}
-
-void launch_lattice_sum(const LatticeSumArgs& a, int grid, cudaStream_t st) {
-    StageScope sc(ST_LATTICE, st);
-    size_t smem = lattice_sum_smem(a.lsum, a.NR, a.offplane != 0);
-    cudaFuncSetAttribute(lattice_sum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    lattice_sum_kernel<<<grid, 256, smem, st>>>(a);
+    return (size_t)NR * 16 + (size_t)256 * nF * 16 + 2 * 256 * 16 + 256 * 8;
 }
 
 void launch_array_solve(const DevPlan& P, const double2* D, size_t ldd, const double* norm, const double2* Tm, int nk,

@@ -21,11 +21,9 @@
 // R(d+1) = (d R(d) + e^-a)/a.
 //
 // Device layout as in lattice.cu: one launch tabulates Treal for the lattice points within the
-// cutoff (a warp per point), one CTA per Bloch vector adds the real-space table with the Bloch
-// phases and the reciprocal sum over G in chunks of 256 points (threads over G evaluate F'_n
-// into shared memory, threads over lm add the chunk in a fixed order). S_lmn is evaluated as a
-// polynomial in beta^2 whose coefficients (powers of -k r_z folded in) come from the host, so
-// shifts on and off the plane take the same path.
+// cutoff (a warp per point); lattice_sum.cu evaluates the reduced integrals and reduces both parts.
+// S_lmn is a polynomial in beta^2 whose coefficients (powers of -k r_z folded in) come from the
+// host, so shifts on and off the plane take the same path.
 #include <cuda_runtime.h>
 
 #include "common.cuh"
@@ -37,8 +35,6 @@ namespace {
 
 constexpr int CK_JMAX = 64;   // Kambe series terms
 constexpr int CK_LADDER = LS_MAXL + 1 + CK_JMAX;
-constexpr int CK_CHUNK = 256;  // reciprocal points per chunk
-constexpr double CK_PI = 3.14159265358979323846;
 
 __device__ __forceinline__ cplx clog_c(cplx z) { return mk(log(hypot(z.x, z.y)), atan2(z.y, z.x)); }
 __device__ __forceinline__ cplx cpow_c(cplx z, double a) {  // principal z^a
@@ -100,40 +96,12 @@ __device__ cplx scaled_gamma_c(double d, cplx a) {
     return csub(cscale(cpow_c(a, -d), tgamma(d)), gamma_series_sum_c(d, a));
 }
 
-// F_(1/2-i)(v, 0) on the outgoing sheet: z = v with a zero imaginary part taken as -0 (lower side),
-// g = Gamma(b, z)/(-z)^b, b = 1/2 - i; odd turns add -2 Gamma(b)/(-z)^b, Im z > 0 flips the sign
-// (lattice/reduced.rs:18-100 with lattice/sheets.rs)
-__device__ cplx reduced_limit_c(int i, cplx z, bool odd_turns) {
-    const double b = 0.5 - i;
-    // 1 / (-z)^b = (-z)^i / sqrt(-z), principal (sqrt(-z) with -z's zero imaginary part as +0);
-    // formed from the positive power, it stays finite next to a threshold at large i
-    const cplx mz = cneg(z);
-    const cplx inv_rp = cmul(cpowi_c(mz, i), cinv(csqrt_p(mz)));
-    cplx g;
-    if (use_fraction(z)) {
-        // Gamma(b, z) = e^-z z^b CF, and z^b / (-z)^b = e^(-+ i pi b) below / above the axis
-        const double ph = (z.y > 0.0 ? 1.0 : -1.0) * CK_PI * b;
-        double s, c;
-        sincos(ph, &s, &c);
-        g = cmul(cmul(cexpz(cneg(z)), mk(c, s)), gamma_fraction_c(b, z));
-    } else {
-        // Gamma(b, z) = Gamma(b) - z^b sum_k (-z)^k/(k! (b + k))
-        const double ph = (z.y > 0.0 ? 1.0 : -1.0) * CK_PI * b;
-        double s, c;
-        sincos(ph, &s, &c);
-        g = csub(cscale(inv_rp, tgamma(b)), cmul(mk(c, s), gamma_series_sum_c(b, z)));
-    }
-    if (odd_turns) g = csub(g, cscale(inv_rp, 2.0 * tgamma(b)));
-    if (z.y > 0.0) g = cneg(g);
-    return g;
-}
-
 // One warp per lattice point: Treal_lm(R) for every l <= lsum, |m| <= l, complex k.
 __global__ void __launch_bounds__(128) real_table_ck_kernel(int lsum, cplx k, double eta, int NR,
                                                             const double2* __restrict__ R, double sx, double sy,
                                                             double sz, const double* __restrict__ norm,
-                                                            const double* __restrict__ reflection,
-                                                            double2* __restrict__ tab) {
+                                                            const double* __restrict__ reflection, int hstep,
+                                                            int row, double2* __restrict__ tab) {
     __shared__ cplx ladder[4][CK_LADDER];
     __shared__ cplx kam[4][LS_MAXL + 1];
     __shared__ cplx Y[4][(LS_MAXL + 1) * (LS_MAXL + 1)];
@@ -184,159 +152,23 @@ __global__ void __launch_bounds__(128) real_table_ck_kernel(int lsum, cplx k, do
         while ((l + 1) * (l + 1) <= lm) ++l;
         const cplx f = cscale(cmul(cpowi_c(kd, l), kam[warp][l]), s2p * norm[lm]);
         const cplx fy = cmul(f, Y[warp][lm]);
-        tab[(size_t)r * T + lm] = mk(fy.y, -fy.x);  // -i f y
-    }
-}
-
-// F'_n = (2 eta^2)^n / (sqrt 2 eta) sum_j tw[j] F_(1/2-n-j)(v, 0), n = 0..nmax, tw[j] = (t/2)^j / j!
-__device__ void reduced_shifted_c(int nmax, int J, const cplx* tw, cplx v, bool odd_turns, double eta, cplx* out) {
-    for (int n = 0; n <= nmax; ++n) out[n] = mk(0.0, 0.0);
-    for (int i = 0; i <= nmax + J; ++i) {
-        const cplx L = reduced_limit_c(i, v, odd_turns);
-        for (int n = min(nmax, i); n >= max(0, i - J); --n) cfma(out[n], tw[i - n], L);
-    }
-    double factor = 1.0 / (1.4142135623730950488 * eta);
-    const double step = 2.0 * eta * eta;
-    for (int n = 0; n <= nmax; ++n) {
-        out[n] = cscale(out[n], factor);
-        factor *= step;
-    }
-}
-
-// Whole turns of v on the outgoing sheet of an order (lattice/sheets.rs): orders whose k^2 - q.q
-// lies in the near sector of the split (|arg| of (k eta)^2 + 1/2 < pi/2) follow arg(k^2 - q.q);
-// the others stay on the principal sheet. Returns whether the number of turns is odd.
-__device__ bool odd_turns_of(const LatticeSumCkArgs& A, double q2, cplx v) {
-    const cplx sq = mk(A.ksq.x - q2, A.ksq.y);
-    const bool near = sq.x > 0.0 && sq.y * sq.y <= A.near * sq.x * sq.x;
-    if (A.has_near && !near) return false;
-    double turn;
-    if (sq.y == 0.0) {
-        turn = sq.x > 0.0 ? 0.0 : CK_PI;
-    } else {
-        turn = atan2(sq.y, sq.x);
-        if (turn < 0.0) turn += 2.0 * CK_PI;
-    }
-    const double sheet = turn - CK_PI - A.turn;
-    const double turns = rint((sheet - atan2(v.y, v.x)) / (2.0 * CK_PI));
-    return fmod(fabs(turns), 2.0) == 1.0;
-}
-
-// One CTA per Bloch vector (complex k).
-__global__ void __launch_bounds__(256) lattice_sum_ck_kernel(LatticeSumCkArgs A) {
-    extern __shared__ double2 ck_smem[];
-    __shared__ cplx tw[LS_TMAX + 1];
-    const int nF = A.lsum + 1;
-    double2* ph = ck_smem;                    // NR
-    double2* gF = ph + A.NR;                  // CK_CHUNK * nF
-    double2* gq = gF + CK_CHUNK * nF;         // CK_CHUNK: (q_x, q_y)
-    double2* gph = gq + CK_CHUNK;             // CK_CHUNK: e^{-i q.r'}
-    double2* gb2 = gph + CK_CHUNK;            // CK_CHUNK: beta^2 = q.q / k^2
-    const int T = (A.lsum + 1) * (A.lsum + 1), nmax = A.lsum;
-    const int tid = threadIdx.x;
-    if (tid == 0) {
-        cplx w = mk(1.0, 0.0);
-        const cplx half_t = cscale(A.t, 0.5);
-        for (int j = 0; j <= A.J; ++j) {
-            if (j > 0) w = cscale(cmul(w, half_t), 1.0 / j);
-            tw[j] = w;
-        }
-    }
-    const cplx kinv = cinv(A.k), kinv2 = cmul(kinv, kinv);
-    for (int kp = blockIdx.x; kp < A.nk; kp += gridDim.x) {
-        const double2 kpar = A.kpar[kp];
-        for (int r = tid; r < A.NR; r += blockDim.x) {
-            double2 R = A.R[r];
-            double s, c;
-            sincos(kpar.x * R.x + kpar.y * R.y, &s, &c);
-            ph[r] = mk(c, s);
-        }
-        __syncthreads();
-        int lm = tid, l = 0, m = 0;
-        const bool active = lm < T;
-        if (active) {
-            while ((l + 1) * (l + 1) <= lm) ++l;
-            m = lm - l * l - l;
-        }
-        const int am = m < 0 ? -m : m;
-        cplx acc = mk(0.0, 0.0);
-        if (active)
-            for (int r = 0; r < A.NR; ++r) cfma(acc, __ldg(&A.realtab[(size_t)r * T + lm]), ph[r]);
-        cplx rec = mk(0.0, 0.0);
-        for (int g0 = 0; g0 < A.NG; g0 += CK_CHUNK) {
-            __syncthreads();
-            const int g = g0 + tid;
-            if (tid < CK_CHUNK && g < A.NG) {
-                const double2 G = A.G[g], Gl = A.Glo[g];
-                double qx, qy, ex, ey;
-                bloch_order(kpar.x, G.x, Gl.x, qx, ex);
-                bloch_order(kpar.y, G.y, Gl.y, qy, ey);
-                const double q2 = qx * qx + qy * qy;
-                const cplx b2 = cscale(kinv2, q2);
-                // v = (q.q - k^2) / (2 eta^2 k^2): Re(q.q - k^2) = (q.q - Re(k)^2) + Im(k)^2 compensated
-                const cplx d = mk(q2_minus_k2(qx, ex, qy, ey, A.k.x) + A.k.y * A.k.y, -2.0 * A.k.x * A.k.y);
-                cplx v = cscale(cmul(d, kinv2), 1.0 / (2.0 * A.eta * A.eta));
-                if (v.y == 0.0) v.y = -0.0;  // lower side (lattice/sheets.rs:12-17)
-                if (hypot(v.x, v.y) <= 1e-14) {
-                    atomicExch(A.status, 9);  // on a diffraction threshold (reciprocal.rs:236-241)
-                    for (int n = 0; n <= nmax; ++n) gF[tid * nF + n] = mk(0.0, 0.0);
-                } else {
-                    reduced_shifted_c(nmax, A.J, tw, v, odd_turns_of(A, q2, v), A.eta, gF + tid * nF);
-                }
-                gb2[tid] = b2;
-                gq[tid] = mk(qx, qy);
-                double ps, pc;
-                sincos(-(qx * A.sx + qy * A.sy), &ps, &pc);
-                gph[tid] = mk(pc, ps);
-            }
-            __syncthreads();
-            if (active) {
-                const cplx* cz = A.coef + (size_t)lm * LS_PMAX * LS_FMAX;
-                const int cnt = min(CK_CHUNK, A.NG - g0);
-                for (int t = 0; t < cnt; ++t) {
-                    const cplx b2 = gb2[t];
-                    const double2* F = gF + t * nF;
-                    cplx s = mk(0.0, 0.0);
-                    // Horner in beta^2 over p = (l - |m| - s)/2; the orders n with n <= s <= 2n
-                    for (int p = (l - am) / 2; p >= 0; --p) {
-                        s = cmul(s, b2);
-                        const int sidx = l - am - 2 * p;
-                        for (int n = (sidx + 1) / 2; n <= sidx; ++n) cfma(s, cz[p * LS_FMAX + n], F[n]);
-                    }
-                    const double2 q = gq[t];
-                    const cplx az = cmul(mk(q.x, m < 0 ? -q.y : q.y), kinv);  // (q_x +- i q_y)/k
-                    cfma(rec, s, cmul(cpowi_c(az, am), gph[t]));
-                }
-            }
-        }
-        if (active) {
-            cplx v = cadd(acc, cmul(A.pref[lm], rec));
-            if (lm == 0) v = cadd(v, A.self0);
-            double cs, cc;  // e^{-i kpar.R0} of the shift reduced into the cell
-            sincos(-(kpar.x * A.R0x + kpar.y * A.R0y), &cs, &cc);
-            A.out[(size_t)kp * A.ldo + lm] = cmul(v, mk(cc, cs));
-        }
-        __syncthreads();
+        // -i f y, where the reduction reads it (in the plane odd l - |m| vanish)
+        const int at = lattice_pair_index(lsum, l, lm - l * l - l, hstep);
+        if (at >= 0) tab[(size_t)r * row + at] = mk(fy.y, -fy.x);
     }
 }
 
 }  // namespace
 
 void launch_real_table_ck(int lsum, cplx k, double eta, int NR, const double2* R, double sx, double sy, double sz,
-                          const double* norm, const double* reflection, double2* tab, cudaStream_t st) {
+                          const double* norm, const double* reflection, bool offplane, double2* tab, cudaStream_t st) {
     StageScope sc(ST_LATTICE, st);
-    real_table_ck_kernel<<<(NR + 3) / 4, 128, 0, st>>>(lsum, k, eta, NR, R, sx, sy, sz, norm, reflection, tab);
+    real_table_ck_kernel<<<(NR + 3) / 4, 128, 0, st>>>(lsum, k, eta, NR, R, sx, sy, sz, norm, reflection,
+                                                       offplane ? 1 : 2, 2 * lattice_pairs(lsum, offplane), tab);
 }
 
 size_t lattice_sum_ck_smem(int lsum, int NR) {
-    return (size_t)NR * 16 + (size_t)CK_CHUNK * (lsum + 1) * 16 + 3 * CK_CHUNK * 16;
-}
-
-void launch_lattice_sum_ck(const LatticeSumCkArgs& a, int grid, cudaStream_t st) {
-    StageScope sc(ST_LATTICE, st);
-    const size_t smem = lattice_sum_ck_smem(a.lsum, a.NR);
-    cudaFuncSetAttribute(lattice_sum_ck_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    lattice_sum_ck_kernel<<<grid, 256, smem, st>>>(a);
+    return (size_t)NR * 16 + (size_t)256 * (lsum + 1) * 16 + 3 * 256 * 16;
 }
 
 }  // namespace tcu
