@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <complex>
 #include <cstdio>
@@ -12,6 +13,7 @@
 #include <set>
 #include <memory>
 #include <mutex>
+#include <new>
 #include <string>
 #include <thread>
 #include <vector>
@@ -73,6 +75,44 @@ struct DevicePool : tcu::DeviceAllocator {
     }
 };
 
+// Pinned ring of a context for large results: the device copies into its slots while host threads
+// copy filled slots out to the caller's pageable memory. A plain cudaMemcpy into pageable memory
+// moves through the driver's own staging on one thread, which also takes the page faults of a fresh
+// result array: 151 MB (1021 array T-matrices) took 32 ms, through this ring 6. From 32 MB on, where
+// the C library returns freed arrays to the system and every result faults anew: 11 MB of lattice sums
+// took 0.6 ms plainly and 1.3 through the ring. 16 MB, made at the first large result and kept until
+// the context is destroyed (calls on a context are serialised).
+struct HostRing {
+    static constexpr size_t SLOT = (size_t)2 << 20;
+    static constexpr int SLOTS = 8;
+    static constexpr size_t LARGE = (size_t)32 << 20;  // smaller results: the plain copy
+    char* mem = nullptr;
+    cudaEvent_t full[SLOTS] = {};
+    bool ready() {
+        if (mem) return true;
+        if (cudaHostAlloc((void**)&mem, SLOT * SLOTS, cudaHostAllocDefault) != cudaSuccess) {
+            cudaGetLastError();
+            mem = nullptr;
+            return false;
+        }
+        for (int i = 0; i < SLOTS; ++i)
+            if (cudaEventCreateWithFlags(&full[i], cudaEventDisableTiming) != cudaSuccess) {
+                cudaGetLastError();
+                release();
+                return false;
+            }
+        return true;
+    }
+    void release() {
+        for (cudaEvent_t& e : full) {
+            if (e) cudaEventDestroy(e);
+            e = nullptr;
+        }
+        if (mem) cudaFreeHost(mem);
+        mem = nullptr;
+    }
+};
+
 struct DevPlanStore {
     HostPlan host;
     DevPlan dev{};
@@ -90,6 +130,7 @@ void set_error_message(const char* msg) { g_last_error = msg; }
 struct tcu_context {
     Profiler prof;
     DevicePool pool;
+    HostRing ring;
     int device = 0;
     cudaStream_t stream = nullptr;
     std::recursive_mutex mu;
@@ -288,6 +329,75 @@ struct DevBuf {
         if (p) ctx->pool.free(p);
     }
 };
+
+// A result of the call to the caller's memory, on the context's stream; returns when it is there.
+tcu_status copy_out(tcu_context* ctx, void* dst, const void* src, size_t bytes, const char* what) {
+    typedef HostRing Ring;
+    cudaPointerAttributes at;
+    const bool pageable = cudaPointerGetAttributes(&at, dst) != cudaSuccess || at.type == cudaMemoryTypeUnregistered;
+    cudaGetLastError();
+    if (bytes < Ring::LARGE || !pageable || !ctx->ring.ready()) {
+        CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream), what);
+        return sync_status(ctx, what);
+    }
+    const size_t chunks = (bytes + Ring::SLOT - 1) / Ring::SLOT;
+    std::atomic<size_t> issued{0}, next{0};
+    std::atomic<bool> stop{false};
+    std::atomic<int> error{(int)cudaSuccess};
+    std::unique_ptr<std::atomic<unsigned char>[]> done(new (std::nothrow) std::atomic<unsigned char>[chunks]);
+    if (!done) {
+        CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream), what);
+        return sync_status(ctx, what);
+    }
+    for (size_t c = 0; c < chunks; ++c) done[c].store(0, std::memory_order_relaxed);
+    auto work = [&] {
+        cudaSetDevice(ctx->device);
+        for (;;) {
+            const size_t c = next.fetch_add(1);
+            if (c >= chunks) return;
+            while (issued.load(std::memory_order_acquire) <= c) {
+                if (stop.load()) return;
+                std::this_thread::yield();
+            }
+            const cudaError_t e = cudaEventSynchronize(ctx->ring.full[c % Ring::SLOTS]);
+            if (e != cudaSuccess) {
+                error = (int)e;
+                stop = true;
+                return;
+            }
+            const size_t off = c * Ring::SLOT;
+            memcpy((char*)dst + off, ctx->ring.mem + (c % Ring::SLOTS) * Ring::SLOT, std::min(Ring::SLOT, bytes - off));
+            done[c].store(1, std::memory_order_release);
+        }
+    };
+    std::vector<std::thread> threads;
+    const unsigned cores = std::max(1u, std::thread::hardware_concurrency());
+    const size_t want = std::min<size_t>({(size_t)8, std::max<size_t>(1, cores / 2), chunks});
+    try {
+        for (size_t t = 0; t < want; ++t) threads.emplace_back(work);
+    } catch (const std::exception&) {  // fewer threads, or none: the copy below
+    }
+    cudaError_t e = cudaSuccess;
+    if (threads.empty()) {
+        e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream);
+    } else {
+        for (size_t c = 0; c < chunks && e == cudaSuccess && !stop; ++c) {
+            if (c >= (size_t)Ring::SLOTS)  // the slot's previous chunk has been copied out
+                while (!done[c - Ring::SLOTS].load(std::memory_order_acquire) && !stop) std::this_thread::yield();
+            const size_t off = c * Ring::SLOT;
+            const int slot = (int)(c % Ring::SLOTS);
+            e = cudaMemcpyAsync(ctx->ring.mem + slot * Ring::SLOT, (const char*)src + off,
+                                std::min(Ring::SLOT, bytes - off), cudaMemcpyDeviceToHost, ctx->stream);
+            if (e == cudaSuccess) e = cudaEventRecord(ctx->ring.full[slot], ctx->stream);
+            if (e == cudaSuccess) issued.store(c + 1, std::memory_order_release);
+        }
+        if (e != cudaSuccess) stop = true;
+        for (std::thread& t : threads) t.join();
+        if (e == cudaSuccess) e = (cudaError_t)error.load();
+    }
+    CK(e, what);
+    return sync_status(ctx, what);
+}
 
 // Sub-buffers of one allocation, each on a 256-byte boundary.
 struct Arena {
@@ -863,6 +973,7 @@ tcu_status tcu_context_destroy(tcu_context* ctx) {
     for (tcu_context* w : ctx->workers) tcu_context_destroy(w);
     for (auto& kv : ctx->plans) cudaFree(kv.second->mem);
     ctx->pool.release();
+    ctx->ring.release();
     cudaFree(ctx->d_partial);
     cudaFree(ctx->d_cpartial);
     cudaFree(ctx->d_small);
@@ -1217,8 +1328,7 @@ tcu_status tcu_cluster_operator(tcu_context* ctx, int lmax, double k0, size_t N,
     if ((s = read_status(ctx, "Mie coefficients"))) return s;
     launch_assemble(*P, (int)N, k0, pos, T, A, n, false, ctx->stream);
     ctx->launches += 2;
-    CK(cudaMemcpyAsync(out, A, n * n * 16, cudaMemcpyDeviceToHost, ctx->stream), "copy");
-    return sync_status(ctx, "cluster operator");
+    return copy_out(ctx, out, A, n * n * 16, "cluster operator");
 }
 
 tcu_status tcu_cluster_apply(tcu_context* ctx, int lmax, double k0, size_t N, const double* radii, const double* eps,
@@ -1573,7 +1683,14 @@ extern "C" tcu_status tcu_iterative_pullback_incident(tcu_context* ctx, int lmax
 // 2D lattice sums at shift 0 and the batched periodic-array solve.
 namespace {
 
-double log_fact(int n) { return std::lgamma((double)n + 1.0); }
+double log_fact(int n) {  // n <= 2 LS_MAXL and the like; lgamma per coefficient took 0.2 ms of a call
+    static const std::vector<double> table = [] {
+        std::vector<double> t(256);
+        for (int i = 0; i < 256; ++i) t[i] = std::lgamma((double)i + 1.0);
+        return t;
+    }();
+    return n >= 0 && n < 256 ? table[n] : std::lgamma((double)n + 1.0);
+}
 
 // Host-side set-up of one batch of lattice sums: split, lattice points within the real-space
 // cutoff, reciprocal vectors within the reciprocal cutoff, and the per-(l, m) constants.
@@ -1937,8 +2054,7 @@ extern "C" tcu_status tcu_lsumsw2d_shift_batch(tcu_context* ctx, int lmax_sum, d
     if ((s = lattice_sums_device(ctx, lmax_sum, k, S, nk, ar.at<double2>(io.p, oK), ar.at<double2>(io.p, oO), nullptr,
                                  scratch)))
         return s;
-    CK(cudaMemcpyAsync(out, ar.at<void>(io.p, oO), nk * T * 16, cudaMemcpyDeviceToHost, ctx->stream), "copy");
-    return sync_status(ctx, "lattice sums");
+    return copy_out(ctx, out, ar.at<void>(io.p, oO), nk * T * 16, "lattice sums");
 }
 
 extern "C" tcu_status tcu_lsumsw2d_batch(tcu_context* ctx, int lmax_sum, double k, const double* lattice, size_t nk,
@@ -2199,8 +2315,7 @@ extern "C" tcu_status tcu_lsumsw2d_complex_batch(tcu_context* ctx, int lmax_sum,
     if (stw == 9)
         return fail(TCU_INVALID_INPUT, "lattice sum is at a diffraction threshold; supply a limiting complex wavenumber");
     if (stw) return fail(TCU_DEVICE_ERROR, "lattice sums: device status " + std::to_string(stw));
-    CK(cudaMemcpyAsync(out, ar.at<void>(b, oO), nk * T * 16, cudaMemcpyDeviceToHost, st), "copy");
-    return sync_status(ctx, "lattice sums");
+    return copy_out(ctx, out, ar.at<void>(b, oO), nk * T * 16, "lattice sums");
 }
 
 extern "C" tcu_status tcu_array_solve_batch(tcu_context* ctx, int lmax, double k0, double radius, const double* eps,
@@ -2220,8 +2335,7 @@ extern "C" tcu_status tcu_array_solve_batch(tcu_context* ctx, int lmax, double k
     tcu_status s = array_solve_device(ctx, lmax, k0, radius, eps, lattice, nk, ar.at<double2>(io.p, oK), eta, kpars,
                                       ar.at<double2>(io.p, oX));
     if (s) return s;
-    CK(cudaMemcpyAsync(out, ar.at<void>(io.p, oX), nk * M * M * 16, cudaMemcpyDeviceToHost, ctx->stream), "copy");
-    return sync_status(ctx, "periodic array solve");
+    return copy_out(ctx, out, ar.at<void>(io.p, oX), nk * M * M * 16, "periodic array solve");
 }
 
 extern "C" tcu_status tcu_context_set_learned_weights(tcu_context* ctx, double reach_diameters, size_t count,
