@@ -171,39 +171,53 @@ __device__ __forceinline__ void build_chunk(const DevPlan& P, int order, int N, 
     }
 }
 
-// Term lists of the plan, Mie block and the alpha / beta / zadd epilogue: thread per
-// (destination, d) of the DI destinations from i0, with G of destination il at
-// Gs + il * tsize * 2 nsrc (rows: table index, columns: source lm and helicity).
+// Term lists of the plan, Mie block and the alpha / beta / zadd epilogue: W lanes per (destination, d)
+// of the DI destinations from i0, each lane the source lm s = lane, lane + W, ..., summed by shuffles in
+// a fixed order, with G of destination il at Gs + il * tsize * 2 nsrc (rows: table index, columns:
+// source lm and helicity). W is what the CTA's threads allow, at most 16: a thread alone walks a
+// chain of 200 dependent gathers at lmax 4, about 5 us, as long as the product itself below some
+// hundred spheres (40 spheres, 96 columns: 0.71 -> 0.45 ms an application).
 __device__ __forceinline__ void terms_epilogue(const DevPlan& P, const SubOp& O, const cplx* Gs, int DI, int i0,
                                                int N, const cplx* __restrict__ T, const cplx* __restrict__ xc,
                                                size_t coff, const cplx* __restrict__ zadd, double alpha,
                                                double beta, bool singular, cplx* __restrict__ y, int tid,
                                                int nthr) {
     const int nlm = P.nlm, M = 2 * O.nsrc, ts = (O.order + 1) * (O.order + 1);
-    const int ndst = O.ndst;
-    for (int it = tid; it < DI * ndst; it += nthr) {
+    const int ndst = O.ndst, tasks = DI * ndst;
+    int W = 1;
+    while (W < 16 && 2 * W * tasks <= nthr && 2 * W <= O.nsrc) W *= 2;
+    const int end = (tasks * W + 31) / 32 * 32;  // whole warps take part in the shuffles
+    for (int t0 = tid; t0 < end; t0 += nthr) {
+        const int it = min(t0 / W, tasks - 1), part = t0 % W;
         const int il = it / ndst, d = it - il * ndst, i = i0 + il;
-        if (i >= N) continue;
         const cplx* G = Gs + (size_t)il * ts * M;
         cplx sp = mk(0.0, 0.0), sn = mk(0.0, 0.0);
-        for (int s = 0; s < O.nsrc; ++s) {
-            const int2 cb = __ldg(&P.combo[s * nlm + d]);
-            int t = cb.x;
-            const int na = cb.y & 0xffff, nb = cb.y >> 16;
-            const cplx* g = G + 2 * s;
-            for (int e = 0; e < na; ++e, ++t) {
-                const cplx w = __ldg(&P.w[t]);
-                const cplx* ge = g + (size_t)__ldg(&P.idx[t]) * M;
-                cfma(sp, w, ge[0]);
-                cfma(sn, w, ge[1]);
+        if (i < N)
+            for (int s = part; s < O.nsrc; s += W) {
+                const int2 cb = __ldg(&P.combo[s * nlm + d]);
+                int t = cb.x;
+                const int na = cb.y & 0xffff, nb = cb.y >> 16;
+                const cplx* g = G + 2 * s;
+                for (int e = 0; e < na; ++e, ++t) {
+                    const cplx w = __ldg(&P.w[t]);
+                    const cplx* ge = g + (size_t)__ldg(&P.idx[t]) * M;
+                    cfma(sp, w, ge[0]);
+                    cfma(sn, w, ge[1]);
+                }
+                for (int e = 0; e < nb; ++e, ++t) {
+                    const cplx w = __ldg(&P.w[t]);
+                    const cplx* ge = g + (size_t)__ldg(&P.idx[t]) * M;
+                    cfma(sp, w, ge[0]);
+                    cfma(sn, cneg(w), ge[1]);
+                }
             }
-            for (int e = 0; e < nb; ++e, ++t) {
-                const cplx w = __ldg(&P.w[t]);
-                const cplx* ge = g + (size_t)__ldg(&P.idx[t]) * M;
-                cfma(sp, w, ge[0]);
-                cfma(sn, cneg(w), ge[1]);
-            }
+        for (int o = W / 2; o > 0; o >>= 1) {
+            sp.x += __shfl_xor_sync(0xffffffffu, sp.x, o);
+            sp.y += __shfl_xor_sync(0xffffffffu, sp.y, o);
+            sn.x += __shfl_xor_sync(0xffffffffu, sn.x, o);
+            sn.y += __shfl_xor_sync(0xffffffffu, sn.y, o);
         }
+        if (i >= N || part != 0 || t0 >= tasks * W) continue;
         // the input at (i, d) exists for source lm only (d < nsrc), the output for d < ndst
         const size_t row = (size_t)i * O.ldout + 2 * d, rin = (size_t)i * O.ldin + 2 * d;
         const cplx x0 = d < O.nsrc ? xc[rin] : mk(0.0, 0.0), x1 = d < O.nsrc ? xc[rin + 1] : mk(0.0, 0.0);
@@ -311,17 +325,8 @@ __global__ void __launch_bounds__(512, 1)
 // source % 4). The inputs are packed per call in the B-fragment order (lane = 4 * column % 8 +
 // source % 4), so every fragment load of a warp reads 512 contiguous bytes.
 constexpr int SRC_CHUNK = 16;  // sources per stored chunk
-constexpr int AS_STAGES = 3;   // cp.async ring of the stored product
+constexpr int AS_STAGES = 3;   // ring of the stored product (2 CTAs per SM at lmax <= 4)
 
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int K>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(K) : "memory");
-}
 // c += a b on one 8 x 8 FP64 tile (m8n8k4, A row-major, B column-major)
 __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
     asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
@@ -359,7 +364,7 @@ __global__ void __launch_bounds__(256) table_store_kernel(DevPlan P, int order, 
             const int row = o * 8 + (lane >> 2), kk = qc * 4 + (lane & 3);  // qc = 4 c + q
             const cplx v = row < rows ? Zs[(size_t)kk * ZLD + row] : mk(0.0, 0.0);
             const size_t slab = (size_t)(j0 / SRC_CHUNK) * 4 + qc;  // chunk * 4 + q
-            Zb[(slab * RO + o) * 32 + lane] = v;
+            if (slab < (size_t)NC * 4) Zb[(slab * RO + o) * 32 + lane] = v;  // the last build chunk may be half past N
         }
     }
 }
@@ -392,93 +397,9 @@ __global__ void pack_sources_kernel(const cplx* __restrict__ x, size_t ldx, int 
 }
 
 // y = zadd + alpha x + beta T C x (or the sub-operator O) from the stored tables: CTA = DI
-// destinations x one column, a warp per RPW row octets with CT column octets (complex
-// accumulators as re and im 8 x 8 FP64 tiles, four m8n8k4 products per complex step:
-// re += a.re b.re + a.im (-b.im), im += a.re b.im + a.im b.re, each B fragment used for RPW
-// row octets); chunks of 16 sources through a 3-stage cp.async ring; then the term lists.
-template <int CT, int RPW>
-__global__ void __launch_bounds__(256, 1)
-    apply_stored_kernel(DevPlan P, SubOp O, int N, const cplx* __restrict__ Z, const cplx* __restrict__ Xf, int NC,
-                        int DI, int RO, const cplx* __restrict__ T, const cplx* __restrict__ x, size_t ldx,
-                        const cplx* __restrict__ zadd, double alpha, double beta, bool singular,
-                        cplx* __restrict__ y) {
-    extern __shared__ __align__(16) unsigned char as_smem[];
-    const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, o0 = (tid >> 5) * RPW;
-    const int ABLK = RO * 128, BBLK = CT * 128, SBLK = ABLK + BBLK;  // complex entries per chunk
-    cplx* ring = reinterpret_cast<cplx*>(as_smem);
-    const cplx* Zb = Z + (size_t)blockIdx.x * NC * ABLK;
-    const cplx* Xb = Xf + (size_t)blockIdx.y * NC * BBLK;
-    auto load = [&](int stage, int kc) {
-        cplx* dst = ring + (size_t)stage * SBLK;
-        const cplx* sa = Zb + (size_t)kc * ABLK;
-        const cplx* sb = Xb + (size_t)kc * BBLK;
-        for (int t = tid; t < SBLK; t += nthr) cp_async16(dst + t, t < ABLK ? sa + t : sb + (t - ABLK));
-    };
-    double re[RPW][CT][2], im[RPW][CT][2];
-#pragma unroll
-    for (int r = 0; r < RPW; ++r)
-#pragma unroll
-        for (int c = 0; c < CT; ++c) re[r][c][0] = re[r][c][1] = im[r][c][0] = im[r][c][1] = 0.0;
-    // row octets past RO (the last warp of an odd count) skip their products, warp-uniformly
-    const int nr = min(RPW, RO - o0);
-#pragma unroll
-    for (int s = 0; s < AS_STAGES - 1; ++s) {
-        if (s < NC) load(s, s);
-        cp_async_commit();
-    }
-    for (int kc = 0; kc < NC; ++kc) {
-        cp_async_wait<AS_STAGES - 2>();
-        __syncthreads();  // chunk kc landed for every thread; the stage of chunk kc - 1 is free
-        if (kc + AS_STAGES - 1 < NC) load((kc + AS_STAGES - 1) % AS_STAGES, kc + AS_STAGES - 1);
-        cp_async_commit();
-        const cplx* As = ring + (size_t)(kc % AS_STAGES) * SBLK;
-        const cplx* Bs = As + ABLK;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            cplx a[RPW];
-#pragma unroll
-            for (int r = 0; r < RPW; ++r) a[r] = r < nr ? As[(q * RO + o0 + r) * 32 + lane] : mk(0.0, 0.0);
-#pragma unroll
-            for (int c = 0; c < CT; ++c) {
-                const cplx b = Bs[(q * CT + c) * 32 + lane];
-#pragma unroll
-                for (int r = 0; r < RPW; ++r) {
-                    if (r < nr) {
-                        dmma(re[r][c], a[r].x, b.x);
-                        dmma(re[r][c], a[r].y, -b.y);
-                        dmma(im[r][c], a[r].x, b.y);
-                        dmma(im[r][c], a[r].y, b.x);
-                    }
-                }
-            }
-        }
-    }
-    cp_async_wait<0>();
-    __syncthreads();  // the ring is free for G
-    cplx* Gs = reinterpret_cast<cplx*>(as_smem);
-    const int M = 2 * O.nsrc, rows = DI * (O.order + 1) * (O.order + 1);
-#pragma unroll
-    for (int r = 0; r < RPW; ++r) {
-        const int row = (o0 + r) * 8 + (lane >> 2);
-        if (row < rows) {
-#pragma unroll
-            for (int c = 0; c < CT; ++c) {
-                const int col = c * 8 + 2 * (lane & 3);
-                if (col < M) {
-                    Gs[(size_t)row * M + col] = mk(re[r][c][0], im[r][c][0]);
-                    Gs[(size_t)row * M + col + 1] = mk(re[r][c][1], im[r][c][1]);
-                }
-            }
-        }
-    }
-    __syncthreads();
-    const size_t coff = (size_t)blockIdx.y * ldx;
-    terms_epilogue(P, O, Gs, DI, blockIdx.x * DI, N, T, x + coff, coff, zadd, alpha, beta, singular, y, tid, nthr);
-}
-
+// destinations x one column, complex accumulators as re and im 8 x 8 FP64 tiles, four m8n8k4 products
+// per complex step: re += a.re b.re + a.im (-b.im), im += a.re b.im + a.im b.re; then the term lists.
 // ---- bulk-copy pipeline of the stored product ---------------------------------------------
-constexpr int AT_STAGES = AS_STAGES;  // ring depth of the bulk-copy pipeline (2 CTAs per SM at lmax <= 4)
-
 __device__ __forceinline__ uint32_t as_smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void as_mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
@@ -533,19 +454,24 @@ __device__ __forceinline__ void as_bulk_load(uint32_t dst, const void* src, uint
 // sits in the loop. Every wait is bounded (2 s): on a timeout the kernel records status 8,
 // waits (bounded) for the copies in flight and returns without writing y.
 // On success the product Z X is in Gs = smem (rows < rows, columns < cols, row-major).
-template <int CT, int RPW>
+// CG 1: a warp takes RPW row octets and all CT column octets. CG 2: eight warps, row octets in four
+// parts of at most RPW, columns in two halves, the second half's parts in reverse order: warp w runs on
+// scheduler w % 4, and 11 row octets by twos (lmax 4) leave the four DMMA pipes 4, 3, 2 and 2 of them,
+// 69 % busy at most, the parts 5, 6, 6 and 5.
+template <int CT, int RPW, int CG>
 __device__ __forceinline__ bool stored_product(unsigned char* smem, const cplx* __restrict__ Zb,
                                                const cplx* __restrict__ Xb, int NC, int RO, int rows, int cols,
                                                int* __restrict__ status) {
-    __shared__ __align__(8) uint64_t bars[2 * AT_STAGES];
+    __shared__ __align__(8) uint64_t bars[2 * AS_STAGES];
     __shared__ int s_abort;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int W = (RO + RPW - 1) / RPW;  // product warps; warp W loads
+    constexpr int CW = CT / CG;  // column octets of a warp
+    const int W = CG == 1 ? (RO + RPW - 1) / RPW : 4 * CG;  // product warps; warp W loads
     const int ABLK = RO * 128, BBLK = CT * 128, SBLK = ABLK + BBLK;  // complex entries per chunk
     cplx* ring = reinterpret_cast<cplx*>(smem);
-    const uint32_t full0 = as_smem_u32(bars), empty0 = full0 + 8 * AT_STAGES;
+    const uint32_t full0 = as_smem_u32(bars), empty0 = full0 + 8 * AS_STAGES;
     if (tid == 0) {
-        for (int s = 0; s < AT_STAGES; ++s) {
+        for (int s = 0; s < AS_STAGES; ++s) {
             as_mbar_init(full0 + 8 * s, 1);
             as_mbar_init(empty0 + 8 * s, W);
         }
@@ -554,18 +480,24 @@ __device__ __forceinline__ bool stored_product(unsigned char* smem, const cplx* 
     }
     __syncthreads();
     volatile int* abort_flag = &s_abort;
-    double re[RPW][CT][2], im[RPW][CT][2];
+    double re[RPW][CW][2], im[RPW][CW][2];
 #pragma unroll
     for (int r = 0; r < RPW; ++r)
 #pragma unroll
-        for (int c = 0; c < CT; ++c) re[r][c][0] = re[r][c][1] = im[r][c][0] = im[r][c][1] = 0.0;
-    const int o0 = warp * RPW;
+        for (int c = 0; c < CW; ++c) re[r][c][0] = re[r][c][1] = im[r][c][0] = im[r][c][1] = 0.0;
+    int o0 = warp * RPW, nr = min(RPW, RO - o0), c0 = 0;  // the warp's row and column octets
+    if (CG > 1) {
+        const int part = (warp >> 2) & 1 ? 3 - (warp & 3) : warp & 3, base = RO / 4, extra = RO % 4;
+        o0 = part * base + min(part, extra);
+        nr = base + (part < extra ? 1 : 0);
+        c0 = (warp >> 2) * CW;
+    }
     if (warp == W) {
         if (lane == 0) {
             int kc = 0;
             for (; kc < NC; ++kc) {
-                const int s = kc % AT_STAGES;
-                if (!as_mbar_wait(empty0 + 8 * s, ((kc / AT_STAGES) & 1) ^ 1, abort_flag)) break;
+                const int s = kc % AS_STAGES;
+                if (!as_mbar_wait(empty0 + 8 * s, ((kc / AS_STAGES) & 1) ^ 1, abort_flag)) break;
                 const uint32_t dst = as_smem_u32(ring + (size_t)s * SBLK);
                 as_mbar_expect_tx(full0 + 8 * s, (uint32_t)SBLK * 16u);
                 as_bulk_load(dst, Zb + (size_t)kc * ABLK, (uint32_t)ABLK * 16u, full0 + 8 * s);
@@ -574,17 +506,16 @@ __device__ __forceinline__ bool stored_product(unsigned char* smem, const cplx* 
             if (*abort_flag) {
                 // drain: the last load issued into every stage lands before the CTA exits
                 volatile int never = 0;
-                for (int s = 0; s < AT_STAGES; ++s) {
-                    const int last = kc - 1 - ((kc - 1 - s) % AT_STAGES + AT_STAGES) % AT_STAGES;
-                    if (last >= 0) as_mbar_wait(full0 + 8 * s, (last / AT_STAGES) & 1, &never);
+                for (int s = 0; s < AS_STAGES; ++s) {
+                    const int last = kc - 1 - ((kc - 1 - s) % AS_STAGES + AS_STAGES) % AS_STAGES;
+                    if (last >= 0) as_mbar_wait(full0 + 8 * s, (last / AS_STAGES) & 1, &never);
                 }
             }
         }
     } else if (warp < W) {
-        const int nr = min(RPW, RO - o0);
         for (int kc = 0; kc < NC; ++kc) {
-            const int s = kc % AT_STAGES;
-            if (!as_mbar_wait(full0 + 8 * s, (kc / AT_STAGES) & 1, abort_flag)) break;
+            const int s = kc % AS_STAGES;
+            if (!as_mbar_wait(full0 + 8 * s, (kc / AS_STAGES) & 1, abort_flag)) break;
             const cplx* As = ring + (size_t)s * SBLK;
             const cplx* Bs = As + ABLK;
 #pragma unroll
@@ -593,8 +524,8 @@ __device__ __forceinline__ bool stored_product(unsigned char* smem, const cplx* 
 #pragma unroll
                 for (int r = 0; r < RPW; ++r) a[r] = r < nr ? As[(q * RO + o0 + r) * 32 + lane] : mk(0.0, 0.0);
 #pragma unroll
-                for (int c = 0; c < CT; ++c) {
-                    const cplx b = Bs[(q * CT + c) * 32 + lane];
+                for (int c = 0; c < CW; ++c) {
+                    const cplx b = Bs[(q * CT + c0 + c) * 32 + lane];
 #pragma unroll
                     for (int r = 0; r < RPW; ++r) {
                         if (r < nr) {
@@ -620,10 +551,10 @@ __device__ __forceinline__ bool stored_product(unsigned char* smem, const cplx* 
 #pragma unroll
         for (int r = 0; r < RPW; ++r) {
             const int row = (o0 + r) * 8 + (lane >> 2);
-            if (row < rows) {
+            if (r < nr && row < rows) {
 #pragma unroll
-                for (int c = 0; c < CT; ++c) {
-                    const int col = c * 8 + 2 * (lane & 3);
+                for (int c = 0; c < CW; ++c) {
+                    const int col = (c0 + c) * 8 + 2 * (lane & 3);
                     if (col < cols) Gs[(size_t)row * cols + col] = mk(re[r][c][0], im[r][c][0]);
                     if (col + 1 < cols) Gs[(size_t)row * cols + col + 1] = mk(re[r][c][1], im[r][c][1]);
                 }
@@ -634,15 +565,15 @@ __device__ __forceinline__ bool stored_product(unsigned char* smem, const cplx* 
     return true;
 }
 
-template <int CT, int RPW>
-__global__ void __launch_bounds__(288, 1)
+template <int CT, int RPW, int CG>
+__global__ void __launch_bounds__(288, CT <= 6 ? 2 : 1)
     apply_stored_tma_kernel(DevPlan P, SubOp O, int N, const cplx* __restrict__ Z, const cplx* __restrict__ Xf,
                             int NC, int DI, int RO, const cplx* __restrict__ T, const cplx* __restrict__ x, size_t ldx,
                             const cplx* __restrict__ zadd, double alpha, double beta, bool singular,
                             cplx* __restrict__ y, int* __restrict__ status) {
     extern __shared__ __align__(128) unsigned char at_smem[];
     const int M = 2 * O.nsrc, rows = DI * (O.order + 1) * (O.order + 1);
-    if (!stored_product<CT, RPW>(at_smem, Z + (size_t)blockIdx.x * NC * RO * 128,
+    if (!stored_product<CT, RPW, CG>(at_smem, Z + (size_t)blockIdx.x * NC * RO * 128,
                                  Xf + (size_t)blockIdx.y * NC * CT * 128, NC, RO, rows, M, status))
         return;
     const size_t coff = (size_t)blockIdx.y * ldx;
@@ -665,7 +596,7 @@ __global__ void __launch_bounds__(512, 1)
     extern __shared__ __align__(128) unsigned char sp_smem[];
     const int i = blockIdx.x / parts, part = blockIdx.x - i * parts, s0 = (part >> 1) * cnt;
     const int ns = min(cnt, P.nlm - s0), nlm = P.nlm;
-    if (!stored_product<CT, RPW>(sp_smem, Z + (size_t)i * NC * RO * 128,
+    if (!stored_product<CT, RPW, 1>(sp_smem, Z + (size_t)i * NC * RO * 128,
                                  Xf + (size_t)blockIdx.y * per_col + (size_t)part * NC * CT * 128, NC, RO, P.tsize, cnt,
                                  status))
         return;
@@ -817,7 +748,7 @@ StoredLayout stored_layout(const DevPlan& P, int N, int kind) {
     }
     l.CT = ((l.parts > 1 ? l.cnt : 2 * l.O.nsrc) + 7) / 8;
     l.RPW = 2;
-    l.NC = (N + l.KJ - 1) / l.KJ * (l.KJ / SRC_CHUNK);
+    l.NC = (N + SRC_CHUNK - 1) / SRC_CHUNK;
     l.nblk = (N + l.DI - 1) / l.DI;
     l.z_elems = (size_t)l.nblk * l.NC * l.RO * 128;
     l.xf_per_col = (size_t)l.parts * l.NC * l.CT * 128;
@@ -887,24 +818,18 @@ void launch_apply_stored(const DevPlan& P, int N, int kind, const cplx* Z, const
         return;
     }
     const dim3 grid((unsigned)l.nblk, (unsigned)ncol);
-    // bulk-copy pipeline, except at 6 column octets (lmax 4) where the cp.async ring measured
-    // faster (1.43 against 1.58 ms at 1024 spheres); TCU_STORED_PIPE=cpasync or tma forces one
-    const char* pipe = getenv("TCU_STORED_PIPE");
-    const bool cpasync = pipe ? strcmp(pipe, "cpasync") == 0 : l.CT == 6;
-#define TCU_STORED(CT, RPW)                                                                                       \
-    if (cpasync)                                                                                                  \
-        apply_stored_kernel<CT, RPW><<<grid, threads, smem, st>>>(P, l.O, N, Z, Xf, l.NC, l.DI, l.RO, T, x, ldx,   \
-                                                                 zadd, alpha, beta, singular, y);                  \
-    else                                                                                                          \
-        apply_stored_tma_kernel<CT, RPW><<<grid, threads + 32, smem, st>>>(P, l.O, N, Z, Xf, l.NC, l.DI, l.RO, T, \
-                                                                          x, ldx, zadd, alpha, beta, singular, y,  \
-                                                                          status)
+    // column octets, row octets per warp, column groups (stored_product); at lmax 3 two column groups
+    // measured slower (4096 spheres: 7.8 against 7.6 ms), at lmax 4 faster (512 spheres, 3 columns: 0.81
+    // against 1.05 ms of the row octets by twos, 200 spheres, 17 columns: 0.79 against 1.03)
+#define TCU_STORED(CT, RPW, CG)                                                                                   \
+    apply_stored_tma_kernel<CT, RPW, CG><<<grid, CG > 1 ? 288 : threads + 32, smem, st>>>(                         \
+        P, l.O, N, Z, Xf, l.NC, l.DI, l.RO, T, x, ldx, zadd, alpha, beta, singular, y, status)
     switch (l.CT) {
-        case 1: TCU_STORED(1, 2); break;
-        case 2: TCU_STORED(2, 2); break;
-        case 4: TCU_STORED(4, 2); break;
-        case 6: TCU_STORED(6, 2); break;
-        default: TCU_STORED(9, 2); break;
+        case 1: TCU_STORED(1, 2, 1); break;
+        case 2: TCU_STORED(2, 2, 1); break;
+        case 4: TCU_STORED(4, 2, 1); break;
+        case 6: TCU_STORED(6, 3, 2); break;
+        default: TCU_STORED(9, 2, 1); break;
     }
 #undef TCU_STORED
 }
@@ -915,16 +840,11 @@ void apply_gemm_init_attributes() {
     cudaFuncSetAttribute(apply_gemm_kernel<4, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     cudaFuncSetAttribute(apply_gemm_kernel<4, 5>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     cudaFuncSetAttribute(table_store_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(apply_stored_kernel<1, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(apply_stored_tma_kernel<1, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(apply_stored_kernel<2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(apply_stored_tma_kernel<2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(apply_stored_kernel<4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(apply_stored_tma_kernel<4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(apply_stored_kernel<6, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(apply_stored_tma_kernel<6, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(apply_stored_kernel<9, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(apply_stored_tma_kernel<9, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(apply_stored_tma_kernel<1, 2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(apply_stored_tma_kernel<2, 2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(apply_stored_tma_kernel<4, 2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(apply_stored_tma_kernel<6, 3, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(apply_stored_tma_kernel<9, 2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     cudaFuncSetAttribute(apply_split_kernel<6, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     cudaFuncSetAttribute(apply_split_kernel<4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
 }
