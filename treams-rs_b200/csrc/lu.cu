@@ -13,8 +13,7 @@
 //     blocked inverse of L11 (tri_inverse_l_kernel) and a tensor-core GEMM (gemm_tf32.cu).
 //  4. trailing update A22 -= L21 U12: FP64 DMMA (mma.sync m8n8k4 f64) complex GEMM, or in
 //     the mixed path the 3-pass split tcgen05 GEMM of gemm_tf32.cu.
-// The permutation is composed from the pivots afterwards; the triangular solves with the
-// factors are in solve.cu.
+// The triangular solves with the factors are in solve.cu.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -221,7 +220,7 @@ __global__ void __launch_bounds__(PANEL_THREADS) panel_kernel(typename Cx<R>::T*
             s_inv[0] = den > 0.0 ? pivot.x / den : 0.0;
             s_inv[1] = den > 0.0 ? -pivot.y / den : 0.0;
             if (b == 0) {
-                piv[gj] = pr;  // the row permutation is composed from piv after the factorization
+                piv[gj] = pr;
                 if (!(den > 0.0)) atomicCAS(status, 0, 5);
             }
         }
@@ -344,8 +343,21 @@ __global__ void __launch_bounds__(PANEL_THREADS) panel_kernel(typename Cx<R>::T*
 namespace tcu {
 
 // ---- row swaps outside the panel ------------------------------------------------------------
+// (and on the row permutation, which the thread after the last column takes as one more column)
+template <typename T>
+__device__ __forceinline__ void swap_entries(T* a, int k0, int w, const int* sp) {
+    for (int j = 0; j < w; ++j) {
+        const int p = sp[j];
+        if (p != k0 + j) {
+            const T t = a[k0 + j];
+            a[k0 + j] = a[p];
+            a[p] = t;
+        }
+    }
+}
 template <typename C>
-__global__ void laswp_kernel(C* A, size_t lda, int n, int k0, int w, const int* __restrict__ piv) {
+__global__ void laswp_kernel(C* A, size_t lda, int n, int k0, int w, const int* __restrict__ piv,
+                             int* __restrict__ perm) {
     __shared__ int sp[128];
     __shared__ int any;
     if (threadIdx.x == 0) any = 0;
@@ -357,18 +369,19 @@ __global__ void laswp_kernel(C* A, size_t lda, int n, int k0, int w, const int* 
     __syncthreads();
     if (!any) return;
     int col = blockIdx.x * blockDim.x + threadIdx.x;
+    if (col == n) swap_entries(perm, k0, w, sp);
     if (col >= n || (col >= k0 && col < k0 + w)) return;
-    C* a = A + (size_t)col * lda;
-    for (int j = 0; j < w; ++j) {
-        int p = sp[j];
-        if (p != k0 + j) {
-            C t = a[k0 + j];
-            a[k0 + j] = a[p];
-            a[p] = t;
-        }
-    }
+    swap_entries(A + (size_t)col * lda, k0, w, sp);
+}
+__global__ void iota_kernel(int* __restrict__ perm, int n) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) perm[i] = i;
 }
 
+// A warp solves TRSM_COLS columns at a time, so that their chains of w dependent steps overlap; the
+// grid takes enough CTAs to cover the SMs twice (64 columns a CTA left half of them idle at n = 4270:
+// 45 us a panel against 17).
+constexpr int TRSM_COLS = 2;
 // ---- U12 = L11^-1 A12 ---------------------------------------------------------------------
 template <typename R, int NB>
 __global__ void __launch_bounds__(256) trsm_kernel(typename Cx<R>::T* A, size_t lda, int k0, int w, int n,
@@ -385,51 +398,65 @@ __global__ void __launch_bounds__(256) trsm_kernel(typename Cx<R>::T* A, size_t 
     constexpr int S = NB / 32;
     int cbeg = k0 + w + blockIdx.x * cols_per_cta;
     int cend = min(n, cbeg + cols_per_cta);
-    for (int col = cbeg + warp; col < cend; col += blockDim.x >> 5) {
-        C* a = A + (size_t)col * lda + k0;
-        R xr[S], xi[S];
+    for (int col = cbeg + warp * TRSM_COLS; col < cend; col += (blockDim.x >> 5) * TRSM_COLS) {
+        const int nc = min(TRSM_COLS, cend - col);
+        R xr[TRSM_COLS][S], xi[TRSM_COLS][S];
 #pragma unroll
-        for (int s = 0; s < S; ++s) {
-            int i = lane + 32 * s;
-            C v = (i < w) ? a[i] : cx_make<C>(0.0, 0.0);
-            xr[s] = v.x;
-            xi[s] = v.y;
-        }
+        for (int c = 0; c < TRSM_COLS; ++c)
+#pragma unroll
+            for (int s = 0; s < S; ++s) {
+                const int i = lane + 32 * s;
+                const C v = (i < w && c < nc) ? A[(size_t)(col + c) * lda + k0 + i] : cx_make<C>(0.0, 0.0);
+                xr[c][s] = v.x;
+                xi[c][s] = v.y;
+            }
 #pragma unroll
         for (int kb = 0; kb < S; ++kb) {
             for (int kk = 0; kk < 32; ++kk) {
-                int k = kb * 32 + kk;
+                const int k = kb * 32 + kk;
                 if (k >= w) break;
-                R br = __shfl_sync(0xffffffffu, xr[kb], kk);
-                R bi = __shfl_sync(0xffffffffu, xi[kb], kk);
+                C l[S];
 #pragma unroll
                 for (int s = kb; s < S; ++s) {
-                    int i = lane + 32 * s;
-                    if (i > k && i < w) {
-                        C l = Ls[k * NB + i];
-                        xr[s] -= l.x * br - l.y * bi;
-                        xi[s] -= l.x * bi + l.y * br;
+                    const int i = lane + 32 * s;
+                    l[s] = (i > k && i < w) ? Ls[k * NB + i] : cx_make<C>(0.0, 0.0);
+                }
+#pragma unroll
+                for (int c = 0; c < TRSM_COLS; ++c) {
+                    const R br = __shfl_sync(0xffffffffu, xr[c][kb], kk);
+                    const R bi = __shfl_sync(0xffffffffu, xi[c][kb], kk);
+#pragma unroll
+                    for (int s = kb; s < S; ++s) {
+                        xr[c][s] -= l[s].x * br - l[s].y * bi;
+                        xi[c][s] -= l[s].x * bi + l[s].y * br;
                     }
                 }
             }
         }
 #pragma unroll
-        for (int s = 0; s < S; ++s) {
-            int i = lane + 32 * s;
-            if (i < w) {
-                C v;
-                v.x = xr[s];
-                v.y = xi[s];
-                a[i] = v;
+        for (int c = 0; c < TRSM_COLS; ++c)
+#pragma unroll
+            for (int s = 0; s < S; ++s) {
+                const int i = lane + 32 * s;
+                if (i < w && c < nc) {
+                    C v;
+                    v.x = xr[c][s];
+                    v.y = xi[c][s];
+                    A[(size_t)(col + c) * lda + k0 + i] = v;
+                }
             }
-        }
     }
 }
 
 // ---- FP64 complex GEMM on DMMA: A22 -= L21 U12 -------------------------------------------
-// CTA tile 64 x 64 complex; K = w complex in chunks of 16 staged by cp.async (2 stages).
-// The complex product runs as a real GEMM of the 2x2-embedded L21 (rows re/im interleaved)
-// with U12 read as interleaved reals: D[2mu+c][nu] = sum_k Lemb[2mu+c][2k+c'] U[2k+c'][nu].
+// CTA tile 64 x 64 complex, K = w complex in chunks of 16 through a 3-stage cp.async ring; 8 warps
+// of 32 x 16 complex, real and imaginary accumulators as 8 x 8 FP64 tiles, four m8n8k4 products per
+// complex step: re += a.re b.re + a.im (-b.im), im += a.re b.im + a.im b.re. The copies write both
+// operands into shared memory in fragment order (per 4-deep k step and octet of rows or columns 32
+// entries, entry 4 (row % 8) + k % 4), so a fragment is one conflict-free 16-byte load of each lane
+// and 6 loads feed 32 products. Reading the real 2 x 2 embedding from a plain [k][row] layout took 10
+// loads and 32 selects per 16 products and kept the DMMA pipe 52 % busy; bound by that pipe:
+// n = 4270 all updates 10.1 -> 8.0 ms (20.6 -> 26 TFLOP/s, cuBLAS complex128 36.9).
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool valid) {
     unsigned s = (unsigned)__cvta_generic_to_shared(smem);
     int sz = valid ? 16 : 0;
@@ -441,207 +468,103 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-constexpr int ZG_T = 64;   // tile rows/cols (complex)
-constexpr int ZG_KC = 16;  // K chunk (complex)
-constexpr size_t ZG_SMEM = 4 * ZG_KC * ZG_T * sizeof(double2);
+constexpr int ZG_T = 64;      // tile rows/cols (complex)
+constexpr int ZG_KC = 16;     // K chunk (complex)
+constexpr int ZG_STAGES = 3;
+constexpr size_t ZG_SMEM = (size_t)ZG_STAGES * 2 * ZG_KC * ZG_T * sizeof(double2);
 
-__global__ void __launch_bounds__(256, 2) zgemm_dmma_kernel(double2* A, size_t lda, int k0, int w, int r0, int n) {
-    extern __shared__ __align__(16) unsigned char zg_smem[];
-    double2 (*Ls)[ZG_KC][ZG_T] = (double2 (*)[ZG_KC][ZG_T])zg_smem;                       // [stage][k][row]
-    double2 (*Us)[ZG_KC][ZG_T] = (double2 (*)[ZG_KC][ZG_T])(zg_smem + 2 * ZG_KC * ZG_T * 16);  // [stage][k][col]
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int tr = r0 + blockIdx.x * ZG_T, tc = r0 + blockIdx.y * ZG_T;
-    const int wr = (warp & 1) * 32, wc = (warp >> 1) * 16;  // warp tile: 32 complex rows x 16 cols
-    double acc[8][2][2];
-#pragma unroll
-    for (int a = 0; a < 8; ++a)
-#pragma unroll
-        for (int b = 0; b < 2; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
-    const int nchunks = (w + ZG_KC - 1) / ZG_KC;
-    auto load = [&](int stage, int ch) {
-        int kc = ch * ZG_KC;
-        for (int idx = tid; idx < ZG_KC * ZG_T; idx += 256) {
-            int r = idx % ZG_T, k = idx / ZG_T;
-            int row = tr + r, kk = kc + k;
-            bool ok = row < n && kk < w;
-            cp_async16(&Ls[stage][k][r], A + (size_t)(k0 + (ok ? kk : 0)) * lda + (ok ? row : 0), ok);
-        }
-        for (int idx = tid; idx < ZG_KC * ZG_T; idx += 256) {
-            int k = idx % ZG_KC, c = idx / ZG_KC;
-            int col = tc + c, kk = kc + k;
-            bool ok = col < n && kk < w;
-            cp_async16(&Us[stage][k][c], A + (size_t)(ok ? col : 0) * lda + k0 + (ok ? kk : 0), ok);
-        }
-        cp_async_commit();
-    };
-    load(0, 0);
-    for (int ch = 0; ch < nchunks; ++ch) {
-        int st = ch & 1;
-        if (ch + 1 < nchunks) {
-            load(st ^ 1, ch + 1);
-            cp_async_wait<1>();
-        } else {
-            cp_async_wait<0>();
-        }
-        __syncthreads();
-#pragma unroll
-        for (int ks = 0; ks < 2 * ZG_KC / 4; ++ks) {  // real k steps of 4
-            int kr = ks * 4 + (lane & 3);
-            int kc = kr >> 1, kp = kr & 1;
-            double bfrag[2];
-#pragma unroll
-            for (int cb = 0; cb < 2; ++cb) {
-                double2 u = Us[st][kc][wc + cb * 8 + (lane >> 2)];
-                bfrag[cb] = kp ? u.y : u.x;
-            }
-#pragma unroll
-            for (int rb = 0; rb < 8; ++rb) {
-                int rr = rb * 8 + (lane >> 2);  // real row within the warp's 64
-                int mu = wr + (rr >> 1), rp = rr & 1;
-                double2 l = Ls[st][kc][mu];
-                double a = (rp == kp) ? l.x : (rp == 0 ? -l.y : l.y);
-#pragma unroll
-                for (int cb = 0; cb < 2; ++cb) {
-                    asm volatile(
-                        "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-                        : "+d"(acc[rb][cb][0]), "+d"(acc[rb][cb][1])
-                        : "d"(a), "d"(bfrag[cb]));
-                }
-            }
-        }
-        __syncthreads();
-    }
-    // epilogue: lanes (l, l^4) hold the re/im rows of one complex row
-    const bool even = ((lane >> 2) & 1) == 0;
-    const int csel = 2 * (lane & 3) + (even ? 0 : 1);
-    // two halves of 8 read-modify-writes, each with all its loads in flight before its stores
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
-        double2 upd[4][2], old[4][2];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            int rb = half * 4 + q;
-#pragma unroll
-            for (int cb = 0; cb < 2; ++cb) {
-                double d0 = acc[rb][cb][0], d1 = acc[rb][cb][1];
-                double p0 = __shfl_xor_sync(0xffffffffu, d0, 4), p1 = __shfl_xor_sync(0xffffffffu, d1, 4);
-                upd[q][cb] = make_double2(even ? d0 : p1, even ? p0 : d1);
-                int grow = tr + wr + ((rb * 8 + (lane >> 2)) >> 1), gcol = tc + wc + cb * 8 + csel;
-                old[q][cb] = (grow < n && gcol < n) ? A[(size_t)gcol * lda + grow] : make_double2(0.0, 0.0);
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            int rb = half * 4 + q;
-#pragma unroll
-            for (int cb = 0; cb < 2; ++cb) {
-                int grow = tr + wr + ((rb * 8 + (lane >> 2)) >> 1), gcol = tc + wc + cb * 8 + csel;
-                if (grow < n && gcol < n)
-                    A[(size_t)gcol * lda + grow] = make_double2(old[q][cb].x - upd[q][cb].x, old[q][cb].y - upd[q][cb].y);
-            }
-        }
-    }
+// c += a b on one 8 x 8 FP64 tile (m8n8k4, A row-major, B column-major)
+__device__ __forceinline__ void zg_mma(double (&c)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+                 : "+d"(c[0]), "+d"(c[1])
+                 : "d"(a), "d"(b));
 }
 
-// ---- FP64 complex GEMM on DMMA, 128 x 64 complex tiles, 3-stage cp.async ring --------------
-// The same real-embedding product as zgemm_dmma_kernel with a larger tile per CTA (8 warps in
-// 4 x 2, warp tile 64 real rows x 32 columns: 32 m8n8k4 products per 4-deep real k step from
-// 8 A and 4 B fragments; 64 accumulators per lane, ~200 registers, one CTA per SM) and K
-// chunks of 8 complex in a 3-stage cp.async ring (24 KB per stage for 2 Mflop of products).
-// A fragments come from the complex tile: the 32 lanes of a load touch 8
-// distinct 16-byte entries (one shared-memory wavefront), and select Re, -Im or Im.
-constexpr int ZH_M = 128;  // complex rows per CTA
-constexpr int ZH_N = 64;   // columns per CTA
-constexpr int ZH_KC = 8;   // complex K per stage
-constexpr int ZH_STAGES = 3;
-constexpr size_t ZH_SMEM = (size_t)ZH_STAGES * ZH_KC * (ZH_M + ZH_N) * sizeof(double2);
-
-__global__ void __launch_bounds__(256, 1) zgemm_dmma_big_kernel(double2* A, size_t lda, int k0, int w, int r0, int n) {
-    extern __shared__ __align__(16) unsigned char zh_smem[];
-    double2 (*Ls)[ZH_KC][ZH_M] = (double2 (*)[ZH_KC][ZH_M])zh_smem;
-    double2 (*Us)[ZH_KC][ZH_N] = (double2 (*)[ZH_KC][ZH_N])(zh_smem + (size_t)ZH_STAGES * ZH_KC * ZH_M * 16);
+__global__ void __launch_bounds__(256, 2) zgemm_dmma_kernel(double2* A, size_t lda, int k0, int w, int r0, int n) {
+    extern __shared__ __align__(16) double2 zg_smem[];
+    constexpr int OP = ZG_KC * ZG_T;  // entries of one operand in a stage
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int tr = r0 + blockIdx.x * ZH_M, tc = r0 + blockIdx.y * ZH_N;
-    const int wr = (warp & 3) * 64, wc = (warp >> 2) * 32;  // real rows, columns of the warp tile
-    double acc[8][4][2];
+    const int tr = r0 + blockIdx.x * ZG_T, tc = r0 + blockIdx.y * ZG_T;
+    const int wr = (warp & 1) * 4, wc = (warp >> 1) * 2;  // first row and column octet of the warp
+    double re[4][2][2], im[4][2][2];
 #pragma unroll
-    for (int a = 0; a < 8; ++a)
+    for (int a = 0; a < 4; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
-    const int nchunks = (w + ZH_KC - 1) / ZH_KC;
+        for (int b = 0; b < 2; ++b) re[a][b][0] = re[a][b][1] = im[a][b][0] = im[a][b][1] = 0.0;
+    const int nchunks = (w + ZG_KC - 1) / ZG_KC;
+    auto at = [](int k, int r) { return ((k >> 2) * 8 + (r >> 3)) * 32 + 4 * (r & 7) + (k & 3); };
     auto load = [&](int stage, int ch) {
-        const int kc = ch * ZH_KC;
-        for (int idx = tid; idx < ZH_KC * ZH_M; idx += 256) {
-            const int r = idx % ZH_M, k = idx / ZH_M;
+        double2* Ls = zg_smem + (size_t)stage * 2 * OP;
+        double2* Us = Ls + OP;
+        const int kc = ch * ZG_KC;
+#pragma unroll
+        for (int q = 0; q < OP / 256; ++q) {
+            const int idx = tid + q * 256, r = idx % ZG_T, k = idx / ZG_T;
             const int row = tr + r, kk = kc + k;
             const bool ok = row < n && kk < w;
-            cp_async16(&Ls[stage][k][r], A + (size_t)(k0 + (ok ? kk : 0)) * lda + (ok ? row : 0), ok);
+            cp_async16(&Ls[at(k, r)], A + (size_t)(k0 + (ok ? kk : 0)) * lda + (ok ? row : 0), ok);
         }
-        for (int idx = tid; idx < ZH_KC * ZH_N; idx += 256) {
-            const int k = idx % ZH_KC, c = idx / ZH_KC;
+#pragma unroll
+        for (int q = 0; q < OP / 256; ++q) {
+            const int idx = tid + q * 256, k = idx % ZG_KC, c = idx / ZG_KC;
             const int col = tc + c, kk = kc + k;
             const bool ok = col < n && kk < w;
-            cp_async16(&Us[stage][k][c], A + (size_t)(ok ? col : 0) * lda + k0 + (ok ? kk : 0), ok);
+            cp_async16(&Us[at(k, c)], A + (size_t)(ok ? col : 0) * lda + k0 + (ok ? kk : 0), ok);
         }
     };
 #pragma unroll
-    for (int s = 0; s < ZH_STAGES - 1; ++s) {
+    for (int s = 0; s < ZG_STAGES - 1; ++s) {
         if (s < nchunks) load(s, s);
         cp_async_commit();
     }
     for (int ch = 0; ch < nchunks; ++ch) {
-        const int st = ch % ZH_STAGES;
-        if (ch + ZH_STAGES - 1 < nchunks) load((ch + ZH_STAGES - 1) % ZH_STAGES, ch + ZH_STAGES - 1);
+        cp_async_wait<ZG_STAGES - 2>();
+        __syncthreads();  // chunk ch landed for every thread; the stage of chunk ch - 1 is free
+        if (ch + ZG_STAGES - 1 < nchunks) load((ch + ZG_STAGES - 1) % ZG_STAGES, ch + ZG_STAGES - 1);
         cp_async_commit();
-        cp_async_wait<ZH_STAGES - 1>();
-        __syncthreads();
+        const double2* Ls = zg_smem + (size_t)(ch % ZG_STAGES) * 2 * OP;
+        const double2* Us = Ls + OP;
 #pragma unroll
-        for (int ks = 0; ks < 2 * ZH_KC / 4; ++ks) {  // real k steps of 4
-            const int kr = ks * 4 + (lane & 3);
-            const int kc = kr >> 1, kp = kr & 1;
-            double bfrag[4];
+        for (int kq = 0; kq < ZG_KC / 4; ++kq) {
+            double2 a[4], b[2];
 #pragma unroll
-            for (int cb = 0; cb < 4; ++cb) {
-                const double2 u = Us[st][kc][wc + cb * 8 + (lane >> 2)];
-                bfrag[cb] = kp ? u.y : u.x;
-            }
+            for (int r = 0; r < 4; ++r) a[r] = Ls[(kq * 8 + wr + r) * 32 + lane];
 #pragma unroll
-            for (int rb = 0; rb < 8; ++rb) {
-                const int rr = wr + rb * 8 + (lane >> 2);
-                const double2 l = Ls[st][kc][rr >> 1];
-                const int rp = rr & 1;
-                const double a = (rp == kp) ? l.x : (rp == 0 ? -l.y : l.y);
+            for (int c = 0; c < 2; ++c) b[c] = Us[(kq * 8 + wc + c) * 32 + lane];
 #pragma unroll
-                for (int cb = 0; cb < 4; ++cb)
-                    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-                                 : "+d"(acc[rb][cb][0]), "+d"(acc[rb][cb][1])
-                                 : "d"(a), "d"(bfrag[cb]));
+            for (int c = 0; c < 2; ++c) {
+#pragma unroll
+                for (int r = 0; r < 4; ++r) zg_mma(re[r][c], a[r].x, b[c].x);
+#pragma unroll
+                for (int r = 0; r < 4; ++r) zg_mma(im[r][c], a[r].x, b[c].y);
+#pragma unroll
+                for (int r = 0; r < 4; ++r) zg_mma(re[r][c], a[r].y, -b[c].y);
+#pragma unroll
+                for (int r = 0; r < 4; ++r) zg_mma(im[r][c], a[r].y, b[c].x);
             }
         }
-        __syncthreads();
     }
     cp_async_wait<0>();
-    // epilogue: lanes (l, l ^ 4) hold the re/im rows of one complex row
-    const bool even = ((lane >> 2) & 1) == 0;
-    const int csel = 2 * (lane & 3) + (even ? 0 : 1);
+    // a column pair at a time: 8 loads in flight before their stores
 #pragma unroll
-    for (int rb = 0; rb < 8; ++rb) {
-        double2 upd[4], old[4];
-        const int grow = tr + ((wr + rb * 8 + (lane >> 2)) >> 1);
+    for (int c = 0; c < 2; ++c) {
+        const int gcol = tc + (wc + c) * 8 + 2 * (lane & 3);
+        double2 old[4][2];
 #pragma unroll
-        for (int cb = 0; cb < 4; ++cb) {
-            const double d0 = acc[rb][cb][0], d1 = acc[rb][cb][1];
-            const double p0 = __shfl_xor_sync(0xffffffffu, d0, 4), p1 = __shfl_xor_sync(0xffffffffu, d1, 4);
-            upd[cb] = make_double2(even ? d0 : p1, even ? p0 : d1);
-            const int gcol = tc + wc + cb * 8 + csel;
-            old[cb] = (grow < n && gcol < n) ? A[(size_t)gcol * lda + grow] : make_double2(0.0, 0.0);
-        }
+        for (int r = 0; r < 4; ++r)
 #pragma unroll
-        for (int cb = 0; cb < 4; ++cb) {
-            const int gcol = tc + wc + cb * 8 + csel;
-            if (grow < n && gcol < n)
-                A[(size_t)gcol * lda + grow] = make_double2(old[cb].x - upd[cb].x, old[cb].y - upd[cb].y);
-        }
+            for (int e = 0; e < 2; ++e) {
+                const int grow = tr + (wr + r) * 8 + (lane >> 2);
+                old[r][e] = grow < n && gcol + e < n ? A[(size_t)(gcol + e) * lda + grow] : make_double2(0.0, 0.0);
+            }
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int grow = tr + (wr + r) * 8 + (lane >> 2);
+                if (grow < n && gcol + e < n)
+                    A[(size_t)(gcol + e) * lda + grow] = make_double2(old[r][e].x - re[r][c][e], old[r][e].y - im[r][c][e]);
+            }
     }
 }
 
@@ -720,8 +643,6 @@ void launch_barrier_selftest(unsigned* bar, int* status, double limit_s, cudaStr
     barrier_selftest_kernel<<<1, 32, 0, st>>>(bar, status, (unsigned long long)ns);
 }
 
-__global__ void perm_from_piv_kernel(const int* __restrict__ piv, int* __restrict__ perm, int n);
-
 void lu_init_attributes() {
     static PerDeviceOnce done;
     once_per_device(done, [] {
@@ -737,8 +658,6 @@ void lu_init_attributes() {
         cudaFuncSetAttribute(trsm_kernel<double, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         cudaFuncSetAttribute(trsm_kernel<float, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         cudaFuncSetAttribute(zgemm_dmma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ZG_SMEM);
-        cudaFuncSetAttribute(zgemm_dmma_big_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ZH_SMEM);
-        cudaFuncSetAttribute(perm_from_piv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     });
 }
 
@@ -755,16 +674,6 @@ static int panel_rows_per_cta() {
         const char* e = getenv("TCU_PANEL_ROWS");
         const int x = e ? atoi(e) : 0;
         return (x >= 16 && x <= 200) ? x : 32;
-    }();
-    return v;
-}
-
-// FP64 trailing update: 64 x 64 complex tiles, two CTAs per SM; TCU_FP64_GEMM=big selects the
-// 128 x 64 tiles (one CTA per SM), measured 9% slower at 512 spheres (2211 vs 2029 ms of updates).
-static bool fp64_big_tiles() {
-    static const bool v = [] {
-        const char* e = getenv("TCU_FP64_GEMM");
-        return e && std::string(e) == "big";
     }();
     return v;
 }
@@ -885,25 +794,6 @@ static int run_panel(typename Cx<R>::T* A, int n, int k0, int w, LuWork& wk, cud
     return e == cudaSuccess ? 0 : 2;
 }
 
-// perm from the interchanges: perm = iota, then swap perm[k] <-> perm[piv[k]] for k = 0..n-1
-// in shared memory (one CTA; row i of P A is row perm[i] of A).
-__global__ void perm_from_piv_kernel(const int* __restrict__ piv, int* __restrict__ perm, int n) {
-    extern __shared__ int pm[];
-    for (int i = threadIdx.x; i < n; i += blockDim.x) pm[i] = i;
-    __syncthreads();
-    if (threadIdx.x == 0)
-        for (int k = 0; k < n; ++k) {
-            int p = piv[k];
-            if (p != k) {
-                int t = pm[k];
-                pm[k] = pm[p];
-                pm[p] = t;
-            }
-        }
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) perm[i] = pm[i];
-}
-
 void launch_tf32_update(float2* A, int n, int k0, int w, LuWork& wk, cudaStream_t st, long long* launches);
 void launch_tf32_update_region(float2* A, int n, int k0, int w, int r0, int m, int c0, int ncols, LuWork& wk,
                                cudaStream_t st, long long* launches);
@@ -955,6 +845,8 @@ static int lu_factor_impl(typename Cx<R>::T* A, int n, LuWork& wk, cudaStream_t 
     typedef typename Cx<R>::T C;
     lu_init_attributes();
     size_t lda = n;
+    iota_kernel<<<(n + 255) / 256, 256, 0, st>>>(wk.perm, n);  // row i of P A is row perm[i] of A
+    ++*launches;
     // flags of the cluster panels' words: epochs 1 .. n
     cudaMemsetAsync(panel_words(wk), 0, (PC_GKEY + PC_GROW) * sizeof(uint4), st);
     // (the FP16-piece packers hold one 128-column panel, so FP16 pieces keep one update per panel)
@@ -978,7 +870,7 @@ static int lu_factor_impl(typename Cx<R>::T* A, int n, LuWork& wk, cudaStream_t 
                            cudaEventRecord(side->inverse_done, side->stream) == cudaSuccess;
         {
             StageScope sc(ST_SWAP, st);
-            laswp_kernel<C><<<(n + 255) / 256, 256, 0, st>>>(A, lda, n, k0, w, wk.piv);
+            laswp_kernel<C><<<n / 256 + 1, 256, 0, st>>>(A, lda, n, k0, w, wk.piv, wk.perm);
         }
         ++*launches;
         int r0 = k0 + w;
@@ -995,7 +887,8 @@ static int lu_factor_impl(typename Cx<R>::T* A, int n, LuWork& wk, cudaStream_t 
             cudaStreamSynchronize(side->stream);  // ordering by the host instead
         }
         if (r0 >= n) break;
-        int cpc = 64;
+        const int per_pass = 8 * TRSM_COLS;  // columns of a CTA's 8 warps at once
+        const int cpc = per_pass * std::max(1, (cols + per_pass * 2 * g_num_sms - 1) / (per_pass * 2 * g_num_sms));
         size_t smem = (size_t)NB * NB * sizeof(C);
         if (sizeof(R) == 4 && tensor_cores) {
             launch_tf32_trsm((float2*)A, n, k0, w, wk, st, launches, inverse_done, rhs_packed);
@@ -1007,12 +900,7 @@ static int lu_factor_impl(typename Cx<R>::T* A, int n, LuWork& wk, cudaStream_t 
         dim3 grid((cols + ZG_T - 1) / ZG_T, (cols + ZG_T - 1) / ZG_T);
         if constexpr (sizeof(R) == 8) {
             StageScope sc(ST_GEMM, st);
-            if (fp64_big_tiles()) {
-                dim3 g2((cols + ZH_M - 1) / ZH_M, (cols + ZH_N - 1) / ZH_N);
-                zgemm_dmma_big_kernel<<<g2, 256, ZH_SMEM, st>>>((double2*)A, lda, k0, w, r0, n);
-            } else {
-                zgemm_dmma_kernel<<<grid, 256, ZG_SMEM, st>>>((double2*)A, lda, k0, w, r0, n);
-            }
+            zgemm_dmma_kernel<<<grid, 256, ZG_SMEM, st>>>((double2*)A, lda, k0, w, r0, n);
             ++*launches;
         } else {
             if (tensor_cores) {
@@ -1035,11 +923,6 @@ static int lu_factor_impl(typename Cx<R>::T* A, int n, LuWork& wk, cudaStream_t 
                 ++*launches;
             }
         }
-    }
-    {
-        StageScope sc(ST_SWAP, st);
-        perm_from_piv_kernel<<<1, 1024, (size_t)n * sizeof(int), st>>>(wk.piv, wk.perm, n);
-        ++*launches;
     }
     return 0;
 }
