@@ -30,71 +30,73 @@ __device__ __forceinline__ double2 to_d2(C v) {
     return make_double2((double)v.x, (double)v.y);
 }
 
-// One CTA per diagonal block: invert in place in shared memory (FP64), column by column.
-// Lower (unit): columns right to left, X[i][j] = -sum_{k=j+1..i} X[i][k] L[k][j].
-// Upper: columns left to right, X[j][j] = 1/U[j][j], X[i][j] = -sum_{k=i..j-1} X[i][k] U[k][j] X[j][j].
-// Out: column-major 64 x 64 per block (identity beyond the matrix edge).
-template <typename C, bool LOWER>
+// One CTA per diagonal block and triangle (blockIdx.y: 0 L, unit lower; 1 U): its FP64 inverse, out
+// column-major 64 x 64 per block (identity beyond the matrix edge), all of L then all of U. U is
+// turned into a lower triangle by reversing both indices. The four 16 x 16 diagonal blocks are
+// inverted by a warp each (a lane per column of the inverse, a right-looking substitution), then
+// neighbouring inverses are joined, [A 0; B C]^-1 = [A^-1 0; -C^-1 B A^-1 C^-1], at 16 and at 32 rows.
+// One column after the other took 64 dependent steps with two barriers and 64 threads at work:
+// 95 us for each triangle whatever n, against 28 for both.
+constexpr int TBI_LD = SB + 1;
+template <typename C>
 __global__ void __launch_bounds__(256) tri_block_inverse_kernel(const C* __restrict__ A, size_t lda, int n,
                                                                 double2* __restrict__ out) {
     extern __shared__ double2 tbi_smem[];
-    double2 (*M)[SB + 1] = (double2 (*)[SB + 1])tbi_smem;  // M[i][k]
-    double2* col = tbi_smem + SB * (SB + 1);
-    const int b0 = blockIdx.x * SB, bw = min(SB, n - b0);
-    for (int idx = threadIdx.x; idx < SB * SB; idx += blockDim.x) {
-        int i = idx % SB, k = idx / SB;
-        double2 v = (i < bw && k < bw) ? to_d2(A[(size_t)(b0 + k) * lda + b0 + i]) : make_double2(i == k ? 1.0 : 0.0, 0.0);
-        M[i][k] = v;
+    double2* M = tbi_smem;                  // M[i * TBI_LD + k], lower triangle
+    double2* T = tbi_smem + SB * TBI_LD;    // 32 x 32 (two 16 x 16 at the first level)
+    const bool upper = blockIdx.y == 1;
+    const int b0 = blockIdx.x * SB, bw = min(SB, n - b0), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    auto place = [&](int i) { return upper ? SB - 1 - i : i; };  // index in the matrix -> in M
+    for (int idx = tid; idx < SB * SB; idx += blockDim.x) {
+        const int i = idx % SB, k = idx / SB;  // matrix row and column inside the block
+        const bool in = upper ? i <= k : i > k;
+        double2 v = make_double2(0.0, 0.0);
+        if (in && i < bw && k < bw) v = to_d2(A[(size_t)(b0 + k) * lda + b0 + i]);
+        if (i == k && (!upper || i >= bw)) v = make_double2(1.0, 0.0);
+        M[place(i) * TBI_LD + place(k)] = v;
     }
     __syncthreads();
-    const int i = threadIdx.x;  // rows handled by threads 0..63
-    if (LOWER) {
-        if (i < SB) M[i][i] = make_double2(1.0, 0.0);
-        for (int j = SB - 2; j >= 0; --j) {
-            if (i < SB) col[i] = M[i][j];
-            __syncthreads();
-            if (i < SB && i > j) {
-                double2 s = make_double2(0.0, 0.0);
-                for (int k = j + 1; k <= i; ++k) {
-                    double2 x = (k == i) ? make_double2(1.0, 0.0) : M[i][k];
-                    double2 l = col[k];
-                    s.x += x.x * l.x - x.y * l.y;
-                    s.y += x.x * l.y + x.y * l.x;
-                }
-                M[i][j] = make_double2(-s.x, -s.y);
-            }
-            __syncthreads();
+    if (warp < SB / 16 && lane < 16) {
+        const int o = warp * 16;
+        double2 x[16], inv[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            x[i] = make_double2(i == lane ? 1.0 : 0.0, 0.0);
+            inv[i] = cinv(M[(o + i) * TBI_LD + o + i]);
         }
-        if (i < SB)
-            for (int k = i + 1; k < SB; ++k) M[i][k] = make_double2(0.0, 0.0);
-    } else {
-        for (int j = 0; j < SB; ++j) {
-            if (i < SB) col[i] = M[i][j];
-            __syncthreads();
-            double2 d = col[j];
-            double den = d.x * d.x + d.y * d.y;
-            double2 inv = make_double2(d.x / den, -d.y / den);
-            if (i < SB && i < j) {
-                double2 s = make_double2(0.0, 0.0);
-                for (int k = i; k < j; ++k) {
-                    double2 x = M[i][k], u = col[k];
-                    s.x += x.x * u.x - x.y * u.y;
-                    s.y += x.x * u.y + x.y * u.x;
-                }
-                M[i][j] = make_double2(-(s.x * inv.x - s.y * inv.y), -(s.x * inv.y + s.y * inv.x));
-            } else if (i == j) {
-                M[i][j] = inv;
-            }
-            __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            x[k] = cmul(x[k], inv[k]);
+#pragma unroll
+            for (int i = k + 1; i < 16; ++i) cfma(x[i], cneg(M[(o + i) * TBI_LD + o + k]), x[k]);
         }
-        if (i < SB)
-            for (int k = 0; k < i; ++k) M[i][k] = make_double2(0.0, 0.0);
+        __syncwarp(0xffffu);  // every lane has read the block
+#pragma unroll
+        for (int i = 0; i < 16; ++i) M[(o + i) * TBI_LD + o + lane] = x[i];
     }
     __syncthreads();
-    double2* o = out + (size_t)blockIdx.x * SB * SB;
-    for (int idx = threadIdx.x; idx < SB * SB; idx += blockDim.x) {
-        int ii = idx % SB, k = idx / SB;
-        o[idx] = M[ii][k];
+    for (int s = 16; s < SB; s *= 2) {
+        const int pairs = SB / (2 * s);
+        for (int idx = tid; idx < pairs * s * s; idx += blockDim.x) {  // T = B A^-1
+            const int q = idx / (s * s), e = idx - q * s * s, k = e % s, i = e / s, a0 = 2 * s * q, c0 = a0 + s;
+            double2 t = make_double2(0.0, 0.0);
+            for (int m = k; m < s; ++m) cfma(t, M[(c0 + i) * TBI_LD + a0 + m], M[(a0 + m) * TBI_LD + a0 + k]);
+            T[idx] = t;
+        }
+        __syncthreads();
+        for (int idx = tid; idx < pairs * s * s; idx += blockDim.x) {  // -C^-1 T over B
+            const int q = idx / (s * s), e = idx - q * s * s, k = e % s, i = e / s, a0 = 2 * s * q, c0 = a0 + s;
+            double2 t = make_double2(0.0, 0.0);
+            for (int m = 0; m <= i; ++m) cfma(t, M[(c0 + i) * TBI_LD + c0 + m], T[q * s * s + m * s + k]);
+            M[(c0 + i) * TBI_LD + a0 + k] = cneg(t);
+        }
+        __syncthreads();
+    }
+    double2* o = out + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * SB * SB;
+    for (int idx = tid; idx < SB * SB; idx += blockDim.x) {
+        const int i = idx % SB, k = idx / SB;
+        const bool in = upper ? i <= k : i >= k;
+        o[idx] = in ? M[place(i) * TBI_LD + place(k)] : make_double2(0.0, 0.0);
     }
 }
 
@@ -455,17 +457,14 @@ template <typename C>
 static void inverses_impl(const C* A, int n, double2* inv, cudaStream_t st, long long* launches) {
     int nb = (n + SB - 1) / SB;
     StageScope sc(ST_SOLVE, st);
-    const size_t smem = (size_t)(SB * (SB + 1) + SB) * sizeof(double2);
+    const size_t smem = (size_t)(SB * TBI_LD + 32 * 32) * sizeof(double2);
     static PerDeviceOnce attr;
     once_per_device(attr, [&] {
-        cudaFuncSetAttribute(tri_block_inverse_kernel<double2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        cudaFuncSetAttribute(tri_block_inverse_kernel<double2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        cudaFuncSetAttribute(tri_block_inverse_kernel<float2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        cudaFuncSetAttribute(tri_block_inverse_kernel<float2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(tri_block_inverse_kernel<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(tri_block_inverse_kernel<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     });
-    tri_block_inverse_kernel<C, true><<<nb, 256, smem, st>>>(A, n, n, inv);
-    tri_block_inverse_kernel<C, false><<<nb, 256, smem, st>>>(A, n, n, inv + (size_t)nb * SB * SB);
-    *launches += 2;
+    tri_block_inverse_kernel<C><<<dim3(nb, 2), 256, smem, st>>>(A, n, n, inv);
+    *launches += 1;
 }
 void lu_block_inverses_fp64(const double2* A, int n, double2* inv, cudaStream_t st, long long* launches) {
     inverses_impl<double2>(A, n, inv, st, launches);
