@@ -4,7 +4,7 @@ Workload: the 512-sphere, lmax-4 precision cluster (n = 24,576 unknowns, three p
 incidences), seeded synthetic geometry. One step = assemble I - T C, factor it and solve
 the three columns to an FP64 residual <= 1e-13 |T b| (relative error well below 1e-10):
 `tcu_sphere_cluster_factor_dev` + `tcu_factor_solve_dev`. The headline is the mixed
-path (complex64 LU with split-TF32 tensor-core trailing updates + FP64 refinement); the
+path (complex64 LU with split-bfloat16 tensor-core trailing updates + FP64 refinement); the
 same run then times the plain FP64 drop-in on the same inputs (`fp64` and
 `speedup_vs_fp64` in the JSON line, `--no-compare` skips it) beside two library yardsticks
 (cuSOLVER zgetrf through torch.linalg.lu_factor on the same complex128 operator, and the
@@ -641,17 +641,20 @@ def _measure_impl(args, precision, steps, warmup, with_e2e, *, ctx, lib, stream,
     if prec == t.MIXED:
         # the update runs inside a seconds-long step: the sustained bf16 rate under the power cap
         bf16 = pk.get("bf16_tflops_sustained") or pk.get("bf16_tflops", 1590.0)
-        tensor_peak = bf16 / 2.0  # TF32 dense = half of bf16 dense
-        passes = 3.0 if os.environ.get("TCU_SPLIT") in ("tf32x3", "f16") else 2.0
+        split = os.environ.get("TCU_SPLIT")
+        tf32 = split in ("tf32x2", "tf32x3")
+        tensor_peak = bf16 / 2.0 if tf32 else bf16  # TF32 dense = half of bf16 dense
+        passes = 2.0 if split == "tf32x2" else 3.0
         executed = passes * flops
         achieved = executed / (gemm[1] / 1e3) / 1e12 if gemm[1] else None
         roof = {"bound": "tensor", "achieved": achieved, "peak": tensor_peak, "unit": "TFLOP/s",
                 "frac": achieved / tensor_peak if achieved else None,
                 "traffic": TF32_TRAFFIC["ratio"] * update_launch_bytes(n, nb, os.environ.get("TCU_LU_PAIRS") != "0"),
                 "traffic_note": TF32_TRAFFIC["note"],
-                "kernel": f"tf32_update_kernel: split-TF32 tcgen05 trailing update ({passes:.0f} passes executed)",
+                "kernel": f"tf32_update_kernel: split-{'TF32' if tf32 else 'FP16' if split == 'f16' else 'bfloat16'} "
+                          f"tcgen05 trailing update ({passes:.0f} passes executed)",
                 "useful_tflops": flops / (gemm[1] / 1e3) / 1e12 if gemm[1] else None,
-                "peak_note": f"TF32 dense peak = half the sustained bf16 GEMM rate, {bf16} TFLOP/s "
+                "peak_note": f"{'half ' if tf32 else ''}the sustained bf16 GEMM rate of {bf16} TFLOP/s "
                              f"(of measured: {pk.get('source')})"}
     else:
         achieved = flops / (gemm[1] / 1e3) / 1e12 if gemm[1] else None

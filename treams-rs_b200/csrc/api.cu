@@ -447,10 +447,9 @@ tcu_status factor_impl(tcu_context* ctx, int L, double k0, size_t N, const doubl
     f->n = n;
     f->precision = precision;
     f->k0 = k0;
-    // reduced: the piece formats the environment may ask for (FP16 pieces, two-pass TF32);
-    // the refinement's fallback factor takes the three-pass TF32 split instead
-    f->wk.f16_pieces = reduced && split_f16_default();
-    f->wk.two_pass = reduced && !f->wk.f16_pieces && split_two_pass_default();
+    // reduced: the default piece format or the one the environment asks for; the refinement's
+    // fallback factor takes the three-pass TF32 split instead
+    f->wk.pieces = reduced ? split_default() : PIECES_TF32X3;
     f->wk.panel_rows = ctx->panel_rows;
     auto cleanup = [&]() {
         for (void* q : {(void*)f->d_pos, (void*)f->d_radii, (void*)f->d_eps, (void*)f->d_T, f->d_A,
@@ -560,10 +559,16 @@ tcu_status factor_impl(tcu_context* ctx, int L, double k0, size_t N, const doubl
 // Refinement state of the columns of one solve in groups of 8 that converge separately: a group
 // takes another sweep while its worst relative residual is above the target, the last sweep
 // halved it and sweeps are left; afterwards its columns and their residuals stay as they are.
+// settle: a group that has met the target with less than a factor 10 to spare takes one sweep more
+// if its sweeps still gain a factor 16 each. Factors of the bfloat16 split start at a residual of 2e-7 and meet
+// 1e-13 at 6e-14 in two sweeps; the third ends at the rounding level (1e-16 to 9e-15), as the three sweeps of
+// the two-pass TF32 split (from 2e-6) do, for one product and one pair of sweeps. A line at a factor 64
+// cost adjoint solves (rounding level 7e-15) a fourth sweep: 18.8 against 16.4 ms for 17 columns each way
+// at 9600 modes.
 struct RefineGroups {
     static constexpr int WIDTH = 8;
     struct Group {
-        bool active = true;
+        bool active = true, settled = false;
         int sweeps = 1, left = 0;
         double prev = INFINITY;
     };
@@ -571,7 +576,9 @@ struct RefineGroups {
     std::vector<double> rn;  // residual norms of the columns' current solutions
     int p;
     double target;
-    RefineGroups(int p_, double target_, int max_sweeps) : g((p_ + WIDTH - 1) / WIDTH), rn(p_), p(p_), target(target_) {
+    bool settle;
+    RefineGroups(int p_, double target_, int max_sweeps, bool settle_)
+        : g((p_ + WIDTH - 1) / WIDTH), rn(p_), p(p_), target(target_), settle(settle_) {
         for (Group& q : g) q.left = max_sweeps;
     }
     size_t first(size_t q) const { return q * WIDTH; }
@@ -588,7 +595,12 @@ struct RefineGroups {
             if (!g[q].active) continue;
             for (int c = (int)first(q); c < (int)first(q) + width(q); ++c) rn[c] = r[c];
             const double w = worst(q, r, bn);
-            if (g[q].left == 0 || w <= target || !(w < 0.5 * g[q].prev)) {
+            bool stop = g[q].left == 0 || !(w < 0.5 * g[q].prev);
+            if (!stop && w <= target) {
+                stop = !settle || g[q].settled || w <= target / 10 || !(w < g[q].prev / 16);
+                g[q].settled = true;
+            }
+            if (stop) {
                 g[q].active = false;
                 continue;
             }
@@ -605,6 +617,15 @@ struct RefineGroups {
         return false;
     }
 };
+
+// most refinement sweeps of a solve: 2 on FP64 factors, 10 on mixed ones with FP32-accurate updates, 20 with
+// updates of about 2^-12 or 2^-17 a term
+int max_refinement_sweeps(const tcu_factor* f) {
+    if (f->precision != TCU_MIXED) return 2;
+    return f->wk.pieces == PIECES_TF32X2 || f->wk.pieces == PIECES_BF16 ? 20 : 10;
+}
+
+bool settles(const tcu_factor* f) { return f->precision == TCU_MIXED && f->wk.pieces == PIECES_BF16; }
 
 // device scratch of vec_norms over p columns: p norms and 256 partial sums a column
 size_t norm_scratch(int p) { return (size_t)p * 257 * sizeof(double); }
@@ -685,9 +706,8 @@ tcu_status solve_impl(tcu_factor* f, const double* B, int p, double* X, tcu_cert
     CK(cudaMemcpyAsync(x, tb, per * 16, cudaMemcpyDeviceToDevice, ctx->stream), "copy");
     lu_apply(x);
     if ((s = residual())) return s;
-    // iterative refinement in FP64: up to 10 sweeps on mixed factors (20 with two-pass updates), 2 on
-    // FP64 factors
-    RefineGroups groups(p, ctx->refine_target, f->precision == TCU_MIXED ? (f->wk.two_pass ? 20 : 10) : 2);
+    // iterative refinement in FP64
+    RefineGroups groups(p, ctx->refine_target, max_refinement_sweeps(f), settles(f));
     while (groups.advance(rn, bn)) {
         lu_apply(r);
         for (size_t g = 0; g < groups.g.size(); ++g)
@@ -699,17 +719,17 @@ tcu_status solve_impl(tcu_factor* f, const double* B, int p, double* X, tcu_cert
     }
     if (f->precision == TCU_MIXED) {
         // refinement stalled above the FP64 target (an ill-scaled operator beyond the reach of
-        // the TF32 factors): finish with an FP64 factor of the same cluster, kept for later solves
+        // the mixed factors): finish with an FP64 factor of the same cluster, kept for later solves
         if (groups.any_above(bn, ctx->fallback_above)) {
-            // FP16 pieces first fall back to a mixed factor with TF32 pieces (which keep 22
-            // bits relative to every element), that one in turn to FP64
+            // the other pieces first fall back to a mixed factor with three passes of TF32 pieces
+            // (which keep 22 bits relative to every element), that one in turn to FP64
             if (!f->fallback) {
                 std::vector<double> hr(f->N), he(2 * (size_t)f->N), hp(3 * (size_t)f->N);
                 CK(cudaMemcpyAsync(hr.data(), f->d_radii, f->N * 8, cudaMemcpyDeviceToHost, ctx->stream), "copy");
                 CK(cudaMemcpyAsync(he.data(), f->d_eps, f->N * 16, cudaMemcpyDeviceToHost, ctx->stream), "copy");
                 CK(cudaMemcpyAsync(hp.data(), f->d_pos, f->N * 24, cudaMemcpyDeviceToHost, ctx->stream), "copy");
                 if ((s = sync_status(ctx, "fallback"))) return s;
-                const bool to_tf32 = f->wk.f16_pieces || f->wk.two_pass;
+                const bool to_tf32 = f->wk.pieces != PIECES_TF32X3;
                 if ((s = factor_impl(ctx, f->L, f->k0, f->N, hr.data(), he.data(), hp.data(), nullptr, nullptr,
                                      nullptr, to_tf32 ? TCU_MIXED : TCU_FP64, &f->fallback, false)))
                     return s;
@@ -809,7 +829,7 @@ tcu_status solve_adjoint_impl(tcu_factor* f, const double* G, int p, double* Y, 
     CK(cudaMemcpyAsync(y, g, per * 16, cudaMemcpyDeviceToDevice, ctx->stream), "copy");
     lu_adjoint(y);
     if ((s = residual())) return s;
-    RefineGroups groups(p, ctx->refine_target, f->precision == TCU_MIXED ? (f->wk.two_pass ? 20 : 10) : 2);
+    RefineGroups groups(p, ctx->refine_target, max_refinement_sweeps(f), settles(f));
     while (groups.advance(rn, bn)) {
         lu_adjoint(r);
         for (size_t q = 0; q < groups.g.size(); ++q)
@@ -826,7 +846,7 @@ tcu_status solve_adjoint_impl(tcu_factor* f, const double* G, int p, double* Y, 
             CK(cudaMemcpyAsync(he.data(), f->d_eps, f->N * 16, cudaMemcpyDeviceToHost, ctx->stream), "copy");
             CK(cudaMemcpyAsync(hp.data(), f->d_pos, f->N * 24, cudaMemcpyDeviceToHost, ctx->stream), "copy");
             if ((s = sync_status(ctx, "fallback"))) return s;
-            const bool to_tf32 = f->wk.f16_pieces || f->wk.two_pass;
+            const bool to_tf32 = f->wk.pieces != PIECES_TF32X3;
             if ((s = factor_impl(ctx, f->L, f->k0, f->N, hr.data(), he.data(), hp.data(), nullptr, nullptr, nullptr,
                                  to_tf32 ? TCU_MIXED : TCU_FP64, &f->fallback, false)))
                 return s;

@@ -6,19 +6,21 @@
 // so that D[2mu+c][nu] is part c of (L21 U12)[mu][nu] and the 2m x n' result maps onto
 // the interleaved storage of A22 (real leading dimension 2n).
 //
-// Precision: every operand is split x = hi + lo into two 11-bit-significand pieces and the
-// passes accumulate in FP32 in TMEM: by default two, hi*hi + lo*hi (the B operand rounded to
-// TF32, about 2^-11 relative per term; the FP64 refinement takes one sweep more), with
-// TCU_SPLIT=tf32x3 or f16 three, hi*hi + hi*lo + lo*hi (the lo*lo term is below FP32
-// rounding). Two piece formats:
-//   FP16 (TCU_SPLIT=f16): each row of each operand (a complex row of L21, a column of U12) is
-//     first scaled by its own power of two 2^(14 - ceil log2 max|row|) (computed in the
-//     packing kernels; no host round trip), hi = f16(x s), lo = f16(x s - hi);
-//     tcgen05.mma kind::f16 runs at twice the TF32 rate and the epilogue multiplies each
-//     accumulator entry by the exact power of two 1/(s_row s_col). Pieces below the FP16
-//     normal range only lose absolute accuracy under 2^-38 of their row's maximum.
-//   TF32 (default): hi = tf32(x), lo = tf32(x - hi), tcgen05.mma kind::tf32.
-// Both give a product accurate to about 2^-22 of max|A| max|B| per term.
+// Precision: every operand is split x = hi + lo into two pieces and the passes accumulate in FP32
+// in TMEM. Formats (TCU_SPLIT):
+//   bfloat16 (default): hi = bf16(x), lo = bf16(x - hi), 16 significant bits at the FP32 exponent range;
+//     three passes hi*hi + hi*lo + lo*hi of tcgen05.mma kind::f16, the dropped lo*lo and the rounding
+//     of lo leave about 2^-17 of |a||b| per term. Twice the TF32 rate: 1.5 TF32 passes of tensor time.
+//   tf32x2: hi = tf32(x), lo = tf32(x - hi), two passes hi*hi + lo*hi of kind::tf32, the B operand rounded
+//     to TF32: about 2^-12 per term at 2 TF32 passes. 24576 modes, all updates of a factorization: 128 ms
+//     and a first residual of 2.5e-6, against 105 ms and 2.1e-7 of the bfloat16 pieces (9600 modes: 8.7 ms and
+//     1.6e-6 against 7.2 ms and 1.7e-7), and the packing kernels write half the bytes (8.1 against 7.0 ms).
+//   tf32x3: the same pieces in three passes, 2^-22 per term; the format of fallback factors.
+//   f16: each row of each operand (a complex row of L21, a column of U12) is first scaled by its own
+//     power of two 2^(14 - ceil log2 max|row|) (computed in the packing kernels; no host round trip),
+//     hi = f16(x s), lo = f16(x s - hi); three passes of kind::f16, and the epilogue multiplies each
+//     accumulator entry by the exact power of two 1/(s_row s_col). Pieces below the FP16 normal
+//     range only lose absolute accuracy under 2^-38 of their row's maximum.
 //
 // Kernel layout (persistent, one CTA per SM, 192 threads):
 //   warp 0     TMA producer: 64-byte-swizzled boxes (64-byte K rows) of the four packed
@@ -33,6 +35,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -150,9 +153,9 @@ __device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t a, uint64_t b,
         "l"(a), "l"(b), "r"(idesc), "r"(acc)
         : "memory");
 }
-template <bool F16>
+template <bool HALF>
 __device__ __forceinline__ void mma_split(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
-    if (F16)
+    if (HALF)
         mma_f16(d_tmem, a, b, idesc, acc);
     else
         mma_tf32(d_tmem, a, b, idesc, acc);
@@ -200,12 +203,16 @@ struct Tf32Args {
     const float* sB;      // FP16 pieces: scale of each row of the B operand (ncols)
 };
 
-template <bool F16, bool TWO>
+template <int PIECES>
 __global__ void __launch_bounds__(192, 1) tf32_update_kernel(const __grid_constant__ CUtensorMap mAhi,
                                                              const __grid_constant__ CUtensorMap mAlo,
                                                              const __grid_constant__ CUtensorMap mBhi,
                                                              const __grid_constant__ CUtensorMap mBlo,
                                                              const __grid_constant__ CUtensorMap mC, Tf32Args args) {
+    // 2-byte pieces (kind::f16), rows with scales, two passes
+    constexpr bool HALF = PIECES == PIECES_F16 || PIECES == PIECES_BF16, F16 = PIECES == PIECES_F16;
+    constexpr bool TWO = PIECES == PIECES_TF32X2;
+    constexpr int KC = HALF ? 2 * TB_K : TB_K;  // K elements of a chunk (64 bytes)
     extern __shared__ uint8_t smem_raw[];
     uint32_t base = smem_u32(smem_raw);
     uint32_t tiles_smem = (base + 1023u) & ~1023u;  // 1024-byte aligned stage ring
@@ -252,10 +259,10 @@ __global__ void __launch_bounds__(192, 1) tf32_update_kernel(const __grid_consta
                     if (!mbar_wait(bar(EMPTY + s), ph ^ 1, abort_flag)) break;
                     uint32_t st = tiles_smem + s * STAGE_BYTES;
                     mbar_expect_tx(bar(s), TWO ? STAGE_BYTES - B_BYTES : STAGE_BYTES);
-                    tma_load_2d(st, &mAhi, kb * TB_K, tm * TB_M, bar(s));
-                    tma_load_2d(st + A_BYTES, &mAlo, kb * TB_K, tm * TB_M, bar(s));
-                    tma_load_2d(st + 2 * A_BYTES, &mBhi, kb * TB_K, tn * TB_N, bar(s));
-                    if (!TWO) tma_load_2d(st + 2 * A_BYTES + B_BYTES, &mBlo, kb * TB_K, tn * TB_N, bar(s));
+                    tma_load_2d(st, &mAhi, kb * KC, tm * TB_M, bar(s));
+                    tma_load_2d(st + A_BYTES, &mAlo, kb * KC, tm * TB_M, bar(s));
+                    tma_load_2d(st + 2 * A_BYTES, &mBhi, kb * KC, tn * TB_N, bar(s));
+                    if (!TWO) tma_load_2d(st + 2 * A_BYTES + B_BYTES, &mBlo, kb * KC, tn * TB_N, bar(s));
                 }
             }
             if (*abort_flag) {
@@ -269,8 +276,8 @@ __global__ void __launch_bounds__(192, 1) tf32_update_kernel(const __grid_consta
         }
     } else if (warp == 1) {
         if (lane == 0) {
-            // D F32; A, B TF32 (2) or F16 (0); K-major; N >> 3 at bit 17, M >> 4 at bit 24
-            const uint32_t ab = F16 ? 0u : 2u;
+            // D F32; A, B TF32 (2), BF16 (1) or F16 (0); K-major; N >> 3 at bit 17, M >> 4 at bit 24
+            const uint32_t ab = F16 ? 0u : (HALF ? 1u : 2u);
             const uint32_t idesc = (1u << 4) | (ab << 7) | (ab << 10) | ((uint32_t)(TB_N >> 3) << 17) |
                                    ((uint32_t)(TB_M >> 4) << 24);
             int step = 0, it = 0;
@@ -296,9 +303,9 @@ __global__ void __launch_bounds__(192, 1) tf32_update_kernel(const __grid_consta
                         uint64_t bhi = swz_desc(st + 2 * A_BYTES + ks * 32);
                         uint64_t blo = swz_desc(st + 2 * A_BYTES + B_BYTES + ks * 32);
                         uint32_t first = (kb == 0 && ks == 0) ? 0u : 1u;
-                        mma_split<F16>(d, ahi, bhi, idesc, first);
-                        if (!TWO) mma_split<F16>(d, ahi, blo, idesc, 1u);
-                        mma_split<F16>(d, alo, bhi, idesc, 1u);
+                        mma_split<HALF>(d, ahi, bhi, idesc, first);
+                        if (!TWO) mma_split<HALF>(d, ahi, blo, idesc, 1u);
+                        mma_split<HALF>(d, alo, bhi, idesc, 1u);
                     }
                     mma_commit(bar(EMPTY + s));
                 }
@@ -432,6 +439,50 @@ __global__ void pack_u_kernel(const float2* __restrict__ A, size_t lda, int r0, 
     if (lo) *(float2*)(lo + o) = make_float2(rl, il);
 }
 
+// The same operands as bfloat16 pieces (kp multiple of 32; K of any number of panels).
+__device__ __forceinline__ void split_bf16(float x, __nv_bfloat16& hi, __nv_bfloat16& lo) {
+    hi = __float2bfloat16_rn(x);
+    lo = __float2bfloat16_rn(x - __bfloat162float(hi));
+}
+__global__ void pack_l_bf16_kernel(const float2* __restrict__ A, size_t lda, int r0, int k0, int m, int w, int kp,
+                                   __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo) {
+    __shared__ float2 tile[32][33];
+    const int mu0 = blockIdx.x * 32, k00 = blockIdx.y * 32;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
+    for (int r = ty; r < 32; r += 8) {
+        const int kk = k00 + r, mu = mu0 + tx;
+        tile[r][tx] = (kk < w && mu < m) ? A[(size_t)(k0 + kk) * lda + r0 + mu] : make_float2(0.f, 0.f);
+    }
+    __syncthreads();
+    for (int r = ty; r < 32; r += 8) {
+        const int mu = mu0 + r, kk = k00 + tx;
+        if (mu >= m || 2 * kk >= kp) continue;
+        const float2 l = tile[tx][r];
+        __nv_bfloat16 rh, rl, ih, il;
+        split_bf16(l.x, rh, rl);
+        split_bf16(l.y, ih, il);
+        const size_t o0 = (size_t)(2 * mu) * kp + 2 * kk, o1 = o0 + kp;
+        *(__nv_bfloat162*)(hi + o0) = __halves2bfloat162(rh, __hneg(ih));
+        *(__nv_bfloat162*)(hi + o1) = __halves2bfloat162(ih, rh);
+        *(__nv_bfloat162*)(lo + o0) = __halves2bfloat162(rl, __hneg(il));
+        *(__nv_bfloat162*)(lo + o1) = __halves2bfloat162(il, rl);
+    }
+}
+__global__ void pack_u_bf16_kernel(const float2* __restrict__ A, size_t lda, int r0, int k0, int ncols, int w, int kp,
+                                   __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo) {
+    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int half = kp / 2;
+    if (t >= (size_t)ncols * half) return;
+    const int nu = (int)(t / half), kk = (int)(t % half);
+    const float2 u = kk < w ? A[(size_t)(r0 + nu) * lda + k0 + kk] : make_float2(0.f, 0.f);
+    __nv_bfloat16 rh, rl, ih, il;
+    split_bf16(u.x, rh, rl);
+    split_bf16(u.y, ih, il);
+    const size_t o = (size_t)nu * kp + 2 * kk;
+    *(__nv_bfloat162*)(hi + o) = __halves2bfloat162(rh, ih);
+    *(__nv_bfloat162*)(lo + o) = __halves2bfloat162(rl, il);
+}
+
 // x <- -x over hi and lo halves (2 count floats starting at p, contiguous)
 __global__ void negate_kernel(float* __restrict__ p, size_t count) {
     size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -541,17 +592,20 @@ static EncodeTiled encoder() {
     return fn;
 }
 
-// K-major operand of `rows` rows of kp elements (4-byte TF32 pieces or 2-byte FP16 pieces);
+// K-major operand of `rows` rows of kp elements (4-byte TF32 pieces or 2-byte FP16 or bfloat16 pieces);
 // boxes are one 64-byte swizzle row deep (16 or 32 elements).
-static bool make_map(CUtensorMap* map, void* base, int rows, int kp, int box_rows, bool f16) {
+static bool make_map(CUtensorMap* map, void* base, int rows, int kp, int box_rows, PieceFormat pieces) {
     EncodeTiled enc = encoder();
     if (!enc) return false;
-    const int eb = f16 ? 2 : 4;
+    const int eb = pieces == PIECES_F16 || pieces == PIECES_BF16 ? 2 : 4;
+    const CUtensorMapDataType type = pieces == PIECES_F16    ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
+                                     : pieces == PIECES_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
+                                                             : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
     cuuint64_t dims[2] = {(cuuint64_t)kp, (cuuint64_t)rows};
     cuuint64_t strides[1] = {(cuuint64_t)kp * eb};
     cuuint32_t box[2] = {(cuuint32_t)(64 / eb), (cuuint32_t)box_rows};
     cuuint32_t estr[2] = {1, 1};
-    return enc(map, f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, base, dims, strides, box,
+    return enc(map, type, 2, base, dims, strides, box,
                estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
@@ -559,29 +613,19 @@ static bool make_map(CUtensorMap* map, void* base, int rows, int kp, int box_row
 __global__ void tri_inverse_l_kernel(const float2* __restrict__ A, size_t lda, int k0, int w, float2* __restrict__ N);
 constexpr size_t TI_SMEM = (size_t)(128 * 129 + 64 * 64) * sizeof(float2);
 
-// TF32 pieces by default; FP16 pieces (twice the tensor rate) with TCU_SPLIT=f16. On the
-// cluster operators measured here the entries of one row of L21 or one column of U12 span
-// more than 2^20 even after equilibration, and FP16 pieces (8 exponent bits fewer) then leave
-// the FP64 refinement stalled, so every solve fell back to TF32 pieces.
-// Two passes hi*hi + lo*hi (the B operand, U12, rounded to TF32) unless TCU_SPLIT asks for
-// three TF32 passes (tf32x3) or FP16 pieces (f16): a third fewer tensor-core passes and no B lo
-// loads, for an update accurate to about 2^-11 relative to max|A| max|B| per term. The FP64
-// refinement then takes one sweep more (512 spheres lmax 4: 3 instead of 2, factor 279 instead
-// of 320 ms), and a stall falls back to the three-pass factor.
-bool split_two_pass_default() {
-    static const bool on = [] {
+// bfloat16 pieces are the fastest and as accurate as FP32 panels allow (see the top). FP16 pieces reach the
+// same residuals, but their epilogue divides every entry by its scales and they keep one update per panel:
+// 380 ms of updates at 24576 modes. A refinement that stalls on any other format falls back to a three-pass
+// TF32 factor.
+PieceFormat split_default() {
+    static const PieceFormat f = [] {
         const char* e = getenv("TCU_SPLIT");
-        return !(e && (std::strcmp(e, "tf32x3") == 0 || std::strcmp(e, "f16") == 0));
+        if (e && std::strcmp(e, "tf32x3") == 0) return PIECES_TF32X3;
+        if (e && std::strcmp(e, "tf32x2") == 0) return PIECES_TF32X2;
+        if (e && std::strcmp(e, "f16") == 0) return PIECES_F16;
+        return PIECES_BF16;
     }();
-    return on;
-}
-
-bool split_f16_default() {
-    static const bool on = [] {
-        const char* e = getenv("TCU_SPLIT");
-        return e && std::strcmp(e, "f16") == 0;
-    }();
-    return on;
+    return f;
 }
 
 bool tf32_enabled() {
@@ -592,11 +636,13 @@ bool tf32_enabled() {
     if (on == 1) {
         static PerDeviceOnce attr;
         once_per_device(attr, [] {
-            cudaFuncSetAttribute(tf32_update_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            cudaFuncSetAttribute(tf32_update_kernel<PIECES_TF32X3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)TF32_SMEM);
-            cudaFuncSetAttribute(tf32_update_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            cudaFuncSetAttribute(tf32_update_kernel<PIECES_TF32X2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)TF32_SMEM);
-            cudaFuncSetAttribute(tf32_update_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            cudaFuncSetAttribute(tf32_update_kernel<PIECES_F16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)TF32_SMEM);
+            cudaFuncSetAttribute(tf32_update_kernel<PIECES_BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)TF32_SMEM);
             cudaFuncSetAttribute(tri_inverse_l_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TI_SMEM);
         });
@@ -706,14 +752,14 @@ static bool ensure_pack(LuWork& wk, size_t need, cudaStream_t st) {
 }
 
 // C[row0 .. row0+m2) x [col0 .. col0+ncols) -= Apack (m2 x kp) * Bpack (ncols x kp)^T;
-// sA != null selects FP16 pieces (row scales sA of the A operand, sB of the B operand).
+// FP16 pieces have the row scales sA of the A operand, sB of the B operand.
 static void run_gemm(float2* A, int n, int row0, int col0, int m2, int ncols, int kp, void* ahi, void* alo, void* bhi,
                      void* blo, const float* sA, const float* sB, LuWork& wk, cudaStream_t st, long long* launches,
-                     bool two = false) {
-    const bool f16 = sA != nullptr;
+                     PieceFormat pieces) {
+    const bool half = pieces == PIECES_F16 || pieces == PIECES_BF16;
     CUtensorMap mAhi, mAlo, mBhi, mBlo;
-    bool ok = make_map(&mAhi, ahi, m2, kp, TB_M, f16) && make_map(&mAlo, alo, m2, kp, TB_M, f16) &&
-              make_map(&mBhi, bhi, ncols, kp, TB_N, f16) && make_map(&mBlo, blo, ncols, kp, TB_N, f16);
+    bool ok = make_map(&mAhi, ahi, m2, kp, TB_M, pieces) && make_map(&mAlo, alo, m2, kp, TB_M, pieces) &&
+              make_map(&mBhi, bhi, ncols, kp, TB_N, pieces) && make_map(&mBlo, blo, ncols, kp, TB_N, pieces);
     // A viewed as a 2n x n float matrix (column-major): box of 128 real rows x 64 columns
     CUtensorMap mC;
     {
@@ -737,7 +783,7 @@ static void run_gemm(float2* A, int n, int row0, int col0, int m2, int ncols, in
     a.col0 = col0;
     a.m2 = m2;
     a.ncols = ncols;
-    a.kchunks = kp / (f16 ? 32 : TB_K);
+    a.kchunks = kp / (half ? 32 : TB_K);
     a.tiles_m = (m2 + TB_M - 1) / TB_M;
     a.tiles_n = (ncols + TB_N - 1) / TB_N;
     a.tiles = a.tiles_m * a.tiles_n;
@@ -745,12 +791,13 @@ static void run_gemm(float2* A, int n, int row0, int col0, int m2, int ncols, in
     a.sA = sA;
     a.sB = sB;
     int grid = std::min(num_sms(), a.tiles);
-    if (f16)
-        tf32_update_kernel<true, false><<<grid, 192, TF32_SMEM, st>>>(mAhi, mAlo, mBhi, mBlo, mC, a);
-    else if (two)
-        tf32_update_kernel<false, true><<<grid, 192, TF32_SMEM, st>>>(mAhi, mAlo, mBhi, mBlo, mC, a);
-    else
-        tf32_update_kernel<false, false><<<grid, 192, TF32_SMEM, st>>>(mAhi, mAlo, mBhi, mBlo, mC, a);
+    auto launch = [&](auto kernel) { kernel<<<grid, 192, TF32_SMEM, st>>>(mAhi, mAlo, mBhi, mBlo, mC, a); };
+    switch (pieces) {
+        case PIECES_BF16: launch(tf32_update_kernel<PIECES_BF16>); break;
+        case PIECES_F16: launch(tf32_update_kernel<PIECES_F16>); break;
+        case PIECES_TF32X2: launch(tf32_update_kernel<PIECES_TF32X2>); break;
+        default: launch(tf32_update_kernel<PIECES_TF32X3>); break;
+    }
     *launches += 1;
 }
 
@@ -783,7 +830,7 @@ bool launch_tf32_trsm_inverse(float2* A, int n, int k0, int w, LuWork& wk, cudaS
 // inverse of L11 (which it does not need); launch_tf32_trsm(..., rhs_packed = true) then skips
 // it. FP16 pieces keep their packing in launch_tf32_trsm (false here).
 bool launch_tf32_trsm_rhs(float2* A, int n, int k0, int w, LuWork& wk, cudaStream_t st, long long* launches) {
-    if (wk.f16_pieces) return false;
+    if (wk.pieces == PIECES_F16) return false;
     int r0 = k0 + w, ncols = n - r0, kp;
     if (ncols <= 0 || !trsm_buffers(n, k0, w, wk, st, &kp)) return false;
     float* bhi = (float*)wk.pack + (size_t)4 * w * kp;
@@ -816,7 +863,7 @@ void launch_tf32_trsm(float2* A, int n, int k0, int w, LuWork& wk, cudaStream_t 
         }
         dim3 g1((w + 31) / 32, (kp / 2 + 31) / 32);
         size_t tot = (size_t)ncols * (kp / 2);
-        if (wk.f16_pieces) {
+        if (wk.pieces == PIECES_F16) {
             // A operand: -N embedded, so that the update C -= (-N) A12 adds N A12
             __half *h_ahi = (__half*)ahi, *h_alo = h_ahi + (size_t)2 * w * kp;
             __half *h_bhi = h_alo + (size_t)2 * w * kp, *h_blo = h_bhi + (size_t)ncols * kp;
@@ -825,7 +872,8 @@ void launch_tf32_trsm(float2* A, int n, int k0, int w, LuWork& wk, cudaStream_t 
             pack_l16_kernel<<<(w + 31) / 32, 256, 0, st>>>(Nm, (size_t)w, 0, 0, w, w, kp, -1.0f, h_ahi, h_alo, sA);
             pack_u16_kernel<<<(unsigned)(((size_t)ncols * 32 + 255) / 256), 256, 0, st>>>(A, (size_t)n, r0, k0, ncols, w,
                                                                                          kp, h_bhi, h_blo, sB);
-            run_gemm(A, n, 2 * k0, r0, 2 * w, ncols, kp, h_ahi, h_alo, h_bhi, h_blo, sA, sB, wk, st, launches);
+            run_gemm(A, n, 2 * k0, r0, 2 * w, ncols, kp, h_ahi, h_alo, h_bhi, h_blo, sA, sB, wk, st, launches,
+                     PIECES_F16);
             *launches += 3;
         } else {
             pack_l_kernel<<<g1, 256, 0, st>>>(Nm, (size_t)w, 0, 0, w, w, kp, ahi, alo);
@@ -835,7 +883,8 @@ void launch_tf32_trsm(float2* A, int n, int k0, int w, LuWork& wk, cudaStream_t 
                 ++*launches;
             }
             negate_kernel<<<(unsigned)(((size_t)4 * w * kp + 255) / 256), 256, 0, st>>>(ahi, (size_t)4 * w * kp);
-            run_gemm(A, n, 2 * k0, r0, 2 * w, ncols, kp, ahi, alo, bhi, blo, nullptr, nullptr, wk, st, launches);
+            run_gemm(A, n, 2 * k0, r0, 2 * w, ncols, kp, ahi, alo, bhi, blo, nullptr, nullptr, wk, st, launches,
+                     PIECES_TF32X3);
             *launches += 3;
         }
     }
@@ -853,14 +902,20 @@ void launch_tf32_update_region(float2* A, int n, int k0, int w, int r0, int m, i
     float* alo = ahi + (size_t)2 * m * kp;
     float* bhi = alo + (size_t)2 * m * kp;
     float* blo = bhi + (size_t)ncols * kp;
-    const bool f16 = wk.f16_pieces;
     __half *h_ahi = (__half*)ahi, *h_alo = h_ahi + (size_t)2 * m * kp;
     __half *h_bhi = h_alo + (size_t)2 * m * kp, *h_blo = h_bhi + (size_t)ncols * kp;
     float* sA = (float*)(((uintptr_t)(h_blo + (size_t)ncols * kp) + 255) & ~(uintptr_t)255);
     float* sB = (float*)(((uintptr_t)(sA + m) + 255) & ~(uintptr_t)255);
     {
         StageScope sc(ST_PACK, st);
-        if (f16) {
+        if (wk.pieces == PIECES_BF16) {
+            const dim3 g1((m + 31) / 32, (kp / 2 + 31) / 32);
+            const size_t tot = (size_t)ncols * (kp / 2);
+            pack_l_bf16_kernel<<<g1, 256, 0, st>>>(A, (size_t)n, r0, k0, m, w, kp, (__nv_bfloat16*)h_ahi,
+                                                   (__nv_bfloat16*)h_alo);
+            pack_u_bf16_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(
+                A, (size_t)n, c0, k0, ncols, w, kp, (__nv_bfloat16*)h_bhi, (__nv_bfloat16*)h_blo);
+        } else if (wk.pieces == PIECES_F16) {
             pack_l16_kernel<<<(m + 31) / 32, 256, 0, st>>>(A, (size_t)n, r0, k0, m, w, kp, 1.0f, h_ahi, h_alo, sA);
             pack_u16_kernel<<<(unsigned)(((size_t)ncols * 32 + 255) / 256), 256, 0, st>>>(A, (size_t)n, c0, k0, ncols, w,
                                                                                          kp, h_bhi, h_blo, sB);
@@ -869,16 +924,15 @@ void launch_tf32_update_region(float2* A, int n, int k0, int w, int r0, int m, i
             size_t tot = (size_t)ncols * (kp / 2);
             pack_l_kernel<<<g1, 256, 0, st>>>(A, (size_t)n, r0, k0, m, w, kp, ahi, alo);
             pack_u_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(A, (size_t)n, c0, k0, ncols, w, kp, bhi,
-                                                                         wk.two_pass ? nullptr : blo);
+                                                                         wk.pieces == PIECES_TF32X2 ? nullptr : blo);
         }
         *launches += 2;
     }
     StageScope sc(ST_GEMM, st);
-    if (f16)
-        run_gemm(A, n, 2 * r0, c0, 2 * m, ncols, kp, h_ahi, h_alo, h_bhi, h_blo, sA, sB, wk, st, launches);
+    if (wk.pieces == PIECES_BF16 || wk.pieces == PIECES_F16)
+        run_gemm(A, n, 2 * r0, c0, 2 * m, ncols, kp, h_ahi, h_alo, h_bhi, h_blo, sA, sB, wk, st, launches, wk.pieces);
     else
-        run_gemm(A, n, 2 * r0, c0, 2 * m, ncols, kp, ahi, alo, bhi, blo, nullptr, nullptr, wk, st, launches,
-                 wk.two_pass);
+        run_gemm(A, n, 2 * r0, c0, 2 * m, ncols, kp, ahi, alo, bhi, blo, nullptr, nullptr, wk, st, launches, wk.pieces);
 }
 
 void launch_tf32_update(float2* A, int n, int k0, int w, LuWork& wk, cudaStream_t st, long long* launches) {

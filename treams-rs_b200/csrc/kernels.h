@@ -287,6 +287,9 @@ void launch_array_solve(const DevPlan& P, const double2* D, size_t ldd, const do
 
 // lu.cu — dense LU of an n x n column-major complex matrix (lda = n) in FP64 (double2)
 // or FP32 (float2) storage, row permutation kept as perm (row i of P A is row perm[i]).
+// Operand pieces of the mixed path's trailing updates (gemm_tf32.cu): three passes of bfloat16, of FP16
+// (scaled rows) or of TF32 pieces, or two of TF32
+enum PieceFormat { PIECES_TF32X3, PIECES_TF32X2, PIECES_F16, PIECES_BF16 };
 struct LuWork {
     int* piv = nullptr;        // n
     int* perm = nullptr;       // n
@@ -295,14 +298,11 @@ struct LuWork {
     void* cand = nullptr;      // candidate values/rows, double-buffered
     void* pack = nullptr;      // packed GEMM operands (mixed path)
     size_t pack_bytes = 0;
-    bool f16_pieces = false;   // mixed path: FP16 (true) or TF32 (false) pieces of the 3-pass split
-    bool two_pass = false;     // mixed path: two-pass TF32 trailing updates (B operand rounded to TF32)
+    PieceFormat pieces = PIECES_BF16;  // mixed path: the split of the trailing updates' operands
     int panel_rows = 0;        // least rows per panel CTA (0: TCU_PANEL_ROWS or 32)
 };
-// FP16 pieces when the environment asks for them (TCU_SPLIT=f16), else TF32 pieces
-bool split_f16_default();
-// Two-pass TF32 trailing updates unless the environment asks for three passes or FP16 pieces
-bool split_two_pass_default();
+// bfloat16 unless TCU_SPLIT names another format (tf32x3, tf32x2, f16)
+PieceFormat split_default();
 int lu_factor_fp64(double2* A, int n, LuWork& w, cudaStream_t st, long long* launches);
 // The panel's grid barrier with one arrival missing (bar: a zeroed counter); it gives up
 // after limit_s (clamped to [0, 4] s) and records status 8.

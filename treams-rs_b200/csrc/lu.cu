@@ -12,7 +12,7 @@
 //  3. U12 = L11^-1 A12: trsm_kernel (FP64, one warp per column), or in the mixed path the
 //     blocked inverse of L11 (tri_inverse_l_kernel) and a tensor-core GEMM (gemm_tf32.cu).
 //  4. trailing update A22 -= L21 U12: FP64 DMMA (mma.sync m8n8k4 f64) complex GEMM, or in
-//     the mixed path the 3-pass split tcgen05 GEMM of gemm_tf32.cu.
+//     the mixed path the split tcgen05 GEMM of gemm_tf32.cu (three bfloat16 passes).
 // The triangular solves with the factors are in solve.cu.
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -850,7 +850,7 @@ static int lu_factor_impl(typename Cx<R>::T* A, int n, LuWork& wk, cudaStream_t 
     // flags of the cluster panels' words: epochs 1 .. n
     cudaMemsetAsync(panel_words(wk), 0, (PC_GKEY + PC_GROW) * sizeof(uint4), st);
     // (the FP16-piece packers hold one 128-column panel, so FP16 pieces keep one update per panel)
-    const bool pairs = sizeof(R) == 4 && tensor_cores && !wk.f16_pieces && lu_pairs_enabled();
+    const bool pairs = sizeof(R) == 4 && tensor_cores && wk.pieces != PIECES_F16 && lu_pairs_enabled();
     int pend_k0 = -1, pend_w = 0;  // panel a whose update right of panel b is still pending
     for (int k0 = 0; k0 < n; k0 += NB) {
         int w = std::min(NB, n - k0);

@@ -378,7 +378,7 @@ def sphere_cluster_factor(lmax: int, k0: float, radii, eps, positions, precision
                           ctx: Context | None = None) -> InteractionFactor:
     """Assemble and factor I - T C (cluster::sphere_cluster_factor, cluster/spheres.rs:85).
 
-    precision "fp64" is the plain drop-in; "mixed" factors in complex64 with split-TF32
+    precision "fp64" is the plain drop-in; "mixed" factors in complex64 with split-bfloat16
     tensor-core updates and refines every solve in FP64."""
     ctx = ctx or default_context()
     prec = {"fp64": FP64, "mixed": MIXED}.get(precision, precision)
