@@ -483,12 +483,6 @@ __global__ void pack_u_bf16_kernel(const float2* __restrict__ A, size_t lda, int
     *(__nv_bfloat162*)(lo + o) = __halves2bfloat162(rl, il);
 }
 
-// x <- -x over hi and lo halves (2 count floats starting at p, contiguous)
-__global__ void negate_kernel(float* __restrict__ p, size_t count) {
-    size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < count) p[t] = -p[t];
-}
-
 // ---- FP16 pieces -----------------------------------------------------------------------
 // Every row of the A operand (complex row mu of L21, both its real rows) and every row of the
 // B operand (column nu of U12) gets its own power-of-two scale f16_scale(max over its K
@@ -610,8 +604,11 @@ static bool make_map(CUtensorMap* map, void* base, int rows, int kp, int box_row
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-__global__ void tri_inverse_l_kernel(const float2* __restrict__ A, size_t lda, int k0, int w, float2* __restrict__ N);
-constexpr size_t TI_SMEM = (size_t)(128 * 129 + 64 * 64) * sizeof(float2);
+constexpr int TI_W = 128, TI_LD = TI_W + 1;  // order of L11, its row pitch
+constexpr int TI_S = 16, TI_C = 8;           // rows of a block, columns of the inverse per CTA
+constexpr size_t TI_SMEM = (size_t)(TI_W * TI_LD + TI_W * (TI_S + 1) + (TI_W + TI_S) * TI_C) * sizeof(float2);
+__global__ void tri_inverse_l_kernel(const float2* __restrict__ A, size_t lda, int k0, float* __restrict__ hi,
+                                     float* __restrict__ lo, float2* __restrict__ N);
 
 // bfloat16 pieces are the fastest and as accurate as FP32 panels allow (see the top). FP16 pieces reach the
 // same residuals, but their epilogue divides every entry by its scales and they keep one update per panel:
@@ -650,81 +647,102 @@ bool tf32_enabled() {
     return on == 1;
 }
 
-// N = L11^-1 - I for the unit lower w x w (w <= 128) diagonal block of the panel, in FP32
-// in shared memory, by recursive doubling: the eight 16 x 16 diagonal blocks are inverted
-// by one warp each (columns right to left), then pairs of inverted blocks [A 0; B C] are
-// joined level by level (s = 16, 32, 64) with the lower-left block -C^-1 B A^-1 formed as
-// two small dense products. M holds the strictly lower part; unit diagonals are implicit.
-// Stored column-major w x w. U12 = L11^-1 A12 = A12 + N A12 then runs on the tensor cores.
-__device__ __forceinline__ float2 cmulf(float2 a, float2 b) {
-    return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+// N = L11^-1 - I for the unit lower 128 x 128 diagonal block of a panel, in FP32: one CTA per 8 columns of
+// the inverse, none waiting for another. Each inverts the 16 x 16 diagonal blocks it needs (a warp per block,
+// a lane per row and 8 columns) and substitutes downwards block by block, X_i = L_ii^-1 R_i, R -= L_:i X_i,
+// with R in registers (a thread per row and 4 columns): one shared-memory load of L serves four products.
+// U12 = L11^-1 A12 = A12 + N A12 then runs on the tensor cores: hi/lo receive the TF32 pieces of -N,
+// embedded as in pack_l_kernel, and N (where not null) the matrix, column-major.
+// A chain of 16 short steps bounds it. One CTA that joined inverted blocks at 16, 32 and 64 rows read two
+// operands from shared memory per product: 50 us against 13, and packing and negating took two more launches.
+__device__ __forceinline__ void fmac(float2& s, float2 a, float2 b) {
+    s.x += a.x * b.x - a.y * b.y;
+    s.y += a.x * b.y + a.y * b.x;
 }
-__global__ void __launch_bounds__(1024) tri_inverse_l_kernel(const float2* __restrict__ A, size_t lda, int k0, int w,
+__global__ void __launch_bounds__(256) tri_inverse_l_kernel(const float2* __restrict__ A, size_t lda, int k0,
+                                                            float* __restrict__ hi, float* __restrict__ lo,
                                                             float2* __restrict__ N) {
-    extern __shared__ float2 ti_smem[];
-    const int LD = 129;
-    float2* M = ti_smem;             // M[i * LD + k], 128 x 128
-    float2* T = ti_smem + 128 * LD;  // 64 x 64 scratch
+    extern __shared__ __align__(16) float2 ti_smem[];
+    float2* X = ti_smem;               // this CTA's columns of the inverse, X[i * TI_C + c]
+    float2* S = X + TI_W * TI_C;       // R of the block in turn
+    float2* M = S + TI_S * TI_C;       // L11, M[i * TI_LD + k], i > k
+    float2* D = M + TI_W * TI_LD;      // inverted diagonal blocks, D[i * (TI_S + 1) + m], i < 128
+    const int o = blockIdx.x * TI_C, b0 = o / TI_S;  // first column, first block
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int idx = tid; idx < 128 * 128; idx += blockDim.x) {
-        int i = idx % 128, k = idx / 128;
-        M[i * LD + k] = (i > k && i < w && k < w) ? A[(size_t)(k0 + k) * lda + k0 + i] : make_float2(0.f, 0.f);
-    }
+    const int row = tid & (TI_W - 1), g = tid >> 7;  // this thread's R: columns 4 g .. 4 g + 3 of the row
+    for (int k = b0 * TI_S + g; k < row; k += 2)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(&M[row * TI_LD + k])),
+                     "l"(A + (size_t)(k0 + k) * lda + k0 + row)
+                     : "memory");
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    // 16 x 16 diagonal blocks: X[i][j] = -sum_{k=j+1..i} X[i][k] L[k][j], X[i][i] = 1
-    if (warp < 8) {  // one warp per 16 x 16 block; the other warps join at the next barrier
-        __shared__ float2 colbuf[8][16];
-        const int o = warp * 16;
-        for (int j = 14; j >= 0; --j) {
-            if (lane < 16) colbuf[warp][lane] = M[(o + lane) * LD + o + j];
-            __syncwarp();
-            if (lane < 16 && lane > j) {
-                int i = lane;
-                float2 sum = colbuf[warp][i];  // k = i term
-                for (int k = j + 1; k < i; ++k) {
-                    float2 l = colbuf[warp][k], x = M[(o + i) * LD + o + k];
-                    sum.x += x.x * l.x - x.y * l.y;
-                    sum.y += x.x * l.y + x.y * l.x;
-                }
-                M[(o + i) * LD + o + j] = make_float2(-sum.x, -sum.y);
+    if (warp >= b0) {
+        const int d = warp * TI_S, r = lane & 15, c0 = (lane >> 4) * 8;
+        float2 x[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) x[u] = make_float2(r == c0 + u ? 1.0f : 0.0f, 0.0f);
+#pragma unroll 1
+        for (int k = 0; k < TI_S - 1; ++k) {
+            float2 l = make_float2(0.0f, 0.0f);
+            if (r > k) l = M[(d + r) * TI_LD + d + k];
+            l.x = -l.x;
+            l.y = -l.y;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const float2 xk = make_float2(__shfl_sync(0xffffffffu, x[u].x, k, 16),
+                                              __shfl_sync(0xffffffffu, x[u].y, k, 16));
+                fmac(x[u], l, xk);
             }
-            __syncwarp();
         }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) D[(d + r) * (TI_S + 1) + c0 + u] = x[u];
     }
-    __syncthreads();
-    // join pairs: [A 0; B C]^-1 lower-left = -Cinv (B Ainv)
-    for (int s = 16; s < 128; s *= 2) {
-        const int pairs = 128 / (2 * s);
-        // T = B Ainv for every pair (pair p stores at T + p * s * s)
-        for (int idx = tid; idx < pairs * s * s; idx += blockDim.x) {
-            int p = idx / (s * s), e = idx % (s * s), i = e / s, k = e % s;
-            int a0 = p * 2 * s, c0 = a0 + s;
-            float2 sum = M[(c0 + i) * LD + a0 + k];  // m = k, Ainv diagonal 1
-            for (int m = k + 1; m < s; ++m) {
-                float2 b = M[(c0 + i) * LD + a0 + m], x = M[(a0 + m) * LD + a0 + k];
-                sum.x += b.x * x.x - b.y * x.y;
-                sum.y += b.x * x.y + b.y * x.x;
-            }
-            T[p * s * s + i * s + k] = sum;
+    float2 R[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) R[u] = make_float2(row == o + 4 * g + u ? 1.0f : 0.0f, 0.0f);
+    const int pr = tid >> 4, pc = (tid >> 1) & 7, ph = tid & 1;  // product: row, column, half of the sum
+#pragma unroll 1
+    for (int b = b0; b < TI_W / TI_S; ++b) {
+        if (row >> 4 == b) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) S[(row & 15) * TI_C + 4 * g + u] = R[u];
         }
         __syncthreads();
-        // lower-left = -(Cinv T)
-        for (int idx = tid; idx < pairs * s * s; idx += blockDim.x) {
-            int p = idx / (s * s), e = idx % (s * s), i = e / s, k = e % s;
-            int a0 = p * 2 * s, c0 = a0 + s;
-            float2 sum = T[p * s * s + i * s + k];  // m = i, Cinv diagonal 1
-            for (int m = 0; m < i; ++m) {
-                float2 c = M[(c0 + i) * LD + c0 + m], t = T[p * s * s + m * s + k];
-                sum.x += c.x * t.x - c.y * t.y;
-                sum.y += c.x * t.y + c.y * t.x;
-            }
-            M[(c0 + i) * LD + a0 + k] = make_float2(-sum.x, -sum.y);
-        }
+        float2 s = make_float2(0.0f, 0.0f);
+#pragma unroll
+        for (int m = 0; m < 8; ++m) fmac(s, D[(b * TI_S + pr) * (TI_S + 1) + ph * 8 + m], S[(ph * 8 + m) * TI_C + pc]);
+        s.x += __shfl_xor_sync(0xffffffffu, s.x, 1);
+        s.y += __shfl_xor_sync(0xffffffffu, s.y, 1);
+        if (ph == 0) X[(b * TI_S + pr) * TI_C + pc] = s;
         __syncthreads();
+        if (row >> 4 > b) {
+#pragma unroll
+            for (int k = 0; k < TI_S; ++k) {
+                float2 l = M[row * TI_LD + b * TI_S + k];
+                l.x = -l.x;
+                l.y = -l.y;
+                const float4 x01 = *(const float4*)&X[(b * TI_S + k) * TI_C + 4 * g];
+                const float4 x23 = *(const float4*)&X[(b * TI_S + k) * TI_C + 4 * g + 2];
+                fmac(R[0], l, make_float2(x01.x, x01.y));
+                fmac(R[1], l, make_float2(x01.z, x01.w));
+                fmac(R[2], l, make_float2(x23.x, x23.y));
+                fmac(R[3], l, make_float2(x23.z, x23.w));
+            }
+        }
     }
-    for (int idx = tid; idx < w * w; idx += blockDim.x) {
-        int ii = idx % w, k = idx / w;
-        N[(size_t)k * w + ii] = M[ii * LD + k];
+    constexpr int kp = 2 * TI_W;
+    for (int idx = tid; idx < TI_W * TI_C; idx += 256) {
+        const int k = idx % TI_C, i = idx / TI_C;
+        const float2 v = i > o + k ? X[idx] : make_float2(0.0f, 0.0f);
+        float rh, rl, ih, il;
+        split(-v.x, rh, rl);
+        split(-v.y, ih, il);
+        const size_t o0 = (size_t)(2 * i) * kp + 2 * (o + k), o1 = o0 + kp;
+        *(float2*)(hi + o0) = make_float2(rh, -ih);
+        *(float2*)(hi + o1) = make_float2(ih, rh);
+        *(float2*)(lo + o0) = make_float2(rl, -il);
+        *(float2*)(lo + o1) = make_float2(il, rl);
+        if (N) N[(size_t)(o + k) * TI_W + i] = v;
     }
 }
 size_t tf32_pack_bytes(int n) {
@@ -803,24 +821,32 @@ static void run_gemm(float2* A, int n, int row0, int col0, int m2, int ncols, in
 
 // U12 = L11^-1 A12 on the tensor cores: invert L11, then A12 -= (-(L11^-1 - I)) A12 with the
 // operands packed (A12 is read from its packed copy, so the in-place update is race free).
-// Operand buffer of one TRSM step (sized on the host; a reallocation synchronises the device)
-// and the place of N = L11^-1 - I in it; null when it could not be sized.
-static float2* trsm_buffers(int n, int k0, int w, LuWork& wk, cudaStream_t st, int* kp_out) {
-    int r0 = k0 + w, ncols = n - r0;
-    int kp = ((2 * w + 31) / 32) * 32;  // whole 64-byte K rows of FP16 pieces (and of TF32)
-    size_t need = ((size_t)2 * w * kp + (size_t)ncols * kp) * 2 * 4 + (size_t)w * w * 8 + 8192;
-    if (!ensure_pack(wk, need, st)) return nullptr;
-    *kp_out = kp;
-    float* blo = (float*)wk.pack + (size_t)4 * w * kp + (size_t)ncols * kp;
-    return (float2*)(((uintptr_t)(blo + (size_t)ncols * kp) + 255) & ~(uintptr_t)255);
+// Places of one TRSM step in the factor's operand buffer (a trailing block means a full panel, w = 128):
+// the pieces of A12 first, then those of -N and N itself, beyond what the updates between the inverse's
+// launch and the TRSM write (panel b's block rows, the packing of A12). False when the buffer is too small.
+struct TrsmPlaces {
+    float *bhi, *blo, *nhi, *nlo;
+    float2* N;
+};
+static bool trsm_places(int n, int k0, LuWork& wk, cudaStream_t st, TrsmPlaces* t) {
+    const size_t ncols = n - k0 - TI_W, kp = 2 * TI_W, piece = 2 * TI_W * kp;
+    // panel b's update with panel a: pieces of its 128 complex rows and of ncols columns (the largest of them)
+    const size_t before = 2 * (piece + ncols * kp);
+    if (!ensure_pack(wk, (before + 2 * piece) * 4 + (size_t)TI_W * TI_W * 8 + 8192, st)) return false;
+    t->bhi = (float*)wk.pack;
+    t->blo = t->bhi + ncols * kp;
+    t->nhi = (float*)(((uintptr_t)((float*)wk.pack + before) + 255) & ~(uintptr_t)255);
+    t->nlo = t->nhi + piece;
+    t->N = (float2*)(t->nlo + piece);
+    return true;
 }
 
-bool launch_tf32_trsm_inverse(float2* A, int n, int k0, int w, LuWork& wk, cudaStream_t st, cudaStream_t side,
+bool launch_tf32_trsm_inverse(float2* A, int n, int k0, LuWork& wk, cudaStream_t st, cudaStream_t side,
                               long long* launches) {
-    int kp;
-    float2* Nm = trsm_buffers(n, k0, w, wk, st, &kp);
-    if (!Nm) return false;
-    tri_inverse_l_kernel<<<1, 1024, TI_SMEM, side>>>(A, (size_t)n, k0, w, Nm);
+    TrsmPlaces t;
+    if (!trsm_places(n, k0, wk, st, &t)) return false;
+    tri_inverse_l_kernel<<<TI_W / TI_C, 256, TI_SMEM, side>>>(A, (size_t)n, k0, t.nhi, t.nlo,
+                                                        wk.pieces == PIECES_F16 ? t.N : nullptr);
     ++*launches;
     // a refused launch leaves the inverse to the main stream (launch_tf32_trsm, inverse_done false)
     return cudaGetLastError() == cudaSuccess;
@@ -829,64 +855,47 @@ bool launch_tf32_trsm_inverse(float2* A, int n, int k0, int w, LuWork& wk, cudaS
 // The TRSM's right-hand side A12 as TF32 pieces, packed before the main stream waits for the
 // inverse of L11 (which it does not need); launch_tf32_trsm(..., rhs_packed = true) then skips
 // it. FP16 pieces keep their packing in launch_tf32_trsm (false here).
-bool launch_tf32_trsm_rhs(float2* A, int n, int k0, int w, LuWork& wk, cudaStream_t st, long long* launches) {
-    if (wk.pieces == PIECES_F16) return false;
-    int r0 = k0 + w, ncols = n - r0, kp;
-    if (ncols <= 0 || !trsm_buffers(n, k0, w, wk, st, &kp)) return false;
-    float* bhi = (float*)wk.pack + (size_t)4 * w * kp;
-    float* blo = bhi + (size_t)ncols * kp;
-    StageScope sc(ST_TRSM, st);
-    size_t tot = (size_t)ncols * (kp / 2);
-    pack_u_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(A, (size_t)n, r0, k0, ncols, w, kp, bhi, blo);
+static void pack_trsm_rhs(float2* A, int n, int k0, const TrsmPlaces& t, cudaStream_t st, long long* launches) {
+    const int r0 = k0 + TI_W, ncols = n - r0;
+    const size_t tot = (size_t)ncols * TI_W;
+    pack_u_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(A, (size_t)n, r0, k0, ncols, TI_W, 2 * TI_W, t.bhi,
+                                                                 t.blo);
     ++*launches;
+}
+bool launch_tf32_trsm_rhs(float2* A, int n, int k0, LuWork& wk, cudaStream_t st, long long* launches) {
+    TrsmPlaces t;
+    if (wk.pieces == PIECES_F16 || !trsm_places(n, k0, wk, st, &t)) return false;
+    StageScope sc(ST_TRSM, st);
+    pack_trsm_rhs(A, n, k0, t, st, launches);
     return true;
 }
 
-void launch_tf32_trsm(float2* A, int n, int k0, int w, LuWork& wk, cudaStream_t st, long long* launches,
-                      bool inverse_done, bool rhs_packed) {
-    int r0 = k0 + w, ncols = n - r0;
-    int kp;
-    float2* Nm = trsm_buffers(n, k0, w, wk, st, &kp);
-    if (!Nm) return;
-    float* ahi = (float*)wk.pack;
-    float* alo = ahi + (size_t)2 * w * kp;
-    float* bhi = alo + (size_t)2 * w * kp;
-    float* blo = bhi + (size_t)ncols * kp;
-    {
-        StageScope sc(ST_TRSM, st);
-        if (!inverse_done) {
-            tri_inverse_l_kernel<<<1, 1024, TI_SMEM, st>>>(A, (size_t)n, k0, w, Nm);
-            if (cudaGetLastError() != cudaSuccess) {  // U12 would use a stale inverse: stop the factorization
-                cudaMemsetAsync(wk.status, 7, 1, st);
-                return;
-            }
-        }
-        dim3 g1((w + 31) / 32, (kp / 2 + 31) / 32);
-        size_t tot = (size_t)ncols * (kp / 2);
-        if (wk.pieces == PIECES_F16) {
-            // A operand: -N embedded, so that the update C -= (-N) A12 adds N A12
-            __half *h_ahi = (__half*)ahi, *h_alo = h_ahi + (size_t)2 * w * kp;
-            __half *h_bhi = h_alo + (size_t)2 * w * kp, *h_blo = h_bhi + (size_t)ncols * kp;
-            float* sA = (float*)(((uintptr_t)(h_blo + (size_t)ncols * kp) + 255) & ~(uintptr_t)255);
-            float* sB = (float*)(((uintptr_t)(sA + w) + 255) & ~(uintptr_t)255);
-            pack_l16_kernel<<<(w + 31) / 32, 256, 0, st>>>(Nm, (size_t)w, 0, 0, w, w, kp, -1.0f, h_ahi, h_alo, sA);
-            pack_u16_kernel<<<(unsigned)(((size_t)ncols * 32 + 255) / 256), 256, 0, st>>>(A, (size_t)n, r0, k0, ncols, w,
-                                                                                         kp, h_bhi, h_blo, sB);
-            run_gemm(A, n, 2 * k0, r0, 2 * w, ncols, kp, h_ahi, h_alo, h_bhi, h_blo, sA, sB, wk, st, launches,
-                     PIECES_F16);
-            *launches += 3;
-        } else {
-            pack_l_kernel<<<g1, 256, 0, st>>>(Nm, (size_t)w, 0, 0, w, w, kp, ahi, alo);
-            if (!rhs_packed) {
-                pack_u_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(A, (size_t)n, r0, k0, ncols, w, kp, bhi,
-                                                                             blo);
-                ++*launches;
-            }
-            negate_kernel<<<(unsigned)(((size_t)4 * w * kp + 255) / 256), 256, 0, st>>>(ahi, (size_t)4 * w * kp);
-            run_gemm(A, n, 2 * k0, r0, 2 * w, ncols, kp, ahi, alo, bhi, blo, nullptr, nullptr, wk, st, launches,
-                     PIECES_TF32X3);
-            *launches += 3;
-        }
+void launch_tf32_trsm(float2* A, int n, int k0, LuWork& wk, cudaStream_t st, long long* launches, bool inverse_done,
+                      bool rhs_packed) {
+    constexpr int w = TI_W, kp = 2 * TI_W;
+    const int r0 = k0 + w, ncols = n - r0;
+    TrsmPlaces t;
+    if (!trsm_places(n, k0, wk, st, &t)) return;
+    StageScope sc(ST_TRSM, st);
+    if (!inverse_done && !launch_tf32_trsm_inverse(A, n, k0, wk, st, st, launches)) {
+        cudaMemsetAsync(wk.status, 7, 1, st);  // U12 would use a stale inverse: stop the factorization
+        return;
+    }
+    if (wk.pieces == PIECES_F16) {
+        // A operand: -N embedded, so that the update C -= (-N) A12 adds N A12
+        __half *h_ahi = (__half*)wk.pack, *h_alo = h_ahi + (size_t)2 * w * kp;
+        __half *h_bhi = h_alo + (size_t)2 * w * kp, *h_blo = h_bhi + (size_t)ncols * kp;
+        float* sA = (float*)(((uintptr_t)(h_blo + (size_t)ncols * kp) + 255) & ~(uintptr_t)255);
+        float* sB = (float*)(((uintptr_t)(sA + w) + 255) & ~(uintptr_t)255);
+        pack_l16_kernel<<<(w + 31) / 32, 256, 0, st>>>(t.N, (size_t)w, 0, 0, w, w, kp, -1.0f, h_ahi, h_alo, sA);
+        pack_u16_kernel<<<(unsigned)(((size_t)ncols * 32 + 255) / 256), 256, 0, st>>>(A, (size_t)n, r0, k0, ncols, w, kp,
+                                                                                     h_bhi, h_blo, sB);
+        run_gemm(A, n, 2 * k0, r0, 2 * w, ncols, kp, h_ahi, h_alo, h_bhi, h_blo, sA, sB, wk, st, launches, PIECES_F16);
+        *launches += 2;
+    } else {
+        if (!rhs_packed) pack_trsm_rhs(A, n, k0, t, st, launches);
+        run_gemm(A, n, 2 * k0, r0, 2 * w, ncols, kp, t.nhi, t.nlo, t.bhi, t.blo, nullptr, nullptr, wk, st, launches,
+                 PIECES_TF32X3);
     }
 }
 

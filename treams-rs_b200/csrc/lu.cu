@@ -809,10 +809,10 @@ static bool lu_pairs_enabled() {
     }();
     return v;
 }
-bool launch_tf32_trsm_rhs(float2* A, int n, int k0, int w, LuWork& wk, cudaStream_t st, long long* launches);
-void launch_tf32_trsm(float2* A, int n, int k0, int w, LuWork& wk, cudaStream_t st, long long* launches,
+bool launch_tf32_trsm_rhs(float2* A, int n, int k0, LuWork& wk, cudaStream_t st, long long* launches);
+void launch_tf32_trsm(float2* A, int n, int k0, LuWork& wk, cudaStream_t st, long long* launches,
                       bool inverse_done, bool rhs_packed);
-bool launch_tf32_trsm_inverse(float2* A, int n, int k0, int w, LuWork& wk, cudaStream_t st, cudaStream_t side,
+bool launch_tf32_trsm_inverse(float2* A, int n, int k0, LuWork& wk, cudaStream_t st, cudaStream_t side,
                               long long* launches);
 
 // A second stream of this thread and device (created once, kept for the process) on which the
@@ -866,7 +866,7 @@ static int lu_factor_impl(typename Cx<R>::T* A, int n, LuWork& wk, cudaStream_t 
         bool inverse_done = false;
         if (side && cudaEventRecord(side->panel_done, st) == cudaSuccess &&
             cudaStreamWaitEvent(side->stream, side->panel_done, 0) == cudaSuccess)
-            inverse_done = launch_tf32_trsm_inverse((float2*)A, n, k0, w, wk, st, side->stream, launches) &&
+            inverse_done = launch_tf32_trsm_inverse((float2*)A, n, k0, wk, st, side->stream, launches) &&
                            cudaEventRecord(side->inverse_done, side->stream) == cudaSuccess;
         {
             StageScope sc(ST_SWAP, st);
@@ -881,7 +881,7 @@ static int lu_factor_impl(typename Cx<R>::T* A, int n, LuWork& wk, cudaStream_t 
         if (sizeof(R) == 4 && tensor_cores && r0 < n) {
             if (pend_k0 >= 0)  // panel b: its block rows right of it get panel a's update first
                 launch_tf32_update_region((float2*)A, n, pend_k0, pend_w, k0, w, r0, cols, wk, st, launches);
-            rhs_packed = launch_tf32_trsm_rhs((float2*)A, n, k0, w, wk, st, launches);
+            rhs_packed = launch_tf32_trsm_rhs((float2*)A, n, k0, wk, st, launches);
         }
         if (inverse_done && cudaStreamWaitEvent(st, side->inverse_done, 0) != cudaSuccess) {
             cudaStreamSynchronize(side->stream);  // ordering by the host instead
@@ -891,7 +891,7 @@ static int lu_factor_impl(typename Cx<R>::T* A, int n, LuWork& wk, cudaStream_t 
         const int cpc = per_pass * std::max(1, (cols + per_pass * 2 * g_num_sms - 1) / (per_pass * 2 * g_num_sms));
         size_t smem = (size_t)NB * NB * sizeof(C);
         if (sizeof(R) == 4 && tensor_cores) {
-            launch_tf32_trsm((float2*)A, n, k0, w, wk, st, launches, inverse_done, rhs_packed);
+            launch_tf32_trsm((float2*)A, n, k0, wk, st, launches, inverse_done, rhs_packed);
         } else {
             StageScope sc(ST_TRSM, st);
             trsm_kernel<R, NB><<<(cols + cpc - 1) / cpc, 256, smem, st>>>(A, lda, k0, w, n, cpc);
