@@ -116,6 +116,7 @@ struct HostRing {
 struct DevPlanStore {
     HostPlan host;
     DevPlan dev{};
+    ProductBlocks blocks;
     void* mem = nullptr;
 };
 
@@ -291,6 +292,8 @@ tcu_status get_plan(tcu_context* ctx, int L, const DevPlan** out) {
         d.w = (const double2*)(base + off_w);
         d.reflection = (const double*)(base + off_refl);
         d.idx = (const uint16_t*)(base + off_idx);
+        stored_product_blocks(d, h, &store->blocks);
+        d.blocks = &store->blocks;
         it = ctx->plans.emplace(L, std::move(store)).first;
     }
     *out = &it->second->dev;

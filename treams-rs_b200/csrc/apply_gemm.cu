@@ -336,7 +336,8 @@ __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
 
 // CTA = one block of DI destinations x a range of source chunks: builds the chunk tables
 // (degrees <= order) exactly as the on-the-fly product does and writes them out in the stored
-// order.
+// order: the block's destinations side by side, row t * DI + destination, so that row octets ascend in
+// degree (stored_product_blocks).
 __global__ void __launch_bounds__(256) table_store_kernel(DevPlan P, int order, int N, double k,
                                                           const double* __restrict__ pos, bool singular, int DI,
                                                           int KJ, int RO, int NC, int span, cplx* __restrict__ Z) {
@@ -347,10 +348,13 @@ __global__ void __launch_bounds__(256) table_store_kernel(DevPlan P, int order, 
     cplx* Rs = Zs + (size_t)KJ * ZLD;                                     // npair x (order + 1)
     double4* Ds = reinterpret_cast<double4*>(Rs + (size_t)npair * ord1);  // direction, state
     double2* rec = reinterpret_cast<double2*>(Ds + npair);                // ts
+    __shared__ unsigned char place[128];                                  // stored row -> row of Zs
     const int tid = threadIdx.x, nthr = blockDim.x;
     recurrence_table(order, rec, tid, nthr);
     const int i0 = blockIdx.x * DI;
     for (int t = tid; t < KJ * ZLD; t += nthr) Zs[t] = mk(0.0, 0.0);  // padding rows stay zero
+    if (DI > 1)  // at most 128 rows
+        for (int row = tid; row < RO * 8; row += nthr) place[row] = row < rows ? row % DI * ts + row / DI : row;
     const int jbeg = blockIdx.y * span, jend = min(N, jbeg + span);
     cplx* Zb = Z + (size_t)blockIdx.x * NC * RO * 128;
     for (int j0 = jbeg; j0 < jend; j0 += KJ) {
@@ -362,7 +366,7 @@ __global__ void __launch_bounds__(256) table_store_kernel(DevPlan P, int order, 
         for (int it = tid; it < total; it += nthr) {
             const int lane = it & 31, w = it >> 5, o = w % RO, qc = w / RO;
             const int row = o * 8 + (lane >> 2), kk = qc * 4 + (lane & 3);  // qc = 4 c + q
-            const cplx v = row < rows ? Zs[(size_t)kk * ZLD + row] : mk(0.0, 0.0);
+            const cplx v = row < rows ? Zs[(size_t)kk * ZLD + (DI > 1 ? place[row] : row)] : mk(0.0, 0.0);
             const size_t slab = (size_t)(j0 / SRC_CHUNK) * 4 + qc;  // chunk * 4 + q
             if (slab < (size_t)NC * 4) Zb[(slab * RO + o) * 32 + lane] = v;  // the last build chunk may be half past N
         }
@@ -447,26 +451,60 @@ __device__ __forceinline__ void as_bulk_load(uint32_t dst, const void* src, uint
         : "memory");
 }
 
+// most blocks a warp takes (stored_product_blocks over the product warps): 16 / 8, 30 / 8, 41 / 8, 52 / 8,
+// 109 / 16, 103 / 16, 106 / 16
+constexpr int SLOTS_DIPOLE = 2, SLOTS_L2 = 4, SLOTS_L3 = 6, SLOTS_L4 = 7, SLOTS_L5 = 7, SLOTS_L6 = 7, SLOTS_L7 = 7;
+
 // The stored product with a producer warp: lane 0 of the last warp streams the 16-source chunks
 // (table slab and packed inputs, each one contiguous bulk copy) into a 3-stage ring, each stage
 // completing on its full barrier; the product warps take a stage once its full barrier flips
 // and release it through its empty barrier (one arrival per warp), so no CTA-wide barrier
 // sits in the loop. Every wait is bounded (2 s): on a timeout the kernel records status 8,
 // waits (bounded) for the copies in flight and returns without writing y.
-// On success the product Z X is in Gs = smem (rows < rows, columns < cols, row-major).
-// CG 1: a warp takes RPW row octets and all CT column octets. CG 2: eight warps, row octets in four
-// parts of at most RPW, columns in two halves, the second half's parts in reverse order: warp w runs on
-// scheduler w % 4, and 11 row octets by twos (lmax 4) leave the four DMMA pipes 4, 3, 2 and 2 of them,
-// 69 % busy at most, the parts 5, 6, 6 and 5.
-template <int CT, int RPW, int CG>
+// On success the product Z X is in Gs = smem (rows < rows, columns < cols, row-major, the rows of
+// destination 0 first), wherever a term reads it.
+// Work: the 8 x 8 blocks of `blocks`, dealt out evenly to the product warps in row order, at most SLOTS each
+// with its accumulators in registers. A source of degree l reads table degrees l - lmax .. l + lmax only,
+// so a fifth of the blocks are never read (lmax 3: 41 of 52 remain, 4: 52 of 66, 5: 109 of 144, 6: 103 of
+// 132), and warps of equal work keep the four DMMA pipes equally busy (warp w runs on scheduler w % 4; row
+// octets by twos left them 4, 4, 3 and 2 octets at lmax 3). Both fragments of a slot are loaded for four
+// products, 39 % of the shared-memory rate, two slots ahead and without a branch in between: 13 % of the
+// time at lmax 3 and 6. One column: 1184 spheres lmax 3 0.64 -> 0.44 ms, 296 lmax 6 0.43 -> 0.345;
+// 4096 lmax 3 7.6 -> 5.3, the DMMA pipe 84 % busy.
+// A chunk's products of the first USED slots (of the first cnt of them), fragments read two slots ahead.
+template <int SLOTS, int USED>
+__device__ __forceinline__ void product_chunk(const cplx* stage, int da, int db, const int (&oa)[SLOTS],
+                                              const int (&ob)[SLOTS], double (&re)[SLOTS][2], double (&im)[SLOTS][2],
+                                              int cnt = USED) {
+    constexpr int AHEAD = 2, STEPS = 4 * USED;
+    cplx a[AHEAD + 1], b[AHEAD + 1];
+#pragma unroll
+    for (int n = 0; n < STEPS + AHEAD; ++n) {
+        if (n < STEPS) {
+            a[n % (AHEAD + 1)] = stage[n / USED * da + oa[n % USED]];
+            b[n % (AHEAD + 1)] = stage[n / USED * db + ob[n % USED]];
+        }
+        if (n >= AHEAD) {
+            const int j = (n - AHEAD) % USED;
+            const cplx x = a[(n - AHEAD) % (AHEAD + 1)], z = b[(n - AHEAD) % (AHEAD + 1)];
+            if (j < cnt) {
+                dmma(re[j], x.x, z.x);
+                dmma(im[j], x.x, z.y);
+                dmma(re[j], x.y, -z.y);
+                dmma(im[j], x.y, z.x);
+            }
+        }
+    }
+}
+template <int SLOTS>
 __device__ __forceinline__ bool stored_product(unsigned char* smem, const cplx* __restrict__ Zb,
-                                               const cplx* __restrict__ Xb, int NC, int RO, int rows, int cols,
+                                               const cplx* __restrict__ Xb, int NC, int RO, int CT,
+                                               const ProductBlocks& blocks, int list, int DI, int ts, int cols,
                                                int* __restrict__ status) {
     __shared__ __align__(8) uint64_t bars[2 * AS_STAGES];
     __shared__ int s_abort;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    constexpr int CW = CT / CG;  // column octets of a warp
-    const int W = CG == 1 ? (RO + RPW - 1) / RPW : 4 * CG;  // product warps; warp W loads
+    const int W = (blockDim.x >> 5) - 1;  // product warps; warp W loads
     const int ABLK = RO * 128, BBLK = CT * 128, SBLK = ABLK + BBLK;  // complex entries per chunk
     cplx* ring = reinterpret_cast<cplx*>(smem);
     const uint32_t full0 = as_smem_u32(bars), empty0 = full0 + 8 * AS_STAGES;
@@ -480,17 +518,20 @@ __device__ __forceinline__ bool stored_product(unsigned char* smem, const cplx* 
     }
     __syncthreads();
     volatile int* abort_flag = &s_abort;
-    double re[RPW][CW][2], im[RPW][CW][2];
+    double re[SLOTS][2], im[SLOTS][2];
+    int oa[SLOTS], ob[SLOTS];  // places of the slots' fragments in a group of 4 sources
+    int cnt = 0, first = 0;
+    if (warp < W) {
+        const int total = blocks.count[list], base = total / W, extra = total - base * W;
+        cnt = base + (warp < extra ? 1 : 0);
+        first = warp * base + min(warp, extra);
 #pragma unroll
-    for (int r = 0; r < RPW; ++r)
-#pragma unroll
-        for (int c = 0; c < CW; ++c) re[r][c][0] = re[r][c][1] = im[r][c][0] = im[r][c][1] = 0.0;
-    int o0 = warp * RPW, nr = min(RPW, RO - o0), c0 = 0;  // the warp's row and column octets
-    if (CG > 1) {
-        const int part = (warp >> 2) & 1 ? 3 - (warp & 3) : warp & 3, base = RO / 4, extra = RO % 4;
-        o0 = part * base + min(part, extra);
-        nr = base + (part < extra ? 1 : 0);
-        c0 = (warp >> 2) * CW;
+        for (int j = 0; j < SLOTS; ++j) {
+            const int at = min(first + j, total - 1);
+            oa[j] = blocks.row[list][at] * 32 + lane;
+            ob[j] = ABLK + blocks.col[list][at] * 32 + lane;
+            re[j][0] = re[j][1] = im[j][0] = im[j][1] = 0.0;
+        }
     }
     if (warp == W) {
         if (lane == 0) {
@@ -512,31 +553,17 @@ __device__ __forceinline__ bool stored_product(unsigned char* smem, const cplx* 
                 }
             }
         }
-    } else if (warp < W) {
+    } else {
         for (int kc = 0; kc < NC; ++kc) {
             const int s = kc % AS_STAGES;
             if (!as_mbar_wait(full0 + 8 * s, (kc / AS_STAGES) & 1, abort_flag)) break;
-            const cplx* As = ring + (size_t)s * SBLK;
-            const cplx* Bs = As + ABLK;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                cplx a[RPW];
-#pragma unroll
-                for (int r = 0; r < RPW; ++r) a[r] = r < nr ? As[(q * RO + o0 + r) * 32 + lane] : mk(0.0, 0.0);
-#pragma unroll
-                for (int c = 0; c < CW; ++c) {
-                    const cplx b = Bs[(q * CT + c0 + c) * 32 + lane];
-#pragma unroll
-                    for (int r = 0; r < RPW; ++r) {
-                        if (r < nr) {
-                            dmma(re[r][c], a[r].x, b.x);
-                            dmma(re[r][c], a[r].y, -b.y);
-                            dmma(im[r][c], a[r].x, b.y);
-                            dmma(im[r][c], a[r].y, b.x);
-                        }
-                    }
-                }
-            }
+            const cplx* stage = ring + (size_t)s * SBLK;
+            if (cnt == SLOTS)
+                product_chunk<SLOTS, SLOTS>(stage, RO * 32, CT * 32, oa, ob, re, im);
+            else if (cnt == SLOTS - 1)
+                product_chunk<SLOTS, SLOTS - 1>(stage, RO * 32, CT * 32, oa, ob, re, im);
+            else  // lmax 7, first half of the sources
+                product_chunk<SLOTS, (SLOTS > 2 ? SLOTS - 2 : 1)>(stage, RO * 32, CT * 32, oa, ob, re, im, cnt);
             __syncwarp();
             if (lane == 0) as_mbar_arrive(empty0 + 8 * s);
         }
@@ -549,15 +576,13 @@ __device__ __forceinline__ bool stored_product(unsigned char* smem, const cplx* 
     cplx* Gs = ring;
     if (warp < W) {
 #pragma unroll
-        for (int r = 0; r < RPW; ++r) {
-            const int row = (o0 + r) * 8 + (lane >> 2);
-            if (r < nr && row < rows) {
-#pragma unroll
-                for (int c = 0; c < CW; ++c) {
-                    const int col = (c0 + c) * 8 + 2 * (lane & 3);
-                    if (col < cols) Gs[(size_t)row * cols + col] = mk(re[r][c][0], im[r][c][0]);
-                    if (col + 1 < cols) Gs[(size_t)row * cols + col + 1] = mk(re[r][c][1], im[r][c][1]);
-                }
+        for (int j = 0; j < SLOTS; ++j) {
+            const int row = blocks.row[list][min(first + j, blocks.count[list] - 1)] * 8 + (lane >> 2);
+            const int col = blocks.col[list][min(first + j, blocks.count[list] - 1)] * 8 + 2 * (lane & 3);
+            if (j < cnt && row < DI * ts) {
+                cplx* g = Gs + (size_t)(DI > 1 ? row % DI * ts + row / DI : row) * cols;
+                if (col < cols) g[col] = mk(re[j][0], im[j][0]);
+                if (col + 1 < cols) g[col + 1] = mk(re[j][1], im[j][1]);
             }
         }
     }
@@ -565,16 +590,17 @@ __device__ __forceinline__ bool stored_product(unsigned char* smem, const cplx* 
     return true;
 }
 
-template <int CT, int RPW, int CG>
-__global__ void __launch_bounds__(288, CT <= 6 ? 2 : 1)
+template <int SLOTS, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32 + 32, WARPS == 8 ? 2 : 1)
     apply_stored_tma_kernel(DevPlan P, SubOp O, int N, const cplx* __restrict__ Z, const cplx* __restrict__ Xf,
-                            int NC, int DI, int RO, const cplx* __restrict__ T, const cplx* __restrict__ x, size_t ldx,
+                            int NC, int DI, int RO, int CT, const __grid_constant__ ProductBlocks blocks,
+                            const cplx* __restrict__ T, const cplx* __restrict__ x, size_t ldx,
                             const cplx* __restrict__ zadd, double alpha, double beta, bool singular,
                             cplx* __restrict__ y, int* __restrict__ status) {
     extern __shared__ __align__(128) unsigned char at_smem[];
-    const int M = 2 * O.nsrc, rows = DI * (O.order + 1) * (O.order + 1);
-    if (!stored_product<CT, RPW, CG>(at_smem, Z + (size_t)blockIdx.x * NC * RO * 128,
-                                 Xf + (size_t)blockIdx.y * NC * CT * 128, NC, RO, rows, M, status))
+    const int M = 2 * O.nsrc, ts = (O.order + 1) * (O.order + 1);
+    if (!stored_product<SLOTS>(at_smem, Z + (size_t)blockIdx.x * NC * RO * 128,
+                               Xf + (size_t)blockIdx.y * NC * CT * 128, NC, RO, CT, blocks, 0, DI, ts, M, status))
         return;
     const size_t coff = (size_t)blockIdx.y * ldx;
     terms_epilogue(P, O, reinterpret_cast<const cplx*>(at_smem), DI, blockIdx.x * DI, N, T, x + coff, coff, zadd, alpha,
@@ -589,16 +615,17 @@ __global__ void __launch_bounds__(288, CT <= 6 ? 2 : 1)
 // adds the parts in a fixed order and applies the Mie block and the epilogue. The DMMA pipe
 // bounds it as it bounds lmax 2..5. 300 spheres lmax 6, one application: 4.3 ms with the per-pair
 // term sums (CUDA cores, an index, a weight and a gather per term and pair), 0.57 ms here.
-template <int CT, int RPW>
-__global__ void __launch_bounds__(512, 1)
+template <int SLOTS, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32 + 32, 1)
     apply_split_kernel(DevPlan P, int N, const cplx* __restrict__ Z, const cplx* __restrict__ Xf, size_t per_col,
-                       int NC, int RO, int parts, int cnt, cplx* __restrict__ Cp, int* __restrict__ status) {
+                       int NC, int RO, int CT, const __grid_constant__ ProductBlocks blocks, int parts, int cnt,
+                       cplx* __restrict__ Cp, int* __restrict__ status) {
     extern __shared__ __align__(128) unsigned char sp_smem[];
     const int i = blockIdx.x / parts, part = blockIdx.x - i * parts, s0 = (part >> 1) * cnt;
     const int ns = min(cnt, P.nlm - s0), nlm = P.nlm;
-    if (!stored_product<CT, RPW, 1>(sp_smem, Z + (size_t)i * NC * RO * 128,
-                                 Xf + (size_t)blockIdx.y * per_col + (size_t)part * NC * CT * 128, NC, RO, P.tsize, cnt,
-                                 status))
+    if (!stored_product<SLOTS>(sp_smem, Z + (size_t)i * NC * RO * 128,
+                               Xf + (size_t)blockIdx.y * per_col + (size_t)part * NC * CT * 128, NC, RO, CT, blocks,
+                               part >> 1, 1, P.tsize, cnt, status))
         return;
     const cplx* G = reinterpret_cast<const cplx*>(sp_smem);
     // thread (d, group): the group's source lm s = group, group + groups, ...; then a fixed-order sum
@@ -728,7 +755,7 @@ bool stored_kind_ok(const DevPlan& P, int kind) {
 }
 struct StoredLayout {
     SubOp O;
-    int DI, KJ, RO, CT, NC, nblk, RPW;  // RPW: row octets per warp of the product
+    int DI, KJ, RO, CT, NC, nblk;
     int parts, cnt;                     // split product: CTAs per destination, source lm of each (else 1, 0)
     size_t z_elems, xf_per_col, cp_per_col;  // cp: the split product's coupling sums
 };
@@ -747,7 +774,6 @@ StoredLayout stored_layout(const DevPlan& P, int N, int kind) {
         l.cnt = (l.O.nsrc + halves - 1) / halves;
     }
     l.CT = ((l.parts > 1 ? l.cnt : 2 * l.O.nsrc) + 7) / 8;
-    l.RPW = 2;
     l.NC = (N + SRC_CHUNK - 1) / SRC_CHUNK;
     l.nblk = (N + l.DI - 1) / l.DI;
     l.z_elems = (size_t)l.nblk * l.NC * l.RO * 128;
@@ -767,6 +793,45 @@ size_t store_smem(const StoredLayout& l) {
            (size_t)(l.O.order + 1) * (l.O.order + 1) * sizeof(double2);
 }
 }  // namespace
+
+// The blocks of the full coupling operator's product that a term of the plan reads: source lm s and table
+// entry t meet in the term lists of some destination. Natural order of both already gathers them (of
+// random exchanges of rows and columns none found fewer).
+void stored_product_blocks(const DevPlan& P, const HostPlan& h, ProductBlocks* b) {
+    b->count[0] = b->count[1] = 0;
+    if (P.L < 2 || P.L > 7) return;
+    const StoredLayout l = stored_layout(P, 1, STORED_FULL);
+    std::vector<char> read((size_t)h.nlm * P.tsize, 0);
+    for (int c = 0; c < h.nlm * h.nlm; ++c) {
+        const int n = (h.combo[2 * c + 1] & 0xffff) + (h.combo[2 * c + 1] >> 16);
+        for (int e = 0; e < n; ++e) read[(size_t)(c / h.nlm) * P.tsize + h.idx[h.combo[2 * c] + e]] = 1;
+    }
+    for (int list = 0; list < std::max(1, l.parts / 2); ++list)
+        for (int o = 0; o < l.RO; ++o)
+            for (int c = 0; c < l.CT; ++c) {
+                bool any = false;
+                for (int row = o * 8; row < std::min(o * 8 + 8, l.DI * P.tsize); ++row)
+                    for (int col = c * 8; col < c * 8 + 8; ++col) {
+                        if (l.parts > 1 && col >= l.cnt) break;
+                        const int s = l.parts > 1 ? list * l.cnt + col : col / 2;
+                        any = any || (s < h.nlm && read[(size_t)s * P.tsize + row / l.DI]);
+                    }
+                if (!any) continue;
+                b->row[list][b->count[list]] = (unsigned char)o;
+                b->col[list][b->count[list]++] = (unsigned char)c;
+            }
+}
+// every block of a product (the dipole operators: one column octet)
+static ProductBlocks all_blocks(const StoredLayout& l) {
+    ProductBlocks b;
+    b.count[0] = b.count[1] = 0;
+    for (int o = 0; o < l.RO; ++o)
+        for (int c = 0; c < l.CT; ++c) {
+            b.row[0][b.count[0]] = (unsigned char)o;
+            b.col[0][b.count[0]++] = (unsigned char)c;
+        }
+    return b;
+}
 
 size_t stored_tables_bytes(const DevPlan& P, int N, int kind) {
     if (!stored_kind_ok(P, kind) || N <= 0) return 0;
@@ -803,35 +868,35 @@ void launch_apply_stored(const DevPlan& P, int N, int kind, const cplx* Z, const
                      (unsigned)l.parts);
     pack_sources_kernel<<<pgrid, 256, 0, st>>>(x, ldx, l.O.ldin, N, M, l.NC, l.CT, l.parts, l.cnt, l.xf_per_col, Xf);
     const size_t smem = stored_smem(l);
-    const int threads = (l.RO + l.RPW - 1) / l.RPW * 32;
+    const ProductBlocks blocks = kind == STORED_FULL ? *P.blocks : all_blocks(l);
     if (l.parts > 1) {
         cplx* Cp = Xf + l.xf_per_col * ncol;
         const dim3 g((unsigned)(N * l.parts), (unsigned)ncol);
-        if (l.CT == 6)
-            apply_split_kernel<6, 2><<<g, threads + 32, smem, st>>>(P, N, Z, Xf, l.xf_per_col, l.NC, l.RO, l.parts,
-                                                                    l.cnt, Cp, status);
+        auto split = [&](auto kernel, int warps) {
+            kernel<<<g, warps * 32 + 32, smem, st>>>(P, N, Z, Xf, l.xf_per_col, l.NC, l.RO, l.CT, blocks, l.parts, l.cnt,
+                                                     Cp, status);
+        };
+        if (P.L == 6)
+            split(apply_split_kernel<SLOTS_L6, 16>, 16);
         else
-            apply_split_kernel<4, 2><<<g, threads + 32, smem, st>>>(P, N, Z, Xf, l.xf_per_col, l.NC, l.RO, l.parts,
-                                                                    l.cnt, Cp, status);
+            split(apply_split_kernel<SLOTS_L7, 16>, 16);
         const dim3 fg((unsigned)(((size_t)N * P.nlm + 255) / 256), (unsigned)ncol);
         split_finish_kernel<<<fg, 256, 0, st>>>(P, N, l.parts, Cp, T, x, ldx, zadd, alpha, beta, singular, y);
         return;
     }
     const dim3 grid((unsigned)l.nblk, (unsigned)ncol);
-    // column octets, row octets per warp, column groups (stored_product); at lmax 3 two column groups
-    // measured slower (4096 spheres: 7.8 against 7.6 ms), at lmax 4 faster (512 spheres, 3 columns: 0.81
-    // against 1.05 ms of the row octets by twos, 200 spheres, 17 columns: 0.79 against 1.03)
-#define TCU_STORED(CT, RPW, CG)                                                                                   \
-    apply_stored_tma_kernel<CT, RPW, CG><<<grid, CG > 1 ? 288 : threads + 32, smem, st>>>(                         \
-        P, l.O, N, Z, Xf, l.NC, l.DI, l.RO, T, x, ldx, zadd, alpha, beta, singular, y, status)
+    auto apply = [&](auto kernel, int warps) {
+        kernel<<<grid, warps * 32 + 32, smem, st>>>(P, l.O, N, Z, Xf, l.NC, l.DI, l.RO, l.CT, blocks, T, x, ldx, zadd,
+                                                    alpha, beta, singular, y, status);
+    };
+    // 8 warps and two CTAs per SM while the ring allows (lmax 5: 153 KB), 16 warps beyond
     switch (l.CT) {
-        case 1: TCU_STORED(1, 2, 1); break;
-        case 2: TCU_STORED(2, 2, 1); break;
-        case 4: TCU_STORED(4, 2, 1); break;
-        case 6: TCU_STORED(6, 3, 2); break;
-        default: TCU_STORED(9, 2, 1); break;
+        case 1: apply(apply_stored_tma_kernel<SLOTS_DIPOLE, 8>, 8); break;
+        case 2: apply(apply_stored_tma_kernel<SLOTS_L2, 8>, 8); break;
+        case 4: apply(apply_stored_tma_kernel<SLOTS_L3, 8>, 8); break;
+        case 6: apply(apply_stored_tma_kernel<SLOTS_L4, 8>, 8); break;
+        default: apply(apply_stored_tma_kernel<SLOTS_L5, 16>, 16); break;
     }
-#undef TCU_STORED
 }
 
 void apply_gemm_init_attributes() {
@@ -840,13 +905,14 @@ void apply_gemm_init_attributes() {
     cudaFuncSetAttribute(apply_gemm_kernel<4, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     cudaFuncSetAttribute(apply_gemm_kernel<4, 5>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     cudaFuncSetAttribute(table_store_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(apply_stored_tma_kernel<1, 2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(apply_stored_tma_kernel<2, 2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(apply_stored_tma_kernel<4, 2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(apply_stored_tma_kernel<6, 3, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(apply_stored_tma_kernel<9, 2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(apply_split_kernel<6, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(apply_split_kernel<4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    auto allow = [](auto kernel) { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); };
+    allow(apply_stored_tma_kernel<SLOTS_DIPOLE, 8>);
+    allow(apply_stored_tma_kernel<SLOTS_L2, 8>);
+    allow(apply_stored_tma_kernel<SLOTS_L3, 8>);
+    allow(apply_stored_tma_kernel<SLOTS_L4, 8>);
+    allow(apply_stored_tma_kernel<SLOTS_L5, 16>);
+    allow(apply_split_kernel<SLOTS_L6, 16>);
+    allow(apply_split_kernel<SLOTS_L7, 16>);
 }
 
 }  // namespace tcu

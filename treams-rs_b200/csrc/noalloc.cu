@@ -138,6 +138,7 @@ extern "C" tcu_status tcu_cluster_apply_noalloc(void* stream, int lmax, double k
     launch_mie(lmax, k0, (int)N, radii, (const double2*)eps, T, status, st);
     if (!ck(cudaGetLastError())) return noalloc_fail(TCU_DEVICE_ERROR, "Mie coefficients failed to launch");
     DevPlan P;
+    P.blocks = nullptr;
     P.L = lmax;
     P.nlm = h.nlm;
     P.order = h.order;

@@ -21,9 +21,18 @@ struct HostPlan {
 HostPlan build_plan(int L);
 double wigner3j_racah(int j1, int j2, int j3, int m1, int m2, int m3);
 
+// 8 x 8 blocks (row octet, column octet) of a stored product that some term reads, row by row; two
+// lists where the source lm are split in halves (lmax 7), else the first one.
+struct ProductBlocks {
+    static constexpr int MAX = 144;
+    int count[2];
+    unsigned char row[2][MAX], col[2][MAX];
+};
+
 // Device view of a plan (pointers into device memory).
 struct DevPlan {
     int L, nlm, order, tsize;  // tsize = (order + 1)^2
+    const ProductBlocks* blocks;  // host memory: the full coupling operator's stored product (null: none)
     const int2* combo;
     const uint16_t* idx;
     const double2* w;
