@@ -615,18 +615,30 @@ __global__ void __launch_bounds__(WARPS * 32 + 32, WARPS == 8 ? 2 : 1)
 // adds the parts in a fixed order and applies the Mie block and the epilogue. The DMMA pipe
 // bounds it as it bounds lmax 2..5. 300 spheres lmax 6, one application: 4.3 ms with the per-pair
 // term sums (CUDA cores, an index, a weight and a gather per term and pair), 0.57 ms here.
+// One CTA fits an SM. Where the last wave of the (column, destination, part) tiles would leave half of the SMs
+// or more idle, each of its tiles is cut into pieces of the source chunks, as many as there are SMs for them:
+// tiles from `whole` on, whose pieces' sums go to Cx and are added by split_finish_kernel. 300 spheres at lmax 6
+// are 600 tiles on 148 SMs, 4.05 waves: 0.43 -> 0.38 ms a product with 8 tiles in 18 pieces each.
+struct SplitTail {
+    int whole, pieces;
+};
 template <int SLOTS, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32 + 32, 1)
     apply_split_kernel(DevPlan P, int N, const cplx* __restrict__ Z, const cplx* __restrict__ Xf, size_t per_col,
                        int NC, int RO, int CT, const __grid_constant__ ProductBlocks blocks, int parts, int cnt,
-                       cplx* __restrict__ Cp, int* __restrict__ status) {
+                       SplitTail tail, cplx* __restrict__ Cp, cplx* __restrict__ Cx, int* __restrict__ status) {
     extern __shared__ __align__(128) unsigned char sp_smem[];
-    const int i = blockIdx.x / parts, part = blockIdx.x - i * parts, s0 = (part >> 1) * cnt;
+    const int b = blockIdx.x, over = b - tail.whole, q = over >= 0 ? over / tail.pieces : 0;
+    const int tile = over >= 0 ? tail.whole + q : b, piece = over - q * tail.pieces;
+    const int col = tile / (N * parts), i = tile / parts - col * N, part = tile % parts, s0 = (part >> 1) * cnt;
+    const int c0 = over >= 0 ? piece * NC / tail.pieces : 0;
+    const int c1 = over >= 0 ? (piece + 1) * NC / tail.pieces : NC;
     const int ns = min(cnt, P.nlm - s0), nlm = P.nlm;
-    if (!stored_product<SLOTS>(sp_smem, Z + (size_t)i * NC * RO * 128,
-                               Xf + (size_t)blockIdx.y * per_col + (size_t)part * NC * CT * 128, NC, RO, CT, blocks,
-                               part >> 1, 1, P.tsize, cnt, status))
+    if (!stored_product<SLOTS>(sp_smem, Z + ((size_t)i * NC + c0) * RO * 128,
+                               Xf + (size_t)col * per_col + ((size_t)part * NC + c0) * CT * 128, c1 - c0, RO, CT,
+                               blocks, part >> 1, 1, P.tsize, cnt, status))
         return;
+    cplx* out = over >= 0 ? Cx + (size_t)over * nlm : Cp + (((size_t)col * parts + part) * N + i) * nlm;
     const cplx* G = reinterpret_cast<const cplx*>(sp_smem);
     // thread (d, group): the group's source lm s = group, group + groups, ...; then a fixed-order sum
     __shared__ cplx sums[512];
@@ -647,13 +659,13 @@ __global__ void __launch_bounds__(WARPS * 32 + 32, 1)
     if (threadIdx.x < nlm) {
         cplx c = sums[threadIdx.x];
         for (int g = 1; g < groups; ++g) c = cadd(c, sums[g * nlm + threadIdx.x]);
-        Cp[(((size_t)blockIdx.y * parts + part) * N + i) * nlm + threadIdx.x] = c;
+        out[threadIdx.x] = c;
     }
 }
 
 // y from the parts' coupling sums: outgoing, y = zadd + alpha x + beta T c; regular, y = x + c.
-__global__ void split_finish_kernel(DevPlan P, int N, int parts, const cplx* __restrict__ Cp,
-                                    const cplx* __restrict__ T, const cplx* __restrict__ x, size_t ldx,
+__global__ void split_finish_kernel(DevPlan P, int N, int parts, SplitTail tail, const cplx* __restrict__ Cp,
+                                    const cplx* __restrict__ Cx, const cplx* __restrict__ T, const cplx* __restrict__ x, size_t ldx,
                                     const cplx* __restrict__ zadd, double alpha, double beta, bool singular,
                                     cplx* __restrict__ y) {
     const int nlm = P.nlm;
@@ -661,11 +673,19 @@ __global__ void split_finish_kernel(DevPlan P, int N, int parts, const cplx* __r
     if (t >= (size_t)N * nlm) return;
     const size_t i = t / nlm, per = (size_t)N * nlm;
     const int d = (int)(t - i * nlm);
-    const cplx* c = Cp + (size_t)blockIdx.y * parts * per + t;
-    cplx sp = c[0], sn = c[per];
+    const int tile = ((int)blockIdx.y * N + (int)i) * parts;
+    auto sum_of = [&](int p) {
+        const int over = tile + p - tail.whole;
+        if (over < 0) return Cp[((size_t)blockIdx.y * parts + p) * per + t];
+        const cplx* c = Cx + (size_t)over * tail.pieces * nlm + d;
+        cplx v = c[0];
+        for (int k = 1; k < tail.pieces; ++k) v = cadd(v, c[(size_t)k * nlm]);
+        return v;
+    };
+    cplx sp = sum_of(0), sn = sum_of(1);
     for (int p = 2; p < parts; p += 2) {
-        sp = cadd(sp, c[p * per]);
-        sn = cadd(sn, c[(p + 1) * per]);
+        sp = cadd(sp, sum_of(p));
+        sn = cadd(sn, sum_of(p + 1));
     }
     const size_t row = (size_t)blockIdx.y * ldx + 2 * t;
     const cplx x0 = x[row], x1 = x[row + 1];
@@ -838,10 +858,22 @@ size_t stored_tables_bytes(const DevPlan& P, int N, int kind) {
     return stored_layout(P, N, kind).z_elems * sizeof(cplx);
 }
 
+static int num_sms() {
+    static const int sms = [] {
+        int dev = 0, v = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+        return v;
+    }();
+    return sms;
+}
+
 size_t stored_inputs_bytes(const DevPlan& P, int N, int kind, int ncol) {
     if (!stored_kind_ok(P, kind) || N <= 0) return 0;
     const StoredLayout l = stored_layout(P, N, kind);
-    return (l.xf_per_col + l.cp_per_col) * (size_t)ncol * sizeof(cplx);
+    // the pieces of the split product's tail: one coupling sum per SM at most
+    const size_t cx = l.parts > 1 ? (size_t)num_sms() * P.nlm : 0;
+    return ((l.xf_per_col + l.cp_per_col) * (size_t)ncol + cx) * sizeof(cplx);
 }
 
 void build_stored_tables(const DevPlan& P, int N, double k, const double* pos, int kind, cplx* Z, cudaStream_t st,
@@ -871,17 +903,21 @@ void launch_apply_stored(const DevPlan& P, int N, int kind, const cplx* Z, const
     const ProductBlocks blocks = kind == STORED_FULL ? *P.blocks : all_blocks(l);
     if (l.parts > 1) {
         cplx* Cp = Xf + l.xf_per_col * ncol;
-        const dim3 g((unsigned)(N * l.parts), (unsigned)ncol);
+        cplx* Cx = Cp + l.cp_per_col * ncol;
+        const int tiles = N * l.parts * ncol, sms = num_sms(), last = tiles % sms;
+        SplitTail tail{tiles, 1};
+        if (last > 0 && 2 * last <= sms && l.NC > 1) tail = {tiles - last, std::min(sms / last, l.NC)};
+        const int ctas = tail.whole + (tiles - tail.whole) * tail.pieces;
         auto split = [&](auto kernel, int warps) {
-            kernel<<<g, warps * 32 + 32, smem, st>>>(P, N, Z, Xf, l.xf_per_col, l.NC, l.RO, l.CT, blocks, l.parts, l.cnt,
-                                                     Cp, status);
+            kernel<<<ctas, warps * 32 + 32, smem, st>>>(P, N, Z, Xf, l.xf_per_col, l.NC, l.RO, l.CT, blocks, l.parts,
+                                                        l.cnt, tail, Cp, Cx, status);
         };
         if (P.L == 6)
             split(apply_split_kernel<SLOTS_L6, 16>, 16);
         else
             split(apply_split_kernel<SLOTS_L7, 16>, 16);
         const dim3 fg((unsigned)(((size_t)N * P.nlm + 255) / 256), (unsigned)ncol);
-        split_finish_kernel<<<fg, 256, 0, st>>>(P, N, l.parts, Cp, T, x, ldx, zadd, alpha, beta, singular, y);
+        split_finish_kernel<<<fg, 256, 0, st>>>(P, N, l.parts, tail, Cp, Cx, T, x, ldx, zadd, alpha, beta, singular, y);
         return;
     }
     const dim3 grid((unsigned)l.nblk, (unsigned)ncol);
