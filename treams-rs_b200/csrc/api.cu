@@ -138,9 +138,7 @@ struct tcu_context {
     std::map<int, std::unique_ptr<DevPlanStore>> plans;
     long long launches = 0;
     double* d_partial = nullptr;  // reduction scratch (8 * 256 doubles)
-    cplx* d_cpartial = nullptr;   // complex reduction scratch (64 * 256)
     double* d_small = nullptr;    // 64 doubles
-    cplx* d_csmall = nullptr;     // 64 complex
     int* d_status = nullptr;
     double* d_lfac = nullptr;     // sqrt((l-m)!/(l+m)!) table up to degree 16
     // GMRES preconditioner settings (tcu_context_set_learned_weights)
@@ -972,9 +970,7 @@ tcu_status tcu_context_create(int device, tcu_context** out) {
     ctx->device = device;
     CK(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking), "stream");
     CK(cudaMalloc(&ctx->d_partial, 8 * 256 * sizeof(double)), "scratch");
-    CK(cudaMalloc(&ctx->d_cpartial, 64 * 256 * sizeof(cplx)), "scratch");
     CK(cudaMalloc(&ctx->d_small, 64 * sizeof(double)), "scratch");
-    CK(cudaMalloc(&ctx->d_csmall, 64 * sizeof(cplx)), "scratch");
     CK(cudaMalloc(&ctx->d_status, 16), "scratch");
     std::vector<double> lfac(17 * 17);
     for (int l = 0; l <= 16; ++l)
@@ -998,9 +994,7 @@ tcu_status tcu_context_destroy(tcu_context* ctx) {
     ctx->pool.release();
     ctx->ring.release();
     cudaFree(ctx->d_partial);
-    cudaFree(ctx->d_cpartial);
     cudaFree(ctx->d_small);
-    cudaFree(ctx->d_csmall);
     cudaFree(ctx->d_status);
     cudaFree(ctx->d_lfac);
     cudaStreamDestroy(ctx->stream);
@@ -1421,6 +1415,11 @@ tcu_status gmres_device(tcu_context* ctx, const std::function<void(const cplx*, 
     cplx* r = w + n;
     cplx* z = r + n;                      // preconditioned vector
     cplx* Z = z + n;                      // preconditioned basis (restart * n) when pre
+    DevBuf sums(ctx);                     // of any restart length
+    CK(sums.alloc(((size_t)restart * 256 + 2 * restart + 1) * 16 + ARNOLDI_PARTS * 8), "GMRES sums");
+    cplx* partial = (cplx*)sums.p;
+    cplx* coef = partial + (size_t)restart * 256;
+    double* npart = (double*)(coef + 2 * restart + 1);
     cudaStream_t st = ctx->stream;
     CK(cudaMemsetAsync(x, 0, n * 16, st), "zero");
     CK(cudaMemcpyAsync(r, rhs, n * 16, cudaMemcpyDeviceToDevice, st), "copy");
@@ -1434,7 +1433,7 @@ tcu_status gmres_device(tcu_context* ctx, const std::function<void(const cplx*, 
     int iterations = 0;
     std::vector<std::complex<double>> h((size_t)(restart + 1) * restart), g(restart + 1);
     std::vector<std::pair<double, std::complex<double>>> rot;
-    std::vector<std::complex<double>> hp(restart + 1);
+    std::vector<std::complex<double>> hp(2 * restart + 1);
     while (true) {
         cert->iterations = iterations;
         cert->residual_norm = rnorm;
@@ -1459,19 +1458,12 @@ tcu_status gmres_device(tcu_context* ctx, const std::function<void(const cplx*, 
                 vin = Z + (size_t)j * n;
             }
             op(vin, w);
-            for (int pass = 0; pass < 2; ++pass) {
-                vec_dots(V, n, j + 1, w, n, ctx->d_csmall, ctx->d_cpartial, st);
-                vec_gemv_sub(w, V, n, j + 1, ctx->d_csmall, n, st);
-                CK(cudaMemcpyAsync(hp.data(), ctx->d_csmall, (j + 1) * 16, cudaMemcpyDeviceToHost, st), "dots");
-                if ((s = sync_status(ctx, "gmres"))) return s;
-                for (int i = 0; i <= j; ++i) h[(size_t)j * (restart + 1) + i] += hp[i];
-                ctx->launches += 3;
-            }
-            double next = 0;
-            vec_norms(w, n, 1, ctx->d_small, ctx->d_partial, st);
-            CK(cudaMemcpyAsync(&next, ctx->d_small, 8, cudaMemcpyDeviceToHost, st), "norm");
+            vec_arnoldi_step(V, n, j + 1, w, n, V + (size_t)(j + 1) * n, coef, partial, npart, st);
+            CK(cudaMemcpyAsync(hp.data(), coef, (2 * j + 3) * 16, cudaMemcpyDeviceToHost, st), "dots");
             if ((s = sync_status(ctx, "gmres"))) return s;
-            ctx->launches += 2;
+            for (int i = 0; i <= j; ++i) h[(size_t)j * (restart + 1) + i] = hp[i] + hp[j + 1 + i];
+            const double next = hp[2 * j + 2].real();
+            ctx->launches += 5;
             h[(size_t)j * (restart + 1) + j + 1] = next;
             for (size_t i = 0; i < rot.size(); ++i) {
                 size_t off = (size_t)j * (restart + 1) + i;
@@ -1495,16 +1487,14 @@ tcu_status gmres_device(tcu_context* ctx, const std::function<void(const cplx*, 
             used = j + 1;
             iterations += 1;
             if (std::abs(g[j + 1]) <= tol || next == 0.0 || iterations == opt.max_iterations) break;
-            vec_scale_copy(V + (size_t)(j + 1) * n, w, n, 1.0 / next, st);
-            ++ctx->launches;
         }
         for (int i = used - 1; i >= 0; --i) {
             std::complex<double> tail = 0.0;
             for (int jj = i + 1; jj < used; ++jj) tail += h[(size_t)jj * (restart + 1) + i] * g[jj];
             g[i] = (g[i] - tail) / h[(size_t)i * (restart + 1) + i];
         }
-        CK(cudaMemcpyAsync(ctx->d_csmall, g.data(), used * 16, cudaMemcpyHostToDevice, st), "coefficients");
-        vec_lincomb(x, pre ? Z : V, n, used, ctx->d_csmall, n, st);
+        CK(cudaMemcpyAsync(coef, g.data(), used * 16, cudaMemcpyHostToDevice, st), "coefficients");
+        vec_lincomb(x, pre ? Z : V, n, used, coef, n, st);
         // true residual r = rhs - A x
         op(x, r);
         vec_sub(r, rhs, r, n, 1, st);

@@ -506,7 +506,7 @@ class IterativeCoarse : public CoarseSolve {
     const DevPlan* plan = nullptr;
     const double* pos = nullptr;
     const cplx* T = nullptr;
-    DevArray V, w, h, small, dpart;
+    DevArray V, w, h, small, dpart, npart;
     const StoredDipole* stored = nullptr;  // tables of A_cc, when built
     long long* launches = nullptr;
     bool build(const DevPlan& P, int N_, double k, const double* d_pos, const cplx* d_T, int restart,
@@ -521,7 +521,8 @@ class IterativeCoarse : public CoarseSolve {
         max_it = max_iterations;
         rtol = tol;
         return V.alloc((size_t)(m + 1) * nc * sizeof(cplx)) && w.alloc((size_t)nc * sizeof(cplx)) &&
-               h.alloc((size_t)(m + 1) * sizeof(cplx)) && small.alloc(64 * sizeof(double)) &&
+               h.alloc((size_t)(2 * m + 1) * sizeof(cplx)) && small.alloc(64 * sizeof(double)) &&
+               npart.alloc(ARNOLDI_PARTS * sizeof(double)) &&
                dpart.alloc((size_t)std::max(m + 1, 8) * 256 * sizeof(cplx));
     }
     // y = A_cc x = x - R T C P x
@@ -545,27 +546,21 @@ class IterativeCoarse : public CoarseSolve {
         if (!(beta > 0.0)) return TCU_OK;
         cplx* Vb = V.as<cplx>();
         vec_scale_copy(Vb, v, nc, 1.0 / beta, st);
-        std::vector<std::complex<double>> H((size_t)(m + 1) * m, 0.0), g(m + 1, 0.0), hp(m + 1);
+        std::vector<std::complex<double>> H((size_t)(m + 1) * m, 0.0), g(m + 1, 0.0), hp(2 * m + 1);
         std::vector<std::pair<double, std::complex<double>>> rot;
         g[0] = beta;
         int used = 0;
         const int iters = std::min(m, max_it);
         for (int j = 0; j < iters; ++j) {
             matvec(Vb + (size_t)j * nc, w.as<cplx>(), st);
-            for (int pass = 0; pass < 2; ++pass) {
-                vec_dots(Vb, nc, j + 1, w.as<cplx>(), nc, h.as<cplx>(), dpart.as<cplx>(), st);
-                vec_gemv_sub(w.as<cplx>(), Vb, nc, j + 1, h.as<cplx>(), nc, st);
-                if (cudaMemcpyAsync(hp.data(), h.p, (j + 1) * 16, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-                    cudaStreamSynchronize(st) != cudaSuccess)
-                    return TCU_DEVICE_ERROR;
-                for (int i = 0; i <= j; ++i) H[(size_t)j * (m + 1) + i] += hp[i];
-            }
-            double next = 0.0;
-            vec_norms(w.as<cplx>(), nc, 1, small.as<double>(), dpart.as<double>(), st);
-            if (cudaMemcpyAsync(&next, small.p, 8, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+            vec_arnoldi_step(Vb, nc, j + 1, w.as<cplx>(), nc, Vb + (size_t)(j + 1) * nc, h.as<cplx>(), dpart.as<cplx>(),
+                             npart.as<double>(), st);
+            if (cudaMemcpyAsync(hp.data(), h.p, (2 * j + 3) * 16, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
                 cudaStreamSynchronize(st) != cudaSuccess)
                 return TCU_DEVICE_ERROR;
-            if (launches) *launches += 8;
+            for (int i = 0; i <= j; ++i) H[(size_t)j * (m + 1) + i] = hp[i] + hp[j + 1 + i];
+            const double next = hp[2 * j + 2].real();
+            if (launches) *launches += 5;
             H[(size_t)j * (m + 1) + j + 1] = next;
             for (size_t i = 0; i < rot.size(); ++i) {
                 const size_t off = (size_t)j * (m + 1) + i;
@@ -588,7 +583,6 @@ class IterativeCoarse : public CoarseSolve {
             used = j + 1;
             ++inner_iterations;
             if (std::abs(g[j + 1]) <= rtol * beta || next == 0.0) break;
-            vec_scale_copy(Vb + (size_t)(j + 1) * nc, w.as<cplx>(), nc, 1.0 / next, st);
         }
         for (int i = used - 1; i >= 0; --i) {
             std::complex<double> tail = 0.0;

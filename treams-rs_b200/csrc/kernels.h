@@ -334,9 +334,10 @@ void lu_init_attributes();
 void vec_norms(const cplx* x, size_t n, int ncol, double* out_dev, double* partial, cudaStream_t st);
 void vec_axpy(cplx* y, const cplx* x, size_t n, int ncol, cudaStream_t st);
 void vec_sub(cplx* out, const cplx* a, const cplx* b, size_t n, int ncol, cudaStream_t st);
-void vec_dots(const cplx* V, size_t ldv, int nv, const cplx* w, size_t n, cplx* out_dev, cplx* partial,
-              cudaStream_t st);
-void vec_gemv_sub(cplx* w, const cplx* V, size_t ldv, int nv, const cplx* h_dev, size_t n, cudaStream_t st);
+constexpr int ARNOLDI_PARTS = 592;  // partial sums of a norm: four CTAs per SM
+// coef: 2 nv + 1 entries, partial: 256 nv, npart: ARNOLDI_PARTS
+void vec_arnoldi_step(const cplx* V, size_t ldv, int nv, cplx* w, size_t n, cplx* next, cplx* coef, cplx* partial,
+                      double* npart, cudaStream_t st);
 void vec_scale_copy(cplx* out, const cplx* x, size_t n, double s, cudaStream_t st);
 void vec_lincomb(cplx* x, const cplx* V, size_t ldv, int nv, const cplx* g_dev, size_t n, cudaStream_t st);
 void vec_real_dots(const cplx* a, const cplx* b, size_t n, int ncol, double* out_dev, double* partial,
