@@ -227,21 +227,19 @@ __global__ void __launch_bounds__(256) trsv_inv_step_kernel(const C* __restrict_
 // needs until both halves differ, so a step of the chain costs one store and one load through L2
 // and no fence, flag or second read.
 //
-// What bounds it: with few columns the chain of n / 64 dependent steps (a step: poll, one tile,
-// reduction, the diagonal product), with many columns the FP64 arithmetic, n^2 NC / 2 complex
-// multiply-adds a chunk. Hence at most 4 columns a chunk, all chunks side by side on the SMs:
-// a tile of 4 columns takes about 0.5 us of an SM's FP64 rate, below the latency of a step.
+// This kernel serves one and two columns, where the chain of n / 64 dependent steps bounds it (a step:
+// poll, one tile, reduction, the diagonal product: 1.4 us at one column, 1.8 at two) or, with few CTAs, its
+// 0.8 us a tile.
 // Tiles arrive by cp.async (3 stages of 32 KB for FP32 factors, 2 of 64 KB for FP64), padded to 65
 // rows so that the transposed reads of the adjoint sweeps have no bank conflicts either.
-// Measured against one launch per 8 columns with completion flags behind fences (both sides us per
-// triangle): n = 9600, 17 columns, FP32 factor 2320 -> 840; n = 1920, 96 columns, FP64 2340 -> 190;
-// n = 24576, 3 columns, FP32 1980 -> 1150; one column 2.6 -> 1.5 us per block step.
+// Measured against one launch per 8 columns with completion flags behind fences: one column
+// 2.6 -> 1.5 us per block step.
 // Every poll is bounded (4 s): status 8 and all CTAs return.
 constexpr int SW_THREADS = 512;
 constexpr int SW_Q = SW_THREADS / SB;  // contraction groups of a tile
 constexpr int SW_K = SB / SW_Q;        // contraction entries per thread and tile
 constexpr int SW_LD = SB + 1;
-constexpr int SW_MAXC = 4;             // columns per chunk
+constexpr int SW_MAXC = 2;             // columns per chunk
 
 __device__ __forceinline__ unsigned long long sw_ns() {
     unsigned long long t;
@@ -418,6 +416,264 @@ __global__ void __launch_bounds__(SW_THREADS, 1)
     }
 }
 
+// ---- persistent sweeps on the FP64 tensor cores -------------------------------------------
+// The same chain for three and more columns, in chunks of four: the 4 complex columns are the 8 real columns
+// [re y | im y] of m8n8k4 products, acc1 = Re T [re y | im y] and acc2 = Im T [re y | im y], two products per 8
+// rows and 4 entries. Roles instead of CTA-wide barriers: 8 product warps (a row octet each, so no
+// sums cross warps), four that stream the tiles into a ring (16-byte copies; one bulk copy per column of a tile
+// took 2.3 us a tile whatever its size), and four that poll the block solutions, a column each, and lay them out as fragments in a second ring.
+// Bound by the FP64 rate, 0.53 us a tile (1.0 measured), with many block rows per CTA; by the chain (poll, tile,
+// diagonal product, 2.2 us) with few. us per triangle against sweep_kernel at 4 columns a chunk, whose
+// 8-byte copies, conversions and CTA barrier took 1.9 us a tile: n = 9600, 17 columns, FP32 factor 840 -> 485,
+// 64 columns 2305 -> 1230; n = 1920, 96 columns, FP64 190 -> 105; n = 24576, 3 columns, FP32 1140 -> 935.
+// Several chains of products per warp or twice the warps with half of the entries each: no faster.
+// Tile columns are SD_LD entries apart, so that the fragments of a tile and of its adjoint (FP64: of the one
+// the sweep reads) come without bank conflicts. n is even (checked by the launch), so that every column of
+// a tile starts on 16 bytes and is a multiple of them long.
+constexpr int SD_COLS = 4, SD_WARPS = 8, SD_LOADERS = 4, SD_THREADS = (SD_WARPS + SD_COLS + SD_LOADERS) * 32;
+template <typename C>
+constexpr int sd_stages() {
+    return sizeof(C) == 8 ? 5 : 3;
+}
+template <typename C>
+constexpr int sd_yring() {
+    return sizeof(C) == 8 ? 4 : 3;
+}
+template <typename C, bool ADJ>
+constexpr int sd_ld() {
+    return sizeof(C) == 8 || ADJ ? 68 : 66;
+}
+template <typename C, bool ADJ>
+constexpr size_t sd_smem_bytes() {
+    return (size_t)sd_stages<C>() * SB * sd_ld<C, ADJ>() * sizeof(C) + (size_t)(sd_yring<C>() + 2) * 512 * sizeof(double);
+}
+__device__ __forceinline__ void sd_init(uint64_t* bar, int count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(bar)), "r"(count)
+                 : "memory");
+}
+__device__ __forceinline__ void sd_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"((unsigned)__cvta_generic_to_shared(bar)) : "memory");
+}
+__device__ __forceinline__ bool sd_try(uint64_t* bar, unsigned parity) {
+    unsigned ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"((unsigned)__cvta_generic_to_shared(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+// false when the CTA has given up or after 5 s (a poll gives up after 4)
+__device__ __forceinline__ bool sd_wait(uint64_t* bar, unsigned parity, volatile int* gave_up) {
+    if (sd_try(bar, parity)) return true;
+    unsigned long long t0 = 0;
+    for (unsigned it = 1;; ++it) {
+        if (sd_try(bar, parity)) return true;
+        if ((it & 63u) == 0) {
+            if (*gave_up) return false;
+            const unsigned long long now = sw_ns();
+            if (!t0) t0 = now;
+            if (now - t0 > 5000000000ull) {
+                *gave_up = 1;
+                return false;
+            }
+        }
+    }
+}
+__device__ __forceinline__ void sd_dmma(double (&c)[2], double a, double b) {
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+        : "+d"(c[0]), "+d"(c[1])
+        : "d"(a), "d"(b));
+}
+// acc1, acc2 -> this lane's two entries of the complex product: columns 2 q, 2 q + 1 of [re | im], q = lane % 4
+template <bool ADJ>
+__device__ __forceinline__ void sd_join(const double (&a1)[2], const double (&a2)[2], int q, double (&v)[2]) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const double o = __shfl_xor_sync(0xffffffffu, a2[u], 2);
+        v[u] = ((q < 2) != ADJ) ? a1[u] - o : a1[u] + o;
+    }
+}
+
+template <typename C, int OP>
+__global__ void __launch_bounds__(SD_THREADS, 1)
+    sweep_dmma_kernel(const C* __restrict__ A, size_t lda, int n, int nb, int ncol, const double2* __restrict__ dinv,
+                      const double2* __restrict__ rhs, double2* sol, double2* clear, int* status) {
+    constexpr bool DOWN = OP == SW_L || OP == SW_UH, ADJ = OP == SW_UH || OP == SW_LH;
+    constexpr int ST = sd_stages<C>(), YR = sd_yring<C>(), LD = sd_ld<C, ADJ>(), TILE = SB * LD;
+    extern __shared__ __align__(128) unsigned char sd_smem[];
+    C* tiles = reinterpret_cast<C*>(sd_smem);                    // [ST][SB][LD]: column k at k * LD
+    double* ys = reinterpret_cast<double*>(tiles + ST * TILE);   // [YR][16][32]: fragments of y
+    double* ss = ys + YR * 512;                            // [2][16][32]: fragments of a block's sums
+    __shared__ __align__(8) uint64_t bars[2 * ST + 2 * YR];
+    __shared__ int s_gave_up;
+    uint64_t *full = bars, *empty = bars + ST, *yfull = bars + 2 * ST, *yempty = yfull + YR;
+    volatile int* gave_up = &s_gave_up;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int col0 = blockIdx.y * SD_COLS, nc = min(SD_COLS, ncol - col0);
+    rhs += (size_t)col0 * n;
+    sol += (size_t)col0 * n;
+    if (clear) {
+        clear += (size_t)col0 * n;
+        const double e = __longlong_as_double(-1ll);
+        for (size_t i = (size_t)blockIdx.x * SD_THREADS + tid; i < (size_t)nc * n; i += (size_t)gridDim.x * SD_THREADS)
+            clear[i] = make_double2(e, e);
+    }
+    if (tid == 0) {
+        for (int i = 0; i < ST; ++i) {
+            sd_init(full + i, 32 * SD_LOADERS);
+            sd_init(empty + i, SD_WARPS);
+        }
+        for (int i = 0; i < YR; ++i) {
+            sd_init(yfull + i, 32 * SD_COLS);
+            sd_init(yempty + i, SD_WARPS);
+        }
+        s_gave_up = 0;
+    }
+    __syncthreads();
+    auto blk = [&](int t) { return DOWN ? t : nb - 1 - t; };
+    if (warp >= SD_WARPS + SD_COLS) {  // tiles
+        constexpr int PER = 16 / sizeof(C), COLS = 32 * PER == SB ? 1 : 2;  // entries a copy, instructions a column
+        const int lw = warp - SD_WARPS - SD_COLS;
+        int seq = 0;
+        bool ok = true;
+        for (int t = blockIdx.x; ok && t < nb; t += gridDim.x)
+            for (int ts = 0; ts < t; ++ts, ++seq) {
+                const int s = seq % ST;
+                if (!(ok = __all_sync(0xffffffffu, sd_wait(empty + s, ((seq / ST) & 1) ^ 1, gave_up)))) break;
+                const int ri = (ADJ ? blk(ts) : blk(t)) * SB, ci = (ADJ ? blk(t) : blk(ts)) * SB;
+                C* dst = tiles + s * TILE;
+#pragma unroll 8
+                for (int k = lw; k < SB; k += SD_LOADERS)
+#pragma unroll
+                    for (int h = 0; h < COLS; ++h) {
+                        const int row = (h * 32 + lane) * PER;
+                        const bool in = ci + k < n && ri + row < n;  // n is even: both entries of a copy or none
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                                         (unsigned)__cvta_generic_to_shared(dst + k * LD + row)),
+                                     "l"(in ? A + (size_t)(ci + k) * lda + ri + row : A), "r"(in ? 16 : 0)
+                                     : "memory");
+                    }
+                asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(
+                                 (unsigned)__cvta_generic_to_shared(full + s))
+                             : "memory");
+            }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    } else if (warp >= SD_WARPS) {  // block solutions: a column each, two entries a lane
+        const int c = warp - SD_WARPS;
+        const double2* yp = sol + (size_t)min(c, nc - 1) * n;
+        int seq = 0;
+        bool ok = true;
+        double2 pre[2];
+        auto fetch = [&](int ts) {
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int at = blk(ts) * SB + lane + 32 * u;
+                pre[u] = c < nc && at < n ? sw_load(yp + at) : make_double2(0.0, 0.0);
+            }
+        };
+        for (int t = blockIdx.x; ok && t < nb; t += gridDim.x) {
+            if (t > 0) fetch(0);
+            for (int ts = 0; ts < t; ++ts, ++seq) {
+                const int s = seq % YR;
+                unsigned long long t0 = 0;
+                for (unsigned spins = 1;; ++spins) {
+                    const bool e0 = sw_empty(pre[0].x) || sw_empty(pre[0].y), e1 = sw_empty(pre[1].x) || sw_empty(pre[1].y);
+                    if (!__any_sync(0xffffffffu, e0 || e1)) break;
+                    if ((spins & 255u) == 0) {  // the clock is read on long waits only
+                        const unsigned long long now = sw_ns();
+                        if (!t0) t0 = now;
+                        if (__any_sync(0xffffffffu, *(volatile int*)status == 8 || now - t0 > 4000000000ull)) {
+                            atomicExch(status, 8);
+                            ok = false;
+                            break;
+                        }
+                    }
+                    if (e0) pre[0] = sw_load(yp + blk(ts) * SB + lane);
+                    if (e1) pre[1] = sw_load(yp + blk(ts) * SB + lane + 32);
+                }
+                const double2 v0 = pre[0], v1 = pre[1];
+                if (ok && ts + 1 < t) fetch(ts + 1);
+                if (ok) ok = __all_sync(0xffffffffu, sd_wait(yempty + s, ((seq / YR) & 1) ^ 1, gave_up));
+                if (!ok) {
+                    *gave_up = 1;
+                    break;
+                }
+                double* y = ys + s * 512 + (lane >> 2) * 32 + c * 4 + (lane & 3);
+                y[0] = v0.x;
+                y[16] = v0.y;
+                y[256] = v1.x;
+                y[256 + 16] = v1.y;
+                sd_arrive(yfull + s);
+            }
+        }
+    } else {
+        const int r = lane >> 2, q = lane & 3, o = warp * 8 + r;  // this lane's row of a block
+        const int c = (2 * q) & 3;                                // its columns c, c + 1 (re: q < 2, im: q >= 2)
+        int seq = 0, turn = 0;
+        bool ok = true;
+        for (int t = blockIdx.x; t < nb; t += gridDim.x, ++turn) {
+            const int bi = blk(t), r0 = bi * SB;
+            double2 d[16];
+#pragma unroll
+            for (int g = 0; g < 16; ++g)
+                d[g] = __ldg(&dinv[(size_t)bi * SB * SB + (ADJ ? o * SB + 4 * g + q : (4 * g + q) * SB + o)]);
+            double b[2] = {0.0, 0.0};
+            const bool in = r0 + o < n;
+#pragma unroll
+            for (int u = 0; u < 2; ++u)
+                if (in && c + u < nc) {
+                    const double2 v = rhs[(size_t)(c + u) * n + r0 + o];
+                    b[u] = q < 2 ? v.x : v.y;
+                }
+            double a1[2] = {0.0, 0.0}, a2[2] = {0.0, 0.0}, v[2];
+            for (int ts = 0; ts < t; ++ts, ++seq) {
+                const int s = seq % ST, sy = seq % YR;
+                // (a warp that gives up goes on to the barrier of every block row, so that none waits there)
+                ok = ok && sd_wait(full + s, (seq / ST) & 1, gave_up) && sd_wait(yfull + sy, (seq / YR) & 1, gave_up);
+                if (!(ok = __all_sync(0xffffffffu, ok))) break;
+                const C* tile = tiles + s * TILE + (ADJ ? o * LD + q : q * LD + o);
+                const double* y = ys + sy * 512 + lane;
+#pragma unroll
+                for (int g = 0; g < 16; ++g) {
+                    const double2 m = to_d2(tile[ADJ ? 4 * g : 4 * g * LD]);
+                    const double yv = y[g * 32];
+                    sd_dmma(a1, m.x, yv);
+                    sd_dmma(a2, m.y, yv);
+                }
+                __syncwarp();
+                if (lane == 0) {
+                    sd_arrive(empty + s);
+                    sd_arrive(yempty + sy);
+                }
+            }
+            sd_join<ADJ>(a1, a2, q, v);
+            double* sf = ss + (turn & 1) * 512;
+#pragma unroll
+            for (int u = 0; u < 2; ++u) sf[(o >> 2) * 32 + (2 * q + u) * 4 + (o & 3)] = in ? b[u] - v[u] : 0.0;
+            asm volatile("bar.sync 1, 256;" ::: "memory");
+            a1[0] = a1[1] = a2[0] = a2[1] = 0.0;
+#pragma unroll
+            for (int g = 0; g < 16; ++g) {
+                const double sv = sf[g * 32 + lane];
+                sd_dmma(a1, d[g].x, sv);
+                sd_dmma(a2, d[g].y, sv);
+            }
+            sd_join<ADJ>(a1, a2, q, v);
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const double im = __shfl_xor_sync(0xffffffffu, v[u], 2);
+                if (in && q < 2 && c + u < nc)
+                    sw_store(&sol[(size_t)(c + u) * n + r0 + o], make_double2(sw_value(v[u]), sw_value(im)));
+            }
+        }
+    }
+    __syncthreads();
+    if (tid == 0 && s_gave_up) atomicExch(status, 8);
+}
+
 static int g_sms = 0;
 
 template <typename C, bool LOWER, int NC>
@@ -510,12 +766,33 @@ static bool sweep_launch_nc(cudaStream_t st, const C* A, int n, const double2* d
 }
 
 template <typename C, int OP>
+static bool sweep_dmma_launch(cudaStream_t st, const C* A, int n, const double2* dinv, const double2* rhs, double2* sol,
+                              double2* clear, int ncol, int* status) {
+    static PerDeviceOnce attr;
+    constexpr size_t smem = sd_smem_bytes<C, OP == SW_UH || OP == SW_LH>();
+    once_per_device(attr, [&] {
+        cudaFuncSetAttribute(sweep_dmma_kernel<C, OP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    });
+    const int nb = (n + SB - 1) / SB, chunks = (ncol + SD_COLS - 1) / SD_COLS;
+    const int G = std::min(nb, g_sms / chunks);
+    if (G < 1) return false;
+    size_t lda = (size_t)n;
+    void* args[] = {(void*)&A, &lda, &n, (void*)&nb, &ncol, (void*)&dinv, (void*)&rhs, &sol, &clear, &status};
+    return cudaLaunchCooperativeKernel((void*)sweep_dmma_kernel<C, OP>, dim3(G, chunks), dim3(SD_THREADS), args, smem,
+                                       st) == cudaSuccess;
+}
+
+template <typename C, int OP>
 static bool sweep_launch(cudaStream_t st, const C* A, int n, const double2* dinv, const double2* rhs, double2* sol,
                          double2* clear, int ncol, int* status) {
+    // the tensor cores from 3 columns on: they take the time of 4 however many there are (us per triangle at 1, 2, 3
+    // and 4 columns, n = 1920 FP32: 64, 65, 66, 67 against 47, 61, 75, 89; 9600: 315, 315, 330, 341 against
+    // 217, 273, 345, 419). n = 2 nlm spheres is even; an odd order would stay on the other kernel.
+    if (n % 2 == 0 && ncol > SW_MAXC) return sweep_dmma_launch<C, OP>(st, A, n, dinv, rhs, sol, clear, ncol, status);
     switch (std::min(ncol, SW_MAXC)) {
 #define SW_CASE(K) \
     case K: return sweep_launch_nc<C, OP, K>(st, A, n, dinv, rhs, sol, clear, ncol, status);
-        SW_CASE(1) SW_CASE(2) SW_CASE(3) SW_CASE(4)
+        SW_CASE(1) SW_CASE(2)
 #undef SW_CASE
     }
     return false;
