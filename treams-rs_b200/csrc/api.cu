@@ -304,15 +304,18 @@ tcu_status sync_status(tcu_context* ctx, const char* what) {
     return cuda_check(e, what);
 }
 
-tcu_status read_status(tcu_context* ctx, const char* what) {
-    int st = 0;
-    CK(cudaMemcpyAsync(&st, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream), what);
-    tcu_status s = sync_status(ctx, what);
-    if (s != TCU_OK) return s;
+tcu_status status_of(int st, const char* what) {
     if (st == 5) return fail(TCU_SINGULAR, std::string(what) + ": numerically singular");
     if (st == 8) return fail(TCU_TIMEOUT, std::string(what) + ": a device-side wait gave up");
     if (st != 0) return fail(TCU_DEVICE_ERROR, std::string(what) + ": device status " + std::to_string(st));
     return TCU_OK;
+}
+
+tcu_status read_status(tcu_context* ctx, const char* what) {
+    int st = 0;
+    CK(cudaMemcpyAsync(&st, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream), what);
+    tcu_status s = sync_status(ctx, what);
+    return s != TCU_OK ? s : status_of(st, what);
 }
 
 template <typename T>
@@ -486,7 +489,6 @@ tcu_status factor_impl(tcu_context* ctx, int L, double k0, size_t N, const doubl
         CK(cudaMemsetAsync(f->wk.status, 0, sizeof(int), ctx->stream), "status");
         launch_mie(L, k0, (int)N, f->d_radii, f->d_eps, f->d_T, ctx->d_status, ctx->stream);
         ++ctx->launches;
-        if ((e = read_status(ctx, "Mie coefficients"))) break;
         launch_assemble(*P, (int)N, k0, f->d_pos, f->d_T, f->d_A, n, precision == TCU_MIXED, ctx->stream);
         ++ctx->launches;
         if (stored_full_supported(*P) && stored_tables_enabled()) {
@@ -501,6 +503,7 @@ tcu_status factor_impl(tcu_context* ctx, int L, double k0, size_t N, const doubl
                 cudaGetLastError();
             }
         }
+        if ((e = read_status(ctx, "Mie coefficients"))) break;
         {
             // equilibrate when an entry exceeds 10 (then the unit diagonal no longer bounds the
             // spread; linalg/mod.rs:137-228)
@@ -522,6 +525,12 @@ tcu_status factor_impl(tcu_context* ctx, int L, double k0, size_t N, const doubl
             e = fail(TCU_DEVICE_ERROR, "LU panel launch failed (cooperative launch or shared memory)");
             break;
         }
+        // the block inverses run while the host waits for the status (of a failed factor they are not used)
+        if ((e = cuda_check(ctx->pool.alloc((void**)&f->d_inv, lu_inverse_bytes((int)n)), "block inverses"))) break;
+        if (precision == TCU_FP64)
+            lu_block_inverses_fp64((const double2*)f->d_A, (int)n, f->d_inv, ctx->stream, &ctx->launches);
+        else
+            lu_block_inverses_fp32((const float2*)f->d_A, (int)n, f->d_inv, ctx->stream, &ctx->launches);
         int st = 0;
         if ((e = cuda_check(cudaMemcpyAsync(&st, f->wk.status, 4, cudaMemcpyDeviceToHost, ctx->stream), "LU"))) break;
         if ((e = sync_status(ctx, "LU factorization"))) break;
@@ -541,12 +550,6 @@ tcu_status factor_impl(tcu_context* ctx, int L, double k0, size_t N, const doubl
             e = fail(TCU_DEVICE_ERROR, "LU factorization: device status " + std::to_string(st));
             break;
         }
-        if ((e = cuda_check(ctx->pool.alloc((void**)&f->d_inv, lu_inverse_bytes((int)n)), "block inverses"))) break;
-        if (precision == TCU_FP64)
-            lu_block_inverses_fp64((const double2*)f->d_A, (int)n, f->d_inv, ctx->stream, &ctx->launches);
-        else
-            lu_block_inverses_fp32((const float2*)f->d_A, (int)n, f->d_inv, ctx->stream, &ctx->launches);
-        if ((e = sync_status(ctx, "block inverses"))) break;
     } while (0);
     if (e) {
         cleanup();
@@ -628,8 +631,28 @@ int max_refinement_sweeps(const tcu_factor* f) {
 
 bool settles(const tcu_factor* f) { return f->precision == TCU_MIXED && f->wk.pieces == PIECES_BF16; }
 
-// device scratch of vec_norms over p columns: p norms and 256 partial sums a column
-size_t norm_scratch(int p) { return (size_t)p * 257 * sizeof(double); }
+// Norms of a solve's p right-hand-side columns and residuals and a status word, side by side so that one copy
+// brings them to the host: a copy each kept the device idle for about 15 us at a time.
+struct SolveNorms {
+    int p;
+    double* d;  // p + p norms, the status, 256 partial sums a column
+    std::vector<double> h;
+    SolveNorms(int p_, void* mem) : p(p_), d((double*)mem), h(2 * (size_t)p_ + 1) {}
+    static size_t bytes(int p) { return ((size_t)p * 258 + 1) * sizeof(double); }
+    void rhs(const cplx* v, size_t n, cudaStream_t st) { vec_norms(v, n, p, d, d + 2 * p + 1, st); }
+    void residual(const cplx* r, size_t n, cudaStream_t st) { vec_norms(r, n, p, d + p, d + 2 * p + 1, st); }
+    // waits for the stream
+    tcu_status fetch(tcu_context* ctx, const int* status, std::vector<double>& bn, std::vector<double>& rn, int* st) {
+        CK(cudaMemcpyAsync(d + 2 * p, status, sizeof(int), cudaMemcpyDeviceToDevice, ctx->stream), "status");
+        CK(cudaMemcpyAsync(h.data(), d, h.size() * 8, cudaMemcpyDeviceToHost, ctx->stream), "norms");
+        const tcu_status s = sync_status(ctx, "residual");
+        if (s) return s;
+        std::copy(h.begin(), h.begin() + p, bn.begin());
+        std::copy(h.begin() + p, h.begin() + 2 * p, rn.begin());
+        memcpy(st, &h[2 * p], sizeof(int));
+        return TCU_OK;
+    }
+};
 
 tcu_status solve_impl(tcu_factor* f, const double* B, int p, double* X, tcu_certificate* certs, bool device) {
     if (!f || !B || !X || p <= 0) return fail(TCU_INVALID_INPUT, "require a factor and at least one column");
@@ -656,22 +679,21 @@ tcu_status solve_impl(tcu_factor* f, const double* B, int p, double* X, tcu_cert
     DevBuf bufs(ctx);
     size_t per = n * p;
     const size_t xf_bytes = f->d_Z ? stored_inputs_bytes(*P, f->N, STORED_FULL, p) : 0;
-    CK(bufs.alloc(6 * per * sizeof(cplx) + xf_bytes + norm_scratch(p)), "solve buffers");
+    CK(bufs.alloc(6 * per * sizeof(cplx) + xf_bytes + SolveNorms::bytes(p)), "solve buffers");
     cplx* b = (cplx*)bufs.p;
     cplx* tb = b + per;
     cplx* x = tb + per;
     cplx* r = x + per;
     cplx* tmp = r + per;  // 2 per
     cplx* xf = tmp + 2 * per;  // packed inputs of the stored-table residual
-    double* d_norm = (double*)((char*)xf + xf_bytes);  // p norms, then their partial sums
+    SolveNorms norms(p, (char*)xf + xf_bytes);
     CK(cudaMemcpyAsync(b, B, per * 16, device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, ctx->stream),
        "copy rhs");
     launch_apply_t(f->L, f->N, f->d_T, b, p, tb, ctx->stream);
     ++ctx->launches;
     std::vector<double> rn(p), bn(p);
-    vec_norms(tb, n, p, d_norm, d_norm + p, ctx->stream);
+    norms.rhs(tb, n, ctx->stream);
     ctx->launches += 2;
-    CK(cudaMemcpyAsync(bn.data(), d_norm, p * 8, cudaMemcpyDeviceToHost, ctx->stream), "norms");
     auto lu_apply = [&](cplx* v) {
         if (f->scaled) scale_rows(v, f->d_scale, n, p, ctx->stream);  // R v
         if (f->precision == TCU_FP64)
@@ -695,11 +717,9 @@ tcu_status solve_impl(tcu_factor* f, const double* B, int p, double* X, tcu_cert
         } else {
             apply_op(ctx, P, f->N, f->k0, f->d_pos, f->d_T, x, n, p, tb, -1.0, 1.0, true, r);
         }
-        vec_norms(r, n, p, d_norm, d_norm + p, ctx->stream);
+        norms.residual(r, n, ctx->stream);
         ctx->launches += 2;
-        CK(cudaMemcpyAsync(rn.data(), d_norm, p * 8, cudaMemcpyDeviceToHost, ctx->stream), "norms");
-        CK(cudaMemcpyAsync(&sweep_status, f->wk.status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream), "status");
-        tcu_status s2 = sync_status(ctx, "residual");
+        tcu_status s2 = norms.fetch(ctx, f->wk.status, bn, rn, &sweep_status);
         if (s2) return s2;
         if (sweep_status == 8) return fail(TCU_TIMEOUT, "refinement: a device-side wait gave up");
         return TCU_OK;
@@ -794,7 +814,7 @@ tcu_status solve_adjoint_impl(tcu_factor* f, const double* G, int p, double* Y, 
     DevBuf bufs(ctx);
     const size_t tmpc = adjoint_solve_tmp((int)n, p);
     const size_t xfc = f->d_Z ? stored_inputs_bytes(*P, f->N, STORED_FULL, p) / sizeof(cplx) : 0;
-    CK(bufs.alloc((5 * per + tmpc + xfc) * sizeof(cplx) + norm_scratch(p)), "adjoint solve buffers");
+    CK(bufs.alloc((5 * per + tmpc + xfc) * sizeof(cplx) + SolveNorms::bytes(p)), "adjoint solve buffers");
     cplx* g = (cplx*)bufs.p;
     cplx* y = g + per;
     cplx* r = y + per;
@@ -802,12 +822,11 @@ tcu_status solve_adjoint_impl(tcu_factor* f, const double* G, int p, double* Y, 
     cplx* t2 = t1 + per;
     cplx* xf = t2 + per;  // packed inputs of the stored-table coupling product
     cplx* tmp = xf + xfc;
-    double* d_norm = (double*)(tmp + tmpc);  // p norms, then their partial sums
+    SolveNorms norms(p, tmp + tmpc);
     CK(cudaMemsetAsync(ctx->d_status, 0, 4, ctx->stream), "status");
     CK(cudaMemcpyAsync(g, G, per * 16, cudaMemcpyHostToDevice, ctx->stream), "copy rhs");
     std::vector<double> rn(p), bn(p);
-    vec_norms(g, n, p, d_norm, d_norm + p, ctx->stream);
-    CK(cudaMemcpyAsync(bn.data(), d_norm, p * 8, cudaMemcpyDeviceToHost, ctx->stream), "norms");
+    norms.rhs(g, n, ctx->stream);
     auto lu_adjoint = [&](cplx* v) {
         if (f->scaled) scale_rows(v, f->d_scale + n, n, p, ctx->stream);  // C g
         if (f->precision == TCU_FP64)
@@ -822,10 +841,11 @@ tcu_status solve_adjoint_impl(tcu_factor* f, const double* G, int p, double* Y, 
         launch_apply_adjoint(*P, f->N, f->k0, f->d_pos, f->d_T, y, n, p, r, t1, t2, ctx->stream, &ctx->launches,
                              f->d_Z, xf, ctx->d_status);
         vec_sub(r, g, r, n, p, ctx->stream);
-        vec_norms(r, n, p, d_norm, d_norm + p, ctx->stream);
+        norms.residual(r, n, ctx->stream);
         ctx->launches += 3;
-        CK(cudaMemcpyAsync(rn.data(), d_norm, p * 8, cudaMemcpyDeviceToHost, ctx->stream), "norms");
-        return read_status(ctx, "adjoint residual");
+        int st = 0;
+        const tcu_status s2 = norms.fetch(ctx, ctx->d_status, bn, rn, &st);
+        return s2 ? s2 : status_of(st, "adjoint residual");
     };
     CK(cudaMemcpyAsync(y, g, per * 16, cudaMemcpyDeviceToDevice, ctx->stream), "copy");
     lu_adjoint(y);
@@ -1168,8 +1188,9 @@ tcu_status tcu_cross_sections(tcu_context* ctx, int lmax, double k0, size_t N, c
     size_t M = 2 * (size_t)lmax * (lmax + 2), n = N * M, per = n * p;
     DevBuf buf(ctx);
     Arena ar;
-    size_t o_pos = ar.add(N * 24), o_x = ar.add(3 * per * 16);
+    size_t o_pos = ar.add(N * 24), o_x = ar.add(3 * per * 16), o_sum = ar.add((size_t)p * 2 * 257 * 8);
     CK(buf.alloc(ar.total), "cross-section buffers");
+    double* sums = ar.at<double>(buf.p, o_sum);  // 2 p sums, then the partial sums of one after the other
     double* pos = ar.at<double>(buf.p, o_pos);
     cplx* dx = ar.at<cplx>(buf.p, o_x);
     cplx* db = dx + per;
@@ -1178,7 +1199,7 @@ tcu_status tcu_cross_sections(tcu_context* ctx, int lmax, double k0, size_t N, c
     CK(cudaMemcpyAsync(dx, x, per * 16, cudaMemcpyHostToDevice, ctx->stream), "copy");
     CK(cudaMemcpyAsync(db, b, per * 16, cudaMemcpyHostToDevice, ctx->stream), "copy");
     DevBuf zbuf(ctx), xfbuf(ctx);
-    const bool stored = !apply_gemm_supported(*P) && use_stored_tables(*P, (int)N);
+    bool stored = !apply_gemm_supported(*P) && use_stored_tables(*P, (int)N);
     if (stored && zbuf.alloc(stored_tables_bytes(*P, (int)N, STORED_FULL)) == cudaSuccess &&
         xfbuf.alloc(stored_inputs_bytes(*P, (int)N, STORED_FULL, p)) == cudaSuccess) {
         // lmax 6 and 7: the regular operator from its pair tables, like the outgoing one
@@ -1187,22 +1208,22 @@ tcu_status tcu_cross_sections(tcu_context* ctx, int lmax, double k0, size_t N, c
         launch_apply_stored(*P, (int)N, STORED_FULL, (const cplx*)zbuf.p, nullptr, dx, n, p, nullptr, 1.0, 1.0, ox,
                             (cplx*)xfbuf.p, ctx->d_status, ctx->stream, false);
         ctx->launches += 4;
-        if ((s = read_status(ctx, "cross sections"))) return s;
     } else {
         cudaGetLastError();  // no room: the tables per pair
+        stored = false;
         apply_op(ctx, P, (int)N, k0, pos, nullptr, dx, n, p, nullptr, 1.0, 1.0, false, ox);
     }
-    std::vector<double> s1(p), s2(p);
-    vec_real_dots(dx, ox, n, p, ctx->d_small, ctx->d_partial, ctx->stream);
-    CK(cudaMemcpyAsync(s1.data(), ctx->d_small, p * 8, cudaMemcpyDeviceToHost, ctx->stream), "copy");
-    vec_real_dots(db, dx, n, p, ctx->d_small + 32, ctx->d_partial + 4 * 256, ctx->stream);
+    // both sums, then one copy: nothing waits in between
+    std::vector<double> s1(2 * (size_t)p);
+    vec_real_dots(dx, ox, n, p, sums, sums + 2 * p, ctx->stream);
+    vec_real_dots(db, dx, n, p, sums + p, sums + 2 * p, ctx->stream);
     ctx->launches += 4;
-    CK(cudaMemcpyAsync(s2.data(), ctx->d_small + 32, p * 8, cudaMemcpyDeviceToHost, ctx->stream), "copy");
-    s = sync_status(ctx, "cross sections");
+    CK(cudaMemcpyAsync(s1.data(), sums, s1.size() * 8, cudaMemcpyDeviceToHost, ctx->stream), "copy");
+    s = stored ? read_status(ctx, "cross sections") : sync_status(ctx, "cross sections");
     if (s) return s;
     for (int c = 0; c < p; ++c) {
         sca[c] = s1[c] / (k0 * k0);
-        ext[c] = -s2[c] / (k0 * k0);
+        ext[c] = -s1[p + c] / (k0 * k0);
     }
     return TCU_OK;
 }
