@@ -13,7 +13,7 @@
 //     of lo leave about 2^-17 of |a||b| per term. Twice the TF32 rate: 1.5 TF32 passes of tensor time.
 //   tf32x2: hi = tf32(x), lo = tf32(x - hi), two passes hi*hi + lo*hi of kind::tf32, the B operand rounded
 //     to TF32: about 2^-12 per term at 2 TF32 passes. 24576 modes, all updates of a factorization: 128 ms
-//     and a first residual of 2.5e-6, against 105 ms and 2.1e-7 of the bfloat16 pieces (9600 modes: 8.7 ms and
+//     and a first residual of 2.5e-6, against 105 ms and 2.1e-7 of the bfloat16 pieces on single CTAs (9600 modes: 8.7 ms and
 //     1.6e-6 against 7.2 ms and 1.7e-7), and the packing kernels write half the bytes (8.1 against 7.0 ms).
 //   tf32x3: the same pieces in three passes, 2^-22 per term; the format of fallback factors.
 //   f16: each row of each operand (a complex row of L21, a column of U12) is first scaled by its own
@@ -22,15 +22,19 @@
 //     accumulator entry by the exact power of two 1/(s_row s_col). Pieces below the FP16 normal
 //     range only lose absolute accuracy under 2^-38 of their row's maximum.
 //
-// Kernel layout (persistent, one CTA per SM, 192 threads):
-//   warp 0     TMA producer: 64-byte-swizzled boxes (64-byte K rows) of the four packed
-//              operands into a 4-stage shared-memory ring (48 KB per stage), mbarrier complete_tx;
-//   warp 1     TMEM allocator and MMA issuer (one thread): 2 K-steps x 2 or 3 passes per stage
-//              into a 128 x 256 FP32 accumulator, double-buffered in TMEM (512 columns);
-//   warps 2-5  epilogue: tcgen05.ld 32 columns at a time into a shared-memory staging buffer,
-//              TMA reduce-add of -D into A22.
+// Kernel layout (persistent, one CTA per SM, 192 threads, CTAs in pairs): a pair forms a 256 x 256 tile with
+// cta_group::2 products, each CTA staging its 128 rows of the A pieces and half of the B rows, so a chunk
+// brings 32 KB into an SM instead of 48. One CTA per 128 x 256 tile drew 64 bytes a clock and SM from L2, more than
+// L2 gives: 24576 modes 105 -> 90 ms (1.33 PFLOP/s executed, 94 % of the sustained bf16 rate), 17150 modes 37 -> 32.
+//   warp 0     TMA producer of each CTA: 64-byte-swizzled boxes (64-byte K rows) of the four packed operands
+//              into a 6-stage shared-memory ring (32 KB per stage), complete_tx on the leader's mbarrier;
+//   warp 1     TMEM allocator; in the leader the MMA issuer (one thread): 2 K-steps x 2 or 3 passes per stage
+//              into both CTAs' 128 x 256 FP32 accumulators, double-buffered in TMEM (512 columns); its
+//              commits free the stages and publish the accumulators in both CTAs;
+//   warps 2-5  epilogue of the CTA's 128 rows: tcgen05.ld 32 columns at a time into a shared-memory staging
+//              buffer, TMA reduce-add of -D into A22.
 // Every mbarrier wait is bounded; on timeout the kernel records status 8, drains its TMA
-// loads, frees TMEM and returns.
+// loads, frees TMEM and returns (the pair's last barrier is reached by both CTAs in any case).
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -48,13 +52,13 @@
 
 namespace tcu {
 
-constexpr int TB_M = 128;       // real rows per tile (64 complex rows)
-constexpr int TB_N = 256;       // columns per tile
+constexpr int TB_M = 128;       // real rows of a CTA (64 complex rows); a pair of CTAs takes 256
+constexpr int TB_N = 256;       // columns per tile; each CTA of the pair stages half of them
 constexpr int TB_K = 16;        // floats per K chunk (one 64-byte swizzle row); 32 for FP16 pieces
-constexpr int TB_STAGES = 4;
+constexpr int TB_STAGES = 6;
 constexpr int A_BYTES = TB_M * TB_K * 4;   // 8 KB
-constexpr int B_BYTES = TB_N * TB_K * 4;   // 16 KB
-constexpr int STAGE_BYTES = 2 * A_BYTES + 2 * B_BYTES;  // 48 KB
+constexpr int B_BYTES = TB_N / 2 * TB_K * 4;  // 8 KB
+constexpr int STAGE_BYTES = 2 * A_BYTES + 2 * B_BYTES;  // 32 KB
 constexpr int TMEM_COLS = 2 * TB_N;        // two accumulators
 constexpr int EPI_COLS = 32;                         // columns per epilogue staging buffer
 constexpr int EPI_BYTES = TB_M * EPI_COLS * 4;         // 16 KB
@@ -74,9 +78,6 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
 }
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
     uint32_t ok;
@@ -105,9 +106,29 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
 }
 
+// The leader's (rank 0) barrier of the pair, as a shared::cluster address.
+__device__ __forceinline__ uint32_t leader_bar(uint32_t bar) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(bar));
+    return r;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ uint32_t cta_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void pair_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// into this CTA's shared memory, completing on a barrier of either CTA of the pair
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
     asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], "
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], "
         "[%4];" ::"r"(dst),
         "l"((uint64_t)map), "r"(x), "r"(y), "r"(bar)
         : "memory");
@@ -124,7 +145,7 @@ __device__ __forceinline__ uint64_t swz_desc(uint32_t addr) {
     return d;
 }
 
-// Tile t of the persistent loop: groups of 16 M-tiles sweep all N-tiles, so the CTAs in
+// Tile t of the persistent loop: groups of 16 M-tiles (of 256 rows) sweep all N-tiles, so the CTAs in
 // flight share a few A and B tiles in L2.
 constexpr int TILE_GROUP = 16;
 __device__ __forceinline__ void tile_coords(int t, int tiles_m, int tiles_n, int& tm, int& tn) {
@@ -141,7 +162,7 @@ __device__ __forceinline__ void mma_tf32(uint32_t d_tmem, uint64_t a, uint64_t b
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+        "tcgen05.mma.cta_group::2.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
         "l"(a), "l"(b), "r"(idesc), "r"(acc)
         : "memory");
 }
@@ -149,7 +170,7 @@ __device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t a, uint64_t b,
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
         "l"(a), "l"(b), "r"(idesc), "r"(acc)
         : "memory");
 }
@@ -167,8 +188,12 @@ __device__ __forceinline__ float f16_scale(float mx) {
     frexpf(mx, &e);  // mx = f 2^e, 0.5 <= f < 1
     return ldexpf(1.0f, 14 - e);
 }
+// arrives on the barrier at this place in both CTAs of the pair
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+    asm volatile(
+        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+        "h"((uint16_t)3)
+        : "memory");
 }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -204,7 +229,7 @@ struct Tf32Args {
 };
 
 template <int PIECES>
-__global__ void __launch_bounds__(192, 1) tf32_update_kernel(const __grid_constant__ CUtensorMap mAhi,
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1) tf32_update_kernel(const __grid_constant__ CUtensorMap mAhi,
                                                              const __grid_constant__ CUtensorMap mAlo,
                                                              const __grid_constant__ CUtensorMap mBhi,
                                                              const __grid_constant__ CUtensorMap mBlo,
@@ -224,6 +249,7 @@ __global__ void __launch_bounds__(192, 1) tf32_update_kernel(const __grid_consta
     uint32_t* tmem_slot = (uint32_t*)(ctrl + 8 * (2 * TB_STAGES + 4));
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = (int)cta_rank(), pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
     auto bar = [&](int i) { return smem_u32(&bars[i]); };
     constexpr int EMPTY = TB_STAGES, TFULL = 2 * TB_STAGES, TEMPTY = 2 * TB_STAGES + 2;
     if (threadIdx.x == 0) {
@@ -233,24 +259,25 @@ __global__ void __launch_bounds__(192, 1) tf32_update_kernel(const __grid_consta
         }
         for (int a = 0; a < 2; ++a) {
             mbar_init(bar(TFULL + a), 1);
-            mbar_init(bar(TEMPTY + a), 128);
+            mbar_init(bar(TEMPTY + a), 2);  // (the leader's: one arrival per CTA)
         }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                      "r"(TMEM_COLS));
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
     }
     __syncthreads();
+    pair_sync();  // both CTAs' barriers are ready, both have their TMEM
     fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == 0) {
         if (lane == 0) {
             int step = 0;
-            for (int t = blockIdx.x; t < args.tiles && !*abort_flag; t += gridDim.x) {
+            for (int t = pair; t < args.tiles && !*abort_flag; t += pairs) {
                 int tm, tn;
                 tile_coords(t, args.tiles_m, args.tiles_n, tm, tn);
                 for (int kb = 0; kb < args.kchunks; ++kb, ++step) {
@@ -258,15 +285,19 @@ __global__ void __launch_bounds__(192, 1) tf32_update_kernel(const __grid_consta
                     uint32_t ph = (step / TB_STAGES) & 1;
                     if (!mbar_wait(bar(EMPTY + s), ph ^ 1, abort_flag)) break;
                     uint32_t st = tiles_smem + s * STAGE_BYTES;
-                    mbar_expect_tx(bar(s), TWO ? STAGE_BYTES - B_BYTES : STAGE_BYTES);
-                    tma_load_2d(st, &mAhi, kb * KC, tm * TB_M, bar(s));
-                    tma_load_2d(st + A_BYTES, &mAlo, kb * KC, tm * TB_M, bar(s));
-                    tma_load_2d(st + 2 * A_BYTES, &mBhi, kb * KC, tn * TB_N, bar(s));
-                    if (!TWO) tma_load_2d(st + 2 * A_BYTES + B_BYTES, &mBlo, kb * KC, tn * TB_N, bar(s));
+                    // the leader's barrier counts the bytes of both CTAs (the other's may come before this)
+                    if (rank == 0) mbar_expect_tx(bar(s), 2 * (TWO ? STAGE_BYTES - B_BYTES : STAGE_BYTES));
+                    const uint32_t fb = leader_bar(bar(s));
+                    const int ya = (2 * tm + rank) * TB_M, yb = tn * TB_N + rank * (TB_N / 2);
+                    tma_load_2d(st, &mAhi, kb * KC, ya, fb);
+                    tma_load_2d(st + A_BYTES, &mAlo, kb * KC, ya, fb);
+                    tma_load_2d(st + 2 * A_BYTES, &mBhi, kb * KC, yb, fb);
+                    if (!TWO) tma_load_2d(st + 2 * A_BYTES + B_BYTES, &mBlo, kb * KC, yb, fb);
                 }
             }
-            if (*abort_flag) {
-                // drain: wait (bounded) for the loads of every stage still in flight
+            if (*abort_flag && rank == 0) {
+                // drain: wait (bounded) for both CTAs' loads of every stage still in flight; the other CTA
+                // stays until the pair's last barrier
                 volatile int never = 0;
                 for (int s = 0; s < TB_STAGES; ++s) {
                     int last = step - 1 - ((step - 1 - s) % TB_STAGES + TB_STAGES) % TB_STAGES;
@@ -275,13 +306,13 @@ __global__ void __launch_bounds__(192, 1) tf32_update_kernel(const __grid_consta
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (lane == 0 && rank == 0) {
             // D F32; A, B TF32 (2), BF16 (1) or F16 (0); K-major; N >> 3 at bit 17, M >> 4 at bit 24
             const uint32_t ab = F16 ? 0u : (HALF ? 1u : 2u);
             const uint32_t idesc = (1u << 4) | (ab << 7) | (ab << 10) | ((uint32_t)(TB_N >> 3) << 17) |
-                                   ((uint32_t)(TB_M >> 4) << 24);
+                                   ((uint32_t)(2 * TB_M >> 4) << 24);
             int step = 0, it = 0;
-            for (int t = blockIdx.x; t < args.tiles && !*abort_flag; t += gridDim.x, ++it) {
+            for (int t = pair; t < args.tiles && !*abort_flag; t += pairs, ++it) {
                 int acc = it & 1;
                 uint32_t aph = (it >> 1) & 1;
                 if (!mbar_wait(bar(TEMPTY + acc), aph ^ 1, abort_flag)) break;
@@ -323,7 +354,7 @@ __global__ void __launch_bounds__(192, 1) tf32_update_kernel(const __grid_consta
         // FP16 pieces: -1 / (row scale x column scale) undoes the operand scaling exactly
         const int grow = R;  // row of the tile this thread stores
         int it = 0, e = 0;
-        for (int t = blockIdx.x; t < args.tiles; t += gridDim.x, ++it) {
+        for (int t = pair; t < args.tiles; t += pairs, ++it) {
             int acc = it & 1;
             uint32_t aph = (it >> 1) & 1;
             // one thread waits (bounded) and the four warps take its decision together, so a
@@ -334,12 +365,15 @@ __global__ void __launch_bounds__(192, 1) tf32_update_kernel(const __grid_consta
             fence_after();
             int tm, tn;
             tile_coords(t, args.tiles_m, args.tiles_n, tm, tn);
+            const int row0 = (2 * tm + rank) * TB_M;  // this CTA's first row
             float rowneg = -1.0f;
             if (F16) {
-                const int mu = (tm * TB_M + grow) >> 1;
+                const int mu = (row0 + grow) >> 1;
                 rowneg = mu < (args.m2 >> 1) ? -1.0f / __ldg(&args.sA[mu]) : -1.0f;
             }
-            for (int sub = 0; sub < TB_N / EPI_COLS; ++sub, ++e) {
+            // columns and rows past the block: nothing to add
+            const int subs = row0 < args.m2 ? (min(TB_N, args.ncols - tn * TB_N) + EPI_COLS - 1) / EPI_COLS : 0;
+            for (int sub = 0; sub < subs; ++sub, ++e) {
                 const int buf = e & 1;
                 if (issuer) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
                 asm volatile("bar.sync 1, 128;" ::: "memory");
@@ -363,7 +397,7 @@ __global__ void __launch_bounds__(192, 1) tf32_update_kernel(const __grid_consta
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 asm volatile("bar.sync 1, 128;" ::: "memory");
                 if (issuer) {
-                    int x = args.row0 + tm * TB_M, y = args.col0 + tn * TB_N + sub * EPI_COLS;
+                    int x = args.row0 + row0, y = args.col0 + tn * TB_N + sub * EPI_COLS;
                     asm volatile(
                         "cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(
                             (uint64_t)&mC),
@@ -373,15 +407,17 @@ __global__ void __launch_bounds__(192, 1) tf32_update_kernel(const __grid_consta
                 }
             }
             fence_before();
-            mbar_arrive(bar(TEMPTY + acc));
+            asm volatile("bar.sync 1, 128;" ::: "memory");
+            if (issuer) mbar_arrive_cluster(leader_bar(bar(TEMPTY + acc)));
         }
         if (issuer) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     }
     __syncthreads();
+    pair_sync();  // no product still reads the other CTA's stages, no arrival is on its way there
     if (*abort_flag && threadIdx.x == 0) atomicExch(args.status, 8);
     if (warp == 1) {
         fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS));
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS));
     }
 }
 
@@ -750,14 +786,29 @@ size_t tf32_pack_bytes(int n) {
     return ((size_t)2 * n * kp + (size_t)n * kp) * 2 * 4 + (size_t)128 * 128 * 8 + 8192;
 }
 
-static int num_sms() {
-    static const int sms = [] {
-        int dev = 0, v = 0;
+// CTA pairs the device holds at once
+static int num_pairs() {
+    static const int pairs = [] {
+        int dev = 0, sms = 0, n = 0;
         cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-        return v;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(2 * (sms / 2));
+        cfg.blockDim = dim3(192);
+        cfg.dynamicSmemBytes = TF32_SMEM;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 2;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&n, tf32_update_kernel<PIECES_BF16>, &cfg) != cudaSuccess || n < 1) {
+            cudaGetLastError();
+            n = sms / 2;
+        }
+        return std::min(n, sms / 2);
     }();
-    return sms;
+    return pairs;
 }
 
 // The packed operands live in the buffer the factor allocated from its context's pool
@@ -777,7 +828,7 @@ static void run_gemm(float2* A, int n, int row0, int col0, int m2, int ncols, in
     const bool half = pieces == PIECES_F16 || pieces == PIECES_BF16;
     CUtensorMap mAhi, mAlo, mBhi, mBlo;
     bool ok = make_map(&mAhi, ahi, m2, kp, TB_M, pieces) && make_map(&mAlo, alo, m2, kp, TB_M, pieces) &&
-              make_map(&mBhi, bhi, ncols, kp, TB_N, pieces) && make_map(&mBlo, blo, ncols, kp, TB_N, pieces);
+              make_map(&mBhi, bhi, ncols, kp, TB_N / 2, pieces) && make_map(&mBlo, blo, ncols, kp, TB_N / 2, pieces);
     // A viewed as a 2n x n float matrix (column-major): box of 128 real rows x 64 columns
     CUtensorMap mC;
     {
@@ -802,13 +853,13 @@ static void run_gemm(float2* A, int n, int row0, int col0, int m2, int ncols, in
     a.m2 = m2;
     a.ncols = ncols;
     a.kchunks = kp / (half ? 32 : TB_K);
-    a.tiles_m = (m2 + TB_M - 1) / TB_M;
+    a.tiles_m = (m2 + 2 * TB_M - 1) / (2 * TB_M);
     a.tiles_n = (ncols + TB_N - 1) / TB_N;
     a.tiles = a.tiles_m * a.tiles_n;
     a.status = wk.status;
     a.sA = sA;
     a.sB = sB;
-    int grid = std::min(num_sms(), a.tiles);
+    const int grid = 2 * std::min(num_pairs(), a.tiles);
     auto launch = [&](auto kernel) { kernel<<<grid, 192, TF32_SMEM, st>>>(mAhi, mAlo, mBhi, mBlo, mC, a); };
     switch (pieces) {
         case PIECES_BF16: launch(tf32_update_kernel<PIECES_BF16>); break;
