@@ -37,7 +37,7 @@ typedef enum tcu_status {
 
 typedef enum tcu_precision {
     TCU_FP64 = 0,   /* complex128 LU, FP64 DMMA trailing updates */
-    TCU_MIXED = 1,  /* complex64 LU, 3-pass split tcgen05 updates (FP16 or TF32 pieces), FP64 refinement */
+    TCU_MIXED = 1,  /* complex64 LU, tcgen05 updates in three passes of bfloat16 pieces, FP64 refinement */
     TCU_AUTO = 2    /* batch solves only: per cluster, MIXED from the context's crossover on (2048 modes
                        until tcu_context_autotune measures it), else FP64 */
 } tcu_precision;
@@ -79,11 +79,12 @@ const char* tcu_last_error_message(void);
 /* Number of kernel launches the context has issued (a counter for benchmarks). */
 long long tcu_context_launches(tcu_context* ctx);
 /* Refinement tolerances of tcu_factor_solve on this context (no counterpart in the reference):
- * sweeps stop at ||r|| <= target ||T b|| (default 1e-13); a mixed solve left above
+ * sweeps stop at ||r|| <= target ||T b|| (default 1e-13; mixed factors take one sweep more where they met
+ * it by less than a factor 10); a mixed solve left above
  * fallback_above ||T b|| (default 1e-12) is finished with an FP64 factor. */
 tcu_status tcu_context_set_refinement(tcu_context* ctx, double target, double fallback_above);
 /* Number of mixed-precision solves whose FP64 refinement stalled above the fallback tolerance
- * and that were finished by a second factor (TF32 pieces, then FP64) of the same cluster. */
+ * and that were finished by a second factor (three passes of TF32 pieces, then FP64) of the same cluster. */
 long long tcu_context_fallbacks(tcu_context* ctx);
 /* Precision autotuner of batched solves (no counterpart in the reference): times assembly +
  * factorization + one refined solve in FP64 and in mixed precision on synthetic lmax-4 clusters
@@ -155,10 +156,10 @@ tcu_status tcu_sphere_cluster_factor_dev(tcu_context* ctx, int lmax, double k0, 
                                          tcu_factor** out);
 /* Solve (I - T C) X = T B for p incident columns B (n x p), X out (n x p); certificates
  * (p entries) may be NULL. Replaces InteractionFactor::solve (cluster/interaction.rs:214).
- * The solve refines in FP64 until ||r|| <= 1e-13 ||T b|| (at most 10 sweeps on mixed factors, 2 on
+ * The solve refines in FP64 until ||r|| <= 1e-13 ||T b|| (at most 20 sweeps on mixed factors, 2 on
  * FP64 factors, stopping when a sweep does not halve the residual); if a mixed solve is left
  * with ||r|| > 1e-12 ||T b||, it is finished with a second factor of the same cluster, made once
- * and kept: a mixed one with TF32 pieces after FP16 pieces, an FP64 one after TF32 pieces
+ * and kept: a mixed one with three passes of TF32 pieces, then an FP64 one
  * (tcu_context_fallbacks counts these solves). */
 tcu_status tcu_factor_solve(tcu_factor* f, const double* B, int p, double* X, tcu_certificate* certificates);
 tcu_status tcu_factor_solve_dev(tcu_factor* f, const double* B, int p, double* X, tcu_certificate* certificates);
@@ -231,7 +232,7 @@ tcu_status tcu_cluster_apply_noalloc(void* stream, int lmax, double k0, size_t N
                                      const double* eps, const double* positions, int p, const double* x, double* y);
 /* Restarted GMRES on (I - T C) X = T B (cluster/iterative.rs:264-284, linalg/gmres.rs:119).
  * The preconditioner, if any, is applied on the right; certificates report the true
- * unpreconditioned residual. For lmax 2..5 the harmonic tables of all N (N - 1) sphere pairs
+ * unpreconditioned residual. For lmax 2..7 the harmonic tables of all N (N - 1) sphere pairs
  * are built once per call and kept in device memory for the operator applications
  * (N^2 (2 lmax + 1)^2 16 bytes: 14 GB at 4096 spheres and lmax 3), and the two-level
  * preconditioners store those of their dipole blocks too; each set only while it takes at most

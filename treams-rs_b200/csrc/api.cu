@@ -167,7 +167,7 @@ struct tcu_factor {
     double2* d_inv = nullptr;  // inverses of the diagonal blocks of L and U
     LuWork wk;
     double* d_scale = nullptr;       // row scales (n) then column scales (n) when equilibrated
-    cplx* d_Z = nullptr;             // stored pair tables of the refinement's FP64 residual (lmax 2..5)
+    cplx* d_Z = nullptr;             // stored pair tables of the refinement's FP64 residual (lmax 2..7)
     bool scaled = false;
     tcu_factor* fallback = nullptr;  // FP64 factor of a mixed factor whose refinement stalled
 };
