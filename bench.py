@@ -44,12 +44,12 @@ UNIT = "solves/s"
 
 # DRAM traffic of the trailing-update kernel relative to its algorithmic bytes (the
 # complex64 C block read and written once, 16 m^2 bytes), from an ncu capture of the
-# m = 11,776 launch of a 256-sphere solve: 2.395 GB measured for 2.219 GB algorithmic.
+# first paired launch (m = 12,032) of a 256-sphere solve: 2.454 GB measured for 2.316 GB algorithmic.
 # Traffic grows with m^2 like the algorithmic bytes, so the bench scales this ratio to the
 # average launch of the measured workload.
-TF32_TRAFFIC = {"ratio": 2.275 / 2.219,
+TF32_TRAFFIC = {"ratio": 2.454 / 2.316,
                 "note": "dram__bytes_read.sum + dram__bytes_write.sum of tf32_update_kernel per launch: "
-                        "ncu ratio to algorithmic bytes (1.03, two-pass m=11776 launch of a 256-sphere solve) "
+                        "ncu ratio to algorithmic bytes (1.06, paired m=12032 launch of a 256-sphere solve) "
                         "x the average algorithmic bytes (complex64 C read + write) of this workload's "
                         "update launches, paired K = 256 updates included"}
 
@@ -247,15 +247,17 @@ def iterative_workload(ctx, stream, count: int = 4096, with_cpu: bool = True, c1
         os.environ.pop("TCU_APPLY", None)
     per = (stage[3] - stage[1]) / 2.0
     pairs = w.radii.size * (w.radii.size - 1)
-    flops = 8.0 * pairs * (2 * w.lmax + 1) ** 2 * 2 * w.lmax * (w.lmax + 2)
-    tf = flops / (per / 1e3) / 1e12 if per > 0 else None
+    # the 8 x 8 blocks of the product that a term reads, at lmax 3: 41 per source and two destinations
+    flops = 8.0 * pairs * 41 * 64 / 2 if w.lmax == 3 else 0.0
+    tf = flops / (per / 1e3) / 1e12 if per > 0 and flops else None
     out["stored_operator"] = {
         "ms_per_application": per, "table_build_ms": stage[1] - per,
         "table_bytes": pairs * (2 * w.lmax + 1) ** 2 * 16,
         "roofline": {"bound": "fp64 tensor (DMMA)", "achieved": tf, "peak": c128_peak, "unit": "TFLOP/s",
                      "frac": tf / c128_peak if tf and c128_peak else None,
-                     "note": "8 (2L+1)^2 2L(L+2) useful flops per ordered pair (complex products of the table "
-                             "matrix with the coefficients); peak: measured cuBLAS complex128 GEMM rate (of measured)"}}
+                     "note": "executed: 8 flops for each of the 64 complex products of the 41 (of 52) 8 x 8 blocks that "
+                             "a term reads, per source and pair of destinations; peak: measured cuBLAS complex128 "
+                             "GEMM rate (of measured)"}}
     # one matrix-free operator application: device time and the CPU restatement on the host cores
     x = np.ones((w.n, 1), complex)
     _, ms_apply, _ = _timed(stream, lambda: c.apply(x))
