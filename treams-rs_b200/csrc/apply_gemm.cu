@@ -614,7 +614,7 @@ __global__ void __launch_bounds__(WARPS * 32 + 32, WARPS == 8 ? 2 : 1)
 // on (all 48 at lmax 6, 32 at lmax 7) and writes its sums over them to Cp; split_finish_kernel
 // adds the parts in a fixed order and applies the Mie block and the epilogue. The DMMA pipe
 // bounds it as it bounds lmax 2..5. 300 spheres lmax 6, one application: 4.3 ms with the per-pair
-// term sums (CUDA cores, an index, a weight and a gather per term and pair), 0.57 ms here.
+// term sums (CUDA cores, an index, a weight and a gather per term and pair), 0.38 ms here.
 // One CTA fits an SM. Where the last wave of the (column, destination, part) tiles would leave half of the SMs
 // or more idle, each of its tiles is cut into pieces of the source chunks, as many as there are SMs for them:
 // tiles from `whole` on, whose pieces' sums go to Cx and are added by split_finish_kernel. 300 spheres at lmax 6

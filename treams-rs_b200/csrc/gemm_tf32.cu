@@ -54,7 +54,7 @@ namespace tcu {
 
 constexpr int TB_M = 128;       // real rows of a CTA (64 complex rows); a pair of CTAs takes 256
 constexpr int TB_N = 256;       // columns per tile; each CTA of the pair stages half of them
-constexpr int TB_K = 16;        // floats per K chunk (one 64-byte swizzle row); 32 for FP16 pieces
+constexpr int TB_K = 16;        // floats per K chunk (one 64-byte swizzle row); 32 for 2-byte pieces
 constexpr int TB_STAGES = 6;
 constexpr int A_BYTES = TB_M * TB_K * 4;   // 8 KB
 constexpr int B_BYTES = TB_N / 2 * TB_K * 4;  // 8 KB
