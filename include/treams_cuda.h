@@ -96,7 +96,8 @@ tcu_status tcu_context_autotune(tcu_context* ctx, size_t* crossover, int count, 
 /* Failure-detection self-test (no counterpart in the reference): runs the LU panel's grid
  * barrier with one arrival missing, so that its bounded wait gives up after limit_seconds
  * (clamped to [0, 4] s). Returns TCU_TIMEOUT, as a factorization whose CTAs never meet
- * would, and leaves the context usable; any other status means the wait did not give up. */
+ * would, and leaves the context usable; any other status means that the wait did not give up or
+ * that row interchanges with the pivots such a factorization leaves behind moved rows. */
 tcu_status tcu_context_wait_selftest(tcu_context* ctx, double limit_seconds);
 /* Per-stage device timing with CUDA events on the context stream (off by default).
  * Stages: 0 assembly, 1 LU panel, 2 row swaps, 3 triangular block (TRSM), 4 trailing

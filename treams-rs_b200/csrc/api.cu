@@ -2659,7 +2659,18 @@ extern "C" tcu_status tcu_context_wait_selftest(tcu_context* ctx, double limit_s
     CK(cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream), "self-test status");
     tcu_status s2 = sync_status(ctx, "bounded-wait self-test");
     if (s == TCU_OK) return fail(TCU_DEVICE_ERROR, "bounded-wait self-test: the barrier passed with an arrival missing");
-    return s2 ? s2 : s;
+    if (s2) return s2;
+    // what follows a panel that gave up: interchanges with pivots that nobody wrote
+    DevBuf swaps(ctx);
+    CK(swaps.alloc(swap_selftest_bytes()), "self-test interchanges");
+    launch_swap_selftest(swaps.p, ctx->d_status, ctx->stream);
+    ctx->launches += 3;
+    int moved = 0;
+    CK(cudaMemcpyAsync(&moved, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream), "self-test status");
+    CK(cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream), "self-test status");
+    if ((s2 = sync_status(ctx, "self-test interchanges"))) return s2;
+    if (moved) return fail(TCU_DEVICE_ERROR, "bounded-wait self-test: interchanges without valid pivots moved rows");
+    return fail(s, "bounded-wait self-test: a device-side wait gave up");
 }
 
 extern "C" tcu_status tcu_context_set_refinement(tcu_context* ctx, double target, double fallback_above) {

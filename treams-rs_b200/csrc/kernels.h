@@ -308,6 +308,10 @@ int lu_factor_fp64(double2* A, int n, LuWork& w, cudaStream_t st, long long* lau
 // The panel's grid barrier with one arrival missing (bar: a zeroed counter); it gives up
 // after limit_s (clamped to [0, 4] s) and records status 8.
 void launch_barrier_selftest(unsigned* bar, int* status, double limit_s, cudaStream_t st);
+// The row interchanges of a panel that gave up: status 9 if a pivot out of range moved anything.
+// work: swap_selftest_bytes() of device memory.
+size_t swap_selftest_bytes();
+void launch_swap_selftest(void* work, int* status, cudaStream_t st);
 int lu_factor_fp32(float2* A, int n, LuWork& w, cudaStream_t st, long long* launches, bool tensor_cores);
 // solve.cu — inverses of the 64 x 64 diagonal blocks of L and U (FP64, lu_inverse_bytes),
 // then x (n x ncol, FP64) <- A^-1 x, ncol <= SOLVE_MAXC; tmp holds 2 n ncol complex.

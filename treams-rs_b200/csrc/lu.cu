@@ -344,6 +344,9 @@ namespace tcu {
 
 // ---- row swaps outside the panel ------------------------------------------------------------
 // (and on the row permutation, which the thread after the last column takes as one more column)
+// A panel whose waits gave up (status 8) leaves pivots unwritten or writes what it read from messages
+// that never came; the host learns of it only after the whole factorization has been launched. An
+// entry that no panel can have chosen, outside [k0 + j, n), is therefore no interchange.
 template <typename T>
 __device__ __forceinline__ void swap_entries(T* a, int k0, int w, const int* sp) {
     for (int j = 0; j < w; ++j) {
@@ -363,7 +366,8 @@ __global__ void laswp_kernel(C* A, size_t lda, int n, int k0, int w, const int* 
     if (threadIdx.x == 0) any = 0;
     __syncthreads();
     for (int j = threadIdx.x; j < w; j += blockDim.x) {
-        sp[j] = piv[k0 + j];
+        const int p = piv[k0 + j];
+        sp[j] = p >= k0 + j && p < n ? p : k0 + j;
         if (sp[j] != k0 + j) any = 1;
     }
     __syncthreads();
@@ -373,9 +377,10 @@ __global__ void laswp_kernel(C* A, size_t lda, int n, int k0, int w, const int* 
     if (col >= n || (col >= k0 && col < k0 + w)) return;
     swap_entries(A + (size_t)col * lda, k0, w, sp);
 }
-__global__ void iota_kernel(int* __restrict__ perm, int n) {
+// no interchange yet, in the permutation and in the pivots (the workspace comes from a pool)
+__global__ void iota_kernel(int* __restrict__ perm, int* __restrict__ piv, int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) perm[i] = i;
+    if (i < n) perm[i] = piv[i] = i;
 }
 
 // A warp solves TRSM_COLS columns at a time, so that their chains of w dependent steps overlap; the
@@ -643,6 +648,36 @@ void launch_barrier_selftest(unsigned* bar, int* status, double limit_s, cudaStr
     barrier_selftest_kernel<<<1, 32, 0, st>>>(bar, status, (unsigned long long)ns);
 }
 
+// The interchanges of a panel that gave up: laswp_kernel with pivots outside their range, and one valid
+// interchange among them, on a matrix and a permutation whose entries are their own index; anything but that
+// interchange, in a guard of 96 entries on both sides too, records status 9. Panel columns 0 .. 63 of 96 rows.
+constexpr int SWT_N = 96, SWT_W = 64, SWT_A = 10, SWT_B = 80;
+__global__ void swap_selftest_kernel(double2* guarded, int* perm, int* piv, int* status, bool check) {
+    const int bad[8] = {-1, SWT_N, 2147483647, -2147483647 - 1, 0, SWT_N + 7, -5, 1};
+    auto swapped = [](int row) { return row == SWT_A ? SWT_B : (row == SWT_B ? SWT_A : row); };
+    for (int i = threadIdx.x; i < SWT_N * (SWT_N + 2); i += blockDim.x) {
+        const int row = i % SWT_N, col = i / SWT_N - 1;  // columns -1 and SWT_N are the guards
+        const int want = check && col >= SWT_W && col < SWT_N ? i - row + swapped(row) : i;
+        if (!check)
+            guarded[i] = make_double2(i, -i);
+        else if (guarded[i].x != want || guarded[i].y != -want)
+            atomicExch(status, 9);
+    }
+    for (int i = threadIdx.x; i < SWT_N; i += blockDim.x) {
+        if (check && perm[i] != swapped(i)) atomicExch(status, 9);
+        if (!check) perm[i] = i;
+        if (!check) piv[i] = i == SWT_A ? SWT_B : (i < 2 ? i : bad[i % 8]);  // 0 and 1 lie above every row from 2 on
+    }
+}
+size_t swap_selftest_bytes() { return (size_t)SWT_N * (SWT_N + 2) * sizeof(double2) + 2 * SWT_N * sizeof(int); }
+void launch_swap_selftest(void* work, int* status, cudaStream_t st) {
+    double2* guarded = (double2*)work;
+    int *perm = (int*)(guarded + SWT_N * (SWT_N + 2)), *piv = perm + SWT_N;
+    swap_selftest_kernel<<<1, 256, 0, st>>>(guarded, perm, piv, status, false);
+    laswp_kernel<double2><<<1, 256, 0, st>>>(guarded + SWT_N, SWT_N, SWT_N, 0, SWT_W, piv, perm);
+    swap_selftest_kernel<<<1, 256, 0, st>>>(guarded, perm, piv, status, true);
+}
+
 void lu_init_attributes() {
     static PerDeviceOnce done;
     once_per_device(done, [] {
@@ -846,7 +881,7 @@ static int lu_factor_impl(typename Cx<R>::T* A, int n, LuWork& wk, cudaStream_t 
     typedef typename Cx<R>::T C;
     lu_init_attributes();
     size_t lda = n;
-    iota_kernel<<<(n + 255) / 256, 256, 0, st>>>(wk.perm, n);  // row i of P A is row perm[i] of A
+    iota_kernel<<<(n + 255) / 256, 256, 0, st>>>(wk.perm, wk.piv, n);  // row i of P A is row perm[i] of A
     ++*launches;
     // flags of the cluster panels' words: epochs 1 .. n
     cudaMemsetAsync(panel_words(wk), 0, (PC_GKEY + PC_GROW) * sizeof(uint4), st);
