@@ -93,11 +93,12 @@ long long tcu_context_fallbacks(tcu_context* ctx);
  * (ms) go to sizes, ms_fp64, ms_mixed (each may be NULL). Takes about a second. */
 tcu_status tcu_context_autotune(tcu_context* ctx, size_t* crossover, int count, size_t* sizes, double* ms_fp64,
                                 double* ms_mixed);
-/* Failure-detection self-test (no counterpart in the reference): runs the LU panel's grid
- * barrier with one arrival missing, so that its bounded wait gives up after limit_seconds
- * (clamped to [0, 4] s). Returns TCU_TIMEOUT, as a factorization whose CTAs never meet
- * would, and leaves the context usable; any other status means that the wait did not give up or
- * that row interchanges with the pivots such a factorization leaves behind moved rows. */
+/* Failure-detection self-test (no counterpart in the reference): runs every bounded device wait (the LU
+ * panels' grid barrier, messages and words, the triangular sweeps' entries and rings, the rings of the
+ * trailing update and of the stored product) on something that never comes, so that each gives up
+ * after limit_seconds (clamped to [0, 4] s). Returns TCU_TIMEOUT, as a factorization whose CTAs never
+ * meet would, and leaves the context usable; any other status means that a wait did not
+ * give up or that row interchanges with the pivots such a factorization leaves behind moved rows. */
 tcu_status tcu_context_wait_selftest(tcu_context* ctx, double limit_seconds);
 /* Per-stage device timing with CUDA events on the context stream (off by default).
  * Stages: 0 assembly, 1 LU panel, 2 row swaps, 3 triangular block (TRSM), 4 trailing

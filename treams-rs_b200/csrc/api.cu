@@ -2649,28 +2649,35 @@ extern "C" tcu_status tcu_context_wait_selftest(tcu_context* ctx, double limit_s
     if (!ctx || !std::isfinite(limit_seconds) || limit_seconds < 0.0)
         return fail(TCU_INVALID_INPUT, "require a context and a finite limit >= 0");
     std::lock_guard<std::recursive_mutex> lock(ctx->mu);
-    DevBuf bar(ctx);
-    CK(bar.alloc(sizeof(unsigned) * 4), "self-test barrier");
-    CK(cudaMemsetAsync(bar.p, 0, sizeof(unsigned) * 4, ctx->stream), "self-test barrier");
-    CK(cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream), "self-test status");
-    launch_barrier_selftest((unsigned*)bar.p, ctx->d_status, limit_seconds, ctx->stream);
-    ctx->launches += 1;
-    tcu_status s = read_status(ctx, "bounded-wait self-test");
-    CK(cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream), "self-test status");
-    tcu_status s2 = sync_status(ctx, "bounded-wait self-test");
-    if (s == TCU_OK) return fail(TCU_DEVICE_ERROR, "bounded-wait self-test: the barrier passed with an arrival missing");
-    if (s2) return s2;
+    // one status word per wait: a wait also gives up when its word already says so
+    const char* const waits[] = {"panel's grid barrier", "cluster panel's message wait", "cluster panel's word wait",
+                                 "sweeps' entry wait", "sweeps' ring wait", "trailing update's ring wait",
+                                 "stored product's ring wait"};
+    constexpr int COUNT = 7;
+    Arena ar;
+    const size_t o_st = ar.add((COUNT + 1) * sizeof(int)), o_zero = ar.add(16), o_entry = ar.add(16),
+                 o_swap = ar.add(swap_selftest_bytes());
+    DevBuf buf(ctx);
+    CK(buf.alloc(ar.total), "self-test buffers");
+    CK(cudaMemsetAsync(buf.p, 0, o_swap, ctx->stream), "self-test buffers");
+    int* st = ar.at<int>(buf.p, o_st);
+    launch_barrier_selftest(ar.at<unsigned>(buf.p, o_entry), st, limit_seconds, ctx->stream);
+    launch_panel_wait_selftest(ar.at<void>(buf.p, o_zero), st + 1, limit_seconds, ctx->stream);
+    launch_sweep_wait_selftest(st + 3, st + 4, ar.at<void>(buf.p, o_entry), limit_seconds, ctx->stream);
+    launch_update_wait_selftest(st + 5, limit_seconds, ctx->stream);
+    launch_product_wait_selftest(st + 6, limit_seconds, ctx->stream);
     // what follows a panel that gave up: interchanges with pivots that nobody wrote
-    DevBuf swaps(ctx);
-    CK(swaps.alloc(swap_selftest_bytes()), "self-test interchanges");
-    launch_swap_selftest(swaps.p, ctx->d_status, ctx->stream);
-    ctx->launches += 3;
-    int moved = 0;
-    CK(cudaMemcpyAsync(&moved, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream), "self-test status");
-    CK(cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream), "self-test status");
-    if ((s2 = sync_status(ctx, "self-test interchanges"))) return s2;
-    if (moved) return fail(TCU_DEVICE_ERROR, "bounded-wait self-test: interchanges without valid pivots moved rows");
-    return fail(s, "bounded-wait self-test: a device-side wait gave up");
+    launch_swap_selftest(ar.at<void>(buf.p, o_swap), st + COUNT, ctx->stream);
+    ctx->launches += 8;
+    int got[COUNT + 1];
+    CK(cudaMemcpyAsync(got, st, sizeof(got), cudaMemcpyDeviceToHost, ctx->stream), "self-test status");
+    const tcu_status s = sync_status(ctx, "bounded-wait self-test");
+    if (s) return s;
+    for (int i = 0; i < COUNT; ++i)
+        if (got[i] != 8)
+            return fail(TCU_DEVICE_ERROR, std::string("bounded-wait self-test: the ") + waits[i] + " did not give up");
+    if (got[COUNT]) return fail(TCU_DEVICE_ERROR, "bounded-wait self-test: interchanges without valid pivots moved rows");
+    return fail(TCU_TIMEOUT, "bounded-wait self-test: a device-side wait gave up");
 }
 
 extern "C" tcu_status tcu_context_set_refinement(tcu_context* ctx, double target, double fallback_above) {

@@ -426,7 +426,8 @@ __device__ __forceinline__ bool as_mbar_try(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 // Bounded wait on a phase: false after 2 s (recorded in abort_flag) or once another warp gave up.
-__device__ __forceinline__ bool as_mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+__device__ __forceinline__ bool as_mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
+                                             unsigned long long limit_ns = 2000000000ull) {
     if (as_mbar_try(bar, parity)) return true;
     unsigned long long t0;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
@@ -436,12 +437,20 @@ __device__ __forceinline__ bool as_mbar_wait(uint32_t bar, uint32_t parity, vola
             if (*abort_flag) return false;
             unsigned long long t;
             asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-            if (t - t0 > 2000000000ull) {
+            if (t - t0 > limit_ns) {
                 *abort_flag = 1;
                 return false;
             }
         }
     }
+}
+// This wait on a barrier without arrivals.
+__global__ void product_wait_selftest_kernel(int* status, unsigned long long limit_ns) {
+    __shared__ __align__(8) uint64_t bar;
+    __shared__ int abort_flag;
+    as_mbar_init(as_smem_u32(&bar), 1);
+    abort_flag = 0;
+    if (!as_mbar_wait(as_smem_u32(&bar), 0, &abort_flag, limit_ns)) atomicExch(status, 8);
 }
 // contiguous global -> shared copy completing on an mbarrier (16-byte aligned, size % 16 == 0)
 __device__ __forceinline__ void as_bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
@@ -744,6 +753,10 @@ void launch_apply_gemm(const DevPlan& P, int N, double k, const double* pos, con
         case 4: launch_shape<4, 4>(P, O, s, N, k, pos, T, x, ldx, ncol, zadd, alpha, beta, singular, y, st); break;
         default: launch_shape<4, 5>(P, O, s, N, k, pos, T, x, ldx, ncol, zadd, alpha, beta, singular, y, st); break;
     }
+}
+
+void launch_product_wait_selftest(int* status, double limit_s, cudaStream_t st) {
+    product_wait_selftest_kernel<<<1, 1, 0, st>>>(status, selftest_ns(limit_s));
 }
 
 void launch_apply_dipole(const DevPlan& P, int N, double k, const double* pos, const cplx* T, const cplx* z,

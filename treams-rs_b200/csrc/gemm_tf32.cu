@@ -91,19 +91,32 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 // Bounded wait: false after 2 s or when another role has aborted.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
+                                          unsigned long long limit_ns = 2000000000ull) {
     if (mbar_try(bar, parity)) return true;
     unsigned long long t0 = gtimer();
     for (unsigned it = 1;; ++it) {
         if (mbar_try(bar, parity)) return true;
         if ((it & 63u) == 0) {
             if (*abort_flag) return false;
-            if (gtimer() - t0 > 2000000000ull) {
+            if (gtimer() - t0 > limit_ns) {
                 *abort_flag = 1;
                 return false;
             }
         }
     }
+}
+
+// This wait on a barrier without arrivals.
+__global__ void update_wait_selftest_kernel(int* status, unsigned long long limit_ns) {
+    __shared__ __align__(8) uint64_t bar;
+    __shared__ int abort_flag;
+    mbar_init(smem_u32(&bar), 1);
+    abort_flag = 0;
+    if (!mbar_wait(smem_u32(&bar), 0, &abort_flag, limit_ns)) atomicExch(status, 8);
+}
+void launch_update_wait_selftest(int* status, double limit_s, cudaStream_t st) {
+    update_wait_selftest_kernel<<<1, 1, 0, st>>>(status, selftest_ns(limit_s));
 }
 
 // The leader's (rank 0) barrier of the pair, as a shared::cluster address.

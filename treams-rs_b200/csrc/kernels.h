@@ -305,6 +305,15 @@ struct LuWork {
 // bfloat16 unless TCU_SPLIT names another format (tf32x3, tf32x2, f16)
 PieceFormat split_default();
 int lu_factor_fp64(double2* A, int n, LuWork& w, cudaStream_t st, long long* launches);
+// Self-tests of the bounded waits: each waits for what never comes, gives up after limit_s (clamped to
+// [0, 4] s) and records status 8. zeros: 16 zeroed bytes of device memory.
+inline unsigned long long selftest_ns(double limit_s) {
+    return (unsigned long long)((limit_s < 0.0 ? 0.0 : limit_s > 4.0 ? 4.0 : limit_s) * 1e9);
+}
+void launch_panel_wait_selftest(const void* zeros, int* status, double limit_s, cudaStream_t st);  // status: 2 words
+void launch_sweep_wait_selftest(int* entry_status, int* ring_status, void* entry, double limit_s, cudaStream_t st);
+void launch_update_wait_selftest(int* status, double limit_s, cudaStream_t st);
+void launch_product_wait_selftest(int* status, double limit_s, cudaStream_t st);
 // The panel's grid barrier with one arrival missing (bar: a zeroed counter); it gives up
 // after limit_s (clamped to [0, 4] s) and records status 8.
 void launch_barrier_selftest(unsigned* bar, int* status, double limit_s, cudaStream_t st);

@@ -644,8 +644,27 @@ __global__ void barrier_selftest_kernel(unsigned* bar, int* status, unsigned lon
 }
 
 void launch_barrier_selftest(unsigned* bar, int* status, double limit_s, cudaStream_t st) {
-    const double ns = std::min(std::max(limit_s, 0.0), 4.0) * 1e9;
-    barrier_selftest_kernel<<<1, 32, 0, st>>>(bar, status, (unsigned long long)ns);
+    barrier_selftest_kernel<<<1, 32, 0, st>>>(bar, status, selftest_ns(limit_s));
+}
+
+// The cluster panel's two waits on what never comes, a message (an mbarrier without arrivals; status[0]) and
+// another cluster's word (a zeroed one; status[1]).
+__global__ void panel_wait_selftest_kernel(const uint4* word, int* status, unsigned long long limit_ns) {
+    __shared__ __align__(8) uint64_t bar;
+    __shared__ int quit;
+    if (threadIdx.x == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(pc_smem(&bar)) : "memory");
+        quit = 0;
+    }
+    __syncthreads();
+    pc_wait(pc_smem(&bar), 0, status, &quit, limit_ns);
+    __syncthreads();
+    if (threadIdx.x == 0) quit = 0;
+    __syncthreads();
+    pc_get(word, pc_peek(word), 1u, status + 1, &quit, limit_ns);
+}
+void launch_panel_wait_selftest(const void* zeros, int* status, double limit_s, cudaStream_t st) {
+    panel_wait_selftest_kernel<<<1, 32, 0, st>>>((const uint4*)zeros, status, selftest_ns(limit_s));
 }
 
 // The interchanges of a panel that gave up: laswp_kernel with pivots outside their range, and one valid

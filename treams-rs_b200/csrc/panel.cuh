@@ -75,20 +75,22 @@ __device__ __forceinline__ void pc_cluster_barrier() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // A long wait checks the clock and the status word; true when the caller has to give up.
-__device__ __forceinline__ bool pc_expired(unsigned long long& t0, unsigned spins, int* status, volatile int* quit) {
+__device__ __forceinline__ bool pc_expired(unsigned long long& t0, unsigned spins, int* status, volatile int* quit,
+                                           unsigned long long limit_ns = BARRIER_LIMIT_NS) {
     if ((spins & 255u) != 0) return false;
     if (*quit) return true;
     const unsigned long long now = global_ns();
     if (!t0) t0 = now;
-    if (*(volatile int*)status != 8 && now - t0 <= BARRIER_LIMIT_NS) return false;
+    if (*(volatile int*)status != 8 && now - t0 <= limit_ns) return false;
     atomicExch(status, 8);
     *quit = 1;
     return true;
 }
-__device__ __forceinline__ void pc_wait(uint32_t bar, uint32_t parity, int* status, volatile int* quit) {
+__device__ __forceinline__ void pc_wait(uint32_t bar, uint32_t parity, int* status, volatile int* quit,
+                                        unsigned long long limit_ns = BARRIER_LIMIT_NS) {
     unsigned long long t0 = 0;
     for (unsigned spins = 1; !pc_try(bar, parity); ++spins)
-        if (*quit || pc_expired(t0, spins, status, quit)) return;
+        if (*quit || pc_expired(t0, spins, status, quit, limit_ns)) return;
 }
 // global words that carry their own flag
 __device__ __forceinline__ void pc_put(uint4* p, pc_word v, unsigned flag) {
@@ -104,10 +106,11 @@ __device__ __forceinline__ uint4 pc_peek(const uint4* p) {
                  : "memory");
     return v;
 }
-__device__ __forceinline__ pc_word pc_get(const uint4* p, uint4 v, unsigned flag, int* status, volatile int* quit) {
+__device__ __forceinline__ pc_word pc_get(const uint4* p, uint4 v, unsigned flag, int* status, volatile int* quit,
+                                          unsigned long long limit_ns = BARRIER_LIMIT_NS) {
     unsigned long long t0 = 0;
     for (unsigned spins = 1; v.y != flag || v.w != flag; ++spins) {
-        if (*quit || pc_expired(t0, spins, status, quit)) break;
+        if (*quit || pc_expired(t0, spins, status, quit, limit_ns)) break;
         v = pc_peek(p);
     }
     return (pc_word)v.x | ((pc_word)v.z << 32);

@@ -259,13 +259,14 @@ __device__ __forceinline__ double sw_value(double v) {  // never the empty patte
     return sw_empty(v) ? __longlong_as_double(0x7ff8000000000000ll) : v;
 }
 // Polls one entry until it is written; false (and status 8) after 4 s or when another wait gave up.
-__device__ __forceinline__ bool sw_wait(const double2* p, double2& v, int* status) {
+__device__ __forceinline__ bool sw_wait(const double2* p, double2& v, int* status,
+                                        unsigned long long limit_ns = 4000000000ull) {
     unsigned long long t0 = 0;
     for (unsigned spins = 1; sw_empty(v.x) || sw_empty(v.y); ++spins) {
         if ((spins & 255u) == 0) {  // the clock is read on long waits only: it costs about a microsecond
             const unsigned long long now = sw_ns();
             if (!t0) t0 = now;
-            if (*(volatile int*)status == 8 || now - t0 > 4000000000ull) {
+            if (*(volatile int*)status == 8 || now - t0 > limit_ns) {
                 atomicExch(status, 8);
                 return false;
             }
@@ -466,7 +467,8 @@ __device__ __forceinline__ bool sd_try(uint64_t* bar, unsigned parity) {
     return ok != 0;
 }
 // false when the CTA has given up or after 5 s (a poll gives up after 4)
-__device__ __forceinline__ bool sd_wait(uint64_t* bar, unsigned parity, volatile int* gave_up) {
+__device__ __forceinline__ bool sd_wait(uint64_t* bar, unsigned parity, volatile int* gave_up,
+                                        unsigned long long limit_ns = 5000000000ull) {
     if (sd_try(bar, parity)) return true;
     unsigned long long t0 = 0;
     for (unsigned it = 1;; ++it) {
@@ -475,7 +477,7 @@ __device__ __forceinline__ bool sd_wait(uint64_t* bar, unsigned parity, volatile
             if (*gave_up) return false;
             const unsigned long long now = sw_ns();
             if (!t0) t0 = now;
-            if (now - t0 > 5000000000ull) {
+            if (now - t0 > limit_ns) {
                 *gave_up = 1;
                 return false;
             }
@@ -672,6 +674,28 @@ __global__ void __launch_bounds__(SD_THREADS, 1)
     }
     __syncthreads();
     if (tid == 0 && s_gave_up) atomicExch(status, 8);
+}
+
+// The sweeps' two waits on what never comes: a solution entry (the empty pattern, preset here) and a ring
+// stage (an mbarrier without arrivals).
+__global__ void sweep_wait_selftest_kernel(double2* entry, int* entry_status, int* ring_status,
+                                           unsigned long long limit_ns) {
+    __shared__ __align__(8) uint64_t bar;
+    __shared__ int gave_up;
+    if (threadIdx.x == 0) {
+        const double e = __longlong_as_double(-1ll);
+        *entry = make_double2(e, e);
+        sd_init(&bar, 1);
+        gave_up = 0;
+        __threadfence();
+    }
+    __syncthreads();
+    double2 v = sw_load(entry);
+    sw_wait(entry, v, entry_status, limit_ns);
+    if (!sd_wait(&bar, 0, &gave_up, limit_ns)) atomicExch(ring_status, 8);
+}
+void launch_sweep_wait_selftest(int* entry_status, int* ring_status, void* entry, double limit_s, cudaStream_t st) {
+    sweep_wait_selftest_kernel<<<1, 32, 0, st>>>((double2*)entry, entry_status, ring_status, selftest_ns(limit_s));
 }
 
 static int g_sms = 0;

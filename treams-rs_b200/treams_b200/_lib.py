@@ -146,9 +146,8 @@ class Context:
         _check(lib().tcu_context_set_refinement(self.handle, float(target), float(fallback_above)))
 
     def wait_selftest(self, limit: float = 0.05) -> None:
-        """Run the LU panel's grid barrier with one arrival missing; its bounded wait gives up
-        after `limit` seconds and this raises TreamsCudaError (status TCU_TIMEOUT), leaving the
-        context usable."""
+        """Run every bounded device wait on something that never comes; each gives up after `limit`
+        seconds and this raises TreamsCudaError (status TCU_TIMEOUT), leaving the context usable."""
         _check(lib().tcu_context_wait_selftest(self.handle, float(limit)))
 
     def autotune(self) -> dict:
