@@ -97,7 +97,7 @@ tcu_status tcu_context_autotune(tcu_context* ctx, size_t* crossover, int count, 
  * panels' grid barrier, messages and words, the triangular sweeps' entries and rings, the rings of the
  * trailing update and of the stored product) on something that never comes, so that each gives up
  * after limit_seconds (clamped to [0, 4] s). Returns TCU_TIMEOUT, as a factorization whose CTAs never
- * meet would, and leaves the context usable; any other status means that a wait did not
+ * meet would, and leaves the context and its factors usable; any other status means that a wait did not
  * give up or that row interchanges with the pivots such a factorization leaves behind moved rows. */
 tcu_status tcu_context_wait_selftest(tcu_context* ctx, double limit_seconds);
 /* Per-stage device timing with CUDA events on the context stream (off by default).

@@ -687,6 +687,7 @@ tcu_status solve_impl(tcu_factor* f, const double* B, int p, double* X, tcu_cert
     cplx* tmp = r + per;  // 2 per
     cplx* xf = tmp + 2 * per;  // packed inputs of the stored-table residual
     SolveNorms norms(p, (char*)xf + xf_bytes);
+    CK(cudaMemsetAsync(f->wk.status, 0, sizeof(int), ctx->stream), "status");  // of this solve alone
     CK(cudaMemcpyAsync(b, B, per * 16, device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, ctx->stream),
        "copy rhs");
     launch_apply_t(f->L, f->N, f->d_T, b, p, tb, ctx->stream);
@@ -2669,6 +2670,11 @@ extern "C" tcu_status tcu_context_wait_selftest(tcu_context* ctx, double limit_s
     // what follows a panel that gave up: interchanges with pivots that nobody wrote
     launch_swap_selftest(ar.at<void>(buf.p, o_swap), st + COUNT, ctx->stream);
     ctx->launches += 8;
+    // a live factor's next solve finds the word that such a wait of an earlier solve left
+    for (tcu_factor* f : ctx->factors) {
+        launch_sweep_wait_selftest(f->wk.status, st + 4, ar.at<void>(buf.p, o_entry), limit_seconds, ctx->stream);
+        ++ctx->launches;
+    }
     int got[COUNT + 1];
     CK(cudaMemcpyAsync(got, st, sizeof(got), cudaMemcpyDeviceToHost, ctx->stream), "self-test status");
     const tcu_status s = sync_status(ctx, "bounded-wait self-test");
