@@ -908,7 +908,8 @@ tcu_status solve_adjoint_impl(tcu_factor* f, const double* G, int p, double* Y, 
 }
 
 // A factor applied once (no refinement): v <- A^-1 v with the row/column scales; the coarse
-// solve of the two-level preconditioners. Owns the factor.
+// solve of the two-level preconditioners. Owns the factor. A sweep that gives up is recorded in the
+// context's status word, which the entry points read at the end.
 struct FactorCoarse : CoarseSolve {
     tcu_factor* f = nullptr;
     cplx* tmp = nullptr;
@@ -922,10 +923,10 @@ struct FactorCoarse : CoarseSolve {
         if (f->scaled) scale_rows(v, f->d_scale, n, 1, st);
         if (f->precision == TCU_FP64)
             lu_solve_fp64((const double2*)f->d_A, (int)n, f->wk.perm, f->d_inv, v, tmp, 1, st, &ctx->launches,
-                          f->wk.status);
+                          ctx->d_status);
         else
             lu_solve_fp32((const float2*)f->d_A, (int)n, f->wk.perm, f->d_inv, v, tmp, 1, st, &ctx->launches,
-                          f->wk.status);
+                          ctx->d_status);
         if (f->scaled) scale_rows(v, f->d_scale + n, n, 1, st);
         return TCU_OK;
     }
@@ -1600,8 +1601,8 @@ extern "C" tcu_status tcu_iterative_solve(tcu_context* ctx, int lmax, double k0,
         if ((s = make_coarse(ctx, k0, N, radii, eps, positions, &coarse)))
             return fail(s, std::string("coarse dipole system: ") + g_last_error);
         s = make_two_level(ctx->stream, preconditioner == TCU_PRECOND_LEARNED, *P, lmax, (int)N, k0, pos, positions,
-                           radii, eps, T, ctx->precond_reach, ctx->learned_weights, std::move(coarse), &pre,
-                           &ctx->launches);
+                           radii, eps, T, ctx->precond_reach, ctx->learned_weights, std::move(coarse), ctx->d_status,
+                           &pre, &ctx->launches);
         if (s == TCU_OUT_OF_MEMORY) return fail(s, "two-level preconditioner: out of device memory");
         if (s) return fail(s, "two-level preconditioner set-up failed");
     }
@@ -2447,9 +2448,10 @@ extern "C" tcu_status tcu_learned_problem_create(tcu_context* ctx, int lmax, dou
     if ((s = make_coarse(ctx, k0, N, radii, eps, positions, &coarse, true)))
         return fail(s, std::string("coarse dipole system: ") + g_last_error);
     s = p->lp.build(ctx->stream, *P, lmax, (int)N, k0, p->d_pos, positions, radii, eps, p->d_T, ctx->precond_reach,
-                    nprobe, p->d_V, std::move(coarse), &ctx->launches);
+                    nprobe, p->d_V, std::move(coarse), ctx->d_status, &ctx->launches);
     if (s == TCU_OUT_OF_MEMORY) return fail(s, "training problem: out of device memory");
     if (s) return fail(s, "training problem: device failure");
+    if ((s = read_status(ctx, "training problem"))) return s;
     *out = p.release();
     return TCU_OK;
 }

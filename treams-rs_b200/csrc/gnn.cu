@@ -508,6 +508,7 @@ class IterativeCoarse : public CoarseSolve {
     const cplx* T = nullptr;
     DevArray V, w, h, small, dpart, npart;
     const StoredDipole* stored = nullptr;  // tables of A_cc, when built
+    int* status = nullptr;
     long long* launches = nullptr;
     bool build(const DevPlan& P, int N_, double k, const double* d_pos, const cplx* d_T, int restart,
                int max_iterations, double tol) {
@@ -529,7 +530,7 @@ class IterativeCoarse : public CoarseSolve {
     void matvec(const cplx* x, cplx* y, cudaStream_t st) {
         if (stored && stored->ready) {
             launch_apply_stored(*plan, N, STORED_DIPOLE_BLOCK, stored->Z.as<cplx>(), T, x, 0, 1, nullptr, 1.0, -1.0, y,
-                                stored->Xf.as<cplx>(), nullptr, st);
+                                stored->Xf.as<cplx>(), status, st);
             if (launches) *launches += 2;
         } else {
             launch_apply_dipole(*plan, N, k0, pos, T, x, true, nullptr, 1.0, -1.0, y, st);
@@ -607,9 +608,11 @@ struct Coarse {
     DevArray vc;
     StoredDipole zsrc, zcc;  // tables of the correction's dipole sources and of A_cc
     std::unique_ptr<CoarseSolve> solver;
+    int* status = nullptr;
     bool build(const DevPlan& P, int N_, double k, const double* d_pos, const cplx* d_T, std::unique_ptr<CoarseSolve> s,
-               cudaStream_t st, long long* launches) {
+               int* status_, cudaStream_t st, long long* launches) {
         plan = &P;
+        status = status_;
         N = N_;
         M = 2 * P.nlm;
         n = (size_t)N * M;
@@ -625,6 +628,7 @@ struct Coarse {
             auto it = std::make_unique<IterativeCoarse>();
             it->launches = launches;
             it->stored = &zcc;
+            it->status = status;
             // relative tolerance of the inner solve: 3e-2 (the 4096-sphere workload measured 300,
             // 291, 256 and 269 ms at 1e-3, 1e-2, 3e-2 and 1e-1), or TCU_COARSE_RTOL
             const char* e = getenv("TCU_COARSE_RTOL");
@@ -641,7 +645,7 @@ struct Coarse {
         if (s) return s;
         if (zsrc.ready) {
             launch_apply_stored(*plan, N, STORED_DIPOLE_SOURCES, zsrc.Z.as<cplx>(), T, vc.as<cplx>(), 0, 1, v, -1.0, 1.0,
-                                r1, zsrc.Xf.as<cplx>(), nullptr, st);
+                                r1, zsrc.Xf.as<cplx>(), status, st);
             if (launches) *launches += 3;
         } else {
             launch_apply_dipole(*plan, N, k0, pos, T, vc.as<cplx>(), false, v, -1.0, 1.0, r1, st);
@@ -682,7 +686,7 @@ int learned_weight_count(int L) { return layout(L).total; }
 tcu_status make_two_level(cudaStream_t st, bool learned, const DevPlan& P, int L, int N, double k0,
                           const double* d_pos, const double* h_pos, const double* h_radii, const double* h_eps,
                           const double2* d_T, double reach, const std::vector<double>& weights_in,
-                          std::unique_ptr<CoarseSolve> coarse, std::unique_ptr<Preconditioner>* out,
+                          std::unique_ptr<CoarseSolve> coarse, int* status, std::unique_ptr<Preconditioner>* out,
                           long long* launches) {
     auto pre = std::make_unique<TwoLevelPre>();
     pre->T = d_T;
@@ -691,7 +695,7 @@ tcu_status make_two_level(cudaStream_t st, bool learned, const DevPlan& P, int L
     for (int i = 0; i < N; ++i) rmax = std::max(rmax, h_radii[i]);
     const double cutoff = 2.0 * (reach > 0.0 ? reach : LEARNED_REACH) * rmax;
     // the coarse blocks' tables go to the device first; the host builds the graph meanwhile
-    if (!pre->coarse.build(P, N, k0, d_pos, d_T, std::move(coarse), st, launches)) return TCU_OUT_OF_MEMORY;
+    if (!pre->coarse.build(P, N, k0, d_pos, d_T, std::move(coarse), status, st, launches)) return TCU_OUT_OF_MEMORY;
     if (!pre->graph.build(st, P, L, N, k0, d_pos, h_pos, h_radii, h_eps, cutoff, launches)) return TCU_OUT_OF_MEMORY;
     if (!pre->r1.alloc(pre->graph.n * sizeof(cplx)) || !pre->noskip.alloc(std::max<size_t>(pre->graph.nnz, 1)))
         return TCU_OUT_OF_MEMORY;
@@ -724,7 +728,7 @@ LearnedProblem::~LearnedProblem() = default;
 tcu_status LearnedProblem::build(cudaStream_t st, const DevPlan& P, int L_, int N_, double k0_, const double* d_pos_,
                                  const double* h_pos, const double* h_radii, const double* h_eps, const double2* d_T_,
                                  double reach, int nprobe, const double2* d_V, std::unique_ptr<CoarseSolve> cs,
-                                 long long* launches_) {
+                                 int* status, long long* launches_) {
     L = L_;
     N = N_;
     k0 = k0_;
@@ -737,7 +741,7 @@ tcu_status LearnedProblem::build(cudaStream_t st, const DevPlan& P, int L_, int 
     for (int i = 0; i < N; ++i) rmax = std::max(rmax, h_radii[i]);
     const double cutoff = 2.0 * (reach > 0.0 ? reach : LEARNED_REACH) * rmax;
     if (!m.graph.build(st, P, L, N, k0, d_pos, h_pos, h_radii, h_eps, cutoff, launches)) return TCU_OUT_OF_MEMORY;
-    if (!m.coarse.build(P, N, k0, d_pos, d_T, std::move(cs), st, launches)) return TCU_OUT_OF_MEMORY;
+    if (!m.coarse.build(P, N, k0, d_pos, d_T, std::move(cs), status, st, launches)) return TCU_OUT_OF_MEMORY;
     n = m.graph.n;
     m.p = nprobe;
     const size_t vb = n * (size_t)nprobe * sizeof(cplx), nnz = m.graph.nnz;

@@ -37,11 +37,12 @@ struct CoarseSolve {
 // Two-level preconditioner (gnn.cu): coarse dipole correction, then the near field within
 // reach sphere diameters with every (degree, degree) sub-block scaled by the graph network's
 // Theta (learned, weights: the compiled-in weights of lmax when empty; without weights for
-// lmax, Theta = 1) or by 1 (learned false: the untrained two-level method).
+// lmax, Theta = 1) or by 1 (learned false: the untrained two-level method). status: device word that
+// records a bounded wait of its products giving up.
 tcu_status make_two_level(cudaStream_t st, bool learned, const DevPlan& P, int L, int N, double k0,
                           const double* d_pos, const double* h_pos, const double* h_radii, const double* h_eps,
                           const double2* d_T, double reach, const std::vector<double>& weights,
-                          std::unique_ptr<CoarseSolve> coarse, std::unique_ptr<Preconditioner>* out,
+                          std::unique_ptr<CoarseSolve> coarse, int* status, std::unique_ptr<Preconditioner>* out,
                           long long* launches);
 int learned_weight_count(int L);
 
@@ -54,7 +55,8 @@ class LearnedProblem {
     ~LearnedProblem();
     tcu_status build(cudaStream_t st, const DevPlan& P, int L, int N, double k0, const double* d_pos,
                      const double* h_pos, const double* h_radii, const double* h_eps, const double2* d_T, double reach,
-                     int nprobe, const double2* d_V, std::unique_ptr<CoarseSolve> coarse, long long* launches);
+                     int nprobe, const double2* d_V, std::unique_ptr<CoarseSolve> coarse, int* status,
+                     long long* launches);
     tcu_status loss_grad(const double* h_weights, double* loss, double* h_grad, cudaStream_t st);
     tcu_status probes(double2* h_out, cudaStream_t st);
     // y = (I - T C)^H x for ncol <= nprobe device columns (the adjoint operator of the loss)
