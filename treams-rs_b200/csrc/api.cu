@@ -22,6 +22,7 @@
 #include "kernels.h"
 #include "plan.h"
 #include "precond.h"
+#include "refine.h"
 
 using namespace tcu;
 
@@ -559,68 +560,6 @@ tcu_status factor_impl(tcu_context* ctx, int L, double k0, size_t N, const doubl
     ctx->factors.insert(*out);
     return TCU_OK;
 }
-
-// Refinement state of the columns of one solve in groups of 8 that converge separately: a group
-// takes another sweep while its worst relative residual is above the target, the last sweep
-// halved it and sweeps are left; afterwards its columns and their residuals stay as they are.
-// settle: a group that has met the target with less than a factor 10 to spare takes one sweep more
-// if its sweeps still gain a factor 16 each. Factors of the bfloat16 split start at a residual of 2e-7 and meet
-// 1e-13 at 6e-14 in two sweeps; the third ends at the rounding level (1e-16 to 9e-15), as the three sweeps of
-// the two-pass TF32 split (from 2e-6) do, for one product and one pair of sweeps. A line at a factor 64
-// cost adjoint solves (rounding level 7e-15) a fourth sweep: 18.8 against 16.4 ms for 17 columns each way
-// at 9600 modes.
-struct RefineGroups {
-    static constexpr int WIDTH = 8;
-    struct Group {
-        bool active = true, settled = false;
-        int sweeps = 1, left = 0;
-        double prev = INFINITY;
-    };
-    std::vector<Group> g;
-    std::vector<double> rn;  // residual norms of the columns' current solutions
-    int p;
-    double target;
-    bool settle;
-    RefineGroups(int p_, double target_, int max_sweeps, bool settle_)
-        : g((p_ + WIDTH - 1) / WIDTH), rn(p_), p(p_), target(target_), settle(settle_) {
-        for (Group& q : g) q.left = max_sweeps;
-    }
-    size_t first(size_t q) const { return q * WIDTH; }
-    int width(size_t q) const { return std::min(WIDTH, p - (int)q * WIDTH); }
-    double worst(size_t q, const std::vector<double>& r, const std::vector<double>& bn) const {
-        double w = 0.0;
-        for (int c = (int)first(q); c < (int)first(q) + width(q); ++c) w = std::max(w, bn[c] > 0 ? r[c] / bn[c] : r[c]);
-        return w;
-    }
-    // r: norms after the latest sweep; true while a group takes another one
-    bool advance(const std::vector<double>& r, const std::vector<double>& bn) {
-        bool any = false;
-        for (size_t q = 0; q < g.size(); ++q) {
-            if (!g[q].active) continue;
-            for (int c = (int)first(q); c < (int)first(q) + width(q); ++c) rn[c] = r[c];
-            const double w = worst(q, r, bn);
-            bool stop = g[q].left == 0 || !(w < 0.5 * g[q].prev);
-            if (!stop && w <= target) {
-                stop = !settle || g[q].settled || w <= target / 10 || !(w < g[q].prev / 16);
-                g[q].settled = true;
-            }
-            if (stop) {
-                g[q].active = false;
-                continue;
-            }
-            g[q].prev = w;
-            --g[q].left;
-            ++g[q].sweeps;
-            any = true;
-        }
-        return any;
-    }
-    bool any_above(const std::vector<double>& bn, double limit) const {
-        for (size_t q = 0; q < g.size(); ++q)
-            if (!(worst(q, rn, bn) <= limit)) return true;
-        return false;
-    }
-};
 
 // most refinement sweeps of a solve: 2 on FP64 factors, 10 on mixed ones with FP32-accurate updates, 20 with
 // updates of about 2^-12 or 2^-17 a term
