@@ -579,7 +579,7 @@ struct SolveNorms {
     SolveNorms(int p_, void* mem) : p(p_), d((double*)mem), h(2 * (size_t)p_ + 1) {}
     static size_t bytes(int p) { return ((size_t)p * 258 + 1) * sizeof(double); }
     void rhs(const cplx* v, size_t n, cudaStream_t st) { vec_norms(v, n, p, d, d + 2 * p + 1, st); }
-    void residual(const cplx* r, size_t n, cudaStream_t st) { vec_norms(r, n, p, d + p, d + 2 * p + 1, st); }
+    void residual(const cplx* r, size_t n, int cols, cudaStream_t st) { vec_norms(r, n, cols, d + p, d + 2 * p + 1, st); }
     // waits for the stream
     tcu_status fetch(tcu_context* ctx, const int* status, std::vector<double>& bn, std::vector<double>& rn, int* st) {
         CK(cudaMemcpyAsync(d + 2 * p, status, sizeof(int), cudaMemcpyDeviceToDevice, ctx->stream), "status");
@@ -592,6 +592,112 @@ struct SolveNorms {
         return TCU_OK;
     }
 };
+
+// The columns of a solve that have ended, from the packed columns to the caller's memory; neighbours go in one
+// copy (copy(packed column, column, count), a cudaError_t).
+template <class Copy>
+struct ColumnsOut {
+    Copy copy;
+    int from = 0, col = 0, count = 0;
+    cudaError_t error = cudaSuccess;
+    void add(int f, int c, int n) {
+        if (count == 0 || f != from + count || c != col + count) {
+            flush();
+            from = f;
+            col = c;
+        }
+        count += n;
+    }
+    void flush() {
+        if (count > 0 && error == cudaSuccess) error = copy(from, col, count);
+        count = 0;
+    }
+};
+
+// Refines x = A^-1 rhs (n x groups.p, packed): sweep(v, columns) is v <- A^-1 v with the factor, residual(columns,
+// norms) forms r = rhs - A x and its norms. Groups of columns leave when they have converged or stalled; those
+// whose solution stands go to the caller's memory through copy. What is left in groups: sweeps and norms.
+template <class Sweep, class Residual, class Copy>
+tcu_status refine_columns(tcu_context* ctx, RefineGroups& groups, const std::vector<double>& bn, cplx* x, cplx* r,
+                          cplx* rhs, size_t n, double fallback_above, Sweep sweep, Residual residual, Copy copy) {
+    std::vector<double> packed(groups.p), rn(groups.p);
+    ColumnsOut<Copy> out{copy};
+    cudaError_t moved = cudaSuccess;
+    auto stands = [&](size_t q) {
+        for (int c = (int)groups.first(q); c < (int)groups.first(q) + groups.width(q); ++c)
+            if (!std::isfinite(groups.rn[c])) return false;
+        return groups.worst(q, groups.rn, bn) <= fallback_above;
+    };
+    for (;;) {
+        const tcu_status s = residual(groups.columns(), packed);
+        if (s) return s;
+        groups.scatter(packed, rn);
+        const bool more = groups.advance(rn, bn);
+        groups.compact(
+            [&](size_t q, int from) {
+                if (stands(q)) out.add(from, (int)groups.first(q), groups.width(q));
+            },
+            [&](int from, int to, int width) {
+                out.flush();
+                for (cplx* v : {x, r, rhs})
+                    if (moved == cudaSuccess)
+                        moved = cudaMemcpyAsync(v + to * n, v + from * n, width * n * sizeof(cplx),
+                                                cudaMemcpyDeviceToDevice, ctx->stream);
+            });
+        out.flush();
+        CK(out.error, "copy solution");
+        CK(moved, "refinement");
+        if (!more) return TCU_OK;
+        sweep(r, groups.columns());
+        vec_axpy(x, r, n, groups.columns(), ctx->stream);
+        ++ctx->launches;
+    }
+}
+
+// The factor of the same cluster that a mixed factor's stalled columns go on with, kept for later solves: the other
+// pieces first fall back to a mixed factor with three passes of TF32 pieces (which keep 22 bits relative to
+// every element), that one in turn to FP64.
+tcu_status make_fallback(tcu_factor* f) {
+    if (f->fallback) return TCU_OK;
+    tcu_context* ctx = f->ctx;
+    std::vector<double> hr(f->N), he(2 * (size_t)f->N), hp(3 * (size_t)f->N);
+    CK(cudaMemcpyAsync(hr.data(), f->d_radii, f->N * 8, cudaMemcpyDeviceToHost, ctx->stream), "copy");
+    CK(cudaMemcpyAsync(he.data(), f->d_eps, f->N * 16, cudaMemcpyDeviceToHost, ctx->stream), "copy");
+    CK(cudaMemcpyAsync(hp.data(), f->d_pos, f->N * 24, cudaMemcpyDeviceToHost, ctx->stream), "copy");
+    const tcu_status s = sync_status(ctx, "fallback");
+    if (s) return s;
+    const bool to_tf32 = f->wk.pieces != PIECES_TF32X3;
+    return factor_impl(ctx, f->L, f->k0, f->N, hr.data(), he.data(), hp.data(), nullptr, nullptr, nullptr,
+                       to_tf32 ? TCU_MIXED : TCU_FP64, &f->fallback, false);
+}
+
+// After refine_columns: the groups that stalled above fallback_above go on with another factor (again(q, column,
+// count)), the others get their certificates.
+template <class Again>
+tcu_status finish_columns(tcu_factor* f, const RefineGroups& groups, const std::vector<double>& bn,
+                          tcu_certificate* certs, Again again) {
+    tcu_context* ctx = f->ctx;
+    // refinement stalled above the FP64 target: an ill-scaled operator beyond the reach of the mixed factors
+    if (f->precision == TCU_MIXED && groups.any_above(bn, ctx->fallback_above)) {
+        const tcu_status s = make_fallback(f);
+        if (s) return s;
+    }
+    for (size_t q = 0; q < groups.g.size(); ++q) {
+        const int c0 = (int)groups.first(q), w = groups.width(q);
+        if (f->precision == TCU_MIXED && !(groups.worst(q, groups.rn, bn) <= ctx->fallback_above)) {
+            ++ctx->fallbacks;
+            const tcu_status s = again(c0, w);
+            if (s) return s;
+            continue;
+        }
+        for (int c = c0; c < c0 + w; ++c) {
+            if (!std::isfinite(groups.rn[c]))
+                return fail(TCU_SINGULAR, "non-finite solution: numerically singular operator");
+            if (certs) certs[c] = {groups.g[q].sweeps, groups.rn[c], bn[c]};
+        }
+    }
+    return TCU_OK;
+}
 
 tcu_status solve_impl(tcu_factor* f, const double* B, int p, double* X, tcu_certificate* certs, bool device) {
     if (!f || !B || !X || p <= 0) return fail(TCU_INVALID_INPUT, "require a factor and at least one column");
@@ -631,98 +737,54 @@ tcu_status solve_impl(tcu_factor* f, const double* B, int p, double* X, tcu_cert
        "copy rhs");
     launch_apply_t(f->L, f->N, f->d_T, b, p, tb, ctx->stream);
     ++ctx->launches;
-    std::vector<double> rn(p), bn(p);
+    std::vector<double> bn(p);
     norms.rhs(tb, n, ctx->stream);
     ctx->launches += 2;
-    auto lu_apply = [&](cplx* v) {
-        if (f->scaled) scale_rows(v, f->d_scale, n, p, ctx->stream);  // R v
+    auto lu_apply = [&](cplx* v, int cols) {
+        if (f->scaled) scale_rows(v, f->d_scale, n, cols, ctx->stream);  // R v
         if (f->precision == TCU_FP64)
-            lu_solve_fp64((const double2*)f->d_A, (int)n, f->wk.perm, f->d_inv, v, tmp, p, ctx->stream,
+            lu_solve_fp64((const double2*)f->d_A, (int)n, f->wk.perm, f->d_inv, v, tmp, cols, ctx->stream,
                           &ctx->launches, f->wk.status);
         else
-            lu_solve_fp32((const float2*)f->d_A, (int)n, f->wk.perm, f->d_inv, v, tmp, p, ctx->stream,
+            lu_solve_fp32((const float2*)f->d_A, (int)n, f->wk.perm, f->d_inv, v, tmp, cols, ctx->stream,
                           &ctx->launches, f->wk.status);
         if (f->scaled) {
-            scale_rows(v, f->d_scale + n, n, p, ctx->stream);  // C (A')^-1 R v
+            scale_rows(v, f->d_scale + n, n, cols, ctx->stream);  // C (A')^-1 R v
             ctx->launches += 2;
         }
     };
-    int sweep_status = 0;
-    auto residual = [&]() -> tcu_status {
+    auto residual = [&](int cols, std::vector<double>& rn) -> tcu_status {
         // r = T b - (x - T C x)
         if (f->d_Z) {
-            launch_apply_stored(*P, f->N, STORED_FULL, f->d_Z, f->d_T, x, n, p, tb, -1.0, 1.0, r, xf, f->wk.status,
+            launch_apply_stored(*P, f->N, STORED_FULL, f->d_Z, f->d_T, x, n, cols, tb, -1.0, 1.0, r, xf, f->wk.status,
                                 ctx->stream);
             ctx->launches += 2;
         } else {
-            apply_op(ctx, P, f->N, f->k0, f->d_pos, f->d_T, x, n, p, tb, -1.0, 1.0, true, r);
+            apply_op(ctx, P, f->N, f->k0, f->d_pos, f->d_T, x, n, cols, tb, -1.0, 1.0, true, r);
         }
-        norms.residual(r, n, ctx->stream);
+        norms.residual(r, n, cols, ctx->stream);
         ctx->launches += 2;
-        tcu_status s2 = norms.fetch(ctx, f->wk.status, bn, rn, &sweep_status);
+        int st = 0;
+        tcu_status s2 = norms.fetch(ctx, f->wk.status, bn, rn, &st);
         if (s2) return s2;
-        if (sweep_status == 8) return fail(TCU_TIMEOUT, "refinement: a device-side wait gave up");
+        if (st == 8) return fail(TCU_TIMEOUT, "refinement: a device-side wait gave up");
         return TCU_OK;
     };
+    auto copy_out = [&](int from, int col, int cols) {
+        return cudaMemcpyAsync((cplx*)X + col * n, x + from * n, cols * n * 16,
+                               device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, ctx->stream);
+    };
     CK(cudaMemcpyAsync(x, tb, per * 16, cudaMemcpyDeviceToDevice, ctx->stream), "copy");
-    lu_apply(x);
-    if ((s = residual())) return s;
+    lu_apply(x, p);
     // iterative refinement in FP64
     RefineGroups groups(p, ctx->refine_target, max_refinement_sweeps(f), settles(f));
-    while (groups.advance(rn, bn)) {
-        lu_apply(r);
-        for (size_t g = 0; g < groups.g.size(); ++g)
-            if (groups.g[g].active) {
-                vec_axpy(x + groups.first(g) * n, r + groups.first(g) * n, n, groups.width(g), ctx->stream);
-                ++ctx->launches;
-            }
-        if ((s = residual())) return s;
-    }
-    if (f->precision == TCU_MIXED) {
-        // refinement stalled above the FP64 target (an ill-scaled operator beyond the reach of
-        // the mixed factors): finish with an FP64 factor of the same cluster, kept for later solves
-        if (groups.any_above(bn, ctx->fallback_above)) {
-            // the other pieces first fall back to a mixed factor with three passes of TF32 pieces
-            // (which keep 22 bits relative to every element), that one in turn to FP64
-            if (!f->fallback) {
-                std::vector<double> hr(f->N), he(2 * (size_t)f->N), hp(3 * (size_t)f->N);
-                CK(cudaMemcpyAsync(hr.data(), f->d_radii, f->N * 8, cudaMemcpyDeviceToHost, ctx->stream), "copy");
-                CK(cudaMemcpyAsync(he.data(), f->d_eps, f->N * 16, cudaMemcpyDeviceToHost, ctx->stream), "copy");
-                CK(cudaMemcpyAsync(hp.data(), f->d_pos, f->N * 24, cudaMemcpyDeviceToHost, ctx->stream), "copy");
-                if ((s = sync_status(ctx, "fallback"))) return s;
-                const bool to_tf32 = f->wk.pieces != PIECES_TF32X3;
-                if ((s = factor_impl(ctx, f->L, f->k0, f->N, hr.data(), he.data(), hp.data(), nullptr, nullptr,
-                                     nullptr, to_tf32 ? TCU_MIXED : TCU_FP64, &f->fallback, false)))
-                    return s;
-            }
-        }
-    }
-    int done = 0;  // columns before it are in X
-    auto copy_out = [&](int end) {  // columns done .. end - 1
-        const int c0 = done;
-        done = end;
-        return end > c0 ? cudaMemcpyAsync((cplx*)X + c0 * n, x + c0 * n, (end - c0) * n * 16,
-                                          device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
-                                          ctx->stream)
-                        : cudaSuccess;
-    };
-    for (size_t q = 0; q < groups.g.size(); ++q) {
-        const int c0 = (int)groups.first(q), w = groups.width(q);
-        if (f->precision == TCU_MIXED && !(groups.worst(q, groups.rn, bn) <= ctx->fallback_above)) {
-            CK(copy_out(c0), "copy solution");
-            ++ctx->fallbacks;
-            const size_t off = 2 * n * (size_t)c0;
-            if ((s = solve_impl(f->fallback, B + off, w, X + off, certs ? certs + c0 : nullptr, device))) return s;
-            done = c0 + w;
-            continue;
-        }
-        for (int c = c0; c < c0 + w; ++c) {
-            if (!std::isfinite(groups.rn[c]))
-                return fail(TCU_SINGULAR, "non-finite solution: numerically singular operator");
-            if (certs) certs[c] = {groups.g[q].sweeps, groups.rn[c], bn[c]};
-        }
-    }
-    CK(copy_out(p), "copy solution");
+    const double limit = f->precision == TCU_MIXED ? ctx->fallback_above : INFINITY;
+    if ((s = refine_columns(ctx, groups, bn, x, r, tb, n, limit, lu_apply, residual, copy_out))) return s;
+    if ((s = finish_columns(f, groups, bn, certs, [&](int c0, int w) {
+             const size_t off = 2 * n * (size_t)c0;
+             return solve_impl(f->fallback, B + off, w, X + off, certs ? certs + c0 : nullptr, device);
+         })))
+        return s;
     return sync_status(ctx, "solve");
 }
 
@@ -765,84 +827,47 @@ tcu_status solve_adjoint_impl(tcu_factor* f, const double* G, int p, double* Y, 
     SolveNorms norms(p, tmp + tmpc);
     CK(cudaMemsetAsync(ctx->d_status, 0, 4, ctx->stream), "status");
     CK(cudaMemcpyAsync(g, G, per * 16, cudaMemcpyHostToDevice, ctx->stream), "copy rhs");
-    std::vector<double> rn(p), bn(p);
+    std::vector<double> bn(p);
     norms.rhs(g, n, ctx->stream);
-    auto lu_adjoint = [&](cplx* v) {
-        if (f->scaled) scale_rows(v, f->d_scale + n, n, p, ctx->stream);  // C g
+    auto lu_adjoint = [&](cplx* v, int cols) {
+        if (f->scaled) scale_rows(v, f->d_scale + n, n, cols, ctx->stream);  // C g
         if (f->precision == TCU_FP64)
-            lu_solve_adjoint_fp64((const double2*)f->d_A, (int)n, f->wk.perm, f->d_inv, v, tmp, p, ctx->stream,
+            lu_solve_adjoint_fp64((const double2*)f->d_A, (int)n, f->wk.perm, f->d_inv, v, tmp, cols, ctx->stream,
                                   &ctx->launches, ctx->d_status);
         else
-            lu_solve_adjoint_fp32((const float2*)f->d_A, (int)n, f->wk.perm, f->d_inv, v, tmp, p, ctx->stream,
+            lu_solve_adjoint_fp32((const float2*)f->d_A, (int)n, f->wk.perm, f->d_inv, v, tmp, cols, ctx->stream,
                                   &ctx->launches, ctx->d_status);
-        if (f->scaled) scale_rows(v, f->d_scale, n, p, ctx->stream);  // R
+        if (f->scaled) scale_rows(v, f->d_scale, n, cols, ctx->stream);  // R
     };
-    auto residual = [&]() -> tcu_status {  // r = g - A^H y
-        launch_apply_adjoint(*P, f->N, f->k0, f->d_pos, f->d_T, y, n, p, r, t1, t2, ctx->stream, &ctx->launches,
+    auto residual = [&](int cols, std::vector<double>& rn) -> tcu_status {  // r = g - A^H y
+        launch_apply_adjoint(*P, f->N, f->k0, f->d_pos, f->d_T, y, n, cols, r, t1, t2, ctx->stream, &ctx->launches,
                              f->d_Z, xf, ctx->d_status);
-        vec_sub(r, g, r, n, p, ctx->stream);
-        norms.residual(r, n, ctx->stream);
+        vec_sub(r, g, r, n, cols, ctx->stream);
+        norms.residual(r, n, cols, ctx->stream);
         ctx->launches += 3;
         int st = 0;
         const tcu_status s2 = norms.fetch(ctx, ctx->d_status, bn, rn, &st);
         return s2 ? s2 : status_of(st, "adjoint residual");
     };
-    CK(cudaMemcpyAsync(y, g, per * 16, cudaMemcpyDeviceToDevice, ctx->stream), "copy");
-    lu_adjoint(y);
-    if ((s = residual())) return s;
-    RefineGroups groups(p, ctx->refine_target, max_refinement_sweeps(f), settles(f));
-    while (groups.advance(rn, bn)) {
-        lu_adjoint(r);
-        for (size_t q = 0; q < groups.g.size(); ++q)
-            if (groups.g[q].active) {
-                vec_axpy(y + groups.first(q) * n, r + groups.first(q) * n, n, groups.width(q), ctx->stream);
-                ++ctx->launches;
-            }
-        if ((s = residual())) return s;
-    }
-    if (f->precision == TCU_MIXED && groups.any_above(bn, ctx->fallback_above)) {
-        if (!f->fallback) {
-            std::vector<double> hr(f->N), he(2 * (size_t)f->N), hp(3 * (size_t)f->N);
-            CK(cudaMemcpyAsync(hr.data(), f->d_radii, f->N * 8, cudaMemcpyDeviceToHost, ctx->stream), "copy");
-            CK(cudaMemcpyAsync(he.data(), f->d_eps, f->N * 16, cudaMemcpyDeviceToHost, ctx->stream), "copy");
-            CK(cudaMemcpyAsync(hp.data(), f->d_pos, f->N * 24, cudaMemcpyDeviceToHost, ctx->stream), "copy");
-            if ((s = sync_status(ctx, "fallback"))) return s;
-            const bool to_tf32 = f->wk.pieces != PIECES_TF32X3;
-            if ((s = factor_impl(ctx, f->L, f->k0, f->N, hr.data(), he.data(), hp.data(), nullptr, nullptr, nullptr,
-                                 to_tf32 ? TCU_MIXED : TCU_FP64, &f->fallback, false)))
-                return s;
+    auto copy_out = [&](int from, int col, int cols) {
+        const cplx* v = y + from * n;
+        if (th) {  // t1 is free between two residuals
+            launch_apply_th(f->L, f->N, f->d_T, v, n, cols, t1, ctx->stream);
+            ++ctx->launches;
+            v = t1;
         }
-    }
-    if (th) {
-        launch_apply_th(f->L, f->N, f->d_T, y, n, p, r, ctx->stream);
-        ++ctx->launches;
-    }
-    int done = 0;  // columns before it are in Y
-    auto copy_out = [&](int end) {  // columns done .. end - 1
-        const int c0 = done;
-        done = end;
-        return end > c0 ? cudaMemcpyAsync((cplx*)Y + c0 * n, (th ? r : y) + c0 * n, (end - c0) * n * 16,
-                                          cudaMemcpyDeviceToHost,
-                                          ctx->stream)
-                        : cudaSuccess;
+        return cudaMemcpyAsync((cplx*)Y + col * n, v, cols * n * 16, cudaMemcpyDeviceToHost, ctx->stream);
     };
-    for (size_t q = 0; q < groups.g.size(); ++q) {
-        const int c0 = (int)groups.first(q), w = groups.width(q);
-        if (f->precision == TCU_MIXED && !(groups.worst(q, groups.rn, bn) <= ctx->fallback_above)) {
-            CK(copy_out(c0), "copy solution");
-            ++ctx->fallbacks;
-            const size_t off = 2 * n * (size_t)c0;
-            if ((s = solve_adjoint_impl(f->fallback, G + off, w, Y + off, certs ? certs + c0 : nullptr, th))) return s;
-            done = c0 + w;
-            continue;
-        }
-        for (int c = c0; c < c0 + w; ++c) {
-            if (!std::isfinite(groups.rn[c]))
-                return fail(TCU_SINGULAR, "non-finite solution: numerically singular operator");
-            if (certs) certs[c] = {groups.g[q].sweeps, groups.rn[c], bn[c]};
-        }
-    }
-    CK(copy_out(p), "copy solution");
+    CK(cudaMemcpyAsync(y, g, per * 16, cudaMemcpyDeviceToDevice, ctx->stream), "copy");
+    lu_adjoint(y, p);
+    RefineGroups groups(p, ctx->refine_target, max_refinement_sweeps(f), settles(f));
+    const double limit = f->precision == TCU_MIXED ? ctx->fallback_above : INFINITY;
+    if ((s = refine_columns(ctx, groups, bn, y, r, g, n, limit, lu_adjoint, residual, copy_out))) return s;
+    if ((s = finish_columns(f, groups, bn, certs, [&](int c0, int w) {
+             const size_t off = 2 * n * (size_t)c0;
+             return solve_adjoint_impl(f->fallback, G + off, w, Y + off, certs ? certs + c0 : nullptr, th);
+         })))
+        return s;
     return sync_status(ctx, "adjoint solve");
 }
 
