@@ -570,19 +570,19 @@ int max_refinement_sweeps(const tcu_factor* f) {
 
 bool settles(const tcu_factor* f) { return f->precision == TCU_MIXED && f->wk.pieces == PIECES_BF16; }
 
-// Norms of a solve's p right-hand-side columns and residuals and a status word, side by side so that one copy
-// brings them to the host: a copy each kept the device idle for about 15 us at a time.
+// Norms of a solve's p right-hand-side columns and residuals and the solve's own status word, side by side so that
+// one copy brings them to the host: a copy each kept the device idle for about 15 us at a time.
 struct SolveNorms {
     int p;
     double* d;  // p + p norms, the status, 256 partial sums a column
     std::vector<double> h;
     SolveNorms(int p_, void* mem) : p(p_), d((double*)mem), h(2 * (size_t)p_ + 1) {}
     static size_t bytes(int p) { return ((size_t)p * 258 + 1) * sizeof(double); }
+    int* status() const { return (int*)(d + 2 * p); }
     void rhs(const cplx* v, size_t n, cudaStream_t st) { vec_norms(v, n, p, d, d + 2 * p + 1, st); }
     void residual(const cplx* r, size_t n, int cols, cudaStream_t st) { vec_norms(r, n, cols, d + p, d + 2 * p + 1, st); }
     // waits for the stream
-    tcu_status fetch(tcu_context* ctx, const int* status, std::vector<double>& bn, std::vector<double>& rn, int* st) {
-        CK(cudaMemcpyAsync(d + 2 * p, status, sizeof(int), cudaMemcpyDeviceToDevice, ctx->stream), "status");
+    tcu_status fetch(tcu_context* ctx, std::vector<double>& bn, std::vector<double>& rn, int* st) {
         CK(cudaMemcpyAsync(h.data(), d, h.size() * 8, cudaMemcpyDeviceToHost, ctx->stream), "norms");
         const tcu_status s = sync_status(ctx, "residual");
         if (s) return s;
@@ -732,7 +732,7 @@ tcu_status solve_impl(tcu_factor* f, const double* B, int p, double* X, tcu_cert
     cplx* tmp = r + per;  // 2 per
     cplx* xf = tmp + 2 * per;  // packed inputs of the stored-table residual
     SolveNorms norms(p, (char*)xf + xf_bytes);
-    CK(cudaMemsetAsync(f->wk.status, 0, sizeof(int), ctx->stream), "status");  // of this solve alone
+    CK(cudaMemsetAsync(norms.status(), 0, sizeof(double), ctx->stream), "status");
     CK(cudaMemcpyAsync(b, B, per * 16, device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, ctx->stream),
        "copy rhs");
     launch_apply_t(f->L, f->N, f->d_T, b, p, tb, ctx->stream);
@@ -744,10 +744,10 @@ tcu_status solve_impl(tcu_factor* f, const double* B, int p, double* X, tcu_cert
         if (f->scaled) scale_rows(v, f->d_scale, n, cols, ctx->stream);  // R v
         if (f->precision == TCU_FP64)
             lu_solve_fp64((const double2*)f->d_A, (int)n, f->wk.perm, f->d_inv, v, tmp, cols, ctx->stream,
-                          &ctx->launches, f->wk.status);
+                          &ctx->launches, norms.status());
         else
             lu_solve_fp32((const float2*)f->d_A, (int)n, f->wk.perm, f->d_inv, v, tmp, cols, ctx->stream,
-                          &ctx->launches, f->wk.status);
+                          &ctx->launches, norms.status());
         if (f->scaled) {
             scale_rows(v, f->d_scale + n, n, cols, ctx->stream);  // C (A')^-1 R v
             ctx->launches += 2;
@@ -756,8 +756,8 @@ tcu_status solve_impl(tcu_factor* f, const double* B, int p, double* X, tcu_cert
     auto residual = [&](int cols, std::vector<double>& rn) -> tcu_status {
         // r = T b - (x - T C x)
         if (f->d_Z) {
-            launch_apply_stored(*P, f->N, STORED_FULL, f->d_Z, f->d_T, x, n, cols, tb, -1.0, 1.0, r, xf, f->wk.status,
-                                ctx->stream);
+            launch_apply_stored(*P, f->N, STORED_FULL, f->d_Z, f->d_T, x, n, cols, tb, -1.0, 1.0, r, xf,
+                                norms.status(), ctx->stream);
             ctx->launches += 2;
         } else {
             apply_op(ctx, P, f->N, f->k0, f->d_pos, f->d_T, x, n, cols, tb, -1.0, 1.0, true, r);
@@ -765,7 +765,7 @@ tcu_status solve_impl(tcu_factor* f, const double* B, int p, double* X, tcu_cert
         norms.residual(r, n, cols, ctx->stream);
         ctx->launches += 2;
         int st = 0;
-        tcu_status s2 = norms.fetch(ctx, f->wk.status, bn, rn, &st);
+        tcu_status s2 = norms.fetch(ctx, bn, rn, &st);
         if (s2) return s2;
         if (st == 8) return fail(TCU_TIMEOUT, "refinement: a device-side wait gave up");
         return TCU_OK;
@@ -825,7 +825,7 @@ tcu_status solve_adjoint_impl(tcu_factor* f, const double* G, int p, double* Y, 
     cplx* xf = t2 + per;  // packed inputs of the stored-table coupling product
     cplx* tmp = xf + xfc;
     SolveNorms norms(p, tmp + tmpc);
-    CK(cudaMemsetAsync(ctx->d_status, 0, 4, ctx->stream), "status");
+    CK(cudaMemsetAsync(norms.status(), 0, sizeof(double), ctx->stream), "status");
     CK(cudaMemcpyAsync(g, G, per * 16, cudaMemcpyHostToDevice, ctx->stream), "copy rhs");
     std::vector<double> bn(p);
     norms.rhs(g, n, ctx->stream);
@@ -833,20 +833,20 @@ tcu_status solve_adjoint_impl(tcu_factor* f, const double* G, int p, double* Y, 
         if (f->scaled) scale_rows(v, f->d_scale + n, n, cols, ctx->stream);  // C g
         if (f->precision == TCU_FP64)
             lu_solve_adjoint_fp64((const double2*)f->d_A, (int)n, f->wk.perm, f->d_inv, v, tmp, cols, ctx->stream,
-                                  &ctx->launches, ctx->d_status);
+                                  &ctx->launches, norms.status());
         else
             lu_solve_adjoint_fp32((const float2*)f->d_A, (int)n, f->wk.perm, f->d_inv, v, tmp, cols, ctx->stream,
-                                  &ctx->launches, ctx->d_status);
+                                  &ctx->launches, norms.status());
         if (f->scaled) scale_rows(v, f->d_scale, n, cols, ctx->stream);  // R
     };
     auto residual = [&](int cols, std::vector<double>& rn) -> tcu_status {  // r = g - A^H y
         launch_apply_adjoint(*P, f->N, f->k0, f->d_pos, f->d_T, y, n, cols, r, t1, t2, ctx->stream, &ctx->launches,
-                             f->d_Z, xf, ctx->d_status);
+                             f->d_Z, xf, norms.status());
         vec_sub(r, g, r, n, cols, ctx->stream);
         norms.residual(r, n, cols, ctx->stream);
         ctx->launches += 3;
         int st = 0;
-        const tcu_status s2 = norms.fetch(ctx, ctx->d_status, bn, rn, &st);
+        const tcu_status s2 = norms.fetch(ctx, bn, rn, &st);
         return s2 ? s2 : status_of(st, "adjoint residual");
     };
     auto copy_out = [&](int from, int col, int cols) {
