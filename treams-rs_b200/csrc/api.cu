@@ -461,6 +461,17 @@ tcu_status factor_impl(tcu_context* ctx, int L, double k0, size_t N, const doubl
                         (void*)f->d_inv, (void*)f->wk.piv, f->wk.pack, (void*)f->d_scale, (void*)f->d_Z})
             ctx->pool.free(q);
     };
+    // what the factor needs besides the stored tables: without room they give way
+    auto alloc_beside_tables = [&](void** q, size_t bytes) {
+        cudaError_t a = ctx->pool.alloc(q, bytes);
+        if (a == cudaErrorMemoryAllocation && f->d_Z) {
+            cudaGetLastError();
+            ctx->pool.free(f->d_Z);
+            f->d_Z = nullptr;
+            a = ctx->pool.alloc(q, bytes);
+        }
+        return a;
+    };
     tcu_status e = TCU_OK;
     do {
         if ((e = dev_alloc(ctx, &f->d_pos, 3 * N, "positions"))) break;
@@ -508,9 +519,10 @@ tcu_status factor_impl(tcu_context* ctx, int L, double k0, size_t N, const doubl
         {
             // equilibrate when an entry exceeds 10 (then the unit diagonal no longer bounds the
             // spread; linalg/mod.rs:137-228)
-            if ((e = dev_alloc(ctx, &f->d_scale, 2 * n, "scales"))) break;
+            if ((e = cuda_check(alloc_beside_tables((void**)&f->d_scale, 2 * n * sizeof(double)), "scales"))) break;
             DevBuf eq(ctx);
-            if ((e = cuda_check(eq.alloc(equilibrate_scratch_doubles((int)n) * sizeof(double)), "scales"))) break;
+            if ((e = cuda_check(alloc_beside_tables(&eq.p, equilibrate_scratch_doubles((int)n) * sizeof(double)), "scales")))
+                break;
             if ((e = equilibrate(f->d_A, precision == TCU_MIXED, (int)n, 10.0, f->d_scale, f->d_scale + n,
                                  (double*)eq.p, &f->scaled, ctx->stream, &ctx->launches))) {
                 e = fail(e, "equilibration failed");
@@ -527,7 +539,7 @@ tcu_status factor_impl(tcu_context* ctx, int L, double k0, size_t N, const doubl
             break;
         }
         // the block inverses run while the host waits for the status (of a failed factor they are not used)
-        if ((e = cuda_check(ctx->pool.alloc((void**)&f->d_inv, lu_inverse_bytes((int)n)), "block inverses"))) break;
+        if ((e = cuda_check(alloc_beside_tables((void**)&f->d_inv, lu_inverse_bytes((int)n)), "block inverses"))) break;
         if (precision == TCU_FP64)
             lu_block_inverses_fp64((const double2*)f->d_A, (int)n, f->d_inv, ctx->stream, &ctx->launches);
         else
@@ -699,6 +711,26 @@ tcu_status finish_columns(tcu_factor* f, const RefineGroups& groups, const std::
     return TCU_OK;
 }
 
+// The buffers of a solve: bytes(c) for c columns at a time, as many of the p as there is room for and at least a
+// group. Then the factor's stored tables give way, and its residuals rebuild them per application.
+template <class Bytes>
+tcu_status solve_buffers(tcu_factor* f, int p, Bytes bytes, DevBuf& buf, int* columns) {
+    for (int c = p;;) {
+        const cudaError_t e = buf.alloc(bytes(c));
+        *columns = c;
+        if (e != cudaErrorMemoryAllocation) return cuda_check(e, "solve buffers");
+        cudaGetLastError();
+        if (c > RefineGroups::WIDTH) {
+            c = std::max((int)RefineGroups::WIDTH, c / 2 / RefineGroups::WIDTH * RefineGroups::WIDTH);
+        } else if (f->d_Z) {
+            f->ctx->pool.free(f->d_Z);
+            f->d_Z = nullptr;
+        } else {
+            return cuda_check(e, "solve buffers");
+        }
+    }
+}
+
 tcu_status solve_impl(tcu_factor* f, const double* B, int p, double* X, tcu_certificate* certs, bool device) {
     if (!f || !B || !X || p <= 0) return fail(TCU_INVALID_INPUT, "require a factor and at least one column");
     if (p > SOLVE_MAXC) {
@@ -722,9 +754,20 @@ tcu_status solve_impl(tcu_factor* f, const double* B, int p, double* X, tcu_cert
         return fail(TCU_INVALID_INPUT,
                     "require finite channel-by-illumination columns matching the factorization");
     DevBuf bufs(ctx);
+    auto xf_bytes_of = [&](int c) { return f->d_Z ? stored_inputs_bytes(*P, f->N, STORED_FULL, c) : 0; };
+    int fit = p;
+    if ((s = solve_buffers(f, p, [&](int c) { return 6 * n * c * sizeof(cplx) + xf_bytes_of(c) + SolveNorms::bytes(c); },
+                           bufs, &fit)))
+        return s;
+    if (fit < p) {
+        ctx->pool.free(bufs.p);
+        bufs.p = nullptr;
+        for (int c0 = 0; c0 < p && !s; c0 += fit)
+            s = solve_impl(f, B + 2 * n * c0, std::min(fit, p - c0), X + 2 * n * c0, certs ? certs + c0 : nullptr, device);
+        return s;
+    }
     size_t per = n * p;
-    const size_t xf_bytes = f->d_Z ? stored_inputs_bytes(*P, f->N, STORED_FULL, p) : 0;
-    CK(bufs.alloc(6 * per * sizeof(cplx) + xf_bytes + SolveNorms::bytes(p)), "solve buffers");
+    const size_t xf_bytes = xf_bytes_of(p);
     cplx* b = (cplx*)bufs.p;
     cplx* tb = b + per;
     cplx* x = tb + per;
@@ -814,9 +857,21 @@ tcu_status solve_adjoint_impl(tcu_factor* f, const double* G, int p, double* Y, 
     if (!finite_all(G, 2 * per))
         return fail(TCU_INVALID_INPUT, "require finite channel-by-illumination columns matching the factorization");
     DevBuf bufs(ctx);
-    const size_t tmpc = adjoint_solve_tmp((int)n, p);
-    const size_t xfc = f->d_Z ? stored_inputs_bytes(*P, f->N, STORED_FULL, p) / sizeof(cplx) : 0;
-    CK(bufs.alloc((5 * per + tmpc + xfc) * sizeof(cplx) + SolveNorms::bytes(p)), "adjoint solve buffers");
+    auto xf_of = [&](int c) { return f->d_Z ? stored_inputs_bytes(*P, f->N, STORED_FULL, c) / sizeof(cplx) : 0; };
+    auto bytes = [&](int c) {
+        return (5 * n * c + adjoint_solve_tmp((int)n, c) + xf_of(c)) * sizeof(cplx) + SolveNorms::bytes(c);
+    };
+    int fit = p;
+    if ((s = solve_buffers(f, p, bytes, bufs, &fit))) return s;
+    if (fit < p) {
+        ctx->pool.free(bufs.p);
+        bufs.p = nullptr;
+        for (int c0 = 0; c0 < p && !s; c0 += fit)
+            s = solve_adjoint_impl(f, G + 2 * n * c0, std::min(fit, p - c0), Y + 2 * n * c0, certs ? certs + c0 : nullptr,
+                                   th);
+        return s;
+    }
+    const size_t tmpc = adjoint_solve_tmp((int)n, p), xfc = xf_of(p);
     cplx* g = (cplx*)bufs.p;
     cplx* y = g + per;
     cplx* r = y + per;
