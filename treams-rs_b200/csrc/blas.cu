@@ -11,6 +11,7 @@
 namespace tcu {
 
 constexpr int RG = 256;  // partial sums per reduction (grid size of stage 1)
+constexpr int MAX_ROWS = 65535;  // of a grid: columns per launch of stage 1
 
 __device__ __forceinline__ double block_sum(double v, double* sh) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
@@ -37,12 +38,13 @@ __global__ void norm_stage1(const cplx* __restrict__ x, size_t n, double* __rest
 __global__ void sum_stage2(const double* __restrict__ partial, int ncol, double* __restrict__ out, int do_sqrt) {
     __shared__ double sh[32];
     int c = blockIdx.x;
-    double s = partial[c * RG + threadIdx.x];
+    double s = partial[(size_t)c * RG + threadIdx.x];
     s = block_sum(s, sh);
     if (threadIdx.x == 0) out[c] = do_sqrt ? sqrt(s) : s;
 }
 void vec_norms(const cplx* x, size_t n, int ncol, double* out_dev, double* partial, cudaStream_t st) {
-    norm_stage1<<<dim3(RG, ncol), 256, 0, st>>>(x, n, partial);
+    for (int c = 0; c < ncol; c += MAX_ROWS)
+        norm_stage1<<<dim3(RG, std::min(MAX_ROWS, ncol - c)), 256, 0, st>>>(x + c * n, n, partial + (size_t)c * RG);
     sum_stage2<<<ncol, RG, 0, st>>>(partial, ncol, out_dev, 1);
 }
 
@@ -59,7 +61,9 @@ __global__ void rdot_stage1(const cplx* __restrict__ a, const cplx* __restrict__
 }
 void vec_real_dots(const cplx* a, const cplx* b, size_t n, int ncol, double* out_dev, double* partial,
                    cudaStream_t st) {
-    rdot_stage1<<<dim3(RG, ncol), 256, 0, st>>>(a, b, n, partial);
+    for (int c = 0; c < ncol; c += MAX_ROWS)
+        rdot_stage1<<<dim3(RG, std::min(MAX_ROWS, ncol - c)), 256, 0, st>>>(a + c * n, b + c * n, n,
+                                                                          partial + (size_t)c * RG);
     sum_stage2<<<ncol, RG, 0, st>>>(partial, ncol, out_dev, 0);
 }
 
