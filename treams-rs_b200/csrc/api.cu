@@ -973,6 +973,34 @@ bool use_stored_tables(const DevPlan& P, int N) {
     return bytes <= fr / 2;
 }
 
+// y = alpha x + beta T C x (singular) or x + C x (regular) for p columns from the pair tables, built for this call:
+// 4096 columns per product (the rows of a grid end at 65,535, and the packed inputs of two spheres, padded to 16,
+// take nine times their columns), fewer where the packed inputs have no room. False when there is none at all:
+// nothing has been launched.
+bool apply_from_tables(tcu_context* ctx, const DevPlan& P, int N, double k0, const double* pos, const cplx* T,
+                       const cplx* x, size_t n, int p, double alpha, double beta, bool singular, cplx* y) {
+    DevBuf zbuf(ctx), xfbuf(ctx);
+    int cols = std::min(p, 4096);
+    bool room = zbuf.alloc(stored_tables_bytes(P, N, STORED_FULL)) == cudaSuccess;
+    while (room && xfbuf.alloc(stored_inputs_bytes(P, N, STORED_FULL, cols)) != cudaSuccess) {
+        cudaGetLastError();
+        room = cols > 1;
+        cols = (cols + 1) / 2;
+    }
+    if (!room) {
+        cudaGetLastError();
+        return false;
+    }
+    build_stored_tables(P, N, k0, pos, STORED_FULL, (cplx*)zbuf.p, ctx->stream, singular);
+    ++ctx->launches;
+    for (int c0 = 0; c0 < p; c0 += cols) {
+        launch_apply_stored(P, N, STORED_FULL, (const cplx*)zbuf.p, T, x + c0 * n, n, std::min(cols, p - c0), nullptr,
+                            alpha, beta, y + c0 * n, (cplx*)xfbuf.p, ctx->d_status, ctx->stream, singular);
+        ctx->launches += 2;
+    }
+    return true;
+}
+
 // The dipole (lmax 1) system of a cluster: factored (complex64 from 2048 modes on, else FP64) up
 // to 6144 dipole modes; above, no factor is made (out stays empty) and the two-level
 // preconditioner solves the dipole system by an inner GMRES on its matrix-free dipole block.
@@ -1219,21 +1247,13 @@ tcu_status tcu_cross_sections(tcu_context* ctx, int lmax, double k0, size_t N, c
     CK(cudaMemcpyAsync(pos, positions, N * 24, cudaMemcpyHostToDevice, ctx->stream), "copy");
     CK(cudaMemcpyAsync(dx, x, per * 16, cudaMemcpyHostToDevice, ctx->stream), "copy");
     CK(cudaMemcpyAsync(db, b, per * 16, cudaMemcpyHostToDevice, ctx->stream), "copy");
-    DevBuf zbuf(ctx), xfbuf(ctx);
+    // lmax 6 and 7: the regular operator from its pair tables, like the outgoing one
     bool stored = !apply_gemm_supported(*P) && use_stored_tables(*P, (int)N);
-    if (stored && zbuf.alloc(stored_tables_bytes(*P, (int)N, STORED_FULL)) == cudaSuccess &&
-        xfbuf.alloc(stored_inputs_bytes(*P, (int)N, STORED_FULL, p)) == cudaSuccess) {
-        // lmax 6 and 7: the regular operator from its pair tables, like the outgoing one
+    if (stored) {
         CK(cudaMemsetAsync(ctx->d_status, 0, 4, ctx->stream), "status");
-        build_stored_tables(*P, (int)N, k0, pos, STORED_FULL, (cplx*)zbuf.p, ctx->stream, false);
-        launch_apply_stored(*P, (int)N, STORED_FULL, (const cplx*)zbuf.p, nullptr, dx, n, p, nullptr, 1.0, 1.0, ox,
-                            (cplx*)xfbuf.p, ctx->d_status, ctx->stream, false);
-        ctx->launches += 4;
-    } else {
-        cudaGetLastError();  // no room: the tables per pair
-        stored = false;
-        apply_op(ctx, P, (int)N, k0, pos, nullptr, dx, n, p, nullptr, 1.0, 1.0, false, ox);
+        stored = apply_from_tables(ctx, *P, (int)N, k0, pos, nullptr, dx, n, p, 1.0, 1.0, false, ox);
     }
+    if (!stored) apply_op(ctx, P, (int)N, k0, pos, nullptr, dx, n, p, nullptr, 1.0, 1.0, false, ox);
     // both sums, then one copy: nothing waits in between
     std::vector<double> s1(2 * (size_t)p);
     vec_real_dots(dx, ox, n, p, sums, sums + 2 * p, ctx->stream);
@@ -1420,19 +1440,13 @@ tcu_status tcu_cluster_apply(tcu_context* ctx, int lmax, double k0, size_t N, co
     // Several columns (or TCU_APPLY=stored): the pair tables once, then the stored-table
     // product per column; one column: the product form (building the tables costs about one
     // application, so storing them gains nothing), which ends at lmax 5: at lmax 6 and 7 tables
-    // and product (300 spheres lmax 6: 0.11 + 0.57 ms) beat the term sums (4.3 ms) for one column too.
+    // and product (300 spheres lmax 6: 0.11 + 0.38 ms) beat the term sums (4.3 ms) for one column too.
     const char* form = getenv("TCU_APPLY");
     const bool forced = form && strcmp(form, "stored") == 0;
-    if (stored_full_supported(*P) &&
-        (forced || ((p >= 2 || !apply_gemm_supported(*P)) && use_stored_tables(*P, (int)N)))) {
-        DevBuf zbuf(ctx), xfbuf(ctx);
-        CK(zbuf.alloc(stored_tables_bytes(*P, (int)N, STORED_FULL)), "stored tables");
-        CK(xfbuf.alloc(stored_inputs_bytes(*P, (int)N, STORED_FULL, p)), "packed inputs");
-        build_stored_tables(*P, (int)N, k0, pos, STORED_FULL, (cplx*)zbuf.p, ctx->stream);
-        launch_apply_stored(*P, (int)N, STORED_FULL, (const cplx*)zbuf.p, T, dx, n, p, nullptr, 1.0, -1.0, dy,
-                            (cplx*)xfbuf.p, ctx->d_status, ctx->stream);
-        ctx->launches += 3;
-    } else {
+    const bool tables = stored_full_supported(*P) &&
+                        (forced || ((p >= 2 || !apply_gemm_supported(*P)) && use_stored_tables(*P, (int)N)));
+    if (!tables || !apply_from_tables(ctx, *P, (int)N, k0, pos, T, dx, n, p, 1.0, -1.0, true, dy)) {
+        if (forced && tables) return fail(TCU_OUT_OF_MEMORY, "stored tables: out of device memory");
         apply_op(ctx, P, (int)N, k0, pos, T, dx, n, p, nullptr, 1.0, -1.0, true, dy);
     }
     CK(cudaMemcpyAsync(y, dy, per * 16, cudaMemcpyDeviceToHost, ctx->stream), "copy");
