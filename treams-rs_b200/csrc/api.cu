@@ -291,7 +291,10 @@ tcu_status get_plan(tcu_context* ctx, int L, const DevPlan** out) {
         d.w = (const double2*)(base + off_w);
         d.reflection = (const double*)(base + off_refl);
         d.idx = (const uint16_t*)(base + off_idx);
-        stored_product_blocks(d, h, &store->blocks);
+        if (!stored_product_blocks(d, h, &store->blocks)) {
+            cudaFree(store->mem);
+            return fail(TCU_DEVICE_ERROR, "translation plan: more table blocks than the stored product holds");
+        }
         d.blocks = &store->blocks;
         it = ctx->plans.emplace(L, std::move(store)).first;
     }

@@ -461,7 +461,8 @@ __device__ __forceinline__ void as_bulk_load(uint32_t dst, const void* src, uint
 }
 
 // most blocks a warp takes (stored_product_blocks over the product warps): 16 / 8, 30 / 8, 41 / 8, 52 / 8,
-// 109 / 16, 103 / 16, 106 / 16
+// 109 / 16, 103 / 16, 106 / 16. A block past the last slot would be dropped: stored_product_blocks refuses
+// lists that product_capacity does not hold.
 constexpr int SLOTS_DIPOLE = 2, SLOTS_L2 = 4, SLOTS_L3 = 6, SLOTS_L4 = 7, SLOTS_L5 = 7, SLOTS_L6 = 7, SLOTS_L7 = 7;
 
 // The stored product with a producer warp: lane 0 of the last warp streams the 16-source chunks
@@ -827,12 +828,23 @@ size_t store_smem(const StoredLayout& l) {
 }
 }  // namespace
 
+// blocks that the warps of the full operator's product take (launch_apply_stored)
+static int product_capacity(int L) {
+    switch (L) {
+        case 2: return 8 * SLOTS_L2;
+        case 3: return 8 * SLOTS_L3;
+        case 4: return 8 * SLOTS_L4;
+        case 5: return 16 * SLOTS_L5;
+        case 6: return 16 * SLOTS_L6;
+        default: return 16 * SLOTS_L7;
+    }
+}
 // The blocks of the full coupling operator's product that a term of the plan reads: source lm s and table
 // entry t meet in the term lists of some destination. Natural order of both already gathers them (of
-// random exchanges of rows and columns none found fewer).
-void stored_product_blocks(const DevPlan& P, const HostPlan& h, ProductBlocks* b) {
+// random exchanges of rows and columns none found fewer). False when the product's warps cannot hold them.
+bool stored_product_blocks(const DevPlan& P, const HostPlan& h, ProductBlocks* b) {
     b->count[0] = b->count[1] = 0;
-    if (P.L < 2 || P.L > 7) return;
+    if (P.L < 2 || P.L > 7) return true;
     const StoredLayout l = stored_layout(P, 1, STORED_FULL);
     std::vector<char> read((size_t)h.nlm * P.tsize, 0);
     for (int c = 0; c < h.nlm * h.nlm; ++c) {
@@ -850,9 +862,11 @@ void stored_product_blocks(const DevPlan& P, const HostPlan& h, ProductBlocks* b
                         any = any || (s < h.nlm && read[(size_t)s * P.tsize + row / l.DI]);
                     }
                 if (!any) continue;
+                if (b->count[list] == std::min(product_capacity(P.L), (int)ProductBlocks::MAX)) return false;
                 b->row[list][b->count[list]] = (unsigned char)o;
                 b->col[list][b->count[list]++] = (unsigned char)c;
             }
+    return true;
 }
 // every block of a product (the dipole operators: one column octet)
 static ProductBlocks all_blocks(const StoredLayout& l) {

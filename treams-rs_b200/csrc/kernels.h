@@ -153,7 +153,8 @@ void launch_apply_dipole(const DevPlan& P, int N, double k, const double* pos, c
 enum StoredKind { STORED_FULL = 0, STORED_DIPOLE_SOURCES = 1, STORED_DIPOLE_BLOCK = 2 };
 bool stored_full_supported(const DevPlan& P);  // STORED_FULL exists for this lmax and TCU_APPLY allows it
 bool stored_tables_enabled();  // false when TCU_APPLY is "fly" or "terms" (read at every call)
-void stored_product_blocks(const DevPlan& P, const HostPlan& h, ProductBlocks* b);
+// the list of blocks that the full operator's product forms; false when its warps cannot hold them
+bool stored_product_blocks(const DevPlan& P, const HostPlan& h, ProductBlocks* b);
 size_t stored_tables_bytes(const DevPlan& P, int N, int kind);
 size_t stored_inputs_bytes(const DevPlan& P, int N, int kind, int ncol);
 void build_stored_tables(const DevPlan& P, int N, double k, const double* pos, int kind, cplx* Z, cudaStream_t st,
