@@ -15,7 +15,7 @@
 // instead of once per pair. Work per ordered pair: tsize * 2 nlm complex multiply-adds
 // (1,470 at lmax 3, 3,888 at lmax 4) plus one harmonic table.
 //
-// CTA = DI destination spheres x one right-hand side, RG x CG threads; thread (rg, cg) owns
+// CTA = DI destination spheres x one right-hand side, RG x CG threads in whole warps; thread (rg, cg) owns
 // G rows rg + RG u (u < TR) and columns cg + CG t (t < TC). Per chunk of KJ sources:
 //   A) thread per pair: direction and radial sequence z_p(k r), p <= 2 lmax, to shared memory;
 //   B) thread per (pair, order m >= 0): the order column of the solid harmonics times z_p,
@@ -29,6 +29,7 @@
 #include <cstdlib>
 #include <cstring>
 
+#include "apply_shapes.h"
 #include "common.cuh"
 #include "kernels.h"
 #include "pairtable.cuh"
@@ -37,33 +38,6 @@
 namespace tcu {
 
 namespace {
-
-struct GemmShape {
-    int DI, TR, TC, RG, CG, KJ;
-};
-
-// The product restricted to the first nsrc source lm and the first ndst destination lm (the
-// table then needs degrees p <= order = l_max(src) + l_max(dst)); input vectors hold ldin and
-// output vectors ldout complex entries per sphere. The full operator: nsrc = ndst = nlm.
-struct SubOp {
-    int nsrc, ndst, order, ldin, ldout;
-};
-
-// Tile shapes per lmax: G rows DI * tsize <= TR * RG, columns 2 nlm <= TC * CG
-GemmShape gemm_shape(int L) {
-    switch (L) {
-        case 2: return {4, 4, 2, 25, 8, 32};   // 100 x 16, 200 threads
-        case 3: return {2, 4, 3, 25, 10, 32};  // 98 x 30, 250 threads
-        case 4: return {1, 4, 4, 21, 12, 32};  // 81 x 48, 252 threads
-        default: return {1, 4, 5, 31, 14, 16}; // lmax 5: 121 x 70, 434 threads
-    }
-}
-
-// The dipole-source (and dipole-to-dipole) products: G is (DI (order+1)^2) x 6, about 200 rows
-GemmShape sub_shape(int tsz) {
-    const int DI = std::max(1, 200 / tsz);
-    return {DI, 4, 2, (DI * tsz + 3) / 4, 3, 16};
-}
 
 size_t gemm_smem(const SubOp& o, const GemmShape& s) {
     const size_t tsz = (size_t)(o.order + 1) * (o.order + 1);
@@ -184,8 +158,7 @@ __device__ __forceinline__ void terms_epilogue(const DevPlan& P, const SubOp& O,
                                                int nthr) {
     const int nlm = P.nlm, M = 2 * O.nsrc, ts = (O.order + 1) * (O.order + 1);
     const int ndst = O.ndst, tasks = DI * ndst;
-    int W = 1;
-    while (W < 16 && 2 * W * tasks <= nthr && 2 * W <= O.nsrc) W *= 2;
+    const int W = epilogue_lanes(tasks, nthr, O.nsrc);
     const int end = (tasks * W + 31) / 32 * 32;  // whole warps take part in the shuffles
     for (int t0 = tid; t0 < end; t0 += nthr) {
         const int it = min(t0 / W, tasks - 1), part = t0 % W;
@@ -738,7 +711,7 @@ static void launch_shape(const DevPlan& P, const SubOp& O, const GemmShape& s, i
                          const cplx* T, const cplx* x, size_t ldx, int ncol, const cplx* zadd, double alpha,
                          double beta, bool singular, cplx* y, cudaStream_t st) {
     const dim3 grid((unsigned)((N + s.DI - 1) / s.DI), (unsigned)ncol);
-    apply_gemm_kernel<TR, TC><<<grid, s.RG * s.CG, gemm_smem(O, s), st>>>(P, O, N, k, pos, T, x, ldx, zadd, alpha,
+    apply_gemm_kernel<TR, TC><<<grid, shape_threads(s), gemm_smem(O, s), st>>>(P, O, N, k, pos, T, x, ldx, zadd, alpha,
                                                                           beta, singular, y, s.DI, s.RG, s.CG, s.KJ);
 }
 
