@@ -1887,6 +1887,7 @@ tcu_status lattice_setup(int lsum, double k, const double* lat, size_t nk, const
     const double len1 = std::hypot(a1x, a1y), len2 = std::hypot(a2x, a2y);
     const double hdir = S.area / std::max(len1, len2);
     const double rin = std::hypot(S.sx, S.sy);
+    // at most 129 x 129 points, 64 MB of tables (the kernels take them in tiles); likewise the reciprocal vectors
     long Nd = (long)std::ceil((Rc + rin) / hdir) + 1;
     if (Nd > 64) return fail(TCU_INVALID_INPUT, "lattice too elongated for the device lattice sums");
     for (long s = S.at_origin ? 1 : 0; s <= Nd; ++s)  // cube shells, fixed order; R = 0 when shifted
@@ -2005,8 +2006,6 @@ tcu_status lattice_sums_device(tcu_context* ctx, int lsum, double k, const Latti
     (void)scratch_arena;
     const int T = (lsum + 1) * (lsum + 1);
     const bool offplane = !S.coefz.empty();
-    if (lattice_sum_smem(lsum, (int)S.R.size(), offplane) > 200 * 1024 || S.G.size() > (1u << 20))
-        return fail(TCU_INVALID_INPUT, "lattice too elongated for the device lattice sums");
     const std::vector<double2> coef = lattice_coefficients(lsum, offplane, [&](int l, int am, int pp, int n) {
         const size_t lm = (size_t)l * l + l + am;
         return make_double2(offplane ? S.coefz[(lm * LS_PMAX + pp) * LS_FMAX + n] : S.coef[lm * LS_NMAX + n], 0.0);
@@ -2316,8 +2315,6 @@ extern "C" tcu_status tcu_lsumsw2d_complex_batch(tcu_context* ctx, int lmax_sum,
     tcu_status s = lattice_setup_ck(lmax_sum, kc, lattice, nk, kpars, eta, shift ? shift : zero, S);
     if (s) return s;
     const int T = (lmax_sum + 1) * (lmax_sum + 1);
-    if (lattice_sum_ck_smem(lmax_sum, (int)S.R.size()) > 200 * 1024 || S.G.size() > (1u << 20))
-        return fail(TCU_INVALID_INPUT, "lattice too elongated for the device lattice sums");
     const bool offplane = S.sz != 0.0;
     const std::vector<double2> coef = lattice_coefficients(lmax_sum, offplane, [&](int l, int am, int pp, int n) {
         return S.coef[(((size_t)l * l + l + am) * LS_PMAX + pp) * LS_FMAX + n];

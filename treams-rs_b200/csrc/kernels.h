@@ -263,10 +263,8 @@ struct LatticeSumCkArgs {
 };
 void launch_real_table_ck(int lsum, double2 k, double eta, int NR, const double2* R, double sx, double sy, double sz,
                           const double* norm, const double* reflection, bool offplane, double2* tab, cudaStream_t st);
-size_t lattice_sum_ck_smem(int lsum, int NR);
 void launch_real_table(int lsum, double k, double eta, int NR, const double2* R, double sx, double sy, double sz,
                        const double* norm, const double* reflection, bool offplane, double2* tab, cudaStream_t st);
-size_t lattice_sum_smem(int lsum, int NR, bool offplane);
 // lattice_sum.cu — the reciprocal part and the reduction. The sums run over the (l, |m|) pairs of
 // even l - |m| in the plane, of all off it, in the order of l - |m|, then |m|.
 int lattice_pairs(int lsum, bool offplane);

@@ -388,11 +388,6 @@ void launch_real_table(int lsum, double k, double eta, int NR, const double2* R,
                                                     2 * lattice_pairs(lsum, offplane), tab);
 }
 
-size_t lattice_sum_smem(int lsum, int NR, bool offplane) {
-    const size_t nF = offplane ? lsum + 1 : lsum / 2 + 1;
-    return (size_t)NR * 16 + (size_t)256 * nF * 16 + 2 * 256 * 16 + 256 * 8;
-}
-
 void launch_array_solve(const DevPlan& P, const double2* D, size_t ldd, const double* norm, const double2* Tm, int nk,
                         double2* X, int* status, int grid, cudaStream_t st) {
     StageScope sc(ST_SMALL_LU, st);

@@ -167,8 +167,4 @@ void launch_real_table_ck(int lsum, cplx k, double eta, int NR, const double2* R
                                                        offplane ? 1 : 2, 2 * lattice_pairs(lsum, offplane), tab);
 }
 
-size_t lattice_sum_ck_smem(int lsum, int NR) {
-    return (size_t)NR * 16 + (size_t)256 * (lsum + 1) * 16 + 3 * 256 * 16;
-}
-
 }  // namespace tcu
