@@ -2570,9 +2570,12 @@ extern "C" tcu_status tcu_batch_solve(tcu_context* ctx, size_t count, const tcu_
     for (int w = 0; w < K; ++w) {
         tcu_context* wc = ctx->workers[w];
         wc->refine_target = ctx->refine_target;
-        // 192 rows per panel CTA: panels of up to ~28,000 rows on 148 CTAs, and the panels of
-        // smaller clusters on few enough SMs that the workers' panels run side by side (64
-        // clusters of the sweep: 3.70 s with 32 rows, 3.03 s with 200 rows, 4 workers)
+        // 192 rows per panel CTA, as far as shared memory holds them: the workers' panels take few enough of the
+        // 7 clusters of 16 that two or three run side by side (9,216 rows in FP32 3 clusters instead of 5), for
+        // 5 % more a column of a panel that has the chip to itself. ms, medians in turn, at the default
+        // shape and at 64, 128, 160 and 192 rows: 24 clusters of up to 9,216 modes 76.3, 91.9, 76.2, 73.6, 72.9 with
+        // 4 workers (117.3, 123.6, 118.4, 117.5, 118.9 with 2; 86.2, 100.0, 87.2, 85.0, 84.1 with 6), 96 of up to
+        // 19,200 modes 2920, 3164, 2922, 2849, 2784.
         wc->panel_rows = 192;
         wc->fallback_above = ctx->fallback_above;
         fb0[w] = wc->fallbacks;

@@ -299,7 +299,7 @@ struct LuWork {
     void* pack = nullptr;      // packed GEMM operands (mixed path)
     size_t pack_bytes = 0;
     PieceFormat pieces = PIECES_TF32X3;  // mixed path: the split of the trailing updates' operands
-    int panel_rows = 0;        // least rows per panel CTA (0: TCU_PANEL_ROWS or 32)
+    int panel_rows = 0;        // least rows per panel CTA (0: the default of the panel's kernel)
 };
 // bfloat16 unless TCU_SPLIT names another format (tf32x3, tf32x2, f16)
 PieceFormat split_default();

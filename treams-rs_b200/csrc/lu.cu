@@ -762,7 +762,6 @@ template <typename R, int NB>
 static bool run_panel_cluster(typename Cx<R>::T* A, int n, int k0, int w, LuWork& wk, cudaStream_t st) {
     typedef typename Cx<R>::T C;
     const void* fn = (const void*)panel_cluster_kernel<R, NB>;
-    constexpr size_t LIMIT = 224 * 1024;  // beside about 2 KB of static shared memory
     static int most_clusters = 0;  // clusters of 16 that the device holds at once
     static PerDeviceOnce attr;
     cudaLaunchAttribute at[2];
@@ -776,10 +775,10 @@ static bool run_panel_cluster(typename Cx<R>::T* A, int n, int k0, int w, LuWork
     cfg.stream = st;
     cfg.attrs = at;
     once_per_device(attr, [&] {
-        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LIMIT);
+        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PC_SMEM_LIMIT);
         cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         cfg.gridDim = dim3(16);
-        cfg.dynamicSmemBytes = LIMIT;
+        cfg.dynamicSmemBytes = PC_SMEM_LIMIT;
         cfg.numAttrs = 1;
         int c = 0;
         if (cudaOccupancyMaxActiveClusters(&c, fn, &cfg) != cudaSuccess) {
@@ -788,28 +787,12 @@ static bool run_panel_cluster(typename Cx<R>::T* A, int n, int k0, int w, LuWork
         }
         most_clusters = std::min(c, PC_MAXCL);
     });
-    const int rows = n - k0;
-    // About 64 rows a CTA while one cluster holds them (measured per column at 24, 48, 64 and 96 rows:
-    // 1.22, 1.19, 1.19, 1.21 us at 240 rows FP64; 1.23, 1.22, 1.22, 1.25 at 1920 FP32): fewer rows only add
-    // messages, more rows lengthen the rank-16 update. Beyond one cluster about 128 rows a CTA: every
-    // further cluster adds readers to the global exchange (12288 FP32: 1.87 us at 96 and 128 rows, 1.94 at
-    // 160, 1.96 at 192), so the first cluster panels of 24576 rows, which need all 7 clusters, cost 2.7 us a column.
-    int cs = 1;
-    while (cs < 16 && cs * 64 < rows) cs *= 2;
-    if (most_clusters < 1) return false;
-    int ncl = 1, chunk = 0;
-    auto fits = [&]() {
-        chunk = (rows + cs * ncl - 1) / (cs * ncl);
-        return chunk <= PC_T && panel_cluster_smem<C>(chunk, NB, cs) <= LIMIT;
-    };
-    while (cs < 16 && !fits()) cs *= 2;
-    if (!fits()) {
-        ncl = std::min(most_clusters, (rows + 16 * 128 - 1) / (16 * 128));
-        while (!fits())
-            if (++ncl > most_clusters) return false;
-    }
+    const PanelShape shape = panel_cluster_shape(sizeof(C), n - k0, NB, wk.panel_rows, most_clusters);
+    int cs = shape.cs, chunk = shape.chunk;
+    const int ncl = shape.ncl;
+    if (cs == 0) return false;
     cfg.gridDim = dim3(cs * ncl);
-    cfg.dynamicSmemBytes = panel_cluster_smem<C>(chunk, NB, cs);
+    cfg.dynamicSmemBytes = panel_cluster_smem(sizeof(C), chunk, NB, cs);
     cfg.numAttrs = ncl > 1 ? 2 : 1;
     at[0].val.clusterDim.x = cs;
     size_t lda = (size_t)n;

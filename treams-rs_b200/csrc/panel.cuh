@@ -28,12 +28,9 @@
 // exits while another may still send to it.
 #pragma once
 
-namespace tcu {
+#include "panel_shape.h"
 
-constexpr int PC_T = 256;     // threads, and most rows of a CTA
-constexpr int PC_SUB = 16;    // columns of a sub-block
-constexpr int PC_MAXCL = 8;   // clusters of a panel (a cluster of 16 SMs per GPC)
-constexpr int PC_WARPS = PC_T / 32;
+namespace tcu {
 
 // A candidate message in 16-byte units: 16 entries, {key, row} in the first word of the next unit, the
 // reciprocal. Words are 8 bytes.
@@ -42,6 +39,7 @@ struct PcMsg {
     static constexpr int E = sizeof(C) / 8;
     static constexpr int UNITS = PC_SUB * E / 2;  // of the entries: 8 or 16, a thread each per CTA
     static constexpr int KEY = PC_SUB * E, INV = KEY + 2, WORDS = INV + 2, BYTES = WORDS * 8;
+    static_assert(BYTES == panel_message_bytes(sizeof(C)), "the launch sizes shared memory by it");
 };
 
 typedef unsigned long long pc_word;
@@ -144,12 +142,6 @@ __device__ __forceinline__ double2 pc_sub(double2 x, double2 l, double2 u) {
     return make_double2(fma(-l.x, u.x, fma(l.y, u.y, x.x)), fma(-l.x, u.y, fma(-l.y, u.x, x.y)));
 }
 
-template <typename C>
-size_t panel_cluster_smem(int chunk, int nb, int cs) {
-    typedef PcMsg<C> M;
-    return (size_t)(2 * cs + PC_MAXCL) * M::BYTES + 2 * PC_WARPS * PC_SUB * sizeof(C) +
-           (size_t)PC_SUB * nb * sizeof(C) + (size_t)chunk * (nb + 1) * sizeof(C);
-}
 // global words of the clusters' exchange and of the pivot rows (uint4 each)
 constexpr size_t PC_GKEY = 2 * PC_MAXCL * 36, PC_GROW = 2 * PC_SUB * 128;
 
