@@ -963,9 +963,11 @@ int batch_workers() {
 
 // The stored-table operator for the applications of GMRES: lmax 2..7 in product form, unless
 // TCU_APPLY is "fly" or "terms", and only while the tables take at most half of the free device
-// memory (and at most 64 GB).
-bool use_stored_tables(const DevPlan& P, int N) {
-    if (!stored_full_supported(P) || !stored_tables_enabled()) return false;
+// memory (and at most 64 GB). One sphere has no pairs to tabulate: the plain form up to 16 columns (us of a call
+// with 1, 3 and 50 columns, plain against tables: lmax 3 103, 103, 203 against (3 and 50) 189, 196; 6 113, 120, 397 against
+// 222, 224, 255; 7 122, 129, 459 against 238, 233, 300).
+bool use_stored_tables(const DevPlan& P, int N, int columns = 1) {
+    if ((N < 2 && columns <= 16) || !stored_full_supported(P) || !stored_tables_enabled()) return false;
     const size_t bytes = stored_tables_bytes(P, N, STORED_FULL);
     if (bytes == 0 || bytes > ((size_t)64 << 30)) return false;
     size_t fr = 0, tot = 0;
@@ -1251,7 +1253,7 @@ tcu_status tcu_cross_sections(tcu_context* ctx, int lmax, double k0, size_t N, c
     CK(cudaMemcpyAsync(dx, x, per * 16, cudaMemcpyHostToDevice, ctx->stream), "copy");
     CK(cudaMemcpyAsync(db, b, per * 16, cudaMemcpyHostToDevice, ctx->stream), "copy");
     // lmax 6 and 7: the regular operator from its pair tables, like the outgoing one
-    bool stored = !apply_gemm_supported(*P) && use_stored_tables(*P, (int)N);
+    bool stored = !apply_gemm_supported(*P) && use_stored_tables(*P, (int)N, p);
     if (stored) {
         CK(cudaMemsetAsync(ctx->d_status, 0, 4, ctx->stream), "status");
         stored = apply_from_tables(ctx, *P, (int)N, k0, pos, nullptr, dx, n, p, 1.0, 1.0, false, ox);
@@ -1447,7 +1449,7 @@ tcu_status tcu_cluster_apply(tcu_context* ctx, int lmax, double k0, size_t N, co
     const char* form = getenv("TCU_APPLY");
     const bool forced = form && strcmp(form, "stored") == 0;
     const bool tables = stored_full_supported(*P) &&
-                        (forced || ((p >= 2 || !apply_gemm_supported(*P)) && use_stored_tables(*P, (int)N)));
+                        (forced || ((p >= 2 || !apply_gemm_supported(*P)) && use_stored_tables(*P, (int)N, p)));
     if (!tables || !apply_from_tables(ctx, *P, (int)N, k0, pos, T, dx, n, p, 1.0, -1.0, true, dy)) {
         if (forced && tables) return fail(TCU_OUT_OF_MEMORY, "stored tables: out of device memory");
         apply_op(ctx, P, (int)N, k0, pos, T, dx, n, p, nullptr, 1.0, -1.0, true, dy);
