@@ -675,7 +675,9 @@ def _measure_impl(args, precision, steps, warmup, with_e2e, *, ctx, lib, stream,
             "gpu_launches": int(launches), "clocks": clk}
     if with_e2e:
         line["e2e"] = {"value": world * steps / (ms_e2e / 1e3), "unit": UNIT, "h2d_bytes_per_step": int(h2d),
-                       "d2h_bytes_per_step": int(d2h)}
+                       "d2h_bytes_per_step": int(d2h),
+                       "note": "timed after the device-timed value in the same process, both under the power cap: their "
+                               "clocks differ by more than the copies take, so it can come out ahead of value"}
     X = X_d.cpu().numpy().reshape(n, p, order="F") if precision == args.precision else None
     return {"line": line, "X": X}
 
