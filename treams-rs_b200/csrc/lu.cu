@@ -853,28 +853,33 @@ void launch_tf32_trsm(float2* A, int n, int k0, LuWork& wk, cudaStream_t st, lon
 bool launch_tf32_trsm_inverse(float2* A, int n, int k0, LuWork& wk, cudaStream_t st, cudaStream_t side,
                               long long* launches);
 
-// A second stream of this thread and device (created once, kept for the process) on which the
-// inverse of each step's L11 runs while the main stream applies the row interchanges: the
-// inverse reads only the panel's diagonal block, the interchanges touch only the columns
-// outside the panel.
+// A second stream of this thread and device on which the inverse of each step's L11 runs while the
+// main stream applies the row interchanges: the inverse reads only the panel's diagonal block, the
+// interchanges touch only the columns outside the panel. Made at the thread's first use and given back
+// when the thread ends: a batch starts new threads for every call, and a stream holds about 0.6 MB.
 struct SideStream {
     cudaStream_t stream = nullptr;
     cudaEvent_t panel_done = nullptr, inverse_done = nullptr;
     bool ok = false;
+    SideStream() {
+        ok = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking) == cudaSuccess &&
+             cudaEventCreateWithFlags(&panel_done, cudaEventDisableTiming) == cudaSuccess &&
+             cudaEventCreateWithFlags(&inverse_done, cudaEventDisableTiming) == cudaSuccess;
+    }
+    SideStream(const SideStream&) = delete;
+    SideStream& operator=(const SideStream&) = delete;
+    ~SideStream() {
+        if (inverse_done) cudaEventDestroy(inverse_done);
+        if (panel_done) cudaEventDestroy(panel_done);
+        if (stream) cudaStreamDestroy(stream);
+    }
 };
 static SideStream* side_stream() {
     thread_local std::map<int, SideStream> by_device;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
-    auto it = by_device.find(dev);
-    if (it == by_device.end()) {
-        SideStream s;
-        s.ok = cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking) == cudaSuccess &&
-               cudaEventCreateWithFlags(&s.panel_done, cudaEventDisableTiming) == cudaSuccess &&
-               cudaEventCreateWithFlags(&s.inverse_done, cudaEventDisableTiming) == cudaSuccess;
-        it = by_device.emplace(dev, s).first;
-    }
-    return it->second.ok ? &it->second : nullptr;
+    SideStream& s = by_device[dev];
+    return s.ok ? &s : nullptr;
 }
 
 template <typename R, int NB>
